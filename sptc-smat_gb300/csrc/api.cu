@@ -85,8 +85,7 @@ static void free_handle(smat_bcsr* h) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (PlanDev& pd : h->pc) {
-    void* pp[] = {pd.d_stages, pd.d_panels, pd.d_row_map, pd.sched[1].d_order, pd.sched[1].d_items,
-                  pd.sched[2].d_order, pd.sched[2].d_items};
+    void* pp[] = {pd.d_stages, pd.d_panels, pd.d_row_map, pd.sched[1].d_items, pd.sched[2].d_items};
     for (void* p : pp)
       if (p) cudaFree(p);
   }
@@ -219,23 +218,21 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
       build_work_items(pd.plan, bh, workers, frac, items, order, sc.n_split, sc.n_slabs);
       sc.grid = std::max(1, std::min<int>(workers, (int)items.size()));
       sc.n_items = (int32_t)items.size();
-      SMAT_TRY(upload(&sc.d_items, items.data(), items.size()));
-      SMAT_TRY(upload(&sc.d_order, order.data(), order.size()));
+      const std::vector<WorkItem> dev = device_items({&pd.plan}, items, order);
+      SMAT_TRY(upload(&sc.d_items, dev.data(), dev.size()));
     }
   }
 
-  // A streams, one per requested form: for each stage its blocks in
-  // consumption order in the 32-byte-swizzled shared-memory layout (inside
-  // each 256-byte group of 8 rows of 32 bytes, the two 16-byte halves of
-  // rows 4..7 are swapped), hi then lo blocks for the split form, then the
-  // stage header.
+  // A streams, one per requested form: for each stage its header, then its
+  // blocks in consumption order in the 32-byte-swizzled shared-memory layout
+  // (inside each 256-byte group of 8 rows of 32 bytes, the two 16-byte halves
+  // of rows 4..7 are swapped), hi then lo blocks for the split form.
   const int64_t nnzb = b.nnzb();
   const size_t bsz = (size_t)bh * bw, ablk = (size_t)bh * 32;
   auto stream_layout = [&](const Plan& pl, const std::vector<uint16_t>& hi, const std::vector<uint16_t>* lo,
                            std::vector<uint8_t>& out) {
     const int64_t nst = (int64_t)pl.stages.size();
-    const size_t nops = lo ? 2 : 1;
-    out.assign(std::max<size_t>((size_t)nnzb * ablk * nops + pl.headers.size(), 16), 0);
+    out.assign(std::max<size_t>(pl.a_bytes, 16), 0);
     auto put = [&](const std::vector<uint16_t>& vals, int64_t k, uint8_t* dst) {
       const uint8_t* src = reinterpret_cast<const uint8_t*>(vals.data() + (size_t)pl.stream_blk[k] * bsz);
       for (int r = 0; r < bh; r++)
@@ -245,12 +242,13 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
 #pragma omp parallel for schedule(static)
     for (int64_t si = 0; si < nst; si++) {
       const StageRec& r = pl.stages[si];
-      uint8_t* base = out.data() + (size_t)r.blk_off * ablk * nops + (size_t)r.hdr_off;
+      uint8_t* base = out.data() + (size_t)r.aoff256 * 256;
+      std::memcpy(base, pl.headers.data() + r.hdr_off, (size_t)r.hdr_bytes);
+      base += kStageHdrBytes;
       for (int32_t q = 0; q < r.nblk; q++) {
         put(hi, r.blk_off + q, base + (size_t)q * ablk);
         if (lo) put(*lo, r.blk_off + q, base + ((size_t)r.nblk + q) * ablk);
       }
-      std::memcpy(base + (size_t)r.nblk * ablk * nops, pl.headers.data() + r.hdr_off, (size_t)r.hdr_bytes);
     }
   };
   std::vector<uint8_t> lay;
@@ -290,22 +288,19 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
     SMAT_TRY(quantize_fp8(b, h->fp8_q, h->fp8_scale));
     const Plan& pl = h->pc[2].plan;
     const int64_t nst = (int64_t)pl.stages.size();
-    // per stage: [nblk e4m3 blocks][nblk FP32 scales, padded][header]
-    lay.assign(std::max<size_t>((size_t)nnzb * 256 + pl.headers.size() +
-                                    (nst ? (size_t)pl.stages[nst - 1].scl_off + fp8_scale_bytes(pl.stages[nst - 1].nblk) : 0),
-                                16),
-               0);
+    // per stage: [header][nblk e4m3 blocks][nblk FP32 scales, padded]
+    lay.assign(std::max<size_t>(pl.a_bytes, 16), 0);
 #pragma omp parallel for schedule(static)
     for (int64_t si = 0; si < nst; si++) {
       const StageRec& r = pl.stages[si];
-      uint8_t* base = lay.data() + (size_t)r.blk_off * 256 + (size_t)r.scl_off + (size_t)r.hdr_off;
+      uint8_t* base = lay.data() + (size_t)r.aoff256 * 256;
+      std::memcpy(base, pl.headers.data() + r.hdr_off, (size_t)r.hdr_bytes);
+      base += kStageHdrBytes;
       for (int32_t qb = 0; qb < r.nblk; qb++) {
         const int64_t blk = pl.stream_blk[r.blk_off + qb];
         std::memcpy(base + (size_t)qb * 256, h->fp8_q.data() + (size_t)blk * 256, 256);
         std::memcpy(base + (size_t)r.nblk * 256 + (size_t)qb * 4, &h->fp8_scale[blk], 4);
       }
-      std::memcpy(base + (size_t)r.nblk * 256 + fp8_scale_bytes(r.nblk), pl.headers.data() + r.hdr_off,
-                  (size_t)r.hdr_bytes);
     }
     SMAT_TRY(upload(&h->d_aval[SMAT_FORM_FP8], lay.data(), lay.size()));
   }
@@ -688,7 +683,6 @@ smat_status smat_spmm_packed(const smat_bcsr* A, int32_t form, const void* packe
   std::memset(&args, 0, sizeof(args));
   const WsLayout wl = ws_layout(A, form, N);
   fill_problem(A, form, packed_b, N, C, c_dtype, ldc, nsub, wl, args.one);
-  args.order = sc.d_order;
   args.n_items = sc.n_items;
   args.items = sc.d_items;
   args.err = A->d_err;

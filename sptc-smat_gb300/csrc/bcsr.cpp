@@ -526,7 +526,7 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
   plan.headers.resize(nh);
   plan.n_groups = 0;
   plan.n_tiles = 0;
-  int64_t so = 0, bo = 0, ho = 0, xo = 0;
+  int64_t so = 0, bo = 0, ho = 0, ao = 0;
   for (int32_t p = 0; p < P; p++) {
     Local& L = loc[p];
     L.info.stage_off = (int32_t)so;
@@ -537,16 +537,17 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
       StageRec r = L.stages[c];
       r.blk_off = bo;
       r.hdr_off = ho;
-      r.scl_off = (int32_t)xo;
+      r.aoff256 = (int32_t)ao;
       bo += r.nblk;
       ho += r.hdr_bytes;
-      xo += fp8_scale_bytes(r.nblk);
+      ao += (stage_a_bytes(cls, b.bh, r.nblk) + 255) / 256;
       plan.stages[so + c] = r;
     }
     so += (int64_t)L.stages.size();
     plan.n_groups += L.groups;
     plan.n_tiles += L.tiles;
   }
+  plan.a_bytes = (size_t)ao * 256;
   return SMAT_OK;
 }
 
@@ -640,6 +641,20 @@ void build_work_items(const Plan& pl, int32_t bh, int32_t workers, double max_it
   build_work_items_multi({&pl}, {bh}, workers, max_item_frac, items, order, ns, nl);
   n_split = ns[0];
   n_slabs = nl[0];
+}
+
+std::vector<WorkItem> device_items(const std::vector<const Plan*>& plans, const std::vector<WorkItem>& items,
+                                   const std::vector<int32_t>& order) {
+  std::vector<WorkItem> out;
+  out.reserve(items.size());
+  for (int32_t i : order) {
+    WorkItem w = items[i];
+    const int32_t off = plans[w.prob]->panels[w.panel].stage_off;
+    w.s0 += off;
+    w.s1 += off;
+    out.push_back(w);
+  }
+  return out;
 }
 
 void order_items(const std::vector<double>& cost, std::vector<int32_t>& order) {

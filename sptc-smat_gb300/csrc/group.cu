@@ -30,7 +30,6 @@ struct Launch {
   int bh = 16, R = 16, nsub = 1, kind = 0, grid = 1;
   ProblemDesc* d_probs = nullptr;
   WorkItem* d_items = nullptr;
-  int32_t* d_order = nullptr;
   int32_t n_items = 0;
   int32_t ctr = 0;  // int offset of the launch's next-item counter in d_counters
 };
@@ -58,7 +57,6 @@ static void group_free(smat_group* g) {
   for (Launch& l : g->launches) {
     cudaFree(l.d_probs);
     cudaFree(l.d_items);
-    cudaFree(l.d_order);
   }
   cudaFree(g->d_ws);
   cudaFree(g->d_counters);
@@ -132,7 +130,6 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
   };
   std::vector<Scratch> sc(count);
   std::vector<std::vector<WorkItem>> v_items;
-  std::vector<std::vector<int32_t>> v_order;
   std::vector<std::vector<int32_t>> v_members;
   for (auto& kv : variants) {
     const auto& members = kv.second;
@@ -164,8 +161,7 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
     l.grid = std::max(1, std::min<int>(workers, (int)items.size()));
     l.n_items = (int32_t)items.size();
     g->launches.push_back(l);
-    v_items.push_back(std::move(items));
-    v_order.push_back(std::move(order));
+    v_items.push_back(device_items(plans, items, order));
     v_members.push_back(members);
   }
   // one scratch allocation for all problems, one for all counters: each
@@ -218,7 +214,6 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
     }
     GTRY(upload_vec(&l.d_probs, descs));
     GTRY(upload_vec(&l.d_items, v_items[v]));
-    GTRY(upload_vec(&l.d_order, v_order[v]));
   }
 #undef GTRY
   *out = g;
@@ -243,7 +238,6 @@ smat_status smat_group_run(smat_group* g, void* stream_) {
     SpmmArgs args;
     std::memset(&args, 0, sizeof(args));
     args.probs = l.d_probs;
-    args.order = l.d_order;
     args.n_items = l.n_items;
     args.next_item = g->d_counters + l.ctr;
     args.items = l.d_items;

@@ -109,6 +109,7 @@ struct Plan {
   std::vector<int32_t> row_map;
   int64_t n_groups = 0;              // MMA instructions per pass over A
   int64_t n_tiles = 0;               // B tile loads per pass over A
+  size_t a_bytes = 0;                // bytes of the A stream
 };
 
 // skip (optional): blocks with skip[k] != 0 are left out of the plan (the
@@ -158,8 +159,7 @@ void build_work_items(const Plan& pl, int32_t bh, int32_t workers, double max_it
 struct Sched {
   int grid = 0;
   int32_t n_items = 0;
-  int32_t* d_order = nullptr;  // items by decreasing estimated cost
-  WorkItem* d_items = nullptr;
+  WorkItem* d_items = nullptr;  // by decreasing estimated cost, absolute stage ranges
   int32_t n_split = 0;  // panels split into parts
   int32_t n_slabs = 0;  // parts of split panels
 };
@@ -288,6 +288,12 @@ struct TuneVal {
 bool tune_key_of(const HostBcsr& b, int kind, int64_t N, TuneKey& key);
 bool tune_lookup(const TuneKey& key, TuneVal& val);
 void tune_store(const TuneKey& key, const TuneVal& val);
+
+// The device's list: the items in `order`, their stage ranges counted from
+// the plan's first stage (a role then reads one 32-byte item, not an index,
+// an item and the panel's record one after the other).
+std::vector<WorkItem> device_items(const std::vector<const Plan*>& plans, const std::vector<WorkItem>& items,
+                                   const std::vector<int32_t>& order);
 
 // Item indices by decreasing cost (ties by index).
 void order_items(const std::vector<double>& item_cost, std::vector<int32_t>& order);

@@ -22,19 +22,29 @@
 // engine and the tensor cores is one full/empty barrier pair per stage.
 //
 // Roles (512 threads):
-//   warps 8..15     copy warps: a stage needs one bulk copy for its A blocks
-//                   and list and one per B tile; the copies rotate over the
-//                   eight warps (a warp keeps only about one copy at a time
-//                   in flight).
-//   warps 0..3      MMA issuers, lane 0 each, one per quarter of the panel's
-//                   block rows (one thread issues at most one tcgen05.mma
-//                   per ~80-150 cycles; four keep the tensor pipe at its
-//                   per-instruction rate); warp 0 also owns TMEM.
+//   warps 8..15     copy warps: a stage needs one bulk copy for its list and
+//                   A blocks and one per B tile; the copies rotate over the
+//                   eight warps, each of which waits for the stage's slot
+//                   and counts itself on the stage's full barrier.
+//   warps 0..3      MMA issuers, one elected lane each, one per quarter of the
+//                   panel's block rows (one thread issues at most one
+//                   tcgen05.mma per 64-75 cycles, the tensor pipe takes one of
+//                   this width every 39); warp 0 also owns TMEM.
 //   warps 4..7      epilogue: tcgen05.ld -> row scatter through row_map ->
 //                   FP32 or FP16 stores of C (coalesced along N).
 //
 // Consecutive block rows with a block at the same column form one MMA
 // (N = bh * run length), so dense panels need far fewer instructions.
+//
+// What bounds it: latency of the control code first (a stage's waits, list
+// reads and MMA issues; measured with single-instruction benchmarks, see
+// tc_ptx.cuh), then shared memory: the copies write it and the MMAs read their
+// 128 x 16 operand from it, about 125 us on the R-MAT workload (2^16 rows,
+// 680K blocks, N = 128). Waits whose loop branches on the barrier's own
+// predicate, MMA and copy issue by an elected lane, copy warps that need no
+// barrier among themselves, and work items read whole from the item ring took
+// the step from 256 to 216 us there (plain graph, 2^15 rows, N = 256: 231 to
+// 196 us).
 //
 // Every wait is bounded (see tc_ptx.cuh); on a timeout the kernel raises the
 // CTA's abort flag, records the site in the global error word, lets the
@@ -86,20 +96,17 @@ struct Cfg {
   static constexpr int CLS = KIND == KIND_SPLIT ? 1 : (KIND == KIND_FP8 ? 2 : (NSUB == 2 ? 3 : 0));
   static constexpr int SB = stage_rows(CLS) / BH;         // A blocks per stage (at most)
   static constexpr int ST = stage_tiles(CLS);             // B tiles per stage (at most)
-  static constexpr int HDRMAX = stage_hdr_max(SB);
   static constexpr uint32_t ABLK = BH * 32;               // bytes of one A block (one operand)
   static constexpr uint32_t TILE = BN * 32;               // bytes of one B tile (one operand)
   static constexpr uint32_t TILEB = TILE * NOPS;          // bytes of one B tile slot
   static constexpr bool FP8 = KIND == KIND_FP8;
-  // stage: [A blocks hi | lo | header] [B tiles] [header offset word]; the
-  // FP8 form lands [e4m3 blocks | scales | header] in a staging area after
-  // the A blocks, which the converter warps turn into FP16 A blocks
-  static constexpr uint32_t OFF_STG = SB * ABLK * NOPS;
-  static constexpr uint32_t STG_BYTES = FP8 ? (SB * 256 + fp8_scale_bytes(SB) + HDRMAX + 255) / 256 * 256 : 0;
-  static constexpr uint32_t A_END = FP8 ? OFF_STG + STG_BYTES : OFF_STG + HDRMAX;
-  static constexpr uint32_t OFF_B = (A_END + 1023) / 1024 * 1024;
-  static constexpr uint32_t OFF_HW = OFF_B + ST * TILEB;
-  static constexpr uint32_t STAGE = (OFF_HW + 16 + 1023) / 1024 * 1024;
+  // stage: [header] [A blocks hi | lo] [B tiles]; the header and the blocks
+  // land with one copy. The FP8 form lands [header | e4m3 blocks | scales],
+  // which the converter warps turn into the FP16 A blocks after it.
+  static constexpr uint32_t HDR = kStageHdrBytes;
+  static constexpr uint32_t OFF_A = FP8 ? (HDR + SB * 256 + fp8_scale_bytes(SB) + 255) / 256 * 256 : HDR;
+  static constexpr uint32_t OFF_B = (OFF_A + SB * ABLK * NOPS + 1023) / 1024 * 1024;
+  static constexpr uint32_t STAGE = (OFF_B + ST * TILEB + 1023) / 1024 * 1024;
   static constexpr uint32_t SMEM_AVAIL = 227 * 1024 - 2048;  // minus alignment slack and barriers
   static constexpr int NS_FIT = (int)(SMEM_AVAIL / STAGE);
   static constexpr int NS = NS_FIT < 2 ? 2 : (NS_FIT > 8 ? 8 : NS_FIT);  // stages
@@ -110,9 +117,8 @@ struct Cfg {
   static constexpr int NPROD = 8;                         // copy warps
   static constexpr int NCONV = FP8 ? 4 : 0;               // FP8 converter warps (16..19)
   static constexpr uint32_t SMEM_BARS = 8 * (2 * NS + 4 + NMMA + (FP8 ? 2 * NS : 0) + 2 * kItemRing + 1);
-  // then the TMEM address, the abort flag, stage_ok[NS], the item ring and
-  // the copy warps' current item
-  static constexpr uint32_t SMEM_BYTES = 1024 + NS * STAGE + SMEM_BARS + 8 + 4 * (NS + kItemRing + 1);
+  // then the TMEM address, the abort flag and the ring of work items
+  static constexpr uint32_t SMEM_BYTES = 1024 + NS * STAGE + SMEM_BARS + 24 + kItemRing * sizeof(WorkItem);
   static constexpr int THREADS = 32 * (8 + NPROD + NCONV);  // MMA, epilogue, copy, converter warps
   static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0,
                 "TMEM allocation must be a power of two in [32, 512]");
@@ -120,6 +126,7 @@ struct Cfg {
   static_assert(NSUB == 1 || (NSUB == 2 && KIND == KIND_PLAIN), "256-column tiles: plain form only");
   static_assert(R <= 32, "slot field is 5 bits");
   static_assert(SB <= kMaxStageBlocks, "position field is 5 bits");
+  static_assert(stage_hdr_max(SB) <= (int)HDR, "stage header");
   // a stage tile of NSUB 128-column subtiles is NSUB copies (packed B is
   // [128-column tile][k-block]: the subtiles are not adjacent)
   static_assert(ST * NSUB + 1 <= 2 * NPROD && ST <= kMaxStageTiles,
@@ -128,6 +135,9 @@ struct Cfg {
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
   static_assert(!FP8 || (BH == 16 && NSUB == 1), "FP8 form: 16 x 16 blocks, 128-column tiles");
 };
+
+// Longest wait for a warp's own copies after an abort.
+constexpr uint64_t kDrainNs = 20000000ull;
 
 // Wait used only while draining after an abort: bounded, ignores the flag.
 __device__ __noinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity, int* err, uint64_t lim) {
@@ -141,10 +151,10 @@ __device__ __noinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity, int*
   return true;
 }
 
-// Bounded wait with an inlined fast path for phases that already completed.
+// Bounded wait: a tight poll first, then the timed one.
 __device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, volatile int* abort, int* err,
                                            int where, uint64_t lim) {
-  return mbar_try_wait(bar, parity) || mbar_wait(bar, parity, abort, err, where, lim);
+  return mbar_poll(bar, parity) || mbar_wait(bar, parity, abort, err, where, lim);
 }
 
 __device__ __forceinline__ bool wait_phase_sleepy(uint32_t bar, uint32_t parity, volatile int* abort, int* err,
@@ -152,42 +162,32 @@ __device__ __forceinline__ bool wait_phase_sleepy(uint32_t bar, uint32_t parity,
   return mbar_try_wait(bar, parity) || mbar_wait_sleepy(bar, parity, abort, err, where, lim);
 }
 
-// Item k of the CTA from the item ring, for a role run by lane 0 alone:
-// waits for it, reads it and frees the ring slot. idx = -1: no more work.
+// Item k of the CTA from the item ring, for a role that one lane runs alone:
+// waits for it, reads it and frees the ring slot. panel = -1: no more work.
 // Returns false when the CTA aborted.
-__device__ __forceinline__ bool take_item_lane0(uint64_t* itemfull, uint64_t* itemempty, const volatile int* ring,
-                                                uint32_t k, volatile int* abort, int* err, int where, uint64_t lim,
-                                                int& idx) {
+__device__ __forceinline__ bool take_item_one(uint64_t* itemfull, uint64_t* itemempty, const WorkItem* ring,
+                                              uint32_t k, volatile int* abort, int* err, int where, uint64_t lim,
+                                              WorkItem& wi) {
   const uint32_t r = k % kItemRing;
   if (!wait_phase(smem_u32(&itemfull[r]), (k / kItemRing) & 1, abort, err, where, lim)) return false;
-  idx = ring[r];
+  wi = ring[r];
   mbar_arrive(smem_u32(&itemempty[r]));
   return true;
 }
 
-// The same for a whole warp: lane 0 waits and reads, the warp gets the
-// index by shuffle (so the warp's decision is uniform).
-__device__ __forceinline__ bool take_item_warp(uint64_t* itemfull, uint64_t* itemempty, const volatile int* ring,
+// The same for a whole warp: every lane waits and reads, the vote makes the
+// warp's decision uniform, and one lane frees the slot.
+__device__ __forceinline__ bool take_item_warp(uint64_t* itemfull, uint64_t* itemempty, const WorkItem* ring,
                                                uint32_t k, int lane, volatile int* abort, int* err, int where,
-                                               uint64_t lim, int& idx) {
-  int got = 1, v = -1;
-  if (lane == 0) {
-    const uint32_t r = k % kItemRing;
-    got = wait_phase_sleepy(smem_u32(&itemfull[r]), (k / kItemRing) & 1, abort, err, where, lim) ? 1 : 0;
-    if (got) {
-      v = ring[r];
-      mbar_arrive(smem_u32(&itemempty[r]));
-    }
-  }
-  got = __shfl_sync(0xffffffffu, got, 0);
-  idx = __shfl_sync(0xffffffffu, v, 0);
-  return got != 0;
-}
-
-// The copy index that copy warp pw issues first in stage c: copy j of a
-// stage goes to warp (j + c) mod nprod, so the duties rotate.
-__device__ __forceinline__ int copy_of(int pw, uint32_t c, int nprod) {
-  return (int)(((uint32_t)pw + (uint32_t)nprod - c % (uint32_t)nprod) % (uint32_t)nprod);
+                                               uint64_t lim, bool sleepy, WorkItem& wi) {
+  const uint32_t r = k % kItemRing, bar = smem_u32(&itemfull[r]), par = (k / kItemRing) & 1;
+  const bool got = sleepy ? wait_phase_sleepy(bar, par, abort, err, where, lim)
+                          : wait_phase(bar, par, abort, err, where, lim);
+  if (!__all_sync(0xffffffffu, got)) return false;
+  wi = ring[r];
+  __syncwarp();
+  if (lane == 0) mbar_arrive(smem_u32(&itemempty[r]));
+  return true;
 }
 
 // Bounded wait for a whole warp: lane 0 polls, the warp learns the outcome
@@ -205,11 +205,6 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int lan
 }
 
 __device__ __forceinline__ int shfl_i(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ int64_t shfl_l(int64_t v, int src) {
-  const int lo = __shfl_sync(0xffffffffu, (int)(uint32_t)(uint64_t)v, src);
-  const int hi = __shfl_sync(0xffffffffu, (int)(uint32_t)((uint64_t)v >> 32), src);
-  return (int64_t)(((uint64_t)(uint32_t)hi << 32) | (uint32_t)lo);
-}
 
 // Warp roles: 0..3 MMA issuers (0 also owns TMEM), 4..7 epilogue (TMEM lane
 // quadrants 0..3), then NPROD copy warps, then (FP8) the converter warps.
@@ -235,11 +230,11 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
   uint64_t* stallbar = itemempty + kItemRing;        // nothing arrives here (test stall)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stallbar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* stage_ok = abort_flag + 1;  // [NS]: the copy leader's verdict on the stage's slot
-  volatile int* item_ring = stage_ok + C::NS;     // [kItemRing] item indices (-1: no more work)
-  volatile int* cur_item = item_ring + kItemRing;  // the copy warps' current item
+  // [kItemRing] work items (panel -1: no more work), 16-byte aligned
+  WorkItem* item_ring = reinterpret_cast<WorkItem*>((reinterpret_cast<uintptr_t>(tmem_slot + 2) + 15) &
+                                                    ~static_cast<uintptr_t>(15));
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // uniform for the compiler
   const int lane = threadIdx.x & 31;
   const uint64_t lim = args.wait_ns ? args.wait_ns : kWaitTimeoutNs;
   // stage slots in use (the pipeline depth): all that fit, or fewer when the
@@ -248,7 +243,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::NS; i++) {
-      mbar_init(smem_u32(&full[i]), 1);  // the A copy warp's arrive (+ every copy's bytes)
+      mbar_init(smem_u32(&full[i]), C::NPROD);  // every copy warp's arrive (+ its copies' bytes)
       mbar_init(smem_u32(&empty[i]), C::NMMA);
     }
     for (int i = 0; i < 2; i++) {
@@ -263,7 +258,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       }
     for (int i = 0; i < kItemRing; i++) {
       mbar_init(smem_u32(&itemfull[i]), 1);
-      mbar_init(smem_u32(&itemempty[i]), C::NMMA + 4 + C::NCONV);  // lane 0 of every other warp
+      mbar_init(smem_u32(&itemempty[i]), C::NMMA + 4 + C::NCONV + C::NPROD);  // one lane of every warp
     }
     mbar_init(smem_u32(stallbar), 1);
     *abort_flag = 0;
@@ -292,13 +287,12 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     uint32_t ci = 0;
     bool ok = true;
     for (uint32_t kk = 0; ok; ++kk) {
-      int idx = -1;
-      if (!take_item_warp(itemfull, itemempty, item_ring, kk, lane, abort_flag, err, ERR_ITEM_CONV, lim, idx)) {
+      WorkItem wi;
+      if (!take_item_warp(itemfull, itemempty, item_ring, kk, lane, abort_flag, err, ERR_ITEM_CONV, lim, false, wi)) {
         ok = false;
         break;
       }
-      if (idx < 0) break;
-      const WorkItem wi = args.items[idx];
+      if (wi.panel < 0) break;
       const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
       const int n_tiles = P.n_tiles;
       for (int nt = 0; nt < n_tiles && ok; ++nt) {
@@ -309,24 +303,40 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
             break;
           }
           uint8_t* stp = smem + s * C::STAGE;
-          const uint32_t hw = *reinterpret_cast<const uint32_t*>(stp + C::OFF_HW);
-          const int nblk = *reinterpret_cast<const uint16_t*>(stp + hw + 8);
-          const uint8_t* stg = stp + C::OFF_STG;
+          const int nblk = *reinterpret_cast<const uint16_t*>(stp + 8);
+          const uint8_t* stg = stp + C::HDR;
           const float* scl = reinterpret_cast<const float*>(stg + nblk * 256);
-          for (int x = ct; x < nblk * 32; x += 128) {
-            const int b = x >> 5, r = (x >> 1) & 15, hh = x & 1;  // block, row, 8-column half
-            const uint2 raw = *reinterpret_cast<const uint2*>(stg + b * 256 + r * 16 + hh * 8);
-            const float sc = scl[b];
-            uint32_t w[4];
+          // a thread widens whole 16-value rows; its rows are loaded first, so
+          // that the loads overlap (FP8 stencil 192 against 209 us with one
+          // 8-value piece loaded, widened and stored at a time)
+          constexpr int XN = (C::SB * 16 + 127) / 128;
+          uint4 raw[XN];
+          float sc[XN];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const uint16_t pair = (uint16_t)(((i < 2 ? raw.x : raw.y) >> (16 * (i & 1))) & 0xffffu);
+          for (int q = 0; q < XN; ++q) {
+            const int b = (ct >> 4) + 8 * q;  // block; the row is ct & 15
+            if (b < nblk) {
+              raw[q] = *reinterpret_cast<const uint4*>(stg + b * 256 + (ct & 15) * 16);
+              sc[q] = scl[b];
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < XN; ++q) {
+            const int b = (ct >> 4) + 8 * q, r = ct & 15;
+            if (b >= nblk) break;
+            const uint32_t in[4] = {raw[q].x, raw[q].y, raw[q].z, raw[q].w};
+            uint32_t w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const uint16_t pair = (uint16_t)((in[i >> 1] >> (16 * (i & 1))) & 0xffffu);
               const float2 f = __half22float2(e4m3x2_to_half2(pair));
-              const __half2 o = __floats2half2_rn(f.x * sc, f.y * sc);
+              const __half2 o = __floats2half2_rn(f.x * sc[q], f.y * sc[q]);
               w[i] = *reinterpret_cast<const uint32_t*>(&o);
             }
-            *reinterpret_cast<uint4*>(stp + b * 512 + r * 32 + ((hh ^ ((r >> 2) & 1)) << 4)) =
-                make_uint4(w[0], w[1], w[2], w[3]);
+            uint4* dst = reinterpret_cast<uint4*>(stp + C::OFF_A + b * 512 + r * 32);
+            const int sw = (r >> 2) & 1;
+            dst[sw] = make_uint4(w[0], w[1], w[2], w[3]);
+            dst[sw ^ 1] = make_uint4(w[4], w[5], w[6], w[7]);
           }
           fence_proxy_async_smem();
           __syncwarp();
@@ -336,152 +346,115 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     }
   } else if (warp >= 8) {
     // ---------------------------------------------------------------- copies
-    // Stage number c (counted over the CTA's whole run) needs 1 + ntiles
-    // bulk copies: copy 0 = the A blocks and the MMA list, copy j = B tile
-    // j - 1. Copy warp p issues the copies j with (j + c) % NPROD == p (j and
-    // j + NPROD), so every warp issues one or two copies per stage and the A
-    // copy (from HBM, the slowest) rotates. A warp keeps only about one copy
-    // at a time in flight, so spreading them is what keeps the copy engine
-    // busy. The warp that
-    // issues copy 0 posts the stage's total byte count (arrive.expect_tx) on
-    // the stage's full barrier; the others only add their bytes as they land.
-    // Stage records are read 32 at a time, one per lane, and each lane
-    // prepares what its warp needs from its record.
+    // Stage number c (counted over the CTA's whole run) needs a copy of its
+    // A region (header and blocks) and one per 128-column subtile of its B
+    // tiles. B copy j goes to copy warp (j + c) mod NPROD, so every warp has
+    // at most two per stage, and the A region (from HBM, the slowest) to the
+    // warp for j = NPROD - 1. Every warp waits for the stage's slot itself and
+    // arrives on its full barrier once per stage, adding the bytes it brings:
+    // no warp can run a ring ahead, and none waits for another (a named
+    // barrier among the eight and their leader's wait took about 550 of a
+    // stage's 1,650 cycles). Stage records are read 32 at a time, one per
+    // lane, and each lane prepares what its warp needs from its record.
     const int pw = warp - 8;
     const uint64_t pol_a = make_l2_policy_evict_first();  // A streams through L2 once
     const uint64_t pol_b = make_l2_policy_evict_last();   // B tiles are re-read by many CTAs
-    uint32_t ci = 0;
+    uint32_t ci = 0, slot_s = 0, phase_s = 1;
     bool ok = true;
     uint32_t last_mine = 0xffffffffu;  // last stage this warp copied into (for the drain)
     for (uint32_t kk = 0; ok; ++kk) {
-      // The CTA's next item: lane 0 of the first copy warp takes it from the
-      // launch's order (the CTA's own index first, then the shared
-      // counter), puts it in the item ring for the other roles once they
-      // have read the entry it replaces, and hands it to the copy warps.
-      if (pw == 0 && lane == 0) {
+      // The CTA's next item: the first copy warp takes it from the launch's
+      // list (the CTA's own index first, then the shared counter) and puts it
+      // in the item ring once every role has read the entry it replaces.
+      if (pw == 0) {
         const uint32_t r = kk % kItemRing;
-        int idx = -2;  // -2: aborted
-        if (wait_phase(smem_u32(&itemempty[r]), ((kk / kItemRing) & 1) ^ 1, abort_flag, err, ERR_ITEM_TAKE, lim)) {
-          const int pos = kk == 0 ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(args.next_item, 1);
-          idx = pos < args.n_items ? args.order[pos] : -1;
-          item_ring[r] = idx;
-          mbar_arrive(smem_u32(&itemfull[r]));
+        if (elect_one()) {
+          if (wait_phase(smem_u32(&itemempty[r]), ((kk / kItemRing) & 1) ^ 1, abort_flag, err, ERR_ITEM_TAKE, lim)) {
+            const int pos = kk == 0 ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(args.next_item, 1);
+            WorkItem nw;
+            nw.panel = -1;
+            if (pos < args.n_items) nw = args.items[pos];
+            item_ring[r] = nw;
+            mbar_arrive(smem_u32(&itemfull[r]));
+          }
         }
-        *cur_item = idx;
+        __syncwarp();
       }
-      named_bar_sync(1, 32 * C::NPROD);
-      const int idx = *cur_item;
-      if (idx < 0) {
-        ok = idx == -1;
+      WorkItem wi;
+      if (!take_item_warp(itemfull, itemempty, item_ring, kk, lane, abort_flag, err, ERR_ITEM_TAKE, lim, false, wi)) {
+        ok = false;
         break;
       }
-      const WorkItem wi = args.items[idx];
+      if (wi.panel < 0) break;
       const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
       // fields used after shared-memory stores, held in registers (the stores
       // could alias P for the compiler and force a reload each time)
       const StageRec* const p_stages = P.stages;
       const uint8_t* const p_aval = P.aval;
-      const uint8_t* const p_bpack = P.bpack;
       const int64_t p_kbs = P.bp_kbs;
       const int n_tiles = P.n_tiles;
-      const int stage0 = P.panels[wi.panel].stage_off;
       for (int nt = 0; nt < n_tiles && ok; ++nt) {
-        const int64_t bcol = (int64_t)nt * NSUB;  // first 128-column packed tile of this pass
+        // the packed tiles of this pass ([128-column tile][k-block])
+        const uint8_t* const p_b = P.bpack + (int64_t)nt * NSUB * p_kbs * (4096 * C::NOPS);
+        const int64_t sub_bytes = p_kbs * (4096 * C::NOPS);
         for (int base = wi.s0; base < wi.s1 && ok; base += 32) {
           const int cnt = min(32, wi.s1 - base);
-          // lane l prepares stage ci + l
-          const uint32_t my_ci = ci + (uint32_t)lane;
-          const int j0 = copy_of(pw, my_ci, C::NPROD);
-          int64_t off1 = 0, off2 = 0;
-          int bytes1 = 0, bytes2 = 0, dst1 = 0, dst2 = 0, total = 0, hword = 0;
+          // lane l prepares stage ci + l: this warp's B copies j0 and j0 +
+          // NPROD (copy j brings subtile j % NSUB of tile j / NSUB), and the
+          // A region for the warp of the last copy index
+          const int j0 = (int)(((uint32_t)pw - (ci + (uint32_t)lane)) & (C::NPROD - 1));
+          int kb1 = -1, kb2 = -1, abytes = 0, aoff = 0;
           if (lane < cnt) {
-            const StageRec* rp = p_stages + stage0 + base + lane;
-            const longlong2 r0 = reinterpret_cast<const longlong2*>(rp)[0];  // blk_off, hdr_off
-            const int4 r1 = reinterpret_cast<const int4*>(rp)[1];           // nblk, hdr_bytes, ntiles, -
-            const int ntl = r1.z;
-            if (j0 == 0) {
-              // the stage's A region (blocks, FP8 scales, header) in one copy
-              // (an L2 prefetch of it a few stages ahead measured slower:
-              // it competes with the copies for the copy engine)
-              if (C::FP8) {
-                off1 = r0.x * 256 + r1.w + r0.y;
-                bytes1 = r1.x * 256 + fp8_scale_bytes(r1.x) + r1.y;
-              } else {
-                off1 = r0.x * (int64_t)(C::ABLK * C::NOPS) + r0.y;
-                bytes1 = r1.x * (int)(C::ABLK * C::NOPS) + r1.y;
-              }
-              // header position inside the stage
-              hword = C::FP8 ? (int)C::OFF_STG + r1.x * 256 + fp8_scale_bytes(r1.x) : r1.x * (int)(C::ABLK * C::NOPS);
-              total = bytes1 + ntl * (int)C::TILEB;
-            }
-            // B copies, one per 128-column subtile (several copies in flight
-            // land sooner than one long copy of adjacent tiles): copy c >= 1
-            // brings subtile (c - 1) % NSUB of tile (c - 1) / NSUB; this
-            // warp's are copies j0 and j0 + NPROD
-            if (j0 >= 1 && j0 <= ntl * NSUB) {
-              const int t = (j0 - 1) / NSUB, sub = (j0 - 1) % NSUB;
-              off1 = ((int64_t)(bcol + sub) * p_kbs + rp->kb[t]) * (4096 * C::NOPS);
-              bytes1 = 4096 * C::NOPS;
-              dst1 = t * (int)C::TILEB + sub * 4096 * C::NOPS;
-            }
-            if (j0 + C::NPROD <= ntl * NSUB) {
-              const int t = (j0 + C::NPROD - 1) / NSUB, sub = (j0 + C::NPROD - 1) % NSUB;
-              off2 = ((int64_t)(bcol + sub) * p_kbs + rp->kb[t]) * (4096 * C::NOPS);
-              bytes2 = 4096 * C::NOPS;
-              dst2 = t * (int)C::TILEB + sub * 4096 * C::NOPS;
+            const StageRec* rp = p_stages + base + lane;
+            const int4 r1 = reinterpret_cast<const int4*>(rp)[1];  // nblk, hdr_bytes, ntiles, aoff256
+            const int nc = r1.z * NSUB;
+            if (j0 < nc) kb1 = rp->kb[j0 / NSUB];
+            if (j0 + C::NPROD < nc) kb2 = rp->kb[(j0 + C::NPROD) / NSUB];
+            if (j0 == C::NPROD - 1) {
+              aoff = r1.w;
+              abytes = stage_a_bytes(C::CLS, BH, r1.x);
             }
           }
           for (int i = 0; i < cnt; ++i, ++ci) {
-            const int b1 = shfl_i(bytes1, i);
-            const int b2 = shfl_i(bytes2, i);
-            const int d1 = shfl_i(dst1, i);
-            const int d2 = shfl_i(dst2, i);
-            const int64_t o1 = shfl_l(off1, i);
-            const int64_t o2 = shfl_l(off2, i);
-            const int tot = shfl_i(total, i);
-            const int hw = shfl_i(hword, i);
-            const int j = copy_of(pw, ci, C::NPROD);
-            const uint32_t s = ci % nsr;
-            // The warp with copy 0 waits for the slot and passes its verdict
-            // to the other copy warps through a named barrier (blocked warps
-            // take no issue slots); so all copy warps move stage by stage and
-            // none can run a ring ahead and overwrite a stage still in use.
-            if (j == 0 && lane == 0)
-              stage_ok[s] = wait_phase(smem_u32(&empty[s]), ((ci / nsr) & 1) ^ 1, abort_flag, err, ERR_PROD_A, lim) ? 1 : 0;
-            named_bar_sync(1, 32 * C::NPROD);
-            int good = 1;
-            if (lane == 0) {
-              if (stage_ok[s]) {
-                const uint32_t st = smem0 + s * C::STAGE;
-                const uint32_t fb = smem_u32(&full[s]);
-                if (b1 == 0) {
-                  // no copy for this warp in this stage
-                } else if (j == 0) {
-                  *reinterpret_cast<uint32_t*>(smem + s * C::STAGE + C::OFF_HW) = (uint32_t)hw;
-                  if (C::FP8) {
-                    // the A region on its own barrier (the converters wait
-                    // for it alone), the B tiles on full[s]
-                    const uint32_t ab = smem_u32(&afull[s]);
-                    mbar_arrive_expect_tx(ab, (uint32_t)b1);
-                    bulk_load_hint(st + C::OFF_STG, p_aval + o1, (uint32_t)b1, ab, pol_a);
-                    mbar_arrive_expect_tx(fb, (uint32_t)(tot - b1));
-                  } else {
-                    mbar_arrive_expect_tx(fb, (uint32_t)tot);
-                    bulk_load_hint(st, p_aval + o1, (uint32_t)b1, fb, pol_a);
-                  }
-                } else {
-                  bulk_load_hint(st + C::OFF_B + d1, p_bpack + o1, (uint32_t)b1, fb, pol_b);
-                }
-                if (b2 != 0) bulk_load_hint(st + C::OFF_B + d2, p_bpack + o2, (uint32_t)b2, fb, pol_b);
-                if (b1 != 0 || b2 != 0) last_mine = ci;
-              } else {
-                good = 0;
-              }
-            }
-            good = shfl_i(good, 0);
-            if (!good) {
+            const int k1 = shfl_i(kb1, i), k2 = shfl_i(kb2, i);
+            const int ab = shfl_i(abytes, i), ao = shfl_i(aoff, i);
+            const int j = (int)(((uint32_t)pw - ci) & (C::NPROD - 1));
+            const uint32_t s = slot_s;
+            const bool good = wait_phase(smem_u32(&empty[s]), phase_s, abort_flag, err, ERR_PROD_A, lim);
+            if (!__all_sync(0xffffffffu, good)) {
               ok = false;
               break;
+            }
+            if (elect_one()) {
+              const uint32_t st = smem0 + s * C::STAGE;
+              const uint32_t fb = smem_u32(&full[s]);
+              uint32_t bytes = (k1 >= 0 ? 4096u * C::NOPS : 0u) + (k2 >= 0 ? 4096u * C::NOPS : 0u);
+              if (ab != 0) {
+                if (C::FP8) {
+                  // the A region on its own barrier (the converters wait for
+                  // it alone), the B tiles on full[s]
+                  const uint32_t fa = smem_u32(&afull[s]);
+                  mbar_arrive_expect_tx(fa, (uint32_t)ab);
+                  bulk_load_hint(st, p_aval + (int64_t)ao * 256, (uint32_t)ab, fa, pol_a);
+                } else {
+                  bytes += (uint32_t)ab;
+                }
+              }
+              mbar_arrive_expect_tx(fb, bytes);
+              if (!C::FP8 && ab != 0) bulk_load_hint(st, p_aval + (int64_t)ao * 256, (uint32_t)ab, fb, pol_a);
+              if (k1 >= 0)
+                bulk_load_hint(st + C::OFF_B + j * (4096 * C::NOPS),
+                               p_b + (j % NSUB) * sub_bytes + (int64_t)k1 * (4096 * C::NOPS), 4096 * C::NOPS, fb, pol_b);
+              if (k2 >= 0)
+                bulk_load_hint(st + C::OFF_B + (j + C::NPROD) * (4096 * C::NOPS),
+                               p_b + ((j + C::NPROD) % NSUB) * sub_bytes + (int64_t)k2 * (4096 * C::NOPS),
+                               4096 * C::NOPS, fb, pol_b);
+            }
+            __syncwarp();
+            last_mine = ci;
+            if (++slot_s == nsr) {
+              slot_s = 0;
+              phase_s ^= 1u;
             }
           }
         }
@@ -489,15 +462,18 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     }
     if (!ok && lane == 0 && last_mine != 0xffffffffu) {
       // wait for this warp's own copies still in flight: they can only be in
-      // the last NS stages it copied into
+      // the last NS stages it copied into (a stage that another warp gave up
+      // on never completes, but copies land within microseconds: the wait is
+      // short)
       const uint32_t lo = last_mine + 1 > nsr ? last_mine + 1 - nsr : 0;
+      const uint64_t dl = lim < kDrainNs ? lim : kDrainNs;
       for (uint32_t k = lo; k <= last_mine; ++k) {
-        mbar_wait_drain(smem_u32(&full[k % nsr]), (k / nsr) & 1, err, lim);
-        if (C::FP8) mbar_wait_drain(smem_u32(&afull[k % nsr]), (k / nsr) & 1, err, lim);
+        mbar_wait_drain(smem_u32(&full[k % nsr]), (k / nsr) & 1, err, dl);
+        if (C::FP8) mbar_wait_drain(smem_u32(&afull[k % nsr]), (k / nsr) & 1, err, dl);
       }
     }
   } else if (warp < C::NMMA) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ----------------------------------------------------------- MMA issuers
       // Issuer w runs the MMA groups of its quarter of the panel's block rows,
       // from the list the copy brought in with the stage, and releases every
@@ -507,13 +483,12 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       bool ok = true, issued = false;
       const uint32_t stall = (blockIdx.x == 0 && warp == 0) ? (uint32_t)args.stall_stage : 0u;
       for (uint32_t kk = 0; ok; ++kk) {
-        int idx = -1;
-        if (!take_item_lane0(itemfull, itemempty, item_ring, kk, abort_flag, err, ERR_ITEM_MMA, lim, idx)) {
+        WorkItem wi;
+        if (!take_item_one(itemfull, itemempty, item_ring, kk, abort_flag, err, ERR_ITEM_MMA, lim, wi)) {
           ok = false;
           break;
         }
-        if (idx < 0) break;
-        const WorkItem wi = args.items[idx];
+        if (wi.panel < 0) break;
         const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
         const int n_tiles = P.n_tiles;
         const uint32_t idesc0 = P.idesc;  // without the N field
@@ -532,8 +507,9 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
             const uint32_t s = slot_s;  // == ci % nsr, kept incrementally
             if (stall != 0u && ci + 1 == stall) {
               // test stall: nothing arrives on this barrier, so the wait runs
-              // into its limit and the CTA aborts
-              ok = wait_phase(smem_u32(stallbar), 0, abort_flag, err, ERR_MMA_STALL, lim);
+              // into its limit (half of the others', so that it is the one
+              // that reports) and the CTA aborts
+              ok = wait_phase(smem_u32(stallbar), 0, abort_flag, err, ERR_MMA_STALL, lim / 2);
               if (!ok) break;
             }
             // the stage's copies landed (complete_tx); the MMA reads shared
@@ -545,10 +521,12 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
               break;
             }
             const uint8_t* stp = smem + s * C::STAGE;
-            const uint32_t hw = *reinterpret_cast<const uint32_t*>(stp + C::OFF_HW);
-            const uint32_t wl = *reinterpret_cast<const uint16_t*>(stp + hw + 2 * warp);
+            const uint2 hd = *reinterpret_cast<const uint2*>(stp);  // (first, count) of each warp
+            const uint32_t wl = ((warp & 2 ? hd.y : hd.x) >> (16 * (warp & 1))) & 0xffffu;
             const uint32_t first = wl & 0xffu, cnt = wl >> 8;
-            const uint32_t* ent = reinterpret_cast<const uint32_t*>(stp + hw + kStageHdrFixed) + first;
+            const uint32_t* ent = reinterpret_cast<const uint32_t*>(stp + kStageHdrFixed) + first;
+            // lo blocks follow the stage's nblk hi blocks (split form)
+            const uint32_t lo_off = KIND == KIND_SPLIT ? *reinterpret_cast<const uint16_t*>(stp + 8) * C::ABLK : 0;
             // descriptors of operands inside the stage = stage descriptor + offset / 16
             const uint64_t sdesc = desc_kmajor_sw32(smem0 + s * C::STAGE);
             for (uint32_t e = 0; e < cnt; ++e) {
@@ -556,7 +534,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
               const uint32_t pos = m & 31u, tile = (m >> 5) & 15u, slot = (m >> 9) & 31u;
               const uint32_t len = ((m >> 14) & 15u) + 1u, acc = (m >> 18) & 1u;
               const uint32_t idesc = idesc0 | (((len * BH) >> 3) << 17);
-              const uint64_t a_hi = sdesc + ((pos * C::ABLK) >> 4);
+              const uint64_t a_hi = sdesc + ((C::OFF_A + pos * C::ABLK) >> 4);
               const uint64_t b_hi0 = sdesc + ((C::OFF_B + tile * C::TILEB) >> 4);
 #pragma unroll
               for (int j = 0; j < NSUB; ++j) {
@@ -564,7 +542,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
                 const uint64_t b_hi = b_hi0 + ((j * 128 * 32) >> 4);
                 umma_f16(dcol, b_hi, a_hi, idesc, acc);
                 if (KIND == KIND_SPLIT) {
-                  const uint64_t a_lo = a_hi + ((hw >> 1) >> 4);  // lo blocks follow the nblk hi blocks
+                  const uint64_t a_lo = a_hi + (lo_off >> 4);
                   const uint64_t b_lo = b_hi + (C::TILE >> 4);
                   umma_f16(dcol, b_hi, a_lo, idesc, 1);
                   umma_f16(dcol, b_lo, a_hi, idesc, 1);
@@ -616,13 +594,12 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     uint32_t k = 0;
     bool ok = true;
     for (uint32_t kk = 0; ok; ++kk) {
-      int idx = -1;
-      if (!take_item_warp(itemfull, itemempty, item_ring, kk, lane, abort_flag, err, ERR_ITEM_EPI, lim, idx)) {
+      WorkItem wi;
+      if (!take_item_warp(itemfull, itemempty, item_ring, kk, lane, abort_flag, err, ERR_ITEM_EPI, lim, true, wi)) {
         ok = false;
         break;
       }
-      if (idx < 0) break;
-      const WorkItem wi = args.items[idx];
+      if (wi.panel < 0) break;
       const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
       // fields used between the stores to C, held in registers (the stores
       // could alias P for the compiler and force reloads of every field)

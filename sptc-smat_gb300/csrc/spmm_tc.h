@@ -43,25 +43,29 @@ struct PanelInfo {
 // Per-stage record (96 bytes), read by the copy warps. In the device A
 // stream of a form (ABLK = bh * 32 bytes per block and operand, NOPS = 2 for
 // the split form, else 1) a stage occupies
-//     [nblk * ABLK blocks (hi)][nblk * ABLK blocks (lo, split form only)][header]
-// starting at byte blk_off * ABLK * NOPS + hdr_off, where hdr_off is the sum
-// of the header bytes of all earlier stages. In the FP8 stream (16 x 16
-// blocks) a stage occupies
-//     [nblk * 256 e4m3 blocks][nblk FP32 scales, padded to 16 bytes][header]
-// starting at byte blk_off * 256 + scl_off + hdr_off, where scl_off is the
-// sum of the padded scale bytes of all earlier stages.
+//     [header, kStageHdrBytes][nblk * ABLK blocks (hi)][nblk * ABLK blocks (lo, split form only)]
+// and in the FP8 stream (16 x 16 blocks)
+//     [header, kStageHdrBytes][nblk * 256 e4m3 blocks][nblk FP32 scales, padded to 16 bytes]
+// starting at byte aoff256 * 256 (the stages of the FP8 stream are padded to
+// that), so the header is always at the stage's start and the MMA threads
+// need no word that says where.
+// Padded bytes of the FP32 scales of n FP8 blocks.
+__host__ __device__ constexpr int fp8_scale_bytes(int n) { return (4 * n + 15) / 16 * 16; }
+// Bytes of a stage of nblk blocks in the A stream of plan class cls.
+constexpr int kStageHdrBytes = 256;  // a header's room in the A stream and in shared memory
+__host__ __device__ constexpr int stage_a_bytes(int cls, int bh, int nblk) {
+  return kStageHdrBytes + (cls == 2 ? nblk * 256 + fp8_scale_bytes(nblk) : nblk * bh * 32 * (cls == 1 ? 2 : 1));
+}
 struct StageRec {
-  int64_t blk_off;     // blocks before this stage (stream order)
-  int64_t hdr_off;     // header bytes before this stage
+  int64_t blk_off;     // blocks before this stage (plan order)
+  int64_t hdr_off;     // header bytes before this stage (Plan::headers)
   int32_t nblk;        // A blocks in the stage
   int32_t hdr_bytes;   // bytes of this stage's header (multiple of 16)
   int32_t ntiles;      // B tiles (distinct block columns) of the stage, 1..stage_tiles
-  int32_t scl_off;     // padded FP8 scale bytes before this stage
+  int32_t aoff256;     // start of the stage in the A stream, in units of 256 bytes
   int32_t kb[kMaxStageTiles];  // k-block (column / 16) of each tile
 };
 
-// Padded bytes of the FP32 scales of n FP8 blocks.
-__host__ __device__ constexpr int fp8_scale_bytes(int n) { return (4 * n + 15) / 16 * 16; }
 
 // Stage header (little-endian), kStageHdrFixed bytes then one 32-bit entry
 // per MMA group, grouped by issuing warp:
@@ -84,7 +88,7 @@ __host__ __device__ constexpr int stage_hdr_max(int sb) { return kStageHdrFixed 
 // split index: its parts write partial sums to workspace slabs, and the part
 // that finishes last (an atomic counter per split panel and column tile)
 // adds the slabs and writes C.
-struct WorkItem {
+struct alignas(16) WorkItem {
   int32_t panel;
   int32_t s0, s1;      // stage range, relative to the panel's first stage
   int32_t split;       // -1: the whole panel; else index of the split panel
@@ -118,10 +122,11 @@ struct ProblemDesc {
 // Kernel arguments (one __grid_constant__ parameter). A single SpMM passes
 // its problem by value (one); a grouped launch passes a device array
 // (probs, indexed by WorkItem::prob).
-// A launch: its problems and work items. CTA b takes the items order[b],
-// then order[grid + atomicAdd(next_item, 1)], ... until the list is done:
-// the items are sorted by decreasing estimated cost, so whichever CTA is
-// free first takes the largest item left (the counter is zero at launch).
+// A launch: its problems and work items, by decreasing estimated cost and
+// with the stage range counted from the plan's first stage. CTA b takes item
+// b, then item grid + atomicAdd(next_item, 1), ... until the list is done:
+// whichever CTA is free first takes the largest item left (the counter is
+// zero at launch).
 // wait_ns bounds every device-side wait (0: 4 s); stall_stage k > 0 makes
 // the first MMA-issuing thread of CTA 0 wait, before its k-th stage, on a
 // barrier nothing arrives at (a test of the bounded-wait error path);
@@ -130,7 +135,6 @@ struct ProblemDesc {
 struct SpmmArgs {
   ProblemDesc one;
   const ProblemDesc* probs;
-  const int32_t* order;      // [n_items] item indices by decreasing cost
   int32_t* next_item;        // zero at launch
   const WorkItem* items;
   int* err;
