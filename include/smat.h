@@ -276,9 +276,10 @@ smat_status smat_tiles_destroy(smat_tiles* t);
 /* ---------------------------------------------------------------- step 3 */
 
 /* Bytes of device scratch smat_spmm needs for this form / B dtype / N: the
- * packed copy of B (twice that for the split form), and for panels split
- * over several CTAs for load balance, one counter per split panel and a
- * partial-sum slab per part. */
+ * packed copy of B (twice that for the split form), for panels split over
+ * several CTAs for load balance one counter per split panel and a partial-sum
+ * slab per part, and a byte per 128 x 64 values of B that says whether they
+ * hold an infinite or NaN one. */
 smat_status smat_spmm_workspace_size(const smat_bcsr* A, int32_t form, int32_t b_dtype, int64_t N,
                                      size_t* bytes);
 
@@ -320,9 +321,10 @@ smat_status smat_spmm_packed(const smat_bcsr* A, int32_t form, const void* packe
  * they need no scratch). Same arguments and results as smat_spmm, without
  * workspace; the packed B goes to a fixed device array of
  * SMAT_SPMM_STATIC_SCRATCH_BYTES inside the library, and nothing is
- * allocated. Returns SMAT_ERR_UNSUPPORTED when smat_spmm_workspace_size()
- * exceeds that size (the packed B, K x N x 2 bytes or twice that for the
- * split form, plus the partial sums of panels split for load balance). The
+ * allocated. Returns SMAT_ERR_UNSUPPORTED when the packed B (K x N x 2 bytes
+ * or twice that for the split form, rounded up to tiles) exceeds that size;
+ * where the partial sums of panels split for load balance do not fit beside
+ * it, no panel is split. The
  * first call on a device looks the array's address
  * up (make it before any stream capture), and so does the first call after
  * the device's context was destroyed and created again (cudaDeviceReset).

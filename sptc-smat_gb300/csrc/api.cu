@@ -85,7 +85,8 @@ static void free_handle(smat_bcsr* h) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (PlanDev& pd : h->pc) {
-    void* pp[] = {pd.d_stages, pd.d_panels, pd.d_row_map, pd.sched[1].d_items, pd.sched[2].d_items};
+    void* pp[] = {pd.d_stages, pd.d_panels, pd.d_row_map, pd.d_gcol, pd.d_poison_ptr, pd.d_poison, pd.sched[1].d_items, pd.sched[2].d_items,
+                  pd.sched[1].d_whole, pd.sched[2].d_whole};
     for (void* p : pp)
       if (p) cudaFree(p);
   }
@@ -158,7 +159,7 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
     if (cls == 1 && !(forms & (1u << SMAT_FORM_SPLIT_BF16))) continue;
     if (cls == 2 && !(forms & (1u << SMAT_FORM_FP8))) continue;
     if (cls == 3 && !wide) continue;
-    st = build_plan(h->host, R, cls, h->pc[cls].plan, ((cls == 0 || cls == 3) && h->sp24_on) ? &take24 : nullptr);
+    st = build_plan(h->host, R, cls, h->pc[cls].plan, ((cls == 0 || cls == 3) && h->sp24_on) ? &take24 : nullptr, true);
     if (st != SMAT_OK) {
       delete h;
       return st;
@@ -205,6 +206,11 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
     SMAT_TRY(upload(&pd.d_stages, pd.plan.stages.data(), pd.plan.stages.size()));
     SMAT_TRY(upload(&pd.d_panels, pd.plan.panels.data(), pd.plan.panels.size()));
     SMAT_TRY(upload(&pd.d_row_map, pd.plan.row_map.data(), pd.plan.row_map.size()));
+    if (!pd.plan.gcol.empty()) SMAT_TRY(upload(&pd.d_gcol, pd.plan.gcol.data(), pd.plan.gcol.size()));
+    if (!pd.plan.poison.empty()) {
+      SMAT_TRY(upload(&pd.d_poison_ptr, pd.plan.poison_ptr.data(), pd.plan.poison_ptr.size()));
+      SMAT_TRY(upload(&pd.d_poison, pd.plan.poison.data(), pd.plan.poison.size()));
+    }
     // work items per launch shape (NSUB 1 and 2): heavy panels split into
     // parts so that no CTA gets much more than the average
     const int kind = cls == 1 ? TC_KIND_SPLIT : (cls == 2 ? TC_KIND_FP8 : TC_KIND_PLAIN);
@@ -216,10 +222,19 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
       std::vector<int32_t> order;
       Sched& sc = pd.sched[nsub];
       build_work_items(pd.plan, bh, workers, frac, items, order, sc.n_split, sc.n_slabs);
-      sc.grid = std::max(1, std::min<int>(workers, (int)items.size()));
+      sc.workers = workers;
       sc.n_items = (int32_t)items.size();
-      const std::vector<WorkItem> dev = device_items({&pd.plan}, items, order);
+      std::vector<WorkItem> dev = device_items({&pd.plan}, items, order);
       SMAT_TRY(upload(&sc.d_items, dev.data(), dev.size()));
+      if (sc.n_split > 0) {
+        // the same without split panels, for scratch that has no room for
+        // their partial sums
+        int32_t ns = 0, nl = 0;
+        build_work_items(pd.plan, bh, workers, 1e30, items, order, ns, nl);
+        dev = device_items({&pd.plan}, items, order);
+        sc.n_whole = (int32_t)dev.size();
+        SMAT_TRY(upload(&sc.d_whole, dev.data(), dev.size()));
+      }
     }
   }
 
@@ -234,7 +249,18 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
     const int64_t nst = (int64_t)pl.stages.size();
     out.assign(std::max<size_t>(pl.a_bytes, 16), 0);
     auto put = [&](const std::vector<uint16_t>& vals, int64_t k, uint8_t* dst) {
-      const uint8_t* src = reinterpret_cast<const uint8_t*>(vals.data() + (size_t)pl.stream_blk[k] * bsz);
+      const int32_t blk = pl.stream_blk[k];
+      if (blk < 0) {  // gathered: sixteen columns of the block row's blocks
+        const int64_t* from = pl.gsrc.data() + (size_t)(-(blk + 1)) * 16;
+        for (int q = 0; q < 16; q++) {
+          if (from[q] < 0) continue;
+          const uint16_t* v = vals.data() + (size_t)(from[q] >> 4) * bsz + (from[q] & 15);
+          for (int r = 0; r < bh; r++)
+            std::memcpy(dst + r * 32 + (((q >> 3) ^ ((r >> 2) & 1)) * 16) + (q & 7) * 2, v + r * 16, 2);
+        }
+        return;
+      }
+      const uint8_t* src = reinterpret_cast<const uint8_t*>(vals.data() + (size_t)blk * bsz);
       for (int r = 0; r < bh; r++)
         for (int c = 0; c < 2; c++)
           std::memcpy(dst + r * 32 + ((c ^ ((r >> 2) & 1)) * 16), src + r * 32 + c * 16, 16);
@@ -296,8 +322,20 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
       uint8_t* base = lay.data() + (size_t)r.aoff256 * 256;
       std::memcpy(base, pl.headers.data() + r.hdr_off, (size_t)r.hdr_bytes);
       base += kStageHdrBytes;
+      uint8_t* gscl = base + (size_t)r.nblk * 256 + fp8_scale_bytes(r.nblk);
       for (int32_t qb = 0; qb < r.nblk; qb++) {
         const int64_t blk = pl.stream_blk[r.blk_off + qb];
+        if (blk < 0) {
+          const int64_t* from = pl.gsrc.data() + (size_t)(-(blk + 1)) * 16;
+          for (int q = 0; q < 16; q++) {
+            if (from[q] < 0) continue;
+            const uint8_t* v = h->fp8_q.data() + (size_t)(from[q] >> 4) * 256 + (from[q] & 15);
+            for (int i = 0; i < 16; i++) base[(size_t)qb * 256 + i * 16 + q] = v[i * 16];
+            std::memcpy(gscl + 4 * q, &h->fp8_scale[from[q] >> 4], 4);
+          }
+          gscl += 64;
+          continue;
+        }
         std::memcpy(base + (size_t)qb * 256, h->fp8_q.data() + (size_t)blk * 256, 256);
         std::memcpy(base + (size_t)r.nblk * 256 + (size_t)qb * 4, &h->fp8_scale[blk], 4);
       }
@@ -523,7 +561,7 @@ static bool uses_sp24(const smat_bcsr* A, int32_t form) {
   return A->sp24_on && (form == SMAT_FORM_F16 || form == SMAT_FORM_BF16);
 }
 
-WsLayout smat::ws_layout(const smat_bcsr* A, int32_t form, int64_t N) {
+WsLayout smat::ws_layout(const smat_bcsr* A, int32_t form, int64_t N, bool whole) {
   WsLayout w;
   const bool split = form == SMAT_FORM_SPLIT_BF16;
   const size_t one = (packed_b_bytes(A->host.cols, std::max<int64_t>(N, 1)) + 255) / 256 * 256;
@@ -535,9 +573,11 @@ WsLayout smat::ws_layout(const smat_bcsr* A, int32_t form, int64_t N) {
   const int nsub = pick_nsub(A, N, kind_of(form));
   const Sched& sc = A->pc[plan_class(form, nsub)].sched[nsub];
   const int64_t bn = 128 * nsub, n_tiles = (std::max<int64_t>(N, 1) + bn - 1) / bn;
-  w.counter_bytes = (16 + (size_t)sc.n_split * n_tiles * 4 * sizeof(int32_t) + 255) / 256 * 256;
+  const size_t n_split = whole ? 0 : sc.n_split, n_slabs = whole ? 0 : sc.n_slabs;
+  w.counter_bytes = (16 + n_split * n_tiles * 4 * sizeof(int32_t) + 255) / 256 * 256;
   w.slabs = w.counters + w.counter_bytes;
-  w.total = w.slabs + (size_t)sc.n_slabs * n_tiles * A->R * A->host.bh * bn * sizeof(float);
+  w.flags = w.slabs + n_slabs * n_tiles * A->R * A->host.bh * bn * sizeof(float);
+  w.total = w.flags + (pack_flag_bytes(A->host.cols, std::max<int64_t>(N, 1)) + 255) / 256 * 256;
   return w;
 }
 
@@ -555,18 +595,24 @@ void smat::fill_problem(const smat_bcsr* A, int32_t form, const void* ws_, int64
   P.panels = A->pc[cls].d_panels;
   P.stages = A->pc[cls].d_stages;
   P.row_map = A->pc[cls].d_row_map;
+  P.bflags = ws + wl.flags;
+  P.gcol = A->pc[cls].d_gcol;
+  P.poison_ptr = A->pc[cls].d_poison_ptr;
+  P.poison = reinterpret_cast<const int2*>(A->pc[cls].d_poison);
   P.C = C;
   P.ldc = ldc;
   P.counters = reinterpret_cast<int32_t*>(ws + wl.counters + 16);  // after the next-item counter
   P.slabs = reinterpret_cast<float*>(ws + wl.slabs);
   P.N = (int32_t)N;
   P.n_tiles = (int32_t)((N + bn - 1) / bn);
-  P.nbr = A->pc[cls].plan.n_panels * A->pc[cls].plan.R;  // plan rows (slots)
   P.c_f16 = c_dtype == SMAT_F16;
+  P.K = (int32_t)A->host.cols;
   // instruction descriptor (kind::f16): FP32 accumulator, FP16 (0) or BF16 (1)
-  // operands, both K-major, M = 128; the kernel adds N per MMA group
+  // operands, B's tile MN-major and A's blocks K-major, M = 128; the kernel
+  // adds N per MMA group
   const uint32_t fmt = (form == SMAT_FORM_F16 || form == SMAT_FORM_FP8) ? 0u : 1u;
-  P.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(128 >> 4) << 24);
+  P.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 15) | ((uint32_t)(128 >> 4) << 24);
+  P.b_bf16 = (int32_t)fmt;
 }
 
 extern "C" {
@@ -630,9 +676,11 @@ static smat_status check_common(const smat_bcsr* A, int32_t form, int64_t N) {
   return SMAT_OK;
 }
 
-smat_status smat_spmm_pack_b(const smat_bcsr* A, int32_t form, const void* B, int32_t b_dtype,
-                             int32_t b_layout, int64_t ldb, int64_t N, void* workspace,
-                             size_t workspace_bytes, void* stream_) {
+}  // extern "C"
+
+static smat_status pack_impl(const smat_bcsr* A, int32_t form, const void* B, int32_t b_dtype, int32_t b_layout,
+                             int64_t ldb, int64_t N, void* workspace, size_t workspace_bytes, void* stream_,
+                             bool whole) {
   smat_status st = check_common(A, form, N);
   if (st != SMAT_OK) return st;
   if (!B) return fail(SMAT_ERR_INVALID, "null B");
@@ -641,9 +689,8 @@ smat_status smat_spmm_pack_b(const smat_bcsr* A, int32_t form, const void* B, in
     return fail(SMAT_ERR_INVALID, "B must be F32, F16 or BF16");
   const int64_t K = A->host.cols;
   if (b_layout == SMAT_COL_MAJOR ? ldb < K : ldb < N) return fail(SMAT_ERR_INVALID, "ldb too small");
-  size_t need = 0;
-  smat_spmm_workspace_size(A, form, b_dtype, N, &need);
-  if (!workspace || workspace_bytes < need)
+  const WsLayout wl = ws_layout(A, form, N, whole);
+  if (!workspace || workspace_bytes < wl.total)
     return fail(SMAT_ERR_INVALID, "workspace too small (see smat_spmm_workspace_size)");
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return fail(SMAT_ERR_INVALID, "workspace must be 256-byte aligned");
   DeviceGuard guard(A->device);
@@ -653,18 +700,17 @@ smat_status smat_spmm_pack_b(const smat_bcsr* A, int32_t form, const void* B, in
   const int in_dt = b_dtype == SMAT_F32 ? 0 : (b_dtype == SMAT_F16 ? 1 : 2);
   const int mode = (form == SMAT_FORM_F16 || form == SMAT_FORM_FP8) ? 0 : (split ? 2 : 1);
   cudaError_t e = pack_b(B, in_dt, b_layout == SMAT_COL_MAJOR ? 1 : 0, ldb, mode, out, K, N, A->d_kperm,
-                         static_cast<cudaStream_t>(stream_));
+                         out + wl.flags, static_cast<cudaStream_t>(stream_));
   if (e != cudaSuccess) return cuda_fail(e, "pack_b");
   if (uses_sp24(A, form)) {
-    const WsLayout wl = ws_layout(A, form, N);
     e = pack_b_sw64(out, K, N, out + wl.b64, static_cast<cudaStream_t>(stream_));
     if (e != cudaSuccess) return cuda_fail(e, "pack_b_sw64");
   }
   return SMAT_OK;
 }
 
-smat_status smat_spmm_packed(const smat_bcsr* A, int32_t form, const void* packed_b, int64_t N,
-                             void* C, int32_t c_dtype, int64_t ldc, void* stream_) {
+static smat_status packed_impl(const smat_bcsr* A, int32_t form, const void* packed_b, int64_t N, void* C,
+                               int32_t c_dtype, int64_t ldc, void* stream_, bool whole) {
   smat_status st = check_common(A, form, N);
   if (st != SMAT_OK) return st;
   if (!packed_b || !C) return fail(SMAT_ERR_INVALID, "null argument");
@@ -681,10 +727,13 @@ smat_status smat_spmm_packed(const smat_bcsr* A, int32_t form, const void* packe
   const Sched& sc = A->pc[plan_class(form, nsub)].sched[nsub];
   SpmmArgs args;
   std::memset(&args, 0, sizeof(args));
-  const WsLayout wl = ws_layout(A, form, N);
+  const WsLayout wl = ws_layout(A, form, N, whole);
+  whole = whole && sc.n_split > 0;  // else the list has no split panel
   fill_problem(A, form, packed_b, N, C, c_dtype, ldc, nsub, wl, args.one);
-  args.n_items = sc.n_items;
-  args.items = sc.d_items;
+  const int64_t units = (int64_t)(whole ? sc.n_whole : sc.n_items) * args.one.n_tiles;
+  if (units > INT32_MAX / 2) return fail(SMAT_ERR_UNSUPPORTED, "too many work items");
+  args.n_items = (int32_t)units;
+  args.items = whole ? sc.d_whole : sc.d_items;
   args.err = A->d_err;
   args.wait_ns = A->wait_ns;
   args.stall_stage = const_cast<smat_bcsr*>(A)->stall.exchange(0);
@@ -697,7 +746,8 @@ smat_status smat_spmm_packed(const smat_bcsr* A, int32_t form, const void* packe
     cudaError_t e = cudaMemsetAsync(ctr, 0, wl.counter_bytes, static_cast<cudaStream_t>(stream_));
     if (e != cudaSuccess) return cuda_fail(e, "clearing the work counters");
   }
-  cudaError_t e = tc_launch(bh, R, nsub, kind, args, sc.grid, static_cast<cudaStream_t>(stream_));
+  cudaError_t e = tc_launch(bh, R, nsub, kind, args, (int)std::min<int64_t>(sc.workers, std::max<int64_t>(units, 1)),
+                            static_cast<cudaStream_t>(stream_));
   if (e != cudaSuccess) return cuda_fail(e, "spmm kernel launch");
   if (uses_sp24(A, form)) {
     // the exact-2:4 blocks, added into the C the dense kernel wrote
@@ -729,15 +779,34 @@ smat_status smat_spmm_packed(const smat_bcsr* A, int32_t form, const void* packe
   return SMAT_OK;
 }
 
-smat_status smat_spmm(const smat_bcsr* A, int32_t form, const void* B, int32_t b_dtype,
-                      int32_t b_layout, int64_t ldb, void* C, int32_t c_dtype, int64_t ldc,
-                      int64_t N, void* workspace, size_t workspace_bytes, void* stream) {
+smat_status smat::spmm_impl(const smat_bcsr* A, int32_t form, const void* B, int32_t b_dtype, int32_t b_layout,
+                            int64_t ldb, void* C, int32_t c_dtype, int64_t ldc, int64_t N, void* workspace,
+                            size_t workspace_bytes, void* stream, bool whole) {
   if (!A || !B || !C) return fail(SMAT_ERR_INVALID, "null argument");
   if (c_dtype != SMAT_F32 && c_dtype != SMAT_F16) return fail(SMAT_ERR_INVALID, "C must be F32 or F16");
   if (ldc < N) return fail(SMAT_ERR_INVALID, "ldc < N");
-  smat_status st = smat_spmm_pack_b(A, form, B, b_dtype, b_layout, ldb, N, workspace, workspace_bytes, stream);
+  smat_status st = pack_impl(A, form, B, b_dtype, b_layout, ldb, N, workspace, workspace_bytes, stream, whole);
   if (st != SMAT_OK) return st;
-  return smat_spmm_packed(A, form, workspace, N, C, c_dtype, ldc, stream);
+  return packed_impl(A, form, workspace, N, C, c_dtype, ldc, stream, whole);
+}
+
+extern "C" {
+
+smat_status smat_spmm_pack_b(const smat_bcsr* A, int32_t form, const void* B, int32_t b_dtype,
+                             int32_t b_layout, int64_t ldb, int64_t N, void* workspace,
+                             size_t workspace_bytes, void* stream) {
+  return pack_impl(A, form, B, b_dtype, b_layout, ldb, N, workspace, workspace_bytes, stream, false);
+}
+
+smat_status smat_spmm_packed(const smat_bcsr* A, int32_t form, const void* packed_b, int64_t N,
+                             void* C, int32_t c_dtype, int64_t ldc, void* stream) {
+  return packed_impl(A, form, packed_b, N, C, c_dtype, ldc, stream, false);
+}
+
+smat_status smat_spmm(const smat_bcsr* A, int32_t form, const void* B, int32_t b_dtype,
+                      int32_t b_layout, int64_t ldb, void* C, int32_t c_dtype, int64_t ldc,
+                      int64_t N, void* workspace, size_t workspace_bytes, void* stream) {
+  return spmm_impl(A, form, B, b_dtype, b_layout, ldb, C, c_dtype, ldc, N, workspace, workspace_bytes, stream, false);
 }
 
 smat_status smat_spmm_host(const smat_bcsr* A_, int32_t form, const void* B_host, int32_t b_dtype,

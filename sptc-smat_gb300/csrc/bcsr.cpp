@@ -89,6 +89,7 @@ smat_status build_host_bcsr(const smat_csr& A, int32_t bh, int32_t bw, const int
   out.val.assign(nnzb * bsz, 0.0f);
   out.val_f16.assign(nnzb * bsz, 0);
   out.is24.assign(nnzb, 0);
+  out.colmask.assign(nnzb, 0);
 
   // pass 2: sorted block columns, then values in CSR order
 #pragma omp parallel
@@ -140,6 +141,7 @@ smat_status build_host_bcsr(const smat_csr& A, int32_t bh, int32_t bw, const int
           }
           out.val[off] = vf;
           out.val_f16[off] = vh;
+          if (vf != 0.0f) out.colmask[b] |= 1u << (col % bw);
         }
       }
       // exact 2:4 along the block's columns, judged on the FP16 values
@@ -193,6 +195,7 @@ smat_status build_host_bcsr_from_blocks(int64_t rows, int64_t cols, int32_t bh, 
   out.val.resize(nnzb * split * bsz);
   out.val_f16.resize(nnzb * split * bsz);
   out.is24.assign(nnzb * split, 0);
+  out.colmask.assign(nnzb * split, 0);
   int64_t nnz = 0;
 #pragma omp parallel for schedule(static) reduction(+ : nnz)
   for (int64_t k = 0; k < nnzb; k++) {
@@ -209,6 +212,7 @@ smat_status build_host_bcsr_from_blocks(int64_t rows, int64_t cols, int32_t bh, 
           const bool nz = (v & 0x7fff) != 0;
           nnz += nz;
           grp += nz;
+          if (nz) out.colmask[b] |= 1u << c;
           if ((c & 3) == 3) {
             ok = ok && grp <= 2;
             grp = 0;
@@ -305,7 +309,21 @@ smat_status quantize_fp8(const HostBcsr& b, std::vector<uint8_t>& q, std::vector
   return SMAT_OK;
 }
 
-smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, const std::vector<uint8_t>* skip) {
+// Cost of a choice in clock cycles of one SM, from single-instruction
+// measurements on GB300: shared memory takes 64 bytes a cycle from L2 (4 KB
+// tile: 64 cycles), an MMA of one block 39 cycles, 12 for a block that
+// widens its neighbour's MMA, and a 512-byte A block 8. A gathered column
+// costs a 256-byte row of B (4) and a sixteenth of an MMA and an A block (3).
+namespace {
+constexpr int kCostTile = 64, kCostBlock = 47, kCostJoin = 12, kCostCol = 8;
+inline int cols_of(uint32_t mask) { return __builtin_popcount(mask); }
+// Blocks with at most this many nonzero columns cost less gathered than
+// kept even in a tile that is there anyway.
+constexpr int kSparseCols = (kCostBlock - 1) / kCostCol;
+}  // namespace
+
+smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, const std::vector<uint8_t>* skip,
+                       bool gather) {
   if (R < 1 || R > 32) return fail(SMAT_ERR_INVALID, "panel rows must be in [1, 32]");
   const int64_t nbr = b.nbr();
   plan.R = R;
@@ -335,7 +353,25 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
   std::vector<uint32_t> ext_masks;
   const int32_t per_warp = R / kMmaWarps;
   const bool can_cut = R % kMmaWarps == 0;
-  auto wrow = [&b](int64_t br) { return (int64_t)(b.rowptr[br + 1] - b.rowptr[br]); };
+  if (gather && (b.bw != 16 || (int64_t)b.colmask.size() != b.nnzb())) gather = false;
+  // a block row's weight is its number of MMAs: its blocks, or (gather) about
+  // a sixteenth of an MMA per nonzero column of its sparse blocks
+  std::vector<int32_t> row_mmas;
+  if (gather) {
+    row_mmas.resize(nbr);
+#pragma omp parallel for schedule(static)
+    for (int64_t br = 0; br < nbr; br++) {
+      int64_t w = 0;
+      for (int32_t k = b.rowptr[br]; k < b.rowptr[br + 1]; k++) {
+        const int c = cols_of(b.colmask[k]);
+        w += c > kSparseCols ? 16 : c;
+      }
+      row_mmas[br] = (int32_t)((w + 15) / 16);
+    }
+  }
+  auto wrow = [&b, &row_mmas](int64_t br) {
+    return row_mmas.empty() ? (int64_t)(b.rowptr[br + 1] - b.rowptr[br]) : (int64_t)row_mmas[br];
+  };
   auto is_hub = [](int64_t w, int64_t W) { return w >= kMinCutBlocks && kMmaWarps * w > W; };
   int32_t order[32], first_free[kMmaWarps], end_free[kMmaWarps];
   int64_t load[kMmaWarps];
@@ -409,18 +445,29 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
     if (src.br < 0 || ((ext_masks[q / R] >> (q % R)) & 1u)) continue;
     for (int32_t i = 0; i < b.bh; i++) plan.row_map[q * b.bh + i] = b.row_map[(size_t)src.br * b.bh + i];
   }
+  // An entry of a panel: a block (blk >= 0) in its column's tile, or a
+  // gathered block (blk = -(g + 1), g counted over the panel) with a tile of
+  // its own. `key` orders the stream and is equal for blocks of one tile.
+  struct Ent {
+    int64_t key;
+    int32_t slot, blk;
+    bool operator<(const Ent& o) const { return key != o.key ? key < o.key : slot < o.slot; }
+  };
   struct Local {
     std::vector<StageRec> stages;
     std::vector<uint8_t> hdr;
     std::vector<int32_t> blk;
+    std::vector<int64_t> gsrc;                 // gathered blocks: 16 sources each (block * 16 + column, or -1)
+    std::vector<std::vector<Poison>> poison;   // per slot
     PanelInfo info{};
     int64_t groups = 0, tiles = 0;
   };
   std::vector<Local> loc(P);
 #pragma omp parallel
   {
-    std::vector<std::pair<int64_t, int32_t>> ent;  // (col * 32 + slot, block)
+    std::vector<Ent> ent;
     std::vector<std::pair<uint32_t, uint32_t>> mma;  // (owner, entry) of the stage being built
+    std::vector<int64_t> sparse[32];                 // per slot: nonzero columns of its sparse blocks
 #pragma omp for schedule(dynamic, 16)
     for (int32_t p = 0; p < P; p++) {
       Local& L = loc[p];
@@ -430,20 +477,84 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
       for (int32_t sl = 0; sl < R; sl++) {
         if (S[sl].k1 > S[sl].k0) mask |= 1u << sl;
         for (int32_t k = S[sl].k0; k < S[sl].k1; k += S[sl].step)
-          if (!skip || !(*skip)[k]) ent.push_back({(int64_t)b.colidx[k] * 32 + sl, k});
+          if (!skip || !(*skip)[k]) ent.push_back({(int64_t)b.colidx[k] * 64, sl, k});
       }
       L.info.ext_mask = ext_masks[p];
       std::sort(ent.begin(), ent.end());
+      if (gather) {
+        // choose, tile by tile, the blocks whose nonzero columns are cheaper
+        // gathered: first the sparse ones (unless they join a neighbour's MMA),
+        // then the rest of a tile if it does not pay for itself
+        L.poison.resize(R);
+        for (int32_t sl = 0; sl < R; sl++) sparse[sl].clear();
+        size_t out = 0;
+        for (size_t t = 0; t < ent.size();) {
+          size_t e = t;
+          while (e < ent.size() && ent[e].key == ent[t].key) e++;
+          uint32_t kept = 0;  // slots whose block stays
+          for (size_t i = t; i < e; i++)
+            if (cols_of(b.colmask[ent[i].blk]) > kSparseCols) kept |= 1u << ent[i].slot;
+          auto joins = [&](uint32_t set, int32_t sl) {
+            return (sl > 0 && ((set >> (sl - 1)) & 1u) && owner(sl - 1) == owner(sl)) ||
+                   (sl + 1 < R && ((set >> (sl + 1)) & 1u) && owner(sl + 1) == owner(sl));
+          };
+          const uint32_t dense = kept;
+          int64_t keep_cost = kCostTile, gather_cost = 0;
+          for (size_t i = t; i < e; i++) {
+            const int32_t sl = ent[i].slot;
+            const int c = cols_of(b.colmask[ent[i].blk]);
+            if (!((kept >> sl) & 1u)) {
+              if (joins(dense, sl) && c * kCostCol > kCostJoin) kept |= 1u << sl;
+              else continue;
+            }
+            const bool first = sl == 0 || !((kept >> (sl - 1)) & 1u) || owner(sl - 1) != owner(sl);
+            keep_cost += first ? kCostBlock : kCostJoin;
+            gather_cost += c * kCostCol;
+          }
+          if (gather_cost < keep_cost) kept = 0;
+          for (size_t i = t; i < e; i++) {
+            const int32_t sl = ent[i].slot, k = ent[i].blk;
+            if ((kept >> sl) & 1u) {
+              ent[out++] = ent[i];
+              continue;
+            }
+            const uint32_t cm = b.colmask[k];
+            for (int c = 0; c < 16; c++)
+              if ((cm >> c) & 1u) sparse[sl].push_back((int64_t)k * 16 + c);
+            if (cm != 0xffffu) {
+              int32_t head = sl;
+              while (can_cut && ((L.info.ext_mask >> head) & 1u)) head -= per_warp;
+              L.poison[head].push_back(Poison{b.colidx[k] / 16, (int32_t)(~cm & 0xffffu)});
+            }
+          }
+          t = e;
+        }
+        ent.resize(out);
+        // sixteen columns of a slot make one gathered block; it stands in
+        // the stream where its first column would
+        for (int32_t sl = 0; sl < R; sl++)
+          for (size_t i = 0; i < sparse[sl].size(); i += 16) {
+            const int32_t g = (int32_t)(L.gsrc.size() / 16);
+            for (size_t q = i; q < i + 16; q++) L.gsrc.push_back(q < sparse[sl].size() ? sparse[sl][q] : -1);
+            ent.push_back({(int64_t)b.colidx[sparse[sl][i] / 16] * 64 + 1 + sl, sl, -(g + 1)});
+          }
+        std::sort(ent.begin(), ent.end());
+      }
       L.info.nblk = (int32_t)ent.size();
       L.info.slot_mask = mask;
       // accumulate flags in stream order: the first block of a slot overwrites
       std::vector<uint8_t> acc(ent.size(), 0);
       uint32_t touched = 0;
       for (size_t t = 0; t < ent.size(); t++) {
-        const uint32_t slot = (uint32_t)(ent[t].first % 32);
+        const uint32_t slot = (uint32_t)ent[t].slot;
         if ((touched >> slot) & 1u) acc[t] = 1;
         touched |= 1u << slot;
       }
+      // gathered blocks of one slot and column would share a key: tell them
+      // apart by their number
+      auto same_tile = [&](size_t x, size_t y) {
+        return ent[x].key == ent[y].key && ent[x].blk >= 0 && ent[y].blk >= 0;
+      };
       // stages: whole block columns where they fit
       size_t t = 0;
       int32_t ucols = 0;
@@ -451,22 +562,21 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
         StageRec s{};
         mma.clear();
         while (t < ent.size() && s.ntiles < ST && s.nblk < SB) {
-          const int64_t col = ent[t].first / 32;
-          size_t e = t;
-          while (e < ent.size() && ent[e].first / 32 == col) e++;
+          size_t e = t + 1;
+          while (e < ent.size() && same_tile(t, e)) e++;
           const int32_t run = (int32_t)(e - t);
           const int32_t room = SB - s.nblk;
           if (run > room && s.nblk > 0 && run <= SB) break;  // keep the column whole
           const int32_t take = std::min(run, room);
           const int32_t tile = s.ntiles++;
-          s.kb[tile] = (int32_t)(col / 16);
-          if (t == 0 || ent[t - 1].first / 32 != col) ucols++;
+          s.kb[tile] = ent[t].blk >= 0 ? b.colidx[ent[t].blk] / 16 : ent[t].blk;  // gathered: made global below
+          if (t == 0 || !same_tile(t - 1, t)) ucols++;
           // MMA groups among the taken blocks
           for (int32_t g = 0; g < take;) {
-            const uint32_t slot0 = (uint32_t)(ent[t + g].first % 32);
+            const uint32_t slot0 = (uint32_t)ent[t + g].slot;
             int32_t len = 1;
             while (g + len < take && len < max_len) {
-              const uint32_t sl = (uint32_t)(ent[t + g + len].first % 32);
+              const uint32_t sl = (uint32_t)ent[t + g + len].slot;
               if (sl != slot0 + (uint32_t)len) break;
               if (acc[t + g + len] != acc[t + g]) break;
               if (owner(sl) != owner(slot0)) break;
@@ -479,18 +589,25 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
             L.groups++;
             g += len;
           }
-          for (int32_t q = 0; q < take; q++) L.blk.push_back(ent[t + q].second);
-          s.nblk += take;
+          for (int32_t q = 0; q < take; q++) L.blk.push_back(ent[t + q].blk);
+          s.nblk = (int16_t)(s.nblk + take);
           t += take;
         }
         L.tiles += s.ntiles;
+        // gathered tiles take the last tile numbers of the stage
+        int32_t to[kMaxStageTiles], kb[kMaxStageTiles], na = 0;
+        for (int32_t q = 0; q < s.ntiles; q++) na += s.kb[q] >= 0 ? 1 : 0;
+        for (int32_t q = 0, x = 0, y = na; q < s.ntiles; q++) to[q] = s.kb[q] >= 0 ? x++ : y++;
+        for (int32_t q = 0; q < s.ntiles; q++) kb[to[q]] = s.kb[q];
+        std::copy(kb, kb + s.ntiles, s.kb);
+        for (auto& m : mma) m.second = (m.second & ~(15u << 5)) | ((uint32_t)to[(m.second >> 5) & 15u] << 5);
         // header: per-warp (first, count), nblk, then the entries grouped by warp
         std::stable_sort(mma.begin(), mma.end(),
                          [](const std::pair<uint32_t, uint32_t>& x, const std::pair<uint32_t, uint32_t>& y) {
                            return x.first < y.first;
                          });
         const int32_t ne = (int32_t)mma.size();
-        s.hdr_bytes = (kStageHdrFixed + 4 * ne + 15) / 16 * 16;
+        s.hdr_bytes = (int16_t)((kStageHdrFixed + 4 * ne + 15) / 16 * 16);
         const size_t h0 = L.hdr.size();
         L.hdr.resize(h0 + s.hdr_bytes, 0);
         uint8_t* h = L.hdr.data() + h0;
@@ -505,7 +622,31 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
         const uint16_t nb16 = (uint16_t)s.nblk, nt16 = (uint16_t)s.ntiles;
         std::memcpy(h + 8, &nb16, 2);
         std::memcpy(h + 10, &nt16, 2);
+        uint32_t gmask = 0;
+        for (int32_t q = 0; q < s.nblk; q++)
+          if (L.blk[L.blk.size() - s.nblk + q] < 0) gmask |= 1u << q;
+        std::memcpy(h + 12, &gmask, 4);
+        s.ngath = (int16_t)__builtin_popcount(gmask);
         L.stages.push_back(s);
+      }
+      // gathered blocks numbered in stream order, so that a stage's are
+      // consecutive
+      if (!L.gsrc.empty()) {
+        std::vector<int32_t> to(L.gsrc.size() / 16);
+        std::vector<int64_t> src(L.gsrc.size());
+        int32_t next = 0;
+        for (int32_t& k : L.blk) {
+          if (k >= 0) continue;
+          const int32_t old = -(k + 1);
+          to[old] = next;
+          std::copy(L.gsrc.begin() + (int64_t)old * 16, L.gsrc.begin() + (int64_t)old * 16 + 16,
+                    src.begin() + (int64_t)next * 16);
+          k = -(++next);
+        }
+        for (StageRec& st : L.stages)
+          for (int32_t q = 0; q < st.ntiles; q++)
+            if (st.kb[q] < 0) st.kb[q] = -(to[-(st.kb[q] + 1)] + 1);
+        L.gsrc.swap(src);
       }
       L.info.nstages = (int32_t)L.stages.size();
       L.info.nucol = ucols;
@@ -526,21 +667,44 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
   plan.headers.resize(nh);
   plan.n_groups = 0;
   plan.n_tiles = 0;
+  int64_t ng = 0, npois = 0;
+  for (auto& L : loc) {
+    ng += (int64_t)L.gsrc.size();
+    for (auto& v : L.poison) npois += (int64_t)v.size();
+  }
+  if (ng / 16 >= ((int64_t)1 << 31) - 1 || npois >= ((int64_t)1 << 31) - 1)
+    return fail(SMAT_ERR_UNSUPPORTED, "plan too large");
+  plan.gsrc.clear();
+  plan.gsrc.reserve(ng);
+  plan.poison.clear();
+  plan.poison.reserve(npois);
+  plan.poison_ptr.clear();
+  if (gather) plan.poison_ptr.assign(1, 0);
   int64_t so = 0, bo = 0, ho = 0, ao = 0;
   for (int32_t p = 0; p < P; p++) {
     Local& L = loc[p];
     L.info.stage_off = (int32_t)so;
     plan.panels[p] = L.info;
-    std::copy(L.blk.begin(), L.blk.end(), plan.stream_blk.begin() + bo);
+    const int32_t g0 = (int32_t)(plan.gsrc.size() / 16);  // the panel's first gathered block
+    for (size_t q = 0; q < L.blk.size(); q++)
+      plan.stream_blk[bo + (int64_t)q] = L.blk[q] >= 0 ? L.blk[q] : L.blk[q] - g0;
+    plan.gsrc.insert(plan.gsrc.end(), L.gsrc.begin(), L.gsrc.end());
+    for (auto& v : L.poison) {
+      plan.poison.insert(plan.poison.end(), v.begin(), v.end());
+      plan.poison_ptr.push_back((int32_t)plan.poison.size());
+    }
     std::copy(L.hdr.begin(), L.hdr.end(), plan.headers.begin() + ho);
     for (size_t c = 0; c < L.stages.size(); c++) {
       StageRec r = L.stages[c];
       r.blk_off = bo;
       r.hdr_off = ho;
+      r.g0 = r.ngath ? g0 - (r.kb[r.ntiles - r.ngath] + 1) : 0;  // kb still counts from the panel's first
       r.aoff256 = (int32_t)ao;
+      for (int32_t q = 0; q < r.ntiles; q++)
+        if (r.kb[q] < 0) r.kb[q] -= g0;
       bo += r.nblk;
       ho += r.hdr_bytes;
-      ao += (stage_a_bytes(cls, b.bh, r.nblk) + 255) / 256;
+      ao += (stage_a_bytes(cls, b.bh, r.nblk, r.ngath) + 255) / 256;
       plan.stages[so + c] = r;
     }
     so += (int64_t)L.stages.size();
@@ -548,6 +712,12 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
     plan.n_tiles += L.tiles;
   }
   plan.a_bytes = (size_t)ao * 256;
+  plan.gcol.resize(plan.gsrc.size());
+#pragma omp parallel for schedule(static)
+  for (size_t q = 0; q < plan.gsrc.size(); q++) {
+    const int64_t s = plan.gsrc[q];
+    plan.gcol[q] = s < 0 ? -1 : b.colidx[s / 16] + (int32_t)(s % 16);
+  }
   return SMAT_OK;
 }
 
@@ -644,7 +814,7 @@ void build_work_items(const Plan& pl, int32_t bh, int32_t workers, double max_it
 }
 
 std::vector<WorkItem> device_items(const std::vector<const Plan*>& plans, const std::vector<WorkItem>& items,
-                                   const std::vector<int32_t>& order) {
+                                   const std::vector<int32_t>& order, const std::vector<int32_t>* n_tiles) {
   std::vector<WorkItem> out;
   out.reserve(items.size());
   for (int32_t i : order) {
@@ -652,7 +822,7 @@ std::vector<WorkItem> device_items(const std::vector<const Plan*>& plans, const 
     const int32_t off = plans[w.prob]->panels[w.panel].stage_off;
     w.s0 += off;
     w.s1 += off;
-    out.push_back(w);
+    for (w.nt = 0; w.nt < (n_tiles ? (*n_tiles)[w.prob] : 1); w.nt++) out.push_back(w);
   }
   return out;
 }

@@ -2,17 +2,26 @@
 //
 // B arrives as FP32, FP16 or BF16, row-major (k*ld + n) or column-major
 // (k + n*ld, the reference's layout, src/cuda_hgemm/src/mma/mmaOBT.cu:75).
-// The SpMM's B producer moves one 16-row slab of a 128-column tile with a
-// single 4 KB bulk copy, so B is first packed into caller-provided scratch:
-// tile (kb, t) holds rows k = 16*kb .. 16*kb+15 and columns
-// n = 128*t .. 128*t+127 as 128 rows (one per n) of 16 16-bit k-values
-// (32 bytes each), in the 32-byte-swizzled shared-memory layout the MMA reads
-// (inside every 8-row group the two 16-byte halves of rows 4..7 are swapped).
-// Tiles are ordered [t][kb] (column tile, then k-block: tile t*KB + kb);
-// K is zero-padded to 16 and N to 128 (to 256
-// when there is more than one tile, so that 256-column tiles stay in range).
-// The split form writes hi = bf16(b) and lo = bf16(b - hi) as one 8 KB
-// [hi tile | lo tile] pair per tile, so a tile is still one copy.
+// Packed tile (t, kb) holds rows k = 16*kb .. 16*kb+15 and columns
+// n = 128*t .. 128*t+127 as two halves of 64 columns, each 16 rows (one per k)
+// of 64 16-bit values (128 bytes): the MMA reads its 128 x 16 operand with N
+// contiguous (MN-major, 128-byte swizzle: 16-byte chunk c of row k lies at
+// chunk c ^ (k & 7)). Tiles are ordered [t][kb]. So an aligned tile is one
+// 4 KB copy, and a single row of B is two 128-byte pieces that a gathered tile
+// can bring to any row of its own by undoing one swizzle and applying the
+// other. The split form writes hi = bf16(b) and lo = bf16(b - hi), [hi | lo]
+// inside each half.
+//
+// K is zero-padded to 16 and N to 64 columns; a half without a column below N
+// is neither written nor read.
+//
+// A block packs one UNIT: 8 k-blocks of one half. It also says, in the unit's
+// byte of `flags`, whether any packed value is infinite or NaN: the SpMM then
+// restores what a block's stored zeros make of such a value (spmm_tc.cu).
+//
+// What bounds it: DRAM and L2 traffic of a copy. Row-major B needs no
+// transposition in this layout (a thread moves eight neighbouring columns);
+// column-major B goes through shared memory, 128 x 64 values at a time.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -25,6 +34,9 @@ namespace smat {
 namespace dev {
 
 enum : int { OUT_F16 = 0, OUT_BF16 = 1, OUT_SPLIT = 2 };
+constexpr int kPackThreads = 256;
+constexpr int kUnitK = 16 * kPackUnitBlocks;  // rows of B per unit
+constexpr int kStride = 33;                   // words per k of the transposition buffer (64 values and one word)
 
 template <typename T>
 __device__ __forceinline__ float load_f(const T* p);
@@ -41,86 +53,160 @@ __device__ __forceinline__ float load_f<__nv_bfloat16>(const __nv_bfloat16* p) {
   return __bfloat162float(__ldg(p));
 }
 
-__device__ __forceinline__ uint4 pack8(const uint16_t* h) {
-  return make_uint4(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16), h[4] | ((uint32_t)h[5] << 16),
-                    h[6] | ((uint32_t)h[7] << 16));
-}
-
 // Element i of a 16-byte vector of T, as float.
 template <typename T>
-__device__ __forceinline__ float vec_elem(const uint4* v, int i);
+__device__ __forceinline__ float vec_elem(const uint4& v, int i);
 template <>
-__device__ __forceinline__ float vec_elem<float>(const uint4* v, int i) {
-  return __uint_as_float(reinterpret_cast<const uint32_t*>(v)[i]);
+__device__ __forceinline__ float vec_elem<float>(const uint4& v, int i) {
+  return __uint_as_float(reinterpret_cast<const uint32_t*>(&v)[i]);
 }
 template <>
-__device__ __forceinline__ float vec_elem<__half>(const uint4* v, int i) {
-  return __half2float(__ushort_as_half(reinterpret_cast<const uint16_t*>(v)[i]));
+__device__ __forceinline__ float vec_elem<__half>(const uint4& v, int i) {
+  return __half2float(__ushort_as_half(reinterpret_cast<const uint16_t*>(&v)[i]));
 }
 template <>
-__device__ __forceinline__ float vec_elem<__nv_bfloat16>(const uint4* v, int i) {
-  return __bfloat162float(__ushort_as_bfloat16(reinterpret_cast<const uint16_t*>(v)[i]));
+__device__ __forceinline__ float vec_elem<__nv_bfloat16>(const uint4& v, int i) {
+  return __bfloat162float(__ushort_as_bfloat16(reinterpret_cast<const uint16_t*>(&v)[i]));
 }
 
-// One thread per (tile row n, k-block); 128 threads per tile. In the
-// column-major layout the 16 k-values of a thread are contiguous and are
-// read as 16-byte vectors where they are aligned and inside K.
+// The packed hi (and, split form, lo) bits of x.
+template <int OUT>
+__device__ __forceinline__ uint32_t hi_bits(float x) {
+  return OUT == OUT_F16 ? __half_as_ushort(__float2half_rn(x)) : __bfloat16_as_ushort(__float2bfloat16_rn(x));
+}
+__device__ __forceinline__ uint32_t lo_bits(float x, uint32_t hi) {
+  return __bfloat16_as_ushort(__float2bfloat16_rn(x - __bfloat162float(__ushort_as_bfloat16((uint16_t)hi))));
+}
+// Nonzero when either 16-bit half of w is infinite or NaN.
+template <int OUT>
+__device__ __forceinline__ uint32_t nonfinite2(uint32_t w) {
+  constexpr uint32_t E = OUT == OUT_F16 ? 0x7c00u : 0x7f80u;
+  return ((w & E) == E || ((w >> 16) & E) == E) ? 1u : 0u;
+}
+
+// Eight columns n .. n + 7 of row ks (n a multiple of 8) as packed pairs.
 template <typename T, int OUT>
-__device__ __forceinline__ void pack_tile(const T* __restrict__ in, int layout, int64_t ldi, uint8_t* __restrict__ out,
-                                          int64_t K, int64_t N, int ntiles, int64_t kb, int t, int r,
-                                          const int32_t* __restrict__ kperm) {
-  const int64_t n = (int64_t)t * 128 + r;
-  constexpr int VEC = 16 / sizeof(T);  // elements per 16-byte vector
-  float xv[16];
-  const T* colp = in + kb * 16 + n * ldi;
-  if (!kperm && layout == 1 && n < N && kb * 16 + 16 <= K && (reinterpret_cast<uintptr_t>(colp) & 15) == 0) {
-    uint4 v[16 / VEC];
+__device__ __forceinline__ void row_chunk(const T* __restrict__ in, int64_t ldi, int64_t N, int64_t ks, int64_t n,
+                                          bool vec, bool inside, uint32_t hi[4], uint32_t lo[4]) {
+  float x[8];
+  if (inside && vec && n + 8 <= N) {
+    constexpr int V = 16 / sizeof(T);
+    const uint4* p = reinterpret_cast<const uint4*>(in + ks * ldi + n);
+    uint4 v[8 / V];
 #pragma unroll
-    for (int q = 0; q < 16 / VEC; q++) v[q] = __ldg(reinterpret_cast<const uint4*>(colp) + q);
+    for (int q = 0; q < 8 / V; q++) v[q] = __ldg(p + q);
 #pragma unroll
-    for (int i = 0; i < 16; i++) xv[i] = vec_elem<T>(&v[i / VEC], i % VEC);
+    for (int i = 0; i < 8; i++) x[i] = vec_elem<T>(v[i / V], i % V);
   } else {
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-      const int64_t k = kb * 16 + i;
-      const int64_t ks = (k < K && kperm) ? (int64_t)kperm[k] : k;  // row of B feeding permuted column k
-      xv[i] = (k < K && n < N) ? load_f<T>(layout == 1 ? in + ks + n * ldi : in + ks * ldi + n) : 0.0f;
-    }
+    for (int i = 0; i < 8; i++) x[i] = (inside && n + i < N) ? load_f<T>(in + ks * ldi + n + i) : 0.0f;
   }
-  uint16_t h[16], l[16];
 #pragma unroll
-  for (int i = 0; i < 16; i++) {
-    const float x = xv[i];
-    if (OUT == OUT_F16) {
-      h[i] = __half_as_ushort(__float2half_rn(x));
-    } else {
-      const __nv_bfloat16 b = __float2bfloat16_rn(x);
-      h[i] = __bfloat16_as_ushort(b);
-      if (OUT == OUT_SPLIT) l[i] = __bfloat16_as_ushort(__float2bfloat16_rn(x - __bfloat162float(b)));
+  for (int i = 0; i < 4; i++) {
+    const uint32_t a = hi_bits<OUT>(x[2 * i]), b = hi_bits<OUT>(x[2 * i + 1]);
+    hi[i] = a | (b << 16);
+    if (OUT == OUT_SPLIT) lo[i] = lo_bits(x[2 * i], a) | (lo_bits(x[2 * i + 1], b) << 16);
+  }
+}
+
+// One unit: k-blocks 8 * kc .. 8 * kc + 7 of half hx (columns 64 * hx ..).
+// `tr`: kUnitK * kStride words of shared memory per operand (column-major).
+template <typename T, int OUT>
+__device__ __forceinline__ void pack_unit(const T* __restrict__ in, int layout, int64_t ldi, uint8_t* __restrict__ out,
+                                          int64_t K, int64_t N, int64_t kc, int64_t hx,
+                                          const int32_t* __restrict__ kperm, uint8_t* __restrict__ flags,
+                                          uint32_t* tr) {
+  constexpr int NOPS = OUT == OUT_SPLIT ? 2 : 1;
+  const int tid = threadIdx.x;
+  const int64_t kbs = (K + 15) / 16, n0 = hx * 64, k0 = kc * kUnitK;
+  uint8_t* const half = out + ((hx >> 1) * kbs + kc * kPackUnitBlocks) * (4096 * NOPS) + (hx & 1) * (2048 * NOPS);
+  uint32_t bad = 0;
+  if (layout == 0) {
+    // row-major: chunk q of the unit = row q / 8, columns 8 * (q % 8)
+    const bool vec = ((reinterpret_cast<uintptr_t>(in) | (uint64_t)ldi * sizeof(T)) & 15) == 0;
+#pragma unroll
+    for (int it = 0; it < kUnitK * 8 / kPackThreads; it++) {
+      const int q = tid + it * kPackThreads, kr = q >> 3, c = q & 7;
+      const int64_t k = k0 + kr;
+      if ((k >> 4) < kbs) {
+        const bool inside = k < K;
+        const int64_t ks = (inside && kperm) ? (int64_t)kperm[k] : k;  // row of B feeding permuted column k
+        uint32_t hi[4], lo[4];
+        row_chunk<T, OUT>(in, ldi, N, ks, n0 + 8 * c, vec, inside, hi, lo);
+        uint8_t* dst = half + (kr >> 4) * (4096 * NOPS) + (kr & 15) * 128 + ((c ^ (kr & 7)) << 4);
+        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        if (OUT == OUT_SPLIT) *reinterpret_cast<uint4*>(dst + 2048) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) bad |= nonfinite2<OUT>(hi[i]);
+      }
+    }
+  } else {
+    // column-major: a thread reads V consecutive k of columns n and n + 1 and
+    // leaves them as column pairs in tr[k][pair]; then the chunks are written
+    // as above
+    constexpr int V = 16 / sizeof(T), KV = kUnitK / V;
+    const bool vec = !kperm && ((reinterpret_cast<uintptr_t>(in) | (uint64_t)ldi * sizeof(T)) & 15) == 0;
+#pragma unroll 2
+    for (int q = tid; q < KV * 32; q += kPackThreads) {
+      // 8 vectors along k (128 contiguous bytes) x 4 column pairs per warp
+      const int w = q >> 5, l = q & 31;
+      const int kv = (w % (KV / 8)) * 8 + (l & 7), np = (w / (KV / 8)) * 4 + (l >> 3);
+      const int64_t k = k0 + kv * V, n = n0 + 2 * np;
+      float x[2][V];
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const T* p = in + (n + e) * ldi;
+        if (vec && n + e < N && k + V <= K) {
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(p + k));
+#pragma unroll
+          for (int i = 0; i < V; i++) x[e][i] = vec_elem<T>(v, i);
+        } else {
+#pragma unroll
+          for (int i = 0; i < V; i++)
+            x[e][i] = (n + e < N && k + i < K) ? load_f<T>(p + (kperm ? (int64_t)kperm[k + i] : k + i)) : 0.0f;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < V; i++) {
+        const uint32_t a = hi_bits<OUT>(x[0][i]), b = hi_bits<OUT>(x[1][i]);
+        tr[(kv * V + i) * kStride + np] = a | (b << 16);
+        bad |= nonfinite2<OUT>(a | (b << 16));
+        if (OUT == OUT_SPLIT)
+          tr[(kUnitK + kv * V + i) * kStride + np] = lo_bits(x[0][i], a) | (lo_bits(x[1][i], b) << 16);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < kUnitK * 8 / kPackThreads; it++) {
+      const int q = tid + it * kPackThreads, kr = q >> 3, c = q & 7;
+      if (((k0 + kr) >> 4) >= kbs) continue;
+      uint8_t* dst = half + (kr >> 4) * (4096 * NOPS) + (kr & 15) * 128 + ((c ^ (kr & 7)) << 4);
+#pragma unroll
+      for (int o = 0; o < NOPS; o++) {
+        const uint32_t* s = tr + (o * kUnitK + kr) * kStride + 4 * c;
+        *reinterpret_cast<uint4*>(dst + o * 2048) = make_uint4(s[0], s[1], s[2], s[3]);
+      }
     }
   }
-  const int64_t tile = (int64_t)t * ((K + 15) / 16) + kb;  // [column tile][k-block]
-  const int sw = (r >> 2) & 1;
-  constexpr int64_t kTileBytes = OUT == OUT_SPLIT ? 8192 : 4096;
-  uint4* dst = reinterpret_cast<uint4*>(out + tile * kTileBytes + r * 32);
-  dst[sw] = pack8(h);
-  dst[sw ^ 1] = pack8(h + 8);
-  if (OUT == OUT_SPLIT) {
-    uint4* d2 = reinterpret_cast<uint4*>(out + tile * kTileBytes + 4096 + r * 32);
-    d2[sw] = pack8(l);
-    d2[sw ^ 1] = pack8(l + 8);
-  }
+  const int any = __syncthreads_or((int)bad);
+  const int64_t fs = pack_flag_stride(K);
+  if (tid == 0) flags[hx * fs + kc] = any ? 1 : 0;
+  if (kc == pack_units_k(K) - 1 && tid > 0 && kc + tid < fs) flags[hx * fs + kc + tid] = 0;  // the unused bytes
 }
 
 template <typename T, int OUT>
-__global__ void pack_b_tiles(const T* __restrict__ in, int layout, int64_t ldi, uint8_t* __restrict__ out,
-                             int64_t K, int64_t N, int ntiles, const int32_t* __restrict__ kperm) {
-  pack_tile<T, OUT>(in, layout, ldi, out, K, N, ntiles, blockIdx.y, blockIdx.x, threadIdx.x, kperm);
+__global__ void __launch_bounds__(kPackThreads)
+    pack_b_kernel(const T* __restrict__ in, int layout, int64_t ldi, uint8_t* __restrict__ out, int64_t K, int64_t N,
+                  const int32_t* __restrict__ kperm, uint8_t* __restrict__ flags) {
+  extern __shared__ uint32_t tr[];
+  pack_unit<T, OUT>(in, layout, ldi, out, K, N, blockIdx.x, blockIdx.y, kperm, flags, tr);
 }
 
-// Many B operands in one launch: block g packs tile (kb, t) of the job whose
-// block range holds g (jobs sorted by their first block).
-__global__ void pack_b_grouped_kernel(const PackJob* __restrict__ jobs, int njobs, int64_t total) {
+// Many B operands in one launch: block g packs unit g of the list of all
+// jobs' units (jobs sorted by their first unit).
+__global__ void __launch_bounds__(kPackThreads)
+    pack_b_grouped_kernel(const PackJob* __restrict__ jobs, int njobs, int64_t total) {
+  extern __shared__ uint32_t tr[];
   for (int64_t g = blockIdx.x; g < total; g += gridDim.x) {
     int lo = 0, hi = njobs - 1;
     while (lo < hi) {
@@ -128,14 +214,12 @@ __global__ void pack_b_grouped_kernel(const PackJob* __restrict__ jobs, int njob
       if (jobs[mid].begin <= g) lo = mid; else hi = mid - 1;
     }
     const PackJob& j = jobs[lo];
-    const int64_t local = g - j.begin;
-    const int64_t kb = local / j.ntiles;
-    const int t = (int)(local % j.ntiles);
+    const int64_t nkc = pack_units_k(j.K), kc = (g - j.begin) % nkc, hx = (g - j.begin) / nkc;
 #define SMAT_GPACK(T)                                                                                        \
   switch (j.out_mode) {                                                                                      \
-    case OUT_F16: pack_tile<T, OUT_F16>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, j.ntiles, kb, t, threadIdx.x, j.kperm); break; \
-    case OUT_BF16: pack_tile<T, OUT_BF16>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, j.ntiles, kb, t, threadIdx.x, j.kperm); break; \
-    default: pack_tile<T, OUT_SPLIT>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, j.ntiles, kb, t, threadIdx.x, j.kperm); break; \
+    case OUT_F16: pack_unit<T, OUT_F16>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, kc, hx, j.kperm, j.flags, tr); break; \
+    case OUT_BF16: pack_unit<T, OUT_BF16>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, kc, hx, j.kperm, j.flags, tr); break; \
+    default: pack_unit<T, OUT_SPLIT>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, kc, hx, j.kperm, j.flags, tr); break; \
   }
     switch (j.in_dtype) {
       case 0: SMAT_GPACK(float) break;
@@ -146,57 +230,49 @@ __global__ void pack_b_grouped_kernel(const PackJob* __restrict__ jobs, int njob
   }
 }
 
-// Column-major B with 16-byte aligned columns: warp w of a block packs
-// column n = blockIdx.y * 8 + w for 32 consecutive k-blocks (lane = k-block),
-// so a warp reads 32 consecutive 32-byte pieces of one column (1 KB,
-// contiguous) -- the access shape that also suits B in host memory read over
-// the CPU-GPU link -- and each lane writes its 32-byte row of one tile.
-template <typename T, int OUT>
-__global__ void pack_b_colmajor(const T* __restrict__ in, int64_t ldi, uint8_t* __restrict__ out, int64_t K,
-                                int64_t N, int ntiles, int64_t kbs) {
-  const int64_t kb = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
-  const int64_t n = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
-  if (kb >= kbs || n >= (int64_t)ntiles * 128) return;
-  pack_tile<T, OUT>(in, 1, ldi, out, K, N, ntiles, kb, (int)(n >> 7), (int)(n & 127), nullptr);
+// Shared memory of a block: the transposition buffer, column-major only.
+static size_t pack_smem(int layout, bool split) {
+  return layout == 1 ? (size_t)kUnitK * kStride * 4 * (split ? 2 : 1) : 0;
 }
 
 template <typename T, int OUT>
 static cudaError_t run_pack(const void* in, int layout, int64_t ldi, uint8_t* out, int64_t K, int64_t N,
-                            const int32_t* kperm, cudaStream_t s) {
-  const int ntiles = (int)packed_b_tiles(N);
-  const int64_t kbs = (K + 15) / 16;
-  if (kbs == 0 || ntiles == 0) return cudaSuccess;
-  if (!kperm && layout == 1 && ((reinterpret_cast<uintptr_t>(in) | (uint64_t)ldi * sizeof(T)) & 15) == 0) {
-    dim3 grid((unsigned)((kbs + 31) / 32), (unsigned)((int64_t)ntiles * 128 / 8));
-    pack_b_colmajor<T, OUT><<<grid, 256, 0, s>>>((const T*)in, ldi, out, K, N, ntiles, kbs);
-    return cudaGetLastError();
+                            const int32_t* kperm, uint8_t* flags, cudaStream_t s) {
+  const int64_t nkc = pack_units_k(K), halves = pack_halves(N);
+  if (nkc == 0 || halves == 0) return cudaSuccess;
+  // grid.y is limited to 65,535 halves: wider B goes in several launches
+  for (int64_t h0 = 0; h0 < halves; h0 += 65534) {
+    const int64_t hn = halves - h0 < 65534 ? halves - h0 : 65534;
+    const T* src = (const T*)in + (layout == 1 ? h0 * 64 * ldi : h0 * 64);
+    uint8_t* dst = out + (h0 >> 1) * ((K + 15) / 16) * (OUT == OUT_SPLIT ? 8192 : 4096);
+    pack_b_kernel<T, OUT><<<dim3((unsigned)nkc, (unsigned)hn), kPackThreads, pack_smem(layout, OUT == OUT_SPLIT), s>>>(
+        src, layout, ldi, dst, K, N - h0 * 64, kperm, flags + h0 * pack_flag_stride(K));
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
-  dim3 grid((unsigned)ntiles, (unsigned)kbs);
-  pack_b_tiles<T, OUT><<<grid, 128, 0, s>>>((const T*)in, layout, ldi, out, K, N, ntiles, kperm);
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 // The 2:4 path's B operand from the packed tiles: tile (t, w) holds k-blocks
 // 2w and 2w+1 of column tile t side by side, 128 rows (n) of 64 bytes (32
 // k-values) in the 64-byte swizzle (inside every 8-row group, 16-byte chunk
-// c of row n sits at chunk c ^ ((n >> 1) & 3)). One thread per row.
-__global__ void pack_b_sw64_kernel(const uint8_t* __restrict__ p32, uint8_t* __restrict__ out, int64_t kbs,
+// c of row n sits at chunk c ^ ((n >> 1) & 3)). One thread per row n; the
+// lanes of a warp read neighbouring columns of one row k.
+__global__ void pack_b_sw64_kernel(const uint8_t* __restrict__ p, uint8_t* __restrict__ out, int64_t kbs,
                                    int64_t kw) {
   const int64_t w = blockIdx.x;
   const int64_t t = blockIdx.y;
   const int n = threadIdx.x;
   uint4 c[4];
+  uint16_t* const v = reinterpret_cast<uint16_t*>(c);
 #pragma unroll
   for (int hb = 0; hb < 2; ++hb) {
     const int64_t kb = 2 * w + hb;
-    if (kb < kbs) {
-      const uint4* src = reinterpret_cast<const uint4*>(p32 + (t * kbs + kb) * 4096 + n * 32);
-      const int sw = (n >> 2) & 1;
-      c[2 * hb] = src[sw];
-      c[2 * hb + 1] = src[sw ^ 1];
-    } else {
-      c[2 * hb] = c[2 * hb + 1] = make_uint4(0, 0, 0, 0);
-    }
+    const uint8_t* src = p + (t * kbs + kb) * 4096 + (n >> 6) * 2048 + (n & 7) * 2;
+#pragma unroll
+    for (int k = 0; k < 16; ++k)
+      v[hb * 16 + k] = kb < kbs ? *reinterpret_cast<const uint16_t*>(src + k * 128 + ((((n >> 3) & 7) ^ (k & 7)) << 4))
+                                : (uint16_t)0;
   }
   uint4* dst = reinterpret_cast<uint4*>(out + (t * kw + w) * 8192 + n * 64);
   const int sw = (n >> 1) & 3;
@@ -211,11 +287,11 @@ size_t packed_b64_bytes(int64_t K, int64_t N) {
   return (size_t)kw * (size_t)packed_b_tiles(N) * 8192;
 }
 
-cudaError_t pack_b_sw64(const uint8_t* packed32, int64_t K, int64_t N, uint8_t* out, cudaStream_t s) {
+cudaError_t pack_b_sw64(const uint8_t* packed, int64_t K, int64_t N, uint8_t* out, cudaStream_t s) {
   const int64_t kbs = (K + 15) / 16, kw = (kbs + 1) / 2, nt = packed_b_tiles(N);
   if (kw == 0 || nt == 0) return cudaSuccess;
   dim3 grid((unsigned)kw, (unsigned)nt);
-  dev::pack_b_sw64_kernel<<<grid, 128, 0, s>>>(packed32, out, kbs, kw);
+  dev::pack_b_sw64_kernel<<<grid, 128, 0, s>>>(packed, out, kbs, kw);
   return cudaGetLastError();
 }
 
@@ -228,15 +304,17 @@ size_t packed_b_bytes(int64_t K, int64_t N) {
   return (size_t)((K + 15) / 16) * (size_t)packed_b_tiles(N) * 4096;
 }
 
+size_t pack_flag_bytes(int64_t K, int64_t N) { return (size_t)pack_halves(N) * (size_t)pack_flag_stride(K); }
+
 cudaError_t pack_b(const void* in, int in_dtype, int layout, int64_t ldi, int out_mode, uint8_t* out,
-                   int64_t K, int64_t N, const int32_t* kperm, cudaStream_t s) {
+                   int64_t K, int64_t N, const int32_t* kperm, uint8_t* flags, cudaStream_t s) {
   using namespace dev;
-#define SMAT_PACK(T)                                                                  \
-  switch (out_mode) {                                                                 \
-    case OUT_F16: return run_pack<T, OUT_F16>(in, layout, ldi, out, K, N, kperm, s);     \
-    case OUT_BF16: return run_pack<T, OUT_BF16>(in, layout, ldi, out, K, N, kperm, s);   \
-    case OUT_SPLIT: return run_pack<T, OUT_SPLIT>(in, layout, ldi, out, K, N, kperm, s); \
-    default: return cudaErrorInvalidValue;                                            \
+#define SMAT_PACK(T)                                                                             \
+  switch (out_mode) {                                                                            \
+    case OUT_F16: return run_pack<T, OUT_F16>(in, layout, ldi, out, K, N, kperm, flags, s);     \
+    case OUT_BF16: return run_pack<T, OUT_BF16>(in, layout, ldi, out, K, N, kperm, flags, s);   \
+    case OUT_SPLIT: return run_pack<T, OUT_SPLIT>(in, layout, ldi, out, K, N, kperm, flags, s); \
+    default: return cudaErrorInvalidValue;                                                       \
   }
   switch (in_dtype) {
     case 0: SMAT_PACK(float)
@@ -247,15 +325,13 @@ cudaError_t pack_b(const void* in, int in_dtype, int layout, int64_t ldi, int ou
 #undef SMAT_PACK
 }
 
-}  // namespace smat
-
-namespace smat {
-
-cudaError_t pack_b_grouped(const PackJob* d_jobs, int njobs, int64_t total_blocks, int num_sms, cudaStream_t s) {
-  if (njobs == 0 || total_blocks == 0) return cudaSuccess;
-  const int64_t want = (int64_t)num_sms * 16;
-  const int grid = (int)(total_blocks < want ? total_blocks : want);
-  dev::pack_b_grouped_kernel<<<grid, 128, 0, s>>>(d_jobs, njobs, total_blocks);
+cudaError_t pack_b_grouped(const PackJob* d_jobs, int njobs, int64_t total_units, bool any_col, bool any_split,
+                           int num_sms, cudaStream_t s) {
+  if (njobs == 0 || total_units == 0) return cudaSuccess;
+  const int64_t want = (int64_t)num_sms * 8;
+  const int grid = (int)(total_units < want ? total_units : want);
+  dev::pack_b_grouped_kernel<<<grid, dev::kPackThreads, dev::pack_smem(any_col ? 1 : 0, any_split), s>>>(d_jobs, njobs,
+                                                                                                     total_units);
   return cudaGetLastError();
 }
 

@@ -45,6 +45,7 @@ struct smat_group {
   PackJob* d_jobs = nullptr;
   int njobs = 0;
   int64_t pack_blocks = 0;
+  bool pack_col = false, pack_split = false;  // column-major / split-form operands among them
   int* d_err = nullptr;
   std::vector<Launch> launches;
 };
@@ -126,7 +127,7 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
 
   // work lists per variant; per problem its scratch sizes
   struct Scratch {
-    size_t packed = 0, slabs = 0, ws_off = 0, ctr_off = 0, ctr_n = 0;
+    size_t packed = 0, slabs = 0, flags = 0, ws_off = 0, ctr_off = 0, ctr_n = 0;
   };
   std::vector<Scratch> sc(count);
   std::vector<std::vector<WorkItem>> v_items;
@@ -135,8 +136,9 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
     const auto& members = kv.second;
     const int bh = std::get<0>(kv.first), nsub = std::get<2>(kv.first), kind = std::get<3>(kv.first);
     std::vector<const Plan*> plans;
-    std::vector<int32_t> bhs;
+    std::vector<int32_t> bhs, ntl;
     for (int32_t i : members) {
+      ntl.push_back((int32_t)((probs[i].N + 128 * nsub - 1) / (128 * nsub)));
       plans.push_back(&probs[i].A->pc[plan_class_of_kind(kind, nsub)].plan);
       bhs.push_back(probs[i].A->host.bh);
     }
@@ -151,6 +153,7 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
       const size_t one = (packed_b_bytes(p.A->host.cols, p.N) + 255) / 256 * 256;
       s.packed = kind == TC_KIND_SPLIT ? 2 * one : one;
       s.slabs = (size_t)n_slabs[m] * n_tiles * p.A->R * p.A->host.bh * bn * sizeof(float);
+      s.flags = pack_flag_bytes(p.A->host.cols, p.N);
       s.ctr_n = (size_t)n_split[m] * n_tiles * 4;
     }
     Launch l;
@@ -158,10 +161,10 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
     l.R = std::get<1>(kv.first);
     l.nsub = nsub;
     l.kind = kind;
-    l.grid = std::max(1, std::min<int>(workers, (int)items.size()));
-    l.n_items = (int32_t)items.size();
+    v_items.push_back(device_items(plans, items, order, &ntl));
+    l.n_items = (int32_t)v_items.back().size();
+    l.grid = std::max(1, std::min<int>(workers, l.n_items));
     g->launches.push_back(l);
-    v_items.push_back(device_items(plans, items, order));
     v_members.push_back(members);
   }
   // one scratch allocation for all problems, one for all counters: each
@@ -170,7 +173,7 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
   for (size_t v = 0; v < g->launches.size(); v++) g->launches[v].ctr = (int32_t)(4 * v);
   for (Scratch& s : sc) {
     s.ws_off = ws_total;
-    ws_total += (s.packed + s.slabs + 255) / 256 * 256;
+    ws_total += (s.packed + s.slabs + s.flags + 255) / 256 * 256;
     s.ctr_off = ctr_total;
     ctr_total += s.ctr_n;
   }
@@ -195,8 +198,10 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
     j.in_dtype = p.b_dtype == SMAT_F32 ? 0 : (p.b_dtype == SMAT_F16 ? 1 : 2);
     j.layout = p.b_layout == SMAT_COL_MAJOR ? 1 : 0;
     j.out_mode = (p.form == SMAT_FORM_F16 || p.form == SMAT_FORM_FP8) ? 0 : (p.form == SMAT_FORM_SPLIT_BF16 ? 2 : 1);
-    j.ntiles = (int32_t)packed_b_tiles(p.N);
-    blocks += (int64_t)j.ntiles * ((p.A->host.cols + 15) / 16);
+    j.flags = j.out + sc[i].packed + sc[i].slabs;
+    g->pack_col |= j.layout == 1;
+    g->pack_split |= j.out_mode == 2;
+    blocks += pack_halves(j.N) * pack_units_k(j.K);
   }
   g->njobs = count;
   g->pack_blocks = blocks;
@@ -209,6 +214,7 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
       const smat_problem& p = probs[i];
       WsLayout wl;  // offsets are replaced below
       fill_problem(p.A, p.form, g->d_ws + sc[i].ws_off, p.N, p.C, p.c_dtype, p.ldc, l.nsub, wl, descs[m]);
+      descs[m].bflags = g->d_ws + sc[i].ws_off + sc[i].packed + sc[i].slabs;
       descs[m].slabs = reinterpret_cast<float*>(g->d_ws + sc[i].ws_off + sc[i].packed);
       descs[m].counters = g->d_counters + sc[i].ctr_off;
     }
@@ -227,7 +233,7 @@ smat_status smat_group_run(smat_group* g, void* stream_) {
   if (prev != g->device && cudaSetDevice(g->device) != cudaSuccess) return fail(SMAT_ERR_CUDA, "cudaSetDevice failed");
   const cudaStream_t s = static_cast<cudaStream_t>(stream_);
   smat_status st = SMAT_OK;
-  cudaError_t e = pack_b_grouped(g->d_jobs, g->njobs, g->pack_blocks, g->num_sms, s);
+  cudaError_t e = pack_b_grouped(g->d_jobs, g->njobs, g->pack_blocks, g->pack_col, g->pack_split, g->num_sms, s);
   if (e != cudaSuccess) st = fail(SMAT_ERR_CUDA, std::string("grouped B packing: ") + cudaGetErrorString(e));
   if (st == SMAT_OK && g->counter_bytes) {
     e = cudaMemsetAsync(g->d_counters, 0, g->counter_bytes, s);

@@ -89,7 +89,8 @@ smat_status spmm_entry(Entry& e, const half* B, half* C, size_t N, size_t K) {
   size_t need = 0;
   smat_status st = smat_spmm_workspace_size(e.h, SMAT_FORM_F16, SMAT_F16, (int64_t)N, &need);
   if (st != SMAT_OK) return st;
-  if (need <= (size_t)SMAT_SPMM_STATIC_SCRATCH_BYTES)
+  bool whole = false;
+  if (smat::static_scratch_fits(e.h, SMAT_FORM_F16, (int64_t)N, &whole))
     return smat_spmm_static_scratch(e.h, SMAT_FORM_F16, B, SMAT_F16, SMAT_COL_MAJOR, (int64_t)K, C, SMAT_F16,
                                     (int64_t)N, (int64_t)N, nullptr);
   if (need > e.ws_bytes) {

@@ -77,6 +77,7 @@ struct HostBcsr {
   std::vector<uint16_t> val_f16;     // same, as the FP16 the reference stores
   std::vector<int32_t> row_map;      // rows_p: BCSR row -> original row (or -1)
   std::vector<uint8_t> is24;         // per block: exactly 2:4 (values as FP16)
+  std::vector<uint32_t> colmask;     // per block: bit c set where column c holds a nonzero
   std::vector<int32_t> kperm;        // permuted column -> original column (empty: none)
   int64_t nnzb() const { return (int64_t)colidx.size(); }
   int64_t nbr() const { return rows_p / bh; }
@@ -91,6 +92,13 @@ smat_status build_host_bcsr(const smat_csr& A, int32_t bh, int32_t bw, const int
 smat_status build_host_bcsr_from_blocks(int64_t rows, int64_t cols, int32_t bh, int32_t bw, int64_t nnzb,
                                         const int32_t* row_ptr, const int32_t* col_idx, const uint16_t* vals,
                                         HostBcsr& out);
+
+// Columns of a gathered block that hold no nonzero: a stored zero times an
+// infinite or NaN value of B is NaN, so these columns still count for such B.
+struct Poison {
+  int32_t kb;    // k-block
+  int32_t mask;  // bit c: column 16 kb + c
+};
 
 // Work plan of the tensor-core SpMM. Panels of `R` block rows; the blocks of
 // a panel are ordered by block column (then block row) and cut into stages
@@ -110,12 +118,22 @@ struct Plan {
   int64_t n_groups = 0;              // MMA instructions per pass over A
   int64_t n_tiles = 0;               // B tile loads per pass over A
   size_t a_bytes = 0;                // bytes of the A stream
+  // gathered blocks (stream_blk and StageRec::kb: -(g + 1)): sixteen nonzero
+  // columns of one block row, from whichever of its blocks, side by side;
+  // their B tile holds the sixteen rows of B they need
+  std::vector<int64_t> gsrc;         // [16 g + q]: BCSR block * 16 + its column, or -1 (zeros)
+  std::vector<int32_t> gcol;         // [16 g + q]: row of B, or -1
+  // per plan slot (panel * R + slot; the head slot of a cut row): the all-zero
+  // columns of its gathered blocks
+  std::vector<int32_t> poison_ptr;   // [panels * R + 1], empty without gathering
+  std::vector<Poison> poison;
 };
 
 // skip (optional): blocks with skip[k] != 0 are left out of the plan (the
-// exact-2:4 blocks that the structured-sparse path computes).
+// exact-2:4 blocks that the structured-sparse path computes). gather: blocks
+// with few nonzero columns are taken apart and their columns gathered.
 smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan,
-                       const std::vector<uint8_t>* skip = nullptr);
+                       const std::vector<uint8_t>* skip = nullptr, bool gather = false);
 
 // ------------------------------------------------------------------ 2:4 path
 // The structured-sparse path's units, stages and groups (spmm24.h) and the
@@ -157,9 +175,11 @@ void build_work_items(const Plan& pl, int32_t bh, int32_t workers, double max_it
 // ------------------------------------------------------------------ handle
 // Work list of one launch shape (NSUB).
 struct Sched {
-  int grid = 0;
+  int workers = 1;      // CTAs the device holds at once
   int32_t n_items = 0;
   WorkItem* d_items = nullptr;  // by decreasing estimated cost, absolute stage ranges
+  WorkItem* d_whole = nullptr;  // the same without split panels (null when there are none)
+  int32_t n_whole = 0;
   int32_t n_split = 0;  // panels split into parts
   int32_t n_slabs = 0;  // parts of split panels
 };
@@ -171,6 +191,9 @@ struct PlanDev {
   PanelInfo* d_panels = nullptr;
   StageRec* d_stages = nullptr;
   int32_t* d_row_map = nullptr;
+  int32_t* d_gcol = nullptr;        // gathered blocks' rows of B (null: none)
+  int32_t* d_poison_ptr = nullptr;  // null: no gathering
+  Poison* d_poison = nullptr;
   Sched sched[3];  // by NSUB (1, 2)
 };
 
@@ -245,12 +268,23 @@ int pick_nsub(const smat_bcsr* h, int64_t N, int kind);
 // [the 2:4 path's copy of B, when the handle uses it for this form]
 // [the launch's next-item counter, 16 bytes]
 // [per split panel, column tile and TMEM lane quadrant: an int counter]
-// [per part of a split panel and column tile: an R*bh x BN FP32 slab].
+// [per part of a split panel and column tile: an R*bh x BN FP32 slab]
+// [a byte per packing unit of B: it holds infinite or NaN values].
 struct WsLayout {
-  size_t counters = 0, counter_bytes = 0, slabs = 0, total = 0;
+  size_t counters = 0, counter_bytes = 0, slabs = 0, flags = 0, total = 0;
   size_t b64 = 0;  // the 2:4 path's copy of B (0: none)
 };
-WsLayout ws_layout(const smat_bcsr* A, int32_t form, int64_t N);
+WsLayout ws_layout(const smat_bcsr* A, int32_t form, int64_t N, bool whole = false);
+
+// smat_spmm; `whole`: with no panel split over CTAs, so that the workspace
+// needs no partial sums.
+smat_status spmm_impl(const smat_bcsr* A, int32_t form, const void* B, int32_t b_dtype, int32_t b_layout, int64_t ldb,
+                      void* C, int32_t c_dtype, int64_t ldc, int64_t N, void* workspace, size_t workspace_bytes,
+                      void* stream, bool whole);
+
+// Whether a call's scratch fits the static scratch, and with whole panels
+// only (spmm_static.cu).
+bool static_scratch_fits(const smat_bcsr* A, int32_t form, int64_t N, bool* whole);
 
 // The kernel's view of one SpMM: A's device plan and stream for the form,
 // the packed B and scratch at `ws` (laid out as wl), C.
@@ -292,8 +326,9 @@ void tune_store(const TuneKey& key, const TuneVal& val);
 // The device's list: the items in `order`, their stage ranges counted from
 // the plan's first stage (a role then reads one 32-byte item, not an index,
 // an item and the panel's record one after the other).
+// n_tiles (grouped launches): column tiles per problem, each a unit of its own.
 std::vector<WorkItem> device_items(const std::vector<const Plan*>& plans, const std::vector<WorkItem>& items,
-                                   const std::vector<int32_t>& order);
+                                   const std::vector<int32_t>& order, const std::vector<int32_t>* n_tiles = nullptr);
 
 // Item indices by decreasing cost (ties by index).
 void order_items(const std::vector<double>& item_cost, std::vector<int32_t>& order);

@@ -23,10 +23,9 @@
 // and the array can move), so such a call also belongs outside a capture.
 //
 // Every call on a device shares the one array and leaves its contents
-// behind. The packed B is rewritten in full (padding included) by the pack
-// kernel before the contraction reads it; the only part that must start at
-// zero, the split-panel counters, is cleared by smat_spmm_packed on the
-// call's stream before each contraction. Calls that overlap in time — on
+// behind. The packed B is rewritten by the pack kernel wherever the contraction
+// uses it; the only part that must start at zero, the split-panel counters, is
+// cleared on the call's stream before each contraction. Calls that overlap in time — on
 // different streams, or from different threads — race on the array and
 // corrupt each other's results.
 #include <cuda.h>
@@ -42,7 +41,10 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 
-static __device__ __align__(256) uint8_t g_spmm_scratch[SMAT_SPMM_STATIC_SCRATCH_BYTES];
+// The limit counts the packed B and the partial sums; a byte per packing unit
+// (at most one per 128 bytes of packed B) comes on top.
+constexpr size_t kFlagRoom = SMAT_SPMM_STATIC_SCRATCH_BYTES / 128 + 4096;
+static __device__ __align__(256) uint8_t g_spmm_scratch[SMAT_SPMM_STATIC_SCRATCH_BYTES + kFlagRoom];
 
 std::mutex g_scratch_mu;
 void* g_scratch_addr[kMaxDevices] = {};
@@ -85,6 +87,16 @@ smat_status scratch_on(int dev, void** out) {
 
 }  // namespace
 
+bool smat::static_scratch_fits(const smat_bcsr* A, int32_t form, int64_t N, bool* whole) {
+  // split panels where their partial sums fit, else whole panels
+  for (int w = 0; w < 2; w++) {
+    const WsLayout wl = ws_layout(A, form, N, w != 0);
+    *whole = w != 0;
+    if (wl.flags <= (size_t)SMAT_SPMM_STATIC_SCRATCH_BYTES && wl.total - wl.flags <= kFlagRoom) return true;
+  }
+  return false;
+}
+
 smat_status smat_spmm_static_scratch(const smat_bcsr* A, int32_t form, const void* B, int32_t b_dtype,
                                      int32_t b_layout, int64_t ldb, void* C, int32_t c_dtype, int64_t ldc,
                                      int64_t N, void* stream) {
@@ -92,7 +104,8 @@ smat_status smat_spmm_static_scratch(const smat_bcsr* A, int32_t form, const voi
   size_t need = 0;
   smat_status st = smat_spmm_workspace_size(A, form, b_dtype, N, &need);
   if (st != SMAT_OK) return st;
-  if (need > (size_t)SMAT_SPMM_STATIC_SCRATCH_BYTES)
+  bool whole = false;
+  if (!smat::static_scratch_fits(A, form, N, &whole))
     return smat::fail(SMAT_ERR_UNSUPPORTED,
                       "packed B needs " + std::to_string(need) + " bytes but the static scratch holds " +
                           std::to_string((size_t)SMAT_SPMM_STATIC_SCRATCH_BYTES) +
@@ -100,6 +113,6 @@ smat_status smat_spmm_static_scratch(const smat_bcsr* A, int32_t form, const voi
   void* scratch = nullptr;
   st = scratch_on(smat::bcsr_device(A), &scratch);
   if (st != SMAT_OK) return st;
-  return smat_spmm(A, form, B, b_dtype, b_layout, ldb, C, c_dtype, ldc, N, scratch,
-                   (size_t)SMAT_SPMM_STATIC_SCRATCH_BYTES, stream);
+  return smat::spmm_impl(A, form, B, b_dtype, b_layout, ldb, C, c_dtype, ldc, N, scratch,
+                         (size_t)SMAT_SPMM_STATIC_SCRATCH_BYTES + kFlagRoom, stream, whole);
 }

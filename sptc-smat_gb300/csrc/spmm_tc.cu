@@ -13,38 +13,43 @@
 //
 // Blocks of a panel are visited in order of their block column, so that the
 // B tile of a column is loaded once and used by every block row of the panel
-// that has a block there. The A blocks are stored on the device in exactly
-// that visiting order, already in the shared-memory layout the MMA reads
-// (32-byte swizzle). The pipeline moves STAGES: one stage carries up to 16
-// A blocks (8 of 32 rows), up to 8 packed B tiles those blocks need and the
-// stage's MMA list (precomputed on the host, stored after the stage's A
-// blocks so that one copy brings both), so the hand-off between the copy
-// engine and the tensor cores is one full/empty barrier pair per stage.
+// that has a block there. Blocks with few nonzero columns are taken apart
+// (bcsr.cpp: build_plan): sixteen nonzero columns of a block row, from
+// whichever of its blocks, make one GATHERED block, whose B tile holds the
+// sixteen rows of B they need. The A blocks are stored on the device in
+// exactly the visiting order, already in the shared-memory layout the MMA
+// reads (32-byte swizzle). The pipeline moves STAGES: one stage carries a
+// number of A blocks, the packed B tiles they need and the stage's MMA list
+// (precomputed on the host, stored before the blocks so that one copy brings
+// both), so the hand-off between the copies and the tensor cores is one
+// full/empty barrier pair per stage.
 //
-// Roles (512 threads):
-//   warps 8..15     copy warps: a stage needs one bulk copy for its list and
-//                   A blocks and one per B tile; the copies rotate over the
-//                   eight warps, each of which waits for the stage's slot
-//                   and counts itself on the stage's full barrier.
+// Roles (640 threads):
+//   warps 12..19    copy warps, in pairs that own whole stages: bulk copies for
+//                   the list, the A blocks and the B tiles, 16-byte copies
+//                   through the load path for the rows of gathered tiles.
 //   warps 0..3      MMA issuers, one elected lane each, one per quarter of the
 //                   panel's block rows (one thread issues at most one
 //                   tcgen05.mma per 64-75 cycles, the tensor pipe takes one of
 //                   this width every 39); warp 0 also owns TMEM.
-//   warps 4..7      epilogue: tcgen05.ld -> row scatter through row_map ->
-//                   FP32 or FP16 stores of C (coalesced along N).
+//   warps 4..11     epilogue, a set of four per accumulator buffer: tcgen05.ld
+//                   -> row scatter through row_map -> FP32 or FP16 stores of C
+//                   (coalesced along N).
 //
 // Consecutive block rows with a block at the same column form one MMA
 // (N = bh * run length), so dense panels need far fewer instructions.
 //
-// What bounds it: latency of the control code first (a stage's waits, list
-// reads and MMA issues; measured with single-instruction benchmarks, see
-// tc_ptx.cuh), then shared memory: the copies write it and the MMAs read their
-// 128 x 16 operand from it, about 125 us on the R-MAT workload (2^16 rows,
-// 680K blocks, N = 128). Waits whose loop branches on the barrier's own
-// predicate, MMA and copy issue by an elected lane, copy warps that need no
-// barrier among themselves, and work items read whole from the item ring took
-// the step from 256 to 216 us there (plain graph, 2^15 rows, N = 256: 231 to
-// 196 us).
+// What bounds it (GB300; time of the whole step with the packing of B):
+//   R-MAT, 2^16 rows, 816K blocks, N = 128: 256 us at first; 216 with waits
+//     that branch on the barrier's own predicate, elected issue and no barrier
+//     among the copy warps; 148 with gathered blocks (600K -> 266K MMAs, 1.85
+//     -> 1.0 GB into shared memory); 115 with the drain as a loop, (item,
+//     column tile) units and the roles above. Now the turn of a stage slot
+//     (copy issue, landing, MMAs) sets the pace: 47 bytes a cycle into an SM of
+//     the 70 it can take, tensor pipe busy 30 %.
+//   64^3 stencil, N = 256: 358 -> 187 us, 63 of them packing the FP32 B at 6.4
+//     TB/s; the kernel moves 450 MB of DRAM data in 125.
+//   plain graph, 2^15 rows, 600K entries, N = 256: 231 -> 76 us.
 //
 // Every wait is bounded (see tc_ptx.cuh); on a timeout the kernel raises the
 // CTA's abort flag, records the site in the global error word, lets the
@@ -58,6 +63,7 @@
 #include <atomic>
 #include <cstdint>
 
+#include "convert.h"
 #include "spmm_tc.h"
 #include "tc_ptx.cuh"
 
@@ -86,7 +92,7 @@ enum : int {
 
 // Entries of the CTA's ring of work items (the copy warps take items from
 // the launch's counter and run up to a few items ahead of the other roles).
-constexpr int kItemRing = 4;
+constexpr int kItemRing = 8;
 
 template <int BH, int R, int NSUB, int KIND>
 struct Cfg {
@@ -97,29 +103,34 @@ struct Cfg {
   static constexpr int SB = stage_rows(CLS) / BH;         // A blocks per stage (at most)
   static constexpr int ST = stage_tiles(CLS);             // B tiles per stage (at most)
   static constexpr uint32_t ABLK = BH * 32;               // bytes of one A block (one operand)
-  static constexpr uint32_t TILE = BN * 32;               // bytes of one B tile (one operand)
-  static constexpr uint32_t TILEB = TILE * NOPS;          // bytes of one B tile slot
+  static constexpr uint32_t HALF = 2048 * NOPS;           // bytes of 64 columns of a B tile (hi, then lo)
+  static constexpr uint32_t SUB = 2 * HALF;               // bytes of a 128-column subtile
+  static constexpr uint32_t TILEB = SUB * NSUB;           // bytes of one B tile slot
   static constexpr bool FP8 = KIND == KIND_FP8;
   // stage: [header] [A blocks hi | lo] [B tiles]; the header and the blocks
   // land with one copy. The FP8 form lands [header | e4m3 blocks | scales],
   // which the converter warps turn into the FP16 A blocks after it.
   static constexpr uint32_t HDR = kStageHdrBytes;
-  static constexpr uint32_t OFF_A = FP8 ? (HDR + SB * 256 + fp8_scale_bytes(SB) + 255) / 256 * 256 : HDR;
+  static constexpr uint32_t OFF_A = FP8 ? (HDR + SB * 256 + fp8_scale_bytes(SB) + 64 * ST + 255) / 256 * 256 : HDR;
   static constexpr uint32_t OFF_B = (OFF_A + SB * ABLK * NOPS + 1023) / 1024 * 1024;
   static constexpr uint32_t STAGE = (OFF_B + ST * TILEB + 1023) / 1024 * 1024;
-  static constexpr uint32_t SMEM_AVAIL = 227 * 1024 - 2048;  // minus alignment slack and barriers
+  static constexpr uint32_t SMEM_AVAIL = 227 * 1024 - 14336;  // minus alignment slack, barriers and row tables
   static constexpr int NS_FIT = (int)(SMEM_AVAIL / STAGE);
   static constexpr int NS = NS_FIT < 2 ? 2 : (NS_FIT > 8 ? 8 : NS_FIT);  // stages
   static constexpr uint32_t SUB_COLS = R * BH;            // TMEM columns of one 128-column subtile
   static constexpr uint32_t ACC_COLS = NSUB * SUB_COLS;   // TMEM columns per buffer
   static constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
   static constexpr int NMMA = kMmaWarps;                  // MMA-issuing warps
-  static constexpr int NPROD = 8;                         // copy warps
+  static constexpr int NEPI = 8;                          // epilogue warps: a set of four per accumulator buffer
+  static constexpr int NPROD = FP8 ? 4 : 8;               // copy warps, in pairs
   static constexpr int NCONV = FP8 ? 4 : 0;               // FP8 converter warps (16..19)
   static constexpr uint32_t SMEM_BARS = 8 * (2 * NS + 4 + NMMA + (FP8 ? 2 * NS : 0) + 2 * kItemRing + 1);
-  // then the TMEM address, the abort flag and the ring of work items
-  static constexpr uint32_t SMEM_BYTES = 1024 + NS * STAGE + SMEM_BARS + 24 + kItemRing * sizeof(WorkItem);
-  static constexpr int THREADS = 32 * (8 + NPROD + NCONV);  // MMA, epilogue, copy, converter warps
+  static constexpr int GLIST = (ST + 1) / 2 * 16 * 4;     // bytes of a copy warp's rows of gathered tiles
+  // then the TMEM address, the abort flag, the ring of work items, the
+  // epilogue warps' row tables and the copy warps' gather lists
+  static constexpr uint32_t SMEM_BYTES = 1024 + NS * STAGE + SMEM_BARS + 24 + kItemRing * sizeof(WorkItem) +
+                                         NEPI * R * BH * 4 + NPROD * GLIST;
+  static constexpr int THREADS = 32 * (4 + NEPI + NPROD + NCONV);  // MMA, epilogue, copy, converter warps
   static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0,
                 "TMEM allocation must be a power of two in [32, 512]");
   static_assert(BH == 16 || BH == 32, "block height");
@@ -129,8 +140,8 @@ struct Cfg {
   static_assert(stage_hdr_max(SB) <= (int)HDR, "stage header");
   // a stage tile of NSUB 128-column subtiles is NSUB copies (packed B is
   // [128-column tile][k-block]: the subtiles are not adjacent)
-  static_assert(ST * NSUB + 1 <= 2 * NPROD && ST <= kMaxStageTiles,
-                "1 + ST * NSUB copies per stage, at most two per copy warp");
+  static_assert(ST * NSUB <= 32 && ST <= 16 && ST <= kMaxStageTiles, "a lane per copy, four per gathered tile");
+  static_assert((ST + 1) / 2 * NSUB < 32, "lane 31 is free for the A region");
   static_assert(NS_FIT >= 2, "two stages must fit");
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
   static_assert(!FP8 || (BH == 16 && NSUB == 1), "FP8 form: 16 x 16 blocks, 128-column tiles");
@@ -190,6 +201,28 @@ __device__ __forceinline__ bool take_item_warp(uint64_t* itemfull, uint64_t* ite
   return true;
 }
 
+// Infinite and NaN values of B. A block's stored zeros count: zero times such
+// a value is NaN in every row of the block. The columns that gathering left
+// out (all zero in the block) are looked up here, for a launch whose packed B
+// says that it holds such values: whether column n of C is NaN in the rows of
+// the plan slot whose all-zero columns are poison[q0 .. q1).
+__device__ __noinline__ bool poisoned(const ProblemDesc& P, int nops, int q0, int q1, int64_t n) {
+  const uint32_t E = P.b_bf16 ? 0x7f80u : 0x7c00u;
+  const uint8_t* base =
+      P.bpack + (n >> 7) * P.bp_kbs * (4096 * nops) + ((n >> 6) & 1) * (2048 * nops) + (n & 7) * 2;
+  const uint32_t c = (uint32_t)(n >> 3) & 7u;
+  for (int q = q0; q < q1; ++q) {
+    const int2 e = P.poison[q];
+    for (uint32_t m = (uint32_t)e.y; m != 0; m &= m - 1) {
+      const uint32_t k = (uint32_t)__ffs((int)m) - 1;
+      const uint32_t v = *reinterpret_cast<const uint16_t*>(base + (int64_t)e.x * (4096 * nops) + k * 128 +
+                                                            ((c ^ (k & 7)) << 4));
+      if ((v & E) == E) return true;
+    }
+  }
+  return false;
+}
+
 // Bounded wait for a whole warp: lane 0 polls, the warp learns the outcome
 // by shuffle and leaves converged (lanes that each polled would leave the
 // loop on different iterations and could run the code after it diverged).
@@ -205,6 +238,114 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int lan
 }
 
 __device__ __forceinline__ int shfl_i(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+
+// Stores a column of 16 rows of C: v[m] to row rows[m] (in shared memory, the
+// same for every lane; -1: none) of rows `ldb` bytes apart, base = the
+// column's first element. `full`: no row is missing, and nothing is tested per
+// row.
+template <typename T>
+__device__ __forceinline__ T c_value(float v);
+template <>
+__device__ __forceinline__ float c_value<float>(float v) {
+  return v;
+}
+template <>
+__device__ __forceinline__ __half c_value<__half>(float v) {
+  return __float2half_rn(v);
+}
+template <typename T>
+__device__ __forceinline__ void store_rows16(uint8_t* base, int64_t ldb, const int* rows, bool full, const float* v) {
+  if (full) {
+#pragma unroll
+    for (int m = 0; m < 16; m += 4) {
+      const int4 r = *reinterpret_cast<const int4*>(rows + m);
+      __stcs(reinterpret_cast<T*>(base + r.x * ldb), c_value<T>(v[m]));
+      __stcs(reinterpret_cast<T*>(base + r.y * ldb), c_value<T>(v[m + 1]));
+      __stcs(reinterpret_cast<T*>(base + r.z * ldb), c_value<T>(v[m + 2]));
+      __stcs(reinterpret_cast<T*>(base + r.w * ldb), c_value<T>(v[m + 3]));
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < 16; ++m)
+      if (rows[m] >= 0) __stcs(reinterpret_cast<T*>(base + rows[m] * ldb), c_value<T>(v[m]));
+  }
+}
+
+// Units with at most this many stages: the CTA's next unit is taken when the
+// copies of one begin.
+constexpr int kShortUnit = 24;
+
+// Unit `k` of the CTA into the item ring (one thread): the launch's unit
+// blockIdx.x first, then the next one nobody has taken; panel -1 at the end.
+__device__ __forceinline__ void put_unit(const SpmmArgs& args, uint32_t k, uint64_t* itemfull, uint64_t* itemempty,
+                                         WorkItem* ring, volatile int* abort, int* err, uint64_t lim) {
+  const uint32_t r = k % kItemRing;
+  if (!wait_phase(smem_u32(&itemempty[r]), ((k / kItemRing) & 1) ^ 1, abort, err, ERR_ITEM_TAKE, lim)) return;
+  const int pos = k == 0 ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(args.next_item, 1);
+  WorkItem nw;
+  nw.panel = -1;
+  if (pos < args.n_items) {
+    if (args.probs) {
+      nw = args.items[pos];
+    } else {  // one problem: every item once per column tile
+      const uint32_t it = (uint32_t)pos / (uint32_t)args.one.n_tiles;
+      nw = args.items[it];
+      nw.nt = pos - (int)(it * (uint32_t)args.one.n_tiles);
+    }
+  }
+  ring[r] = nw;
+  mbar_arrive(smem_u32(&itemfull[r]));
+}
+
+// A stage record as its copy warp holds it: the counts in every lane, its bulk
+// tile's k-block in each lane, and (after load_rows) a 16-byte piece of the
+// rows of B of the warp's gathered tiles (every other one, from hf).
+struct StageView {
+  int nblk, ngath, ntiles, aoff, kb, g0;
+  int4 rows0;
+};
+__device__ __forceinline__ void load_stage(StageView& v, const StageRec* recs, int i, int n, int tile) {
+  v.nblk = v.ngath = v.ntiles = v.aoff = v.kb = v.g0 = 0;
+  if (i >= 0 && i < n) {
+    const StageRec* rp = recs + i;
+    const int4 r1 = __ldg(reinterpret_cast<const int4*>(rp) + 1);  // nblk | ntiles, hdr_bytes | ngath, g0, aoff256
+    v.nblk = r1.x & 0xffff;
+    v.ntiles = r1.x >> 16;
+    v.ngath = r1.y >> 16;
+    v.g0 = r1.z;
+    v.aoff = r1.w;
+    v.kb = __ldg(rp->kb + min(tile, kMaxStageTiles - 1));
+  }
+}
+__device__ __forceinline__ void load_rows(StageView& v, const int32_t* gcol, int hf, int lane) {
+  const int t = (lane >> 2) * 2 + hf;  // four pieces per tile
+  if (t < v.ngath) v.rows0 = __ldg(reinterpret_cast<const int4*>(gcol + ((int64_t)v.g0 + t) * 16) + (lane & 3));
+}
+
+// A gathered tile: row r of the tile from row k = list[r] of B (zeros for -1).
+// A lane moves 16-byte chunks: 8 lanes bring the 128 bytes of 64 columns of a
+// row, undoing the swizzle of row k & 7 in the packed B and applying that of
+// row r & 7.
+template <int NOPS>
+__device__ __forceinline__ void gather_tile(uint32_t dst, const uint8_t* b, const int* list, int nh, int lane) {
+  const int c = lane & 7;
+#pragma unroll
+  for (int rr = 0; rr < 4; ++rr) {
+    const int r = rr * 4 + (lane >> 3);
+    const int k = list[r];
+    const int kk = k < 0 ? 0 : k;
+    const uint8_t* src = b + (int64_t)(kk >> 4) * (4096 * NOPS) + (kk & 15) * 128 + ((c ^ (kk & 7)) << 4);
+    const uint32_t d = dst + r * 128 + ((c ^ (r & 7)) << 4);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h < nh) {
+#pragma unroll
+        for (int o = 0; o < NOPS; ++o)
+          cp_async16(d + h * (2048 * NOPS) + o * 2048, src + h * (2048 * NOPS) + o * 2048, k < 0 ? 0u : 16u);
+      }
+    }
+  }
+}
 
 // Warp roles: 0..3 MMA issuers (0 also owns TMEM), 4..7 epilogue (TMEM lane
 // quadrants 0..3), then NPROD copy warps, then (FP8) the converter warps.
@@ -233,6 +374,8 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
   // [kItemRing] work items (panel -1: no more work), 16-byte aligned
   WorkItem* item_ring = reinterpret_cast<WorkItem*>((reinterpret_cast<uintptr_t>(tmem_slot + 2) + 15) &
                                                     ~static_cast<uintptr_t>(15));
+  int* row_tab = reinterpret_cast<int*>(item_ring + kItemRing);  // [NEPI][R * BH] C rows, a table per epilogue warp
+  int* glists = row_tab + C::NEPI * R * BH;                      // [NPROD][GLIST / 4] rows of B of gathered tiles
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // uniform for the compiler
   const int lane = threadIdx.x & 31;
@@ -243,7 +386,9 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::NS; i++) {
-      mbar_init(smem_u32(&full[i]), C::NPROD);  // every copy warp's arrive (+ its copies' bytes)
+      // the stage's two copy warps: 32 arrivals each (+ their bulk copies'
+      // bytes), for a lane's gathered rows count when they land
+      mbar_init(smem_u32(&full[i]), 64);
       mbar_init(smem_u32(&empty[i]), C::NMMA);
     }
     for (int i = 0; i < 2; i++) {
@@ -276,14 +421,14 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
   int* err = args.err;
   const uint32_t smem0 = smem_u32(smem);
 
-  if (C::FP8 && warp >= 8 + C::NPROD) {
+  if (C::FP8 && warp >= 4 + C::NEPI + C::NPROD) {
     // ------------------------------------------------------ FP8 converters
     // Each stage's e4m3 blocks and FP32 scales land in the staging area;
     // these four warps write them to the stage's A area as FP16 (value times
     // its block's scale, one rounding) in the 32-byte-swizzled layout the
     // MMA reads, make the writes visible to the tensor core's async proxy,
     // and release the stage to the MMA warps (conv barrier).
-    const int ct = threadIdx.x - 32 * (8 + C::NPROD);
+    const int ct = threadIdx.x - 32 * (4 + C::NEPI + C::NPROD);
     uint32_t ci = 0;
     bool ok = true;
     for (uint32_t kk = 0; ok; ++kk) {
@@ -293,9 +438,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
         break;
       }
       if (wi.panel < 0) break;
-      const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
-      const int n_tiles = P.n_tiles;
-      for (int nt = 0; nt < n_tiles && ok; ++nt) {
+      {
         for (int c = wi.s0; c < wi.s1; ++c, ++ci) {
           const uint32_t s = ci % nsr;
           if (!warp_wait(smem_u32(&afull[s]), (ci / nsr) & 1, lane, abort_flag, err, ERR_CONV, false, lim)) {
@@ -306,6 +449,9 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
           const int nblk = *reinterpret_cast<const uint16_t*>(stp + 8);
           const uint8_t* stg = stp + C::HDR;
           const float* scl = reinterpret_cast<const float*>(stg + nblk * 256);
+          // gathered blocks: a scale per column, after the blocks' scales
+          const uint32_t gmask = *reinterpret_cast<const uint32_t*>(stp + 12);
+          const float4* gscl = reinterpret_cast<const float4*>(stg + nblk * 256 + fp8_scale_bytes(nblk));
           // a thread widens whole 16-value rows; its rows are loaded first, so
           // that the loads overlap (FP8 stencil 192 against 209 us with one
           // 8-value piece loaded, widened and stored at a time)
@@ -325,13 +471,18 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
             const int b = (ct >> 4) + 8 * q, r = ct & 15;
             if (b >= nblk) break;
             const uint32_t in[4] = {raw[q].x, raw[q].y, raw[q].z, raw[q].w};
+            const bool gat = (gmask >> b) & 1u;
+            const float4* gs = gscl + 4 * __popc(gmask & ((1u << b) - 1));
             uint32_t w[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const uint16_t pair = (uint16_t)((in[i >> 1] >> (16 * (i & 1))) & 0xffffu);
-              const float2 f = __half22float2(e4m3x2_to_half2(pair));
-              const __half2 o = __floats2half2_rn(f.x * sc[q], f.y * sc[q]);
-              w[i] = *reinterpret_cast<const uint32_t*>(&o);
+            for (int i = 0; i < 4; ++i) {
+              const float4 s4 = gat ? gs[i] : make_float4(sc[q], sc[q], sc[q], sc[q]);
+              const float2 f0 = __half22float2(e4m3x2_to_half2((uint16_t)(in[i] & 0xffffu)));
+              const float2 f1 = __half22float2(e4m3x2_to_half2((uint16_t)(in[i] >> 16)));
+              const __half2 o0 = __floats2half2_rn(f0.x * s4.x, f0.y * s4.y);
+              const __half2 o1 = __floats2half2_rn(f1.x * s4.z, f1.y * s4.w);
+              w[2 * i] = *reinterpret_cast<const uint32_t*>(&o0);
+              w[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&o1);
             }
             uint4* dst = reinterpret_cast<uint4*>(stp + C::OFF_A + b * 512 + r * 32);
             const int sw = (r >> 2) & 1;
@@ -344,130 +495,148 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
         }
       }
     }
-  } else if (warp >= 8) {
+  } else if (warp >= 4 + C::NEPI) {
     // ---------------------------------------------------------------- copies
-    // Stage number c (counted over the CTA's whole run) needs a copy of its
-    // A region (header and blocks) and one per 128-column subtile of its B
-    // tiles. B copy j goes to copy warp (j + c) mod NPROD, so every warp has
-    // at most two per stage, and the A region (from HBM, the slowest) to the
-    // warp for j = NPROD - 1. Every warp waits for the stage's slot itself and
-    // arrives on its full barrier once per stage, adding the bytes it brings:
-    // no warp can run a ring ahead, and none waits for another (a named
-    // barrier among the eight and their leader's wait took about 550 of a
-    // stage's 1,650 cycles). Stage records are read 32 at a time, one per
-    // lane, and each lane prepares what its warp needs from its record.
-    const int pw = warp - 8;
+    // Stage number c (counted over the CTA's whole run) belongs to pair c mod
+    // np of copy warps, which bring all of it: a bulk copy for the A region
+    // (header and blocks) and one per 128-column subtile of the B tiles, issued
+    // by the lanes side by side (about 55 cycles each; two warps reach the SM's
+    // 74-78 bytes a cycle), and the rows of the gathered tiles with 16-byte
+    // copies through the load path. The warps of a pair take every other tile;
+    // as many pairs are at work as stages are in flight. (Eight warps that each
+    // brought two of every stage's tiles spent 940 cycles a stage on waits,
+    // shuffles and arrivals.) A stage's record is read two of the pair's stages
+    // ahead, its rows of B one.
+    //
+    // np must not exceed the stages in flight: the wait for a slot tells its
+    // phase by parity, so a warp may not come to it before the use before last
+    // has been consumed, and its own last stage, c - np, shows only that stage
+    // c - np - nsr has.
+    const int pw = warp - 4 - C::NEPI;
     const uint64_t pol_a = make_l2_policy_evict_first();  // A streams through L2 once
     const uint64_t pol_b = make_l2_policy_evict_last();   // B tiles are re-read by many CTAs
-    uint32_t ci = 0, slot_s = 0, phase_s = 1;
-    bool ok = true;
-    uint32_t last_mine = 0xffffffffu;  // last stage this warp copied into (for the drain)
+    const int hf = pw & 1;
+    int* const glist = glists + pw * (C::GLIST / 4);
+    uint32_t ci = 0;           // the item's first stage
+    const uint32_t pair = (uint32_t)pw >> 1, np = min((uint32_t)C::NPROD / 2, nsr);
+    const bool active = pair < np;  // the others only pass the units on
+    uint32_t my_c = pair, slot_s = pair, phase_s = 1u;  // the warp's next stage, its slot and phase
+    bool ok = true, mine = false;
+    uint32_t last_mine = 0;    // last stage this warp copied into (for the drain)
+    uint32_t taken = 0;        // units put in the ring
     for (uint32_t kk = 0; ok; ++kk) {
-      // The CTA's next item: the first copy warp takes it from the launch's
+      // The CTA's next unit: the first copy warp takes it from the launch's
       // list (the CTA's own index first, then the shared counter) and puts it
       // in the item ring once every role has read the entry it replaces.
-      if (pw == 0) {
-        const uint32_t r = kk % kItemRing;
-        if (elect_one()) {
-          if (wait_phase(smem_u32(&itemempty[r]), ((kk / kItemRing) & 1) ^ 1, abort_flag, err, ERR_ITEM_TAKE, lim)) {
-            const int pos = kk == 0 ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(args.next_item, 1);
-            WorkItem nw;
-            nw.panel = -1;
-            if (pos < args.n_items) nw = args.items[pos];
-            item_ring[r] = nw;
-            mbar_arrive(smem_u32(&itemfull[r]));
-          }
-        }
+      if (pw == 0 && taken == kk) {
+        if (elect_one()) put_unit(args, taken, itemfull, itemempty, item_ring, abort_flag, err, lim);
         __syncwarp();
+        ++taken;
       }
       WorkItem wi;
       if (!take_item_warp(itemfull, itemempty, item_ring, kk, lane, abort_flag, err, ERR_ITEM_TAKE, lim, false, wi)) {
         ok = false;
         break;
       }
-      if (wi.panel < 0) break;
+      if (wi.panel < 0) {
+        // the end, once more for the other set of epilogue warps
+        if (pw == 0 && elect_one())
+          put_unit(args, taken, itemfull, itemempty, item_ring, abort_flag, err, lim);
+        __syncwarp();
+        break;
+      }
+      // a short unit: take the next one now, so that its copies follow
+      // without a wait (a long one would be taken from a CTA that is free
+      // earlier)
+      if (pw == 0 && wi.s1 - wi.s0 <= kShortUnit) {
+        if (elect_one()) put_unit(args, taken, itemfull, itemempty, item_ring, abort_flag, err, lim);
+        __syncwarp();
+        ++taken;
+      }
       const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
       // fields used after shared-memory stores, held in registers (the stores
       // could alias P for the compiler and force a reload each time)
-      const StageRec* const p_stages = P.stages;
+      const StageRec* const p_stages = P.stages + wi.s0;
       const uint8_t* const p_aval = P.aval;
-      const int64_t p_kbs = P.bp_kbs;
-      const int n_tiles = P.n_tiles;
-      for (int nt = 0; nt < n_tiles && ok; ++nt) {
-        // the packed tiles of this pass ([128-column tile][k-block])
-        const uint8_t* const p_b = P.bpack + (int64_t)nt * NSUB * p_kbs * (4096 * C::NOPS);
-        const int64_t sub_bytes = p_kbs * (4096 * C::NOPS);
-        for (int base = wi.s0; base < wi.s1 && ok; base += 32) {
-          const int cnt = min(32, wi.s1 - base);
-          // lane l prepares stage ci + l: this warp's B copies j0 and j0 +
-          // NPROD (copy j brings subtile j % NSUB of tile j / NSUB), and the
-          // A region for the warp of the last copy index
-          const int j0 = (int)(((uint32_t)pw - (ci + (uint32_t)lane)) & (C::NPROD - 1));
-          int kb1 = -1, kb2 = -1, abytes = 0, aoff = 0;
-          if (lane < cnt) {
-            const StageRec* rp = p_stages + base + lane;
-            const int4 r1 = reinterpret_cast<const int4*>(rp)[1];  // nblk, hdr_bytes, ntiles, aoff256
-            const int nc = r1.z * NSUB;
-            if (j0 < nc) kb1 = rp->kb[j0 / NSUB];
-            if (j0 + C::NPROD < nc) kb2 = rp->kb[(j0 + C::NPROD) / NSUB];
-            if (j0 == C::NPROD - 1) {
-              aoff = r1.w;
-              abytes = stage_a_bytes(C::CLS, BH, r1.x);
-            }
-          }
-          for (int i = 0; i < cnt; ++i, ++ci) {
-            const int k1 = shfl_i(kb1, i), k2 = shfl_i(kb2, i);
-            const int ab = shfl_i(abytes, i), ao = shfl_i(aoff, i);
-            const int j = (int)(((uint32_t)pw - ci) & (C::NPROD - 1));
-            const uint32_t s = slot_s;
-            const bool good = wait_phase(smem_u32(&empty[s]), phase_s, abort_flag, err, ERR_PROD_A, lim);
-            if (!__all_sync(0xffffffffu, good)) {
-              ok = false;
-              break;
-            }
-            if (elect_one()) {
-              const uint32_t st = smem0 + s * C::STAGE;
-              const uint32_t fb = smem_u32(&full[s]);
-              uint32_t bytes = (k1 >= 0 ? 4096u * C::NOPS : 0u) + (k2 >= 0 ? 4096u * C::NOPS : 0u);
-              if (ab != 0) {
-                if (C::FP8) {
-                  // the A region on its own barrier (the converters wait for
-                  // it alone), the B tiles on full[s]
-                  const uint32_t fa = smem_u32(&afull[s]);
-                  mbar_arrive_expect_tx(fa, (uint32_t)ab);
-                  bulk_load_hint(st, p_aval + (int64_t)ao * 256, (uint32_t)ab, fa, pol_a);
-                } else {
-                  bytes += (uint32_t)ab;
-                }
-              }
-              mbar_arrive_expect_tx(fb, bytes);
-              if (!C::FP8 && ab != 0) bulk_load_hint(st, p_aval + (int64_t)ao * 256, (uint32_t)ab, fb, pol_a);
-              if (k1 >= 0)
-                bulk_load_hint(st + C::OFF_B + j * (4096 * C::NOPS),
-                               p_b + (j % NSUB) * sub_bytes + (int64_t)k1 * (4096 * C::NOPS), 4096 * C::NOPS, fb, pol_b);
-              if (k2 >= 0)
-                bulk_load_hint(st + C::OFF_B + (j + C::NPROD) * (4096 * C::NOPS),
-                               p_b + ((j + C::NPROD) % NSUB) * sub_bytes + (int64_t)k2 * (4096 * C::NOPS),
-                               4096 * C::NOPS, fb, pol_b);
-            }
-            __syncwarp();
-            last_mine = ci;
-            if (++slot_s == nsr) {
-              slot_s = 0;
-              phase_s ^= 1u;
-            }
+      const int32_t* const p_gcol = P.gcol;
+      const int64_t sub_bytes = P.bp_kbs * (int64_t)C::SUB;
+      // the packed tiles of this unit ([128-column tile][k-block]); a half
+      // without a column below N is not copied (its rows of the accumulators
+      // are never stored)
+      const uint8_t* const p_b = P.bpack + (int64_t)wi.nt * NSUB * sub_bytes;
+      const int left = P.N - wi.nt * C::BN;
+      // this lane's bulk copy: subtile sub of the stage's tile bt
+      const int bt = (lane / NSUB) * 2 + hf, sub = lane % NSUB;
+      const uint32_t bbytes = (uint32_t)max(0, min(2, (left - sub * 128 + 63) >> 6)) * C::HALF;
+      const uint8_t* const lane_b = p_b + sub * sub_bytes;
+      uint32_t tile_bytes = 0;  // bulk bytes of one tile
+#pragma unroll
+      for (int j = 0; j < NSUB; ++j)
+        tile_bytes += (uint32_t)max(0, min(2, (left - j * 128 + 63) >> 6)) * C::HALF;
+      const int nst = active ? wi.s1 - wi.s0 : 0;
+      int i = active ? (int)(my_c - ci) : 0;  // the warp's next stage of the unit (>= 0)
+      StageView cur, nxt;
+      load_stage(cur, p_stages, i, nst, bt);
+      load_stage(nxt, p_stages, i + (int)np, nst, bt);
+      load_rows(cur, p_gcol, hf, lane);
+      for (; i < nst; i += (int)np) {
+        const int na = cur.ntiles - cur.ngath, ng = (cur.ngath + 1 - hf) / 2;  // gathered tiles of this warp
+        const int nb = (na + 1 - hf) / 2;                                     // and bulk ones
+        const int kb = cur.kb, aoff = cur.aoff;
+        const uint32_t abytes = (uint32_t)stage_a_bytes(C::CLS, BH, cur.nblk, cur.ngath);
+        if (lane < ng * 4) reinterpret_cast<int4*>(glist)[lane] = cur.rows0;  // for every lane to look up
+        cur = nxt;
+        load_rows(cur, p_gcol, hf, lane);
+        load_stage(nxt, p_stages, i + 2 * (int)np, nst, bt);
+        const bool good = wait_phase(smem_u32(&empty[slot_s]), phase_s, abort_flag, err, ERR_PROD_A, lim);
+        if (!__all_sync(0xffffffffu, good)) {
+          ok = false;
+          break;
+        }
+        const uint32_t st = smem0 + slot_s * C::STAGE;
+        const uint32_t fb = smem_u32(&full[slot_s]);
+        // One bulk copy per lane: the warp's B tiles on the stage's barrier, and
+        // on lane 31 (the pair's second warp, which has the smaller half) the
+        // A region, which has a barrier of its own in the FP8 form, for the
+        // converters wait for it alone
+        const bool la = hf && lane == 31;
+        const uint32_t fa = C::FP8 ? smem_u32(&afull[slot_s]) : fb;
+        const uint32_t bytes = (uint32_t)nb * tile_bytes + (!C::FP8 && hf ? abytes : 0u);
+        mbar_expect_tx_if(fb, bytes, lane == 0 && bytes != 0);
+        if (C::FP8) mbar_arrive_expect_tx_if(fa, abytes, lane == 0 && hf);
+        bulk_load_hint_if(la ? st : st + C::OFF_B + (bt * NSUB + sub) * C::SUB,
+                          la ? p_aval + (int64_t)aoff * 256 : lane_b + (int64_t)kb * C::SUB, la ? abytes : bbytes,
+                          la ? fa : fb, la ? pol_a : pol_b, la || (bt < na && bbytes != 0));
+#pragma unroll 1
+        for (int g = 0; g < ng; ++g) {
+#pragma unroll
+          for (int j = 0; j < NSUB; ++j) {
+            const int nh = min(2, (left - j * 128 + 63) >> 6);
+            if (nh > 0)
+              gather_tile<C::NOPS>(st + C::OFF_B + ((na + 2 * g + hf) * NSUB + j) * C::SUB, p_b + j * sub_bytes,
+                                   glist + g * 16, nh, lane);
           }
         }
+        cp_async_arrive(fb);
+        __syncwarp();
+        last_mine = my_c;
+        mine = true;
+        my_c += np;
+        slot_s += np;
+        if (slot_s >= nsr) {  // np <= nsr: at most one turn of the ring
+          slot_s -= nsr;
+          phase_s ^= 1u;
+        }
       }
+      ci += (uint32_t)(wi.s1 - wi.s0);
     }
-    if (!ok && lane == 0 && last_mine != 0xffffffffu) {
+    if (!ok) cp_async_wait_all();
+    if (!ok && lane == 0 && mine) {
       // wait for this warp's own copies still in flight: they can only be in
-      // the last NS stages it copied into (a stage that another warp gave up
-      // on never completes, but copies land within microseconds: the wait is
-      // short)
-      const uint32_t lo = last_mine + 1 > nsr ? last_mine + 1 - nsr : 0;
+      // its stages among the last NS
       const uint64_t dl = lim < kDrainNs ? lim : kDrainNs;
-      for (uint32_t k = lo; k <= last_mine; ++k) {
+      for (uint32_t k = last_mine + 1 > nsr ? last_mine + 1 - nsr : 0; k <= last_mine; ++k) {
+        if (k % np != pair) continue;
         mbar_wait_drain(smem_u32(&full[k % nsr]), (k / nsr) & 1, err, dl);
         if (C::FP8) mbar_wait_drain(smem_u32(&afull[k % nsr]), (k / nsr) & 1, err, dl);
       }
@@ -477,8 +646,8 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       // ----------------------------------------------------------- MMA issuers
       // Issuer w runs the MMA groups of its quarter of the panel's block rows,
       // from the list the copy brought in with the stage, and releases every
-      // stage once. One thread issues a tcgen05.mma only every ~80-150
-      // cycles; four keep the tensor pipe near its rate for these narrow MMAs.
+      // stage once. One thread issues a tcgen05.mma only every 64-75 cycles;
+      // four keep the tensor pipe near its rate for these narrow MMAs.
       uint32_t ci = 0, k = 0, slot_s = 0, phase_s = 0;
       bool ok = true, issued = false;
       const uint32_t stall = (blockIdx.x == 0 && warp == 0) ? (uint32_t)args.stall_stage : 0u;
@@ -490,10 +659,10 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
         }
         if (wi.panel < 0) break;
         const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
-        const int n_tiles = P.n_tiles;
         const uint32_t idesc0 = P.idesc;  // without the N field
+        const bool gathers = P.gcol != nullptr;
         const int nstages = wi.s1 - wi.s0;
-        for (int nt = 0; nt < n_tiles && ok; ++nt, ++k) {
+        {
           const uint32_t buf = k & 1;
           const uint32_t dbase = tmem + buf * C::ACC_COLS;
           // use u = k / 2 of this buffer waits for phase u of accempty: the
@@ -520,6 +689,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
               ok = false;
               break;
             }
+            if (gathers) fence_proxy_async_smem();  // gathered rows were written through the generic proxy
             const uint8_t* stp = smem + s * C::STAGE;
             const uint2 hd = *reinterpret_cast<const uint2*>(stp);  // (first, count) of each warp
             const uint32_t wl = ((warp & 2 ? hd.y : hd.x) >> (16 * (warp & 1))) & 0xffffu;
@@ -528,22 +698,23 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
             // lo blocks follow the stage's nblk hi blocks (split form)
             const uint32_t lo_off = KIND == KIND_SPLIT ? *reinterpret_cast<const uint16_t*>(stp + 8) * C::ABLK : 0;
             // descriptors of operands inside the stage = stage descriptor + offset / 16
-            const uint64_t sdesc = desc_kmajor_sw32(smem0 + s * C::STAGE);
+            const uint64_t sdesc = desc_kmajor_sw32(smem0 + s * C::STAGE + C::OFF_A);
+            const uint64_t bdesc = desc_mnmajor_sw128(smem0 + s * C::STAGE + C::OFF_B, C::HALF);
             for (uint32_t e = 0; e < cnt; ++e) {
               const uint32_t m = ent[e];
               const uint32_t pos = m & 31u, tile = (m >> 5) & 15u, slot = (m >> 9) & 31u;
               const uint32_t len = ((m >> 14) & 15u) + 1u, acc = (m >> 18) & 1u;
               const uint32_t idesc = idesc0 | (((len * BH) >> 3) << 17);
-              const uint64_t a_hi = sdesc + ((C::OFF_A + pos * C::ABLK) >> 4);
-              const uint64_t b_hi0 = sdesc + ((C::OFF_B + tile * C::TILEB) >> 4);
+              const uint64_t a_hi = sdesc + ((pos * C::ABLK) >> 4);
+              const uint64_t b_hi0 = bdesc + ((tile * C::TILEB) >> 4);
 #pragma unroll
               for (int j = 0; j < NSUB; ++j) {
                 const uint32_t dcol = dbase + j * C::SUB_COLS + slot * BH;
-                const uint64_t b_hi = b_hi0 + ((j * 128 * 32) >> 4);
+                const uint64_t b_hi = b_hi0 + ((j * C::SUB) >> 4);
                 umma_f16(dcol, b_hi, a_hi, idesc, acc);
                 if (KIND == KIND_SPLIT) {
                   const uint64_t a_lo = a_hi + (lo_off >> 4);
-                  const uint64_t b_lo = b_hi + (C::TILE >> 4);
+                  const uint64_t b_lo = b_hi + (2048 >> 4);
                   umma_f16(dcol, b_hi, a_lo, idesc, 1);
                   umma_f16(dcol, b_lo, a_hi, idesc, 1);
                 }
@@ -558,6 +729,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
           }
           if (!ok) break;
           umma_commit(smem_u32(&accfull[buf]));
+          ++k;
         }
       }
       if (!ok && issued) {
@@ -568,32 +740,37 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     }
   } else if (warp >= 4) {
     // -------------------------------------------------------------- epilogue
-    // Warp 4 + q drains TMEM lane quadrant q (C columns q*32 .. q*32+31 of
-    // each 128-column subtile) for every slot, and writes zeros back: the
-    // accumulators are all zero whenever the MMA warps receive a buffer, so
-    // a part that starts in the middle of a panel accumulates onto zero.
+    // Two sets of four warps, one per accumulator buffer: while one drains a
+    // unit, the other looks up the next one's rows (8,000 cycles of dependent
+    // global loads a unit on the 64^3 stencil) and drains it as soon as its
+    // MMAs are done. Warp q of a set drains TMEM lane quadrant q (C columns
+    // q*32 .. q*32+31 of each 128-column subtile) for every slot, and writes
+    // zeros back: the accumulators are all zero whenever the MMA warps receive
+    // a buffer, so a part that starts in the middle of a panel accumulates
+    // onto zero.
     const uint32_t q = warp & 3;
+    const uint32_t buf = (uint32_t)(warp - 4) >> 2;
     const uint32_t lane_base = tmem + ((q * 32u) << 16);
-    for (uint32_t c = 0; c < 2 * C::ACC_COLS; c += 16) tmem_st_x16_zero(lane_base + c);
+    const uint32_t dbase = lane_base + buf * C::ACC_COLS;
+    for (uint32_t c = 0; c < C::ACC_COLS; c += 16) tmem_st_x16_zero(dbase + c);
     tmem_st_wait();
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) {
-      mbar_arrive(smem_u32(&accempty[0]));
-      mbar_arrive(smem_u32(&accempty[1]));
-    }
+    if (lane == 0) mbar_arrive(smem_u32(&accempty[buf]));
     constexpr int SLAB = R * BH * C::BN;  // floats per slab
     constexpr int PW = (R % kMmaWarps == 0) ? R / kMmaWarps : 0;  // slots per issuing warp
-    constexpr int RPL = (R * BH + 31) / 32;                          // C-row entries per lane
-    // 16-row blocks with at least two slots per issuing warp: the drain reads
-    // two adjacent slots with one 32-column load (one load round trip per
-    // pair; a hub row's later parts are never in their first part's pair).
-    // Not for FP8: its 640-thread CTAs have 96 registers a thread, and the
-    // pair's 32 values would spill.
-    constexpr bool PAIR = BH == 16 && NSUB == 1 && PW >= 2 && R % 2 == 0 && KIND != KIND_FP8;
-    uint32_t k = 0;
+    // A drain step takes 32 TMEM columns (a 32-row slot, or two adjacent
+    // 16-row ones) with one load; 16 where a hub row's later parts may be in
+    // its first part's pair (one slot per issuing warp). The steps are a loop:
+    // unrolled, the drain was about 16,000 instructions a pass, and fetching
+    // them set the kernel's pace (64^3 stencil, N = 256: 235 us with every
+    // copy and MMA in place, 190 us with none).
+    constexpr int STEP = 16;
+    int* const rows = row_tab + (warp - 4) * (R * BH);  // this warp's table of the panel's C rows
     bool ok = true;
-    for (uint32_t kk = 0; ok; ++kk) {
+    int odd_prob = -1;                      // problem that odd_known and odd_val are about
+    uint64_t odd_known = 0, odd_val = 0;  // a bit per column tile below 64
+    for (uint32_t kk = buf; ok; kk += 2) {
       WorkItem wi;
       if (!take_item_warp(itemfull, itemempty, item_ring, kk, lane, abort_flag, err, ERR_ITEM_EPI, lim, true, wi)) {
         ok = false;
@@ -603,165 +780,191 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
       // fields used between the stores to C, held in registers (the stores
       // could alias P for the compiler and force reloads of every field)
-      const int p_N = P.N, p_nbr = P.nbr, p_f16 = P.c_f16;
+      const int p_N = P.N, p_f16 = P.c_f16, n_tiles = P.n_tiles;
       const int64_t p_ldc = P.ldc;
       void* const p_C = P.C;
-      float* const p_slabs = P.slabs;
-      int32_t* const p_counters = P.counters;
-      const int n_tiles = P.n_tiles;
-      const int panel = wi.panel;
+      const int panel = wi.panel, nt = wi.nt;
       const bool split = wi.split >= 0;
       const uint32_t slot_mask = P.panels[panel].slot_mask;
       // a hub row cut over the issuing warps has its parts in slots s, s + PW,
       // s + 2 PW, ...; the parts after the first are added into it here
       const uint32_t ext_mask = P.panels[panel].ext_mask;
-      // the panel's C rows, plan row 32 q + lane in rmap[q] of that lane,
-      // loaded before the accumulators are ready: one global round trip
-      // per item instead of one per slot (the slot loops are unrolled, so
-      // rmap stays in registers)
-      int rmap[RPL];
+      // the panel's C rows, loaded before the accumulators are ready; bit x of
+      // `full`: rows 16 x .. 16 x + 15 are all there
+      uint32_t full = 0;
+      const int elt = p_f16 ? 2 : 4;
+      const int64_t ldb = p_ldc * elt;
 #pragma unroll
-      for (int q2 = 0; q2 < RPL; ++q2) {
-        const int pr = q2 * 32 + lane;
-        rmap[q2] = (pr < R * BH && (int64_t)panel * R * BH + pr < (int64_t)p_nbr * BH)
-                       ? P.row_map[(int64_t)panel * R * BH + pr]
-                       : -1;
+      for (int x = 0; x < R * BH; x += 32) {
+        const int row = P.row_map[(int64_t)panel * R * BH + x + lane];
+        rows[x + lane] = row;
+        const uint32_t there = __ballot_sync(0xffffffffu, row >= 0);
+        full |= ((there & 0xffffu) == 0xffffu ? 1u : 0u) << (x / 16);
+        full |= ((there >> 16) == 0xffffu ? 1u : 0u) << (x / 16 + 1);
       }
-      for (int nt = 0; nt < n_tiles; ++nt, ++k) {
-        const uint32_t buf = k & 1;
-        if (!warp_wait(smem_u32(&accfull[buf]), (k >> 1) & 1, lane, abort_flag, err, ERR_EPI, true, lim)) {
-          ok = false;
-          break;
+      const int32_t* const p_pois = P.poison_ptr;
+      // does the packed B of these columns hold infinite or NaN values?
+      // (looked up once per problem and column tile)
+      bool odd = false;
+      if (p_pois != nullptr) {
+        if (wi.prob != odd_prob) {
+          odd_prob = wi.prob;
+          odd_known = odd_val = 0;
         }
-        tc_fence_after();
-        const uint32_t dbase = lane_base + buf * C::ACC_COLS;
-        // slab of (part, column tile): (first slab of the panel + part) * n_tiles + nt
-        float* slab = split ? p_slabs + ((size_t)(wi.slab + wi.part) * n_tiles + nt) * SLAB : nullptr;
-        float pairv[32];
+        const uint64_t bit = nt < 64 ? 1ull << nt : 0ull;
+        if ((odd_known & bit) == 0) {
+          const int64_t fs = pack_flag_stride(P.K);
+          const int h0 = nt * (2 * NSUB), h1 = min(h0 + 2 * NSUB, (p_N + 63) >> 6);
+          const uint4* fl = reinterpret_cast<const uint4*>(P.bflags + (int64_t)h0 * fs);
+          uint32_t any = 0;
+#pragma unroll 4
+          for (int64_t x = lane; x < (h1 - h0) * fs / 16; x += 32) {
+            const uint4 f = __ldcg(fl + x);
+            any |= f.x | f.y | f.z | f.w;
+          }
+          odd = __any_sync(0xffffffffu, any != 0);
+          odd_known |= bit;
+          if (odd) odd_val |= bit;
+        } else {
+          odd = (odd_val & bit) != 0;
+        }
+      }
+      __syncwarp();
+      if (!warp_wait(smem_u32(&accfull[buf]), (kk >> 1) & 1, lane, abort_flag, err, ERR_EPI, true, lim)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      // slab of (part, column tile): (first slab of the panel + part) * n_tiles + nt
+      float* const slab0 = split ? P.slabs + ((size_t)wi.slab * n_tiles + nt) * SLAB : nullptr;
+      float* const slab = split ? slab0 + (size_t)wi.part * n_tiles * SLAB : nullptr;
+#pragma unroll 1
+      for (int j = 0; j < NSUB; ++j) {
+        const int nl = j * 128 + (int)q * 32 + lane;  // column inside the tile
+        const int n = nt * C::BN + nl;
+        uint8_t* const col = static_cast<uint8_t*>(p_C) + (int64_t)n * elt;
+#pragma unroll 1
+        for (int r0 = 0; r0 < R * BH; r0 += STEP) {
+          float v[STEP];
+          const uint32_t ta = dbase + j * C::SUB_COLS + r0;
+          __syncwarp();  // lanes past N skipped the stores: together again for the aligned loads
+          // an empty slot reads zeros: slots are zeroed after every drain and
+          // no MMA writes an empty one
+          if ((slot_mask >> (r0 / BH)) & (STEP > BH ? 3u : 1u)) {
+            if constexpr (STEP == 32) {
+              tmem_ld_x32(ta, v);
+              tmem_st_x32_zero(ta);
+            } else {
+              tmem_ld_x16(ta, v);
+              tmem_st_x16_zero(ta);
+            }
+          } else {
 #pragma unroll
-        for (int s = 0; s < R; ++s) {
-          const int rb = panel * R + s;
-          if (rb >= p_nbr) break;
-          if constexpr (PAIR) {
-            if ((s & 1) == 0) {
-              // slots s and s + 1 (an empty slot reads zeros: slots are
-              // zeroed after every drain and no MMA writes an empty one)
-              if ((slot_mask >> s) & 3u) {
-                const uint32_t ta = dbase + s * BH;
-                tmem_ld_x32(ta, pairv);
-                tmem_st_x32_zero(ta);
-              } else {
+            for (int m = 0; m < STEP; ++m) v[m] = 0.0f;
+          }
 #pragma unroll
-                for (int m = 0; m < 32; ++m) pairv[m] = 0.0f;
+          for (int g = 0; g < STEP; g += 16) {
+            const int sl = (r0 + g) / BH, h = (r0 + g) % BH;  // slot, row inside it
+            if ((ext_mask >> sl) & 1u) continue;
+            __syncwarp();
+            float* const w = v + g;
+            if constexpr (PW > 0) {
+#pragma unroll 1
+              for (int t = sl + PW; t < R && ((ext_mask >> t) & 1u); t += PW) {
+                if (((slot_mask >> t) & 1u) == 0) continue;
+                float u[16];
+                const uint32_t tb = dbase + j * C::SUB_COLS + t * BH + h;
+                tmem_ld_x16(tb, u);
+                tmem_st_x16_zero(tb);
+#pragma unroll
+                for (int m = 0; m < 16; ++m) w[m] += u[m];
+              }
+            }
+            if (split) {
+              float* const dst = slab + (size_t)(r0 + g) * C::BN + nl;
+#pragma unroll
+              for (int m = 0; m < 16; ++m) __stcg(dst + (size_t)m * C::BN, w[m]);
+            } else {
+              if (odd) {
+                const int q0 = p_pois[panel * R + sl], q1 = p_pois[panel * R + sl + 1];
+                if (q0 < q1 && n < p_N && poisoned(P, C::NOPS, q0, q1, n)) {
+#pragma unroll
+                  for (int m = 0; m < 16; ++m) w[m] = __int_as_float(0x7fffffff);
+                }
+              }
+              const bool fl = (full >> ((r0 + g) / 16)) & 1u;
+              if (n < p_N) {
+                if (p_f16) store_rows16<__half>(col, ldb, rows + r0 + g, fl, w);
+                else store_rows16<float>(col, ldb, rows + r0 + g, fl, w);
               }
             }
           }
-          if ((ext_mask >> s) & 1u) continue;
-          const bool empty_slot = ((slot_mask >> s) & 1u) == 0;
+        }
+      }
+      __syncwarp();
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&accempty[buf]));
+      if (!split) continue;
+      // this warp's part of the slab is written: count it; the warp that
+      // brings the count of its quadrant to nparts adds up all parts
+      __threadfence();
+      __syncwarp();
+      int last = 0;
+      if (lane == 0) {
+        int* ctr = P.counters + ((size_t)wi.split * n_tiles + nt) * 4 + q;
+        last = atomicAdd(ctr, 1) == wi.nparts - 1;
+      }
+      last = __shfl_sync(0xffffffffu, last, 0);
+      if (!last) continue;
+      __threadfence();
+#pragma unroll 1
+      for (int j = 0; j < NSUB; ++j) {
+        const int nl = j * 128 + (int)q * 32 + lane;
+        const int n = nt * C::BN + nl;
+#pragma unroll 1
+        for (int r0 = 0; r0 < R * BH; r0 += 16) {
+          const int sl = r0 / BH;
+          if ((ext_mask >> sl) & 1u) continue;  // added into its first part's slab rows
+          // 16 rows of two parts at a time: their loads are independent and
+          // overlap instead of paying one L2 round trip each
+          float acc[16];
 #pragma unroll
-          for (int j = 0; j < NSUB; ++j) {
-            const int nl = j * 128 + (int)q * 32 + lane;  // column inside the tile
-            const int n = nt * C::BN + nl;
+          for (int m = 0; m < 16; ++m) acc[m] = 0.0f;
+          const float* src = slab0 + (size_t)r0 * C::BN + nl;
+          const size_t step = (size_t)n_tiles * SLAB;
+          int p = 0;
+#pragma unroll 1
+          for (; p + 2 <= wi.nparts; p += 2, src += 2 * step) {
+            float t[32];
 #pragma unroll
-            for (int h = 0; h < BH; h += 16) {
-              float vs[16];
-              float* v = PAIR ? pairv + (s & 1) * 16 : vs;
-              if constexpr (!PAIR) {
-                if (!empty_slot) {
-                  const uint32_t ta = dbase + j * C::SUB_COLS + s * BH + h;
-                  tmem_ld_x16(ta, vs);
-                  tmem_st_x16_zero(ta);
-                } else {
+            for (int m = 0; m < 16; ++m) {
+              t[m] = __ldcg(src + (size_t)m * C::BN);
+              t[16 + m] = __ldcg(src + step + (size_t)m * C::BN);
+            }
 #pragma unroll
-                  for (int m = 0; m < 16; ++m) vs[m] = 0.0f;
-                }
-              }
-              if constexpr (PW > 0) {
-                for (int t = s + PW; t < R && ((ext_mask >> t) & 1u); t += PW) {
-                  if (((slot_mask >> t) & 1u) == 0) continue;
-                  float u[16];
-                  const uint32_t tb = dbase + j * C::SUB_COLS + t * BH + h;
-                  tmem_ld_x16(tb, u);
-                  tmem_st_x16_zero(tb);
+            for (int m = 0; m < 16; ++m) acc[m] = (acc[m] + t[m]) + t[16 + m];
+          }
+          if (p < wi.nparts) {
+            float t[16];
 #pragma unroll
-                  for (int m = 0; m < 16; ++m) v[m] += u[m];
-                }
-              }
-              if (split) {
+            for (int m = 0; m < 16; ++m) t[m] = __ldcg(src + (size_t)m * C::BN);
 #pragma unroll
-                for (int m = 0; m < 16; ++m) __stcg(slab + (size_t)(s * BH + h + m) * C::BN + nl, v[m]);
-              } else {
+            for (int m = 0; m < 16; ++m) acc[m] += t[m];
+          }
+          if (odd) {
+            const int q0 = p_pois[panel * R + sl], q1 = p_pois[panel * R + sl + 1];
+            if (q0 < q1 && n < p_N && poisoned(P, C::NOPS, q0, q1, n)) {
 #pragma unroll
-                for (int m = 0; m < 16; ++m) {
-                  const int pr = s * BH + h + m;  // plan row inside the panel
-                  const int row = __shfl_sync(0xffffffffu, rmap[pr >> 5], pr & 31);
-                  if (row >= 0 && n < p_N) {
-                    const int64_t off = (int64_t)row * p_ldc + n;
-                    if (p_f16)
-                      __stcs(reinterpret_cast<__half*>(p_C) + off, __float2half_rn(v[m]));
-                    else
-                      __stcs(reinterpret_cast<float*>(p_C) + off, v[m]);
-                  }
-                }
-              }
+              for (int m = 0; m < 16; ++m) acc[m] = __int_as_float(0x7fffffff);
             }
           }
-        }
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&accempty[buf]));
-        if (!split) continue;
-        // this warp's part of the slab is written: count it; the warp that
-        // brings the count of its quadrant to nparts adds up all parts
-        __threadfence();
-        __syncwarp();
-        int last = 0;
-        if (lane == 0) {
-          int* ctr = p_counters + ((size_t)wi.split * n_tiles + nt) * 4 + q;
-          last = atomicAdd(ctr, 1) == wi.nparts - 1;
-        }
-        last = __shfl_sync(0xffffffffu, last, 0);
-        if (!last) continue;
-        __threadfence();
-        const float* slab0 = p_slabs + ((size_t)wi.slab * n_tiles + nt) * SLAB;
-#pragma unroll
-        for (int s = 0; s < R; ++s) {
-          const int rb = panel * R + s;
-          if (rb >= p_nbr) break;
-          if ((ext_mask >> s) & 1u) continue;  // added into its first part's slab rows
-#pragma unroll
-          for (int j = 0; j < NSUB; ++j) {
-            const int nl = j * 128 + (int)q * 32 + lane;
-            const int n = nt * C::BN + nl;
-            for (int h = 0; h < BH; h += 16) {
-              // 16 rows at a time: the loads of a part are independent, so
-              // they overlap instead of paying one L2 round trip per row
-              float acc[16];
-#pragma unroll
-              for (int m = 0; m < 16; ++m) acc[m] = 0.0f;
-              const float* src = slab0 + (size_t)(s * BH + h) * C::BN + nl;
-              for (int p = 0; p < wi.nparts; ++p) {
-                float t[16];
-#pragma unroll
-                for (int m = 0; m < 16; ++m) t[m] = __ldcg(src + (size_t)m * C::BN);
-#pragma unroll
-                for (int m = 0; m < 16; ++m) acc[m] += t[m];
-                src += (size_t)n_tiles * SLAB;
-              }
-#pragma unroll
-              for (int m = 0; m < 16; ++m) {
-                const int pr = s * BH + h + m;
-                const int row = __shfl_sync(0xffffffffu, rmap[pr >> 5], pr & 31);
-                if (row >= 0 && n < p_N) {
-                  const int64_t off = (int64_t)row * p_ldc + n;
-                  if (p_f16)
-                    __stcs(reinterpret_cast<__half*>(p_C) + off, __float2half_rn(acc[m]));
-                  else
-                    __stcs(reinterpret_cast<float*>(p_C) + off, acc[m]);
-                }
-              }
-            }
+          const bool fl = (full >> (r0 / 16)) & 1u;
+          uint8_t* const col = static_cast<uint8_t*>(p_C) + (int64_t)n * elt;
+          if (n < p_N) {
+            if (p_f16) store_rows16<__half>(col, ldb, rows + r0, fl, acc);
+            else store_rows16<float>(col, ldb, rows + r0, fl, acc);
           }
         }
       }

@@ -46,31 +46,37 @@ struct PanelInfo {
 //     [header, kStageHdrBytes][nblk * ABLK blocks (hi)][nblk * ABLK blocks (lo, split form only)]
 // and in the FP8 stream (16 x 16 blocks)
 //     [header, kStageHdrBytes][nblk * 256 e4m3 blocks][nblk FP32 scales, padded to 16 bytes]
+//     [16 FP32 scales per gathered block (its columns come from several blocks)]
 // starting at byte aoff256 * 256 (the stages of the FP8 stream are padded to
 // that), so the header is always at the stage's start and the MMA threads
 // need no word that says where.
 // Padded bytes of the FP32 scales of n FP8 blocks.
 __host__ __device__ constexpr int fp8_scale_bytes(int n) { return (4 * n + 15) / 16 * 16; }
-// Bytes of a stage of nblk blocks in the A stream of plan class cls.
+// Bytes of a stage of nblk blocks, ngath of them gathered, in the A stream of
+// plan class cls.
 constexpr int kStageHdrBytes = 256;  // a header's room in the A stream and in shared memory
-__host__ __device__ constexpr int stage_a_bytes(int cls, int bh, int nblk) {
-  return kStageHdrBytes + (cls == 2 ? nblk * 256 + fp8_scale_bytes(nblk) : nblk * bh * 32 * (cls == 1 ? 2 : 1));
+__host__ __device__ constexpr int stage_a_bytes(int cls, int bh, int nblk, int ngath) {
+  return kStageHdrBytes +
+         (cls == 2 ? nblk * 256 + fp8_scale_bytes(nblk) + 64 * ngath : nblk * bh * 32 * (cls == 1 ? 2 : 1));
 }
 struct StageRec {
   int64_t blk_off;     // blocks before this stage (plan order)
   int64_t hdr_off;     // header bytes before this stage (Plan::headers)
-  int32_t nblk;        // A blocks in the stage
-  int32_t hdr_bytes;   // bytes of this stage's header (multiple of 16)
-  int32_t ntiles;      // B tiles (distinct block columns) of the stage, 1..stage_tiles
+  int16_t nblk;        // A blocks in the stage
+  int16_t ntiles;      // B tiles of the stage, 1..stage_tiles
+  int16_t hdr_bytes;   // bytes of this stage's header (multiple of 16)
+  int16_t ngath;       // gathered blocks; their tiles come last
+  int32_t g0;          // the first of them (they are consecutive)
   int32_t aoff256;     // start of the stage in the A stream, in units of 256 bytes
-  int32_t kb[kMaxStageTiles];  // k-block (column / 16) of each tile
+  int32_t kb[kMaxStageTiles];  // k-block (column / 16) of each tile; -(g + 1): rows of B of gathered block g
 };
 
 
 // Stage header (little-endian), kStageHdrFixed bytes then one 32-bit entry
 // per MMA group, grouped by issuing warp:
 //   uint16 warp_list[4]   bits 0-7 first entry of warp w, bits 8-15 its entry count
-//   uint16 nblk, ntiles, pad[2]
+//   uint16 nblk, ntiles
+//   uint32 gathered       bit q set: block q of the stage is gathered
 //   uint32 entry[...]
 // A group is a run of consecutive block rows ("slots") with a block at the
 // same block column, the same accumulate flag and the same owner; it is one
@@ -88,6 +94,8 @@ __host__ __device__ constexpr int stage_hdr_max(int sb) { return kStageHdrFixed 
 // split index: its parts write partial sums to workspace slabs, and the part
 // that finishes last (an atomic counter per split panel and column tile)
 // adds the slabs and writes C.
+static_assert(sizeof(StageRec) == 96, "the kernel reads 16-byte pieces");
+
 struct alignas(16) WorkItem {
   int32_t panel;
   int32_t s0, s1;      // stage range, relative to the panel's first stage
@@ -96,12 +104,17 @@ struct alignas(16) WorkItem {
   int32_t nparts;      // parts of the split panel
   int32_t slab;        // first slab of the split panel (one per part and column tile)
   int32_t prob;        // problem of a grouped launch (0 for a single SpMM)
+  int32_t nt = 0;      // column tile (grouped launches; else set when the item is taken)
+  int32_t pad[3] = {};
 };
 
 // Everything the kernel needs about one SpMM problem.
 struct ProblemDesc {
-  const uint8_t* bpack;      // B in 4 KB tiles [128-column tile][k-block] (pack_b); the split
-                             // form stores [hi tile | lo tile] pairs, 8 KB per tile
+  const uint8_t* bpack;      // B in 4 KB tiles [128-column tile][k-block] (pack_b), 8 KB in the split form
+  const uint8_t* bflags;     // a byte per packing unit: holds infinite or NaN values
+  const int32_t* gcol;       // [16 g + q]: row of B of gathered block g's column q, or -1
+  const int32_t* poison_ptr; // [panels * R + 1] per plan slot: its range of `poison`; null without gathering
+  const int2* poison;        // k-block and mask of its all-zero columns, per gathered block
   int64_t bp_kbs;            // k-blocks per 128-column tile in bpack ([column tile][k-block])
   const uint8_t* aval;       // A stream of the form (see StageRec)
   const PanelInfo* panels;
@@ -113,20 +126,22 @@ struct ProblemDesc {
   int32_t* counters;         // [split panels][column tiles][4], zero before the launch
   int32_t N;
   int32_t n_tiles;
-  int32_t nbr;               // plan block rows: panels * R (TMEM slots)
   int32_t c_f16;
   uint32_t idesc;            // instruction descriptor without the N field
-  int32_t pad[3];
+  int32_t K;
+  int32_t b_bf16;            // packed B is BF16 (else FP16)
 };
 
 // Kernel arguments (one __grid_constant__ parameter). A single SpMM passes
 // its problem by value (one); a grouped launch passes a device array
 // (probs, indexed by WorkItem::prob).
 // A launch: its problems and work items, by decreasing estimated cost and
-// with the stage range counted from the plan's first stage. CTA b takes item
-// b, then item grid + atomicAdd(next_item, 1), ... until the list is done:
-// whichever CTA is free first takes the largest item left (the counter is
-// zero at launch).
+// with the stage range counted from the plan's first stage. A unit of work is
+// an item and a column tile (one problem: unit u is item u / n_tiles, tile u %
+// n_tiles; a grouped launch lists every unit). CTA b takes unit b, then unit
+// grid + atomicAdd(next_item, 1), ... until all n_items units are done:
+// whichever CTA is free first takes the largest one left (the counter is zero
+// at launch).
 // wait_ns bounds every device-side wait (0: 4 s); stall_stage k > 0 makes
 // the first MMA-issuing thread of CTA 0 wait, before its k-th stage, on a
 // barrier nothing arrives at (a test of the bounded-wait error path);

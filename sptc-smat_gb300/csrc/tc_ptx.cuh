@@ -280,6 +280,57 @@ __device__ __forceinline__ uint64_t desc_kmajor_sw32(uint32_t saddr) {
   return d;
 }
 
+// Shared-memory matrix descriptor of the M operand stored MN-major with the
+// 128-byte swizzle: K rows of 64 16-bit values (128 bytes), 8-row groups 1,024
+// bytes apart (stride), the next 64 values of M `lead` bytes on (leading
+// dimension). The tile must start on a 1,024-byte boundary.
+__device__ __forceinline__ uint64_t desc_mnmajor_sw128(uint32_t saddr, uint32_t lead) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
+  d |= static_cast<uint64_t>(lead >> 4) << 16;
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;
+  d |= static_cast<uint64_t>(1) << 46;  // descriptor version for tcgen05
+  d |= static_cast<uint64_t>(2) << 61;  // layout: 128-byte swizzle
+  return d;
+}
+
+// 16 bytes global -> shared through the load path, zeros when bytes == 0.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// One arrival on `bar` (counted against its expected arrivals) when this
+// thread's earlier cp.async have landed.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Predicated forms for whole-warp code: a branch around a few lanes' copies
+// splits the warp, and putting it together again costs more than they do (one
+// polling lane in place of 32 took the R-MAT step from 115 to 149 us).
+__device__ __forceinline__ void mbar_expect_tx_if(uint32_t bar, uint32_t bytes, bool pred) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;\n}" ::"r"(
+          bar),
+      "r"(bytes), "r"((uint32_t)pred)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx_if(uint32_t bar, uint32_t bytes, bool pred) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}" ::"r"(
+          bar),
+      "r"(bytes), "r"((uint32_t)pred)
+      : "memory");
+}
+__device__ __forceinline__ void bulk_load_hint_if(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar,
+                                                  uint64_t policy, bool pred) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n"
+      " @p cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], "
+      "%4;\n}" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar), "l"(policy), "r"((uint32_t)pred)
+      : "memory");
+}
+
 // Instruction descriptor, kind::f16: FP32 accumulator, both operands
 // K-major, A/B format 0 = FP16, 1 = BF16.
 __host__ __device__ constexpr uint32_t idesc_f16(int M, int N, uint32_t ab_format) {
