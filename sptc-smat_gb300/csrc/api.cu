@@ -86,7 +86,7 @@ static void free_handle(smat_bcsr* h) {
     if (p) cudaFree(p);
   for (PlanDev& pd : h->pc) {
     void* pp[] = {pd.d_stages, pd.d_panels, pd.d_row_map, pd.d_gcol, pd.d_poison_ptr, pd.d_poison, pd.sched[1].d_items, pd.sched[2].d_items,
-                  pd.sched[1].d_whole, pd.sched[2].d_whole};
+                  pd.sched[1].d_whole, pd.sched[2].d_whole, pd.sched[1].d_splits, pd.sched[2].d_splits};
     for (void* p : pp)
       if (p) cudaFree(p);
   }
@@ -227,6 +227,8 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
       std::vector<WorkItem> dev = device_items({&pd.plan}, items, order);
       SMAT_TRY(upload(&sc.d_items, dev.data(), dev.size()));
       if (sc.n_split > 0) {
+        dev = split_items(items);
+        SMAT_TRY(upload(&sc.d_splits, dev.data(), dev.size()));
         // the same without split panels, for scratch that has no room for
         // their partial sums
         int32_t ns = 0, nl = 0;
@@ -573,9 +575,8 @@ WsLayout smat::ws_layout(const smat_bcsr* A, int32_t form, int64_t N, bool whole
   const int nsub = pick_nsub(A, N, kind_of(form));
   const Sched& sc = A->pc[plan_class(form, nsub)].sched[nsub];
   const int64_t bn = 128 * nsub, n_tiles = (std::max<int64_t>(N, 1) + bn - 1) / bn;
-  const size_t n_split = whole ? 0 : sc.n_split, n_slabs = whole ? 0 : sc.n_slabs;
-  w.counter_bytes = (16 + n_split * n_tiles * 4 * sizeof(int32_t) + 255) / 256 * 256;
-  w.slabs = w.counters + w.counter_bytes;
+  const size_t n_slabs = whole ? 0 : sc.n_slabs;
+  w.slabs = w.counters + 256;
   w.flags = w.slabs + n_slabs * n_tiles * A->R * A->host.bh * bn * sizeof(float);
   w.total = w.flags + (pack_flag_bytes(A->host.cols, std::max<int64_t>(N, 1)) + 255) / 256 * 256;
   return w;
@@ -601,7 +602,6 @@ void smat::fill_problem(const smat_bcsr* A, int32_t form, const void* ws_, int64
   P.poison = reinterpret_cast<const int2*>(A->pc[cls].d_poison);
   P.C = C;
   P.ldc = ldc;
-  P.counters = reinterpret_cast<int32_t*>(ws + wl.counters + 16);  // after the next-item counter
   P.slabs = reinterpret_cast<float*>(ws + wl.slabs);
   P.N = (int32_t)N;
   P.n_tiles = (int32_t)((N + bn - 1) / bn);
@@ -700,7 +700,7 @@ static smat_status pack_impl(const smat_bcsr* A, int32_t form, const void* B, in
   const int in_dt = b_dtype == SMAT_F32 ? 0 : (b_dtype == SMAT_F16 ? 1 : 2);
   const int mode = (form == SMAT_FORM_F16 || form == SMAT_FORM_FP8) ? 0 : (split ? 2 : 1);
   cudaError_t e = pack_b(B, in_dt, b_layout == SMAT_COL_MAJOR ? 1 : 0, ldb, mode, out, K, N, A->d_kperm,
-                         out + wl.flags, static_cast<cudaStream_t>(stream_));
+                         out + wl.flags, reinterpret_cast<int32_t*>(out + wl.counters), static_cast<cudaStream_t>(stream_));
   if (e != cudaSuccess) return cuda_fail(e, "pack_b");
   if (uses_sp24(A, form)) {
     e = pack_b_sw64(out, K, N, out + wl.b64, static_cast<cudaStream_t>(stream_));
@@ -710,7 +710,7 @@ static smat_status pack_impl(const smat_bcsr* A, int32_t form, const void* B, in
 }
 
 static smat_status packed_impl(const smat_bcsr* A, int32_t form, const void* packed_b, int64_t N, void* C,
-                               int32_t c_dtype, int64_t ldc, void* stream_, bool whole) {
+                               int32_t c_dtype, int64_t ldc, void* stream_, bool whole, bool behind_pack) {
   smat_status st = check_common(A, form, N);
   if (st != SMAT_OK) return st;
   if (!packed_b || !C) return fail(SMAT_ERR_INVALID, "null argument");
@@ -740,15 +740,28 @@ static smat_status packed_impl(const smat_bcsr* A, int32_t form, const void* pac
   args.depth = A->depth;
   uint8_t* ctr = static_cast<uint8_t*>(const_cast<void*>(packed_b)) + wl.counters;
   args.next_item = reinterpret_cast<int32_t*>(ctr);
-  {
-    // the next-item counter and the split panels' counters start at zero
-    // in every launch
-    cudaError_t e = cudaMemsetAsync(ctr, 0, wl.counter_bytes, static_cast<cudaStream_t>(stream_));
-    if (e != cudaSuccess) return cuda_fail(e, "clearing the work counters");
+  if (!behind_pack) {
+    // the next-unit counter starts at zero in every launch (packing B sets it
+    // to zero for the launch right behind)
+    cudaError_t e = cudaMemsetAsync(ctr, 0, 16, static_cast<cudaStream_t>(stream_));
+    if (e != cudaSuccess) return cuda_fail(e, "clearing the work counter");
   }
   cudaError_t e = tc_launch(bh, R, nsub, kind, args, (int)std::min<int64_t>(sc.workers, std::max<int64_t>(units, 1)),
-                            static_cast<cudaStream_t>(stream_));
+                            behind_pack, static_cast<cudaStream_t>(stream_));
   if (e != cudaSuccess) return cuda_fail(e, "spmm kernel launch");
+  if (!whole && sc.n_split > 0) {
+    SumArgs sa;
+    std::memset(&sa, 0, sizeof(sa));
+    sa.one = args.one;
+    sa.splits = sc.d_splits;
+    sa.n_units = sc.n_split * args.one.n_tiles;
+    sa.bh = bh;
+    sa.R = R;
+    sa.nsub = nsub;
+    sa.nops = kind == TC_KIND_SPLIT ? 2 : 1;
+    e = tc_sum_parts(sa, static_cast<cudaStream_t>(stream_));
+    if (e != cudaSuccess) return cuda_fail(e, "split panel sums");
+  }
   if (uses_sp24(A, form)) {
     // the exact-2:4 blocks, added into the C the dense kernel wrote
     Sp24Args a24;
@@ -787,7 +800,8 @@ smat_status smat::spmm_impl(const smat_bcsr* A, int32_t form, const void* B, int
   if (ldc < N) return fail(SMAT_ERR_INVALID, "ldc < N");
   smat_status st = pack_impl(A, form, B, b_dtype, b_layout, ldb, N, workspace, workspace_bytes, stream, whole);
   if (st != SMAT_OK) return st;
-  return packed_impl(A, form, workspace, N, C, c_dtype, ldc, stream, whole);
+  // a matrix without columns has no B to pack, and nothing launched before
+  return packed_impl(A, form, workspace, N, C, c_dtype, ldc, stream, whole, A->host.cols > 0);
 }
 
 extern "C" {
@@ -800,7 +814,7 @@ smat_status smat_spmm_pack_b(const smat_bcsr* A, int32_t form, const void* B, in
 
 smat_status smat_spmm_packed(const smat_bcsr* A, int32_t form, const void* packed_b, int64_t N,
                              void* C, int32_t c_dtype, int64_t ldc, void* stream) {
-  return packed_impl(A, form, packed_b, N, C, c_dtype, ldc, stream, false);
+  return packed_impl(A, form, packed_b, N, C, c_dtype, ldc, stream, false, false);
 }
 
 smat_status smat_spmm(const smat_bcsr* A, int32_t form, const void* B, int32_t b_dtype,

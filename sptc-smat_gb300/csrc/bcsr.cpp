@@ -827,6 +827,14 @@ std::vector<WorkItem> device_items(const std::vector<const Plan*>& plans, const 
   return out;
 }
 
+std::vector<WorkItem> split_items(const std::vector<WorkItem>& items, const std::vector<int32_t>* n_tiles) {
+  std::vector<WorkItem> out;
+  for (WorkItem w : items)
+    if (w.split >= 0 && w.part == 0)
+      for (w.nt = 0; w.nt < (n_tiles ? (*n_tiles)[w.prob] : 1); w.nt++) out.push_back(w);
+  return out;
+}
+
 void order_items(const std::vector<double>& cost, std::vector<int32_t>& order) {
   order.resize(cost.size());
   std::iota(order.begin(), order.end(), 0);

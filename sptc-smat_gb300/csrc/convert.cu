@@ -29,6 +29,7 @@
 #include <cstdint>
 
 #include "convert.h"
+#include "tc_ptx.cuh"
 
 namespace smat {
 namespace dev {
@@ -197,16 +198,22 @@ __device__ __forceinline__ void pack_unit(const T* __restrict__ in, int layout, 
 template <typename T, int OUT>
 __global__ void __launch_bounds__(kPackThreads)
     pack_b_kernel(const T* __restrict__ in, int layout, int64_t ldi, uint8_t* __restrict__ out, int64_t K, int64_t N,
-                  const int32_t* __restrict__ kperm, uint8_t* __restrict__ flags) {
+                  const int32_t* __restrict__ kperm, uint8_t* __restrict__ flags, int32_t* __restrict__ counters) {
   extern __shared__ uint32_t tr[];
+  grid_release();  // the SpMM launched behind may be set up
+  if (counters && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kLaunchCounters) counters[threadIdx.x] = 0;
   pack_unit<T, OUT>(in, layout, ldi, out, K, N, blockIdx.x, blockIdx.y, kperm, flags, tr);
 }
 
 // Many B operands in one launch: block g packs unit g of the list of all
 // jobs' units (jobs sorted by their first unit).
 __global__ void __launch_bounds__(kPackThreads)
-    pack_b_grouped_kernel(const PackJob* __restrict__ jobs, int njobs, int64_t total) {
+    pack_b_grouped_kernel(const PackJob* __restrict__ jobs, int njobs, int64_t total, int32_t* __restrict__ counters,
+                          int n_counters) {
   extern __shared__ uint32_t tr[];
+  grid_release();
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < n_counters; i += kPackThreads) counters[i] = 0;
   for (int64_t g = blockIdx.x; g < total; g += gridDim.x) {
     int lo = 0, hi = njobs - 1;
     while (lo < hi) {
@@ -237,7 +244,7 @@ static size_t pack_smem(int layout, bool split) {
 
 template <typename T, int OUT>
 static cudaError_t run_pack(const void* in, int layout, int64_t ldi, uint8_t* out, int64_t K, int64_t N,
-                            const int32_t* kperm, uint8_t* flags, cudaStream_t s) {
+                            const int32_t* kperm, uint8_t* flags, int32_t* counters, cudaStream_t s) {
   const int64_t nkc = pack_units_k(K), halves = pack_halves(N);
   if (nkc == 0 || halves == 0) return cudaSuccess;
   // grid.y is limited to 65,535 halves: wider B goes in several launches
@@ -246,7 +253,7 @@ static cudaError_t run_pack(const void* in, int layout, int64_t ldi, uint8_t* ou
     const T* src = (const T*)in + (layout == 1 ? h0 * 64 * ldi : h0 * 64);
     uint8_t* dst = out + (h0 >> 1) * ((K + 15) / 16) * (OUT == OUT_SPLIT ? 8192 : 4096);
     pack_b_kernel<T, OUT><<<dim3((unsigned)nkc, (unsigned)hn), kPackThreads, pack_smem(layout, OUT == OUT_SPLIT), s>>>(
-        src, layout, ldi, dst, K, N - h0 * 64, kperm, flags + h0 * pack_flag_stride(K));
+        src, layout, ldi, dst, K, N - h0 * 64, kperm, flags + h0 * pack_flag_stride(K), counters);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -307,13 +314,13 @@ size_t packed_b_bytes(int64_t K, int64_t N) {
 size_t pack_flag_bytes(int64_t K, int64_t N) { return (size_t)pack_halves(N) * (size_t)pack_flag_stride(K); }
 
 cudaError_t pack_b(const void* in, int in_dtype, int layout, int64_t ldi, int out_mode, uint8_t* out,
-                   int64_t K, int64_t N, const int32_t* kperm, uint8_t* flags, cudaStream_t s) {
+                   int64_t K, int64_t N, const int32_t* kperm, uint8_t* flags, int32_t* counters, cudaStream_t s) {
   using namespace dev;
 #define SMAT_PACK(T)                                                                             \
   switch (out_mode) {                                                                            \
-    case OUT_F16: return run_pack<T, OUT_F16>(in, layout, ldi, out, K, N, kperm, flags, s);     \
-    case OUT_BF16: return run_pack<T, OUT_BF16>(in, layout, ldi, out, K, N, kperm, flags, s);   \
-    case OUT_SPLIT: return run_pack<T, OUT_SPLIT>(in, layout, ldi, out, K, N, kperm, flags, s); \
+    case OUT_F16: return run_pack<T, OUT_F16>(in, layout, ldi, out, K, N, kperm, flags, counters, s);     \
+    case OUT_BF16: return run_pack<T, OUT_BF16>(in, layout, ldi, out, K, N, kperm, flags, counters, s);   \
+    case OUT_SPLIT: return run_pack<T, OUT_SPLIT>(in, layout, ldi, out, K, N, kperm, flags, counters, s); \
     default: return cudaErrorInvalidValue;                                                       \
   }
   switch (in_dtype) {
@@ -326,12 +333,11 @@ cudaError_t pack_b(const void* in, int in_dtype, int layout, int64_t ldi, int ou
 }
 
 cudaError_t pack_b_grouped(const PackJob* d_jobs, int njobs, int64_t total_units, bool any_col, bool any_split,
-                           int num_sms, cudaStream_t s) {
-  if (njobs == 0 || total_units == 0) return cudaSuccess;
+                           int num_sms, int32_t* counters, int n_counters, cudaStream_t s) {
   const int64_t want = (int64_t)num_sms * 8;
-  const int grid = (int)(total_units < want ? total_units : want);
-  dev::pack_b_grouped_kernel<<<grid, dev::kPackThreads, dev::pack_smem(any_col ? 1 : 0, any_split), s>>>(d_jobs, njobs,
-                                                                                                     total_units);
+  const int grid = (int)(total_units < 1 ? 1 : (total_units < want ? total_units : want));
+  dev::pack_b_grouped_kernel<<<grid, dev::kPackThreads, dev::pack_smem(any_col ? 1 : 0, any_split), s>>>(
+      d_jobs, njobs, total_units, counters, n_counters);
   return cudaGetLastError();
 }
 

@@ -36,8 +36,11 @@ size_t pack_flag_bytes(int64_t K, int64_t N);
 // kperm (device, optional): row kperm[k] of `in` feeds packed row k (a
 // column permutation of A; gathered with scalar loads).
 // flags: pack_flag_bytes() bytes; the units' bytes are written.
+// counters (optional): kLaunchCounters integers set to zero, for the SpMM
+// launched behind.
+constexpr int kLaunchCounters = 4;
 cudaError_t pack_b(const void* in, int in_dtype, int layout, int64_t ldi, int out_mode, uint8_t* out,
-                   int64_t K, int64_t N, const int32_t* kperm, uint8_t* flags, cudaStream_t s);
+                   int64_t K, int64_t N, const int32_t* kperm, uint8_t* flags, int32_t* counters, cudaStream_t s);
 
 // The 2:4 path's copy of B: 8 KB tiles ordered [128-column tile][window],
 // window w = k-blocks 2w and 2w+1 (32 k-values; the second half zero past
@@ -60,7 +63,8 @@ struct PackJob {
 
 // Packs every job in one launch (jobs sorted by begin, in device memory).
 // any_col / any_split: whether a job is column-major / of the split form.
+// counters: n_counters integers set to zero, for the SpMMs launched behind.
 cudaError_t pack_b_grouped(const PackJob* d_jobs, int njobs, int64_t total_units, bool any_col, bool any_split,
-                           int num_sms, cudaStream_t s);
+                           int num_sms, int32_t* counters, int n_counters, cudaStream_t s);
 
 }  // namespace smat

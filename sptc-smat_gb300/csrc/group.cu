@@ -6,10 +6,10 @@
 // assignment to the CTAs, so that small and large problems share the GPU),
 // the per-problem descriptors the kernel reads, the packed-B / partial-sum
 // scratch and the jobs of the grouped B packing. smat_group_run then issues
-// one grouped B-packing launch, one memset of the split-panel counters and
-// one SpMM launch per kernel variant among the problems (one for a group of
-// FP16 / BF16 problems with N <= 128), and allocates nothing, so it can be
-// captured in a CUDA graph. The pointers B and C are fixed at creation.
+// one grouped B-packing launch, one SpMM launch per kernel variant among the
+// problems (one for a group of FP16 / BF16 problems with N <= 128) and one that
+// sums each variant's split panels, and allocates nothing, so it can be captured
+// in a CUDA graph. The pointers B and C are fixed at creation.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,7 +31,8 @@ struct Launch {
   ProblemDesc* d_probs = nullptr;
   WorkItem* d_items = nullptr;
   int32_t n_items = 0;
-  int32_t ctr = 0;  // int offset of the launch's next-item counter in d_counters
+  WorkItem* d_splits = nullptr;  // split panels x column tiles
+  int32_t n_splits = 0;
 };
 
 }  // namespace
@@ -40,8 +41,7 @@ struct smat_group {
   int device = 0;
   int num_sms = 0;
   uint8_t* d_ws = nullptr;       // packed B and partial sums of every problem
-  int32_t* d_counters = nullptr;  // split-panel counters of every problem
-  size_t counter_bytes = 0;
+  int32_t* d_counters = nullptr;  // each launch's next-unit counter, 16 bytes apart
   PackJob* d_jobs = nullptr;
   int njobs = 0;
   int64_t pack_blocks = 0;
@@ -58,6 +58,7 @@ static void group_free(smat_group* g) {
   for (Launch& l : g->launches) {
     cudaFree(l.d_probs);
     cudaFree(l.d_items);
+    cudaFree(l.d_splits);
   }
   cudaFree(g->d_ws);
   cudaFree(g->d_counters);
@@ -127,10 +128,10 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
 
   // work lists per variant; per problem its scratch sizes
   struct Scratch {
-    size_t packed = 0, slabs = 0, flags = 0, ws_off = 0, ctr_off = 0, ctr_n = 0;
+    size_t packed = 0, slabs = 0, flags = 0, ws_off = 0;
   };
   std::vector<Scratch> sc(count);
-  std::vector<std::vector<WorkItem>> v_items;
+  std::vector<std::vector<WorkItem>> v_items, v_splits;
   std::vector<std::vector<int32_t>> v_members;
   for (auto& kv : variants) {
     const auto& members = kv.second;
@@ -154,7 +155,6 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
       s.packed = kind == TC_KIND_SPLIT ? 2 * one : one;
       s.slabs = (size_t)n_slabs[m] * n_tiles * p.A->R * p.A->host.bh * bn * sizeof(float);
       s.flags = pack_flag_bytes(p.A->host.cols, p.N);
-      s.ctr_n = (size_t)n_split[m] * n_tiles * 4;
     }
     Launch l;
     l.bh = bh;
@@ -162,24 +162,21 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
     l.nsub = nsub;
     l.kind = kind;
     v_items.push_back(device_items(plans, items, order, &ntl));
+    v_splits.push_back(split_items(items, &ntl));
+    l.n_splits = (int32_t)v_splits.back().size();
     l.n_items = (int32_t)v_items.back().size();
     l.grid = std::max(1, std::min<int>(workers, l.n_items));
     g->launches.push_back(l);
     v_members.push_back(members);
   }
-  // one scratch allocation for all problems, one for all counters: each
-  // launch's next-item counter (16 bytes apart), then the split panels'
-  size_t ws_total = 0, ctr_total = 4 * g->launches.size();
-  for (size_t v = 0; v < g->launches.size(); v++) g->launches[v].ctr = (int32_t)(4 * v);
+  // one scratch allocation for all problems
+  size_t ws_total = 0;
   for (Scratch& s : sc) {
     s.ws_off = ws_total;
     ws_total += (s.packed + s.slabs + s.flags + 255) / 256 * 256;
-    s.ctr_off = ctr_total;
-    ctr_total += s.ctr_n;
   }
   GTRY(cudaMalloc(reinterpret_cast<void**>(&g->d_ws), std::max<size_t>(ws_total, 256)));
-  g->counter_bytes = ctr_total * sizeof(int32_t);
-  GTRY(cudaMalloc(reinterpret_cast<void**>(&g->d_counters), std::max<size_t>(g->counter_bytes, 256)));
+  GTRY(cudaMalloc(reinterpret_cast<void**>(&g->d_counters), std::max<size_t>(16 * g->launches.size(), 256)));
   GTRY(cudaMalloc(reinterpret_cast<void**>(&g->d_err), sizeof(int)));
   GTRY(cudaMemset(g->d_err, 0, sizeof(int)));
   // descriptors and pack jobs
@@ -216,10 +213,10 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
       fill_problem(p.A, p.form, g->d_ws + sc[i].ws_off, p.N, p.C, p.c_dtype, p.ldc, l.nsub, wl, descs[m]);
       descs[m].bflags = g->d_ws + sc[i].ws_off + sc[i].packed + sc[i].slabs;
       descs[m].slabs = reinterpret_cast<float*>(g->d_ws + sc[i].ws_off + sc[i].packed);
-      descs[m].counters = g->d_counters + sc[i].ctr_off;
     }
     GTRY(upload_vec(&l.d_probs, descs));
     GTRY(upload_vec(&l.d_items, v_items[v]));
+    GTRY(upload_vec(&l.d_splits, v_splits[v]));
   }
 #undef GTRY
   *out = g;
@@ -233,23 +230,34 @@ smat_status smat_group_run(smat_group* g, void* stream_) {
   if (prev != g->device && cudaSetDevice(g->device) != cudaSuccess) return fail(SMAT_ERR_CUDA, "cudaSetDevice failed");
   const cudaStream_t s = static_cast<cudaStream_t>(stream_);
   smat_status st = SMAT_OK;
-  cudaError_t e = pack_b_grouped(g->d_jobs, g->njobs, g->pack_blocks, g->pack_col, g->pack_split, g->num_sms, s);
+  cudaError_t e = pack_b_grouped(g->d_jobs, g->njobs, g->pack_blocks, g->pack_col, g->pack_split, g->num_sms,
+                                 g->d_counters, (int)(4 * g->launches.size()), s);
   if (e != cudaSuccess) st = fail(SMAT_ERR_CUDA, std::string("grouped B packing: ") + cudaGetErrorString(e));
-  if (st == SMAT_OK && g->counter_bytes) {
-    e = cudaMemsetAsync(g->d_counters, 0, g->counter_bytes, s);
-    if (e != cudaSuccess) st = fail(SMAT_ERR_CUDA, "clearing the split-panel counters");
-  }
   for (size_t v = 0; v < g->launches.size() && st == SMAT_OK; v++) {
     const Launch& l = g->launches[v];
     SpmmArgs args;
     std::memset(&args, 0, sizeof(args));
     args.probs = l.d_probs;
     args.n_items = l.n_items;
-    args.next_item = g->d_counters + l.ctr;
+    args.next_item = g->d_counters + 4 * v;
     args.items = l.d_items;
     args.err = g->d_err;
-    e = tc_launch(l.bh, l.R, l.nsub, l.kind, args, l.grid, s);
+    e = tc_launch(l.bh, l.R, l.nsub, l.kind, args, l.grid, true, s);
     if (e != cudaSuccess) st = fail(SMAT_ERR_CUDA, std::string("grouped spmm launch: ") + cudaGetErrorString(e));
+  }
+  for (size_t v = 0; v < g->launches.size() && st == SMAT_OK; v++) {
+    const Launch& l = g->launches[v];
+    SumArgs sa;
+    std::memset(&sa, 0, sizeof(sa));
+    sa.probs = l.d_probs;
+    sa.splits = l.d_splits;
+    sa.n_units = l.n_splits;
+    sa.bh = l.bh;
+    sa.R = l.R;
+    sa.nsub = l.nsub;
+    sa.nops = l.kind == TC_KIND_SPLIT ? 2 : 1;
+    e = tc_sum_parts(sa, s);
+    if (e != cudaSuccess) st = fail(SMAT_ERR_CUDA, std::string("grouped split panel sums: ") + cudaGetErrorString(e));
   }
   if (prev >= 0 && prev != g->device) cudaSetDevice(prev);
   return st;

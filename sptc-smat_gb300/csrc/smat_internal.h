@@ -180,6 +180,7 @@ struct Sched {
   WorkItem* d_items = nullptr;  // by decreasing estimated cost, absolute stage ranges
   WorkItem* d_whole = nullptr;  // the same without split panels (null when there are none)
   int32_t n_whole = 0;
+  WorkItem* d_splits = nullptr;  // the split panels, an item each (n_split)
   int32_t n_split = 0;  // panels split into parts
   int32_t n_slabs = 0;  // parts of split panels
 };
@@ -266,12 +267,11 @@ int pick_nsub(const smat_bcsr* h, int64_t N, int kind);
 
 // Workspace layout of one SpMM: [packed B (x2 for the split form)]
 // [the 2:4 path's copy of B, when the handle uses it for this form]
-// [the launch's next-item counter, 16 bytes]
-// [per split panel, column tile and TMEM lane quadrant: an int counter]
+// [the launch's next-unit counter, 256 bytes]
 // [per part of a split panel and column tile: an R*bh x BN FP32 slab]
 // [a byte per packing unit of B: it holds infinite or NaN values].
 struct WsLayout {
-  size_t counters = 0, counter_bytes = 0, slabs = 0, flags = 0, total = 0;
+  size_t counters = 0, slabs = 0, flags = 0, total = 0;
   size_t b64 = 0;  // the 2:4 path's copy of B (0: none)
 };
 WsLayout ws_layout(const smat_bcsr* A, int32_t form, int64_t N, bool whole = false);
@@ -329,6 +329,10 @@ void tune_store(const TuneKey& key, const TuneVal& val);
 // n_tiles (grouped launches): column tiles per problem, each a unit of its own.
 std::vector<WorkItem> device_items(const std::vector<const Plan*>& plans, const std::vector<WorkItem>& items,
                                    const std::vector<int32_t>& order, const std::vector<int32_t>* n_tiles = nullptr);
+
+// One item per split panel (its first part's), and column tile when n_tiles is
+// given: what sum_parts goes over.
+std::vector<WorkItem> split_items(const std::vector<WorkItem>& items, const std::vector<int32_t>* n_tiles = nullptr);
 
 // Item indices by decreasing cost (ties by index).
 void order_items(const std::vector<double>& item_cost, std::vector<int32_t>& order);

@@ -24,10 +24,9 @@
 //
 // Every call on a device shares the one array and leaves its contents
 // behind. The packed B is rewritten by the pack kernel wherever the contraction
-// uses it; the only part that must start at zero, the split-panel counters, is
-// cleared on the call's stream before each contraction. Calls that overlap in time — on
-// different streams, or from different threads — race on the array and
-// corrupt each other's results.
+// uses it, and so is the one counter that must start at zero. Calls that
+// overlap in time — on different streams, or from different threads — race on
+// the array and corrupt each other's results.
 #include <cuda.h>
 #include <cuda_runtime.h>
 

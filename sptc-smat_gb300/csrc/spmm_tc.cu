@@ -417,6 +417,8 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_release();  // the kernel that sums split panels may be set up
+  grid_wait();     // B is packed, the next-unit counter is zero, C is free
 
   int* err = args.err;
   const uint32_t smem0 = smem_u32(smem);
@@ -836,8 +838,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       }
       tc_fence_after();
       // slab of (part, column tile): (first slab of the panel + part) * n_tiles + nt
-      float* const slab0 = split ? P.slabs + ((size_t)wi.slab * n_tiles + nt) * SLAB : nullptr;
-      float* const slab = split ? slab0 + (size_t)wi.part * n_tiles * SLAB : nullptr;
+      float* const slab = split ? P.slabs + ((size_t)(wi.slab + wi.part) * n_tiles + nt) * SLAB : nullptr;
 #pragma unroll 1
       for (int j = 0; j < NSUB; ++j) {
         const int nl = j * 128 + (int)q * 32 + lane;  // column inside the tile
@@ -881,6 +882,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
               }
             }
             if (split) {
+              if (((slot_mask >> sl) & 1u) == 0) continue;  // taken as zeros
               float* const dst = slab + (size_t)(r0 + g) * C::BN + nl;
 #pragma unroll
               for (int m = 0; m < 16; ++m) __stcg(dst + (size_t)m * C::BN, w[m]);
@@ -906,68 +908,6 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&accempty[buf]));
-      if (!split) continue;
-      // this warp's part of the slab is written: count it; the warp that
-      // brings the count of its quadrant to nparts adds up all parts
-      __threadfence();
-      __syncwarp();
-      int last = 0;
-      if (lane == 0) {
-        int* ctr = P.counters + ((size_t)wi.split * n_tiles + nt) * 4 + q;
-        last = atomicAdd(ctr, 1) == wi.nparts - 1;
-      }
-      last = __shfl_sync(0xffffffffu, last, 0);
-      if (!last) continue;
-      __threadfence();
-#pragma unroll 1
-      for (int j = 0; j < NSUB; ++j) {
-        const int nl = j * 128 + (int)q * 32 + lane;
-        const int n = nt * C::BN + nl;
-#pragma unroll 1
-        for (int r0 = 0; r0 < R * BH; r0 += 16) {
-          const int sl = r0 / BH;
-          if ((ext_mask >> sl) & 1u) continue;  // added into its first part's slab rows
-          // 16 rows of two parts at a time: their loads are independent and
-          // overlap instead of paying one L2 round trip each
-          float acc[16];
-#pragma unroll
-          for (int m = 0; m < 16; ++m) acc[m] = 0.0f;
-          const float* src = slab0 + (size_t)r0 * C::BN + nl;
-          const size_t step = (size_t)n_tiles * SLAB;
-          int p = 0;
-#pragma unroll 1
-          for (; p + 2 <= wi.nparts; p += 2, src += 2 * step) {
-            float t[32];
-#pragma unroll
-            for (int m = 0; m < 16; ++m) {
-              t[m] = __ldcg(src + (size_t)m * C::BN);
-              t[16 + m] = __ldcg(src + step + (size_t)m * C::BN);
-            }
-#pragma unroll
-            for (int m = 0; m < 16; ++m) acc[m] = (acc[m] + t[m]) + t[16 + m];
-          }
-          if (p < wi.nparts) {
-            float t[16];
-#pragma unroll
-            for (int m = 0; m < 16; ++m) t[m] = __ldcg(src + (size_t)m * C::BN);
-#pragma unroll
-            for (int m = 0; m < 16; ++m) acc[m] += t[m];
-          }
-          if (odd) {
-            const int q0 = p_pois[panel * R + sl], q1 = p_pois[panel * R + sl + 1];
-            if (q0 < q1 && n < p_N && poisoned(P, C::NOPS, q0, q1, n)) {
-#pragma unroll
-              for (int m = 0; m < 16; ++m) acc[m] = __int_as_float(0x7fffffff);
-            }
-          }
-          const bool fl = (full >> (r0 / 16)) & 1u;
-          uint8_t* const col = static_cast<uint8_t*>(p_C) + (int64_t)n * elt;
-          if (n < p_N) {
-            if (p_f16) store_rows16<__half>(col, ldb, rows + r0, fl, acc);
-            else store_rows16<float>(col, ldb, rows + r0, fl, acc);
-          }
-        }
-      }
     }
   }
 
@@ -979,6 +919,80 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, C::TMEM_COLS);
+  }
+}
+
+// C of the split panels: block (unit, 16 plan rows) adds the parts' slab rows
+// in part order, a thread per column. What bounds it: latency of its one or
+// two rounds of loads; the slabs (96 parts of 128 KB at most per problem and
+// column tile) are in L2. Adding them at the end of the SpMM kernel, by the
+// part that came last, took 15-20 us of one SM's time on the R-MAT workload
+// and on 24 grouped matrices while the other SMs were done.
+__global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ SumArgs a) {
+  grid_wait();
+  const int u = (int)blockIdx.x, r0 = (int)blockIdx.y * 16;
+  WorkItem w;
+  if (a.probs) {
+    w = a.splits[u];
+  } else {
+    w = a.splits[u / a.one.n_tiles];
+    w.nt = u % a.one.n_tiles;
+  }
+  const ProblemDesc& P = a.probs ? a.probs[w.prob] : a.one;
+  const int sl = r0 / a.bh, bn = 128 * a.nsub;
+  const uint32_t slot_mask = P.panels[w.panel].slot_mask, ext_mask = P.panels[w.panel].ext_mask;
+  if ((ext_mask >> sl) & 1u) return;  // added into its first part's rows
+  const int n = w.nt * bn + (int)threadIdx.x;
+  float acc[16];
+#pragma unroll
+  for (int m = 0; m < 16; ++m) acc[m] = 0.0f;
+  if ((slot_mask >> sl) & 1u) {
+    const size_t step = (size_t)P.n_tiles * (a.R * a.bh * bn);
+    const float* src = P.slabs + ((size_t)w.slab * P.n_tiles + w.nt) * (a.R * a.bh * bn) + (size_t)r0 * bn + threadIdx.x;
+    int p = 0;
+    for (; p + 2 <= w.nparts; p += 2, src += 2 * step) {
+      float t[32];
+#pragma unroll
+      for (int m = 0; m < 16; ++m) {
+        t[m] = __ldcg(src + (size_t)m * bn);
+        t[16 + m] = __ldcg(src + step + (size_t)m * bn);
+      }
+#pragma unroll
+      for (int m = 0; m < 16; ++m) acc[m] = (acc[m] + t[m]) + t[16 + m];
+    }
+    if (p < w.nparts) {
+#pragma unroll
+      for (int m = 0; m < 16; ++m) acc[m] += __ldcg(src + (size_t)m * bn);
+    }
+  }
+  if (P.poison_ptr != nullptr) {
+    const int q0 = P.poison_ptr[w.panel * a.R + sl], q1 = P.poison_ptr[w.panel * a.R + sl + 1];
+    if (q0 < q1) {
+      const int64_t fs = pack_flag_stride(P.K);
+      const int h0 = w.nt * (2 * a.nsub), h1 = min(h0 + 2 * a.nsub, (P.N + 63) >> 6);
+      const uint4* fl = reinterpret_cast<const uint4*>(P.bflags + (int64_t)h0 * fs);
+      uint32_t any = 0;
+      for (int64_t x = threadIdx.x; x < (h1 - h0) * fs / 16; x += blockDim.x) {
+        const uint4 f = __ldcg(fl + x);
+        any |= f.x | f.y | f.z | f.w;
+      }
+      if (__syncthreads_or((int)any) && n < P.N && poisoned(P, a.nops, q0, q1, n)) {
+#pragma unroll
+        for (int m = 0; m < 16; ++m) acc[m] = __int_as_float(0x7fffffff);
+      }
+    }
+  }
+  if (n >= P.N) return;
+  const int32_t* rows = P.row_map + (int64_t)w.panel * a.R * a.bh + r0;
+#pragma unroll
+  for (int m = 0; m < 16; ++m) {
+    const int row = __ldg(rows + m);
+    if (row < 0) continue;
+    const int64_t off = (int64_t)row * P.ldc + n;
+    if (P.c_f16)
+      __stcs(reinterpret_cast<__half*>(P.C) + off, __float2half_rn(acc[m]));
+    else
+      __stcs(reinterpret_cast<float*>(P.C) + off, acc[m]);
   }
 }
 
@@ -1003,13 +1017,14 @@ static cudaError_t prepare_one() {
 }
 
 template <int BH, int R, int NSUB, int KIND>
-static cudaError_t launch_one(const SpmmArgs& args, int grid, cudaStream_t stream) {
+static cudaError_t launch_one(const SpmmArgs& args, int grid, bool behind, cudaStream_t stream) {
   using C = Cfg<BH, R, NSUB, KIND>;
   auto kfn = spmm_tc_kernel<BH, R, NSUB, KIND>;
   cudaError_t e = prepare_one<BH, R, NSUB, KIND>();
   if (e != cudaSuccess) return e;
-  kfn<<<grid, C::THREADS, C::SMEM_BYTES, stream>>>(args);
-  return cudaGetLastError();
+  void* params[] = {const_cast<SpmmArgs*>(&args)};
+  return launch_kernel(reinterpret_cast<const void*>(kfn), dim3((unsigned)grid), dim3(C::THREADS), C::SMEM_BYTES, stream,
+                       behind, params);
 }
 
 // Co-resident CTAs per SM: limited by TMEM (512 columns per SM) and by what
@@ -1030,6 +1045,31 @@ static int ctas_per_sm_one() {
 }
 
 }  // namespace dev
+
+cudaError_t launch_kernel(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool behind,
+                          void** args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = behind ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
+  const cudaError_t last = cudaGetLastError();  // do not leave the error for the next call to find
+  return e != cudaSuccess ? e : last;
+}
+
+cudaError_t tc_sum_parts(const SumArgs& args, cudaStream_t stream) {
+  if (args.n_units == 0) return cudaSuccess;
+  void* params[] = {const_cast<SumArgs*>(&args)};
+  return launch_kernel(reinterpret_cast<const void*>(dev::sum_parts_kernel),
+                       dim3((unsigned)args.n_units, (unsigned)(args.R * args.bh / 16)), dim3((unsigned)(128 * args.nsub)), 0,
+                       stream, true, params);
+}
 
 #define SMAT_TC_VARIANTS(X) \
   X(16, 4, 1, 0)            \
@@ -1064,11 +1104,11 @@ int tc_ctas_per_sm(int bh, int R, int nsub, int kind) {
   return 1;
 }
 
-cudaError_t tc_launch(int bh, int R, int nsub, int kind, const SpmmArgs& args, int grid,
+cudaError_t tc_launch(int bh, int R, int nsub, int kind, const SpmmArgs& args, int grid, bool behind,
                       cudaStream_t stream) {
 #define SMAT_TC_LAUNCH(BH, R_, NS, K)                             \
   if (bh == BH && R == R_ && nsub == NS && kind == K) \
-    return dev::launch_one<BH, R_, NS, K>(args, grid, stream);
+    return dev::launch_one<BH, R_, NS, K>(args, grid, behind, stream);
   SMAT_TC_VARIANTS(SMAT_TC_LAUNCH)
 #undef SMAT_TC_LAUNCH
   return cudaErrorInvalidValue;

@@ -91,9 +91,8 @@ __host__ __device__ constexpr int stage_hdr_max(int sb) { return kStageHdrFixed 
 
 // A unit of work of one CTA: stages [s0, s1) of a panel. A panel whose
 // stages are split over several items ("parts", for load balance) has a
-// split index: its parts write partial sums to workspace slabs, and the part
-// that finishes last (an atomic counter per split panel and column tile)
-// adds the slabs and writes C.
+// split index: its parts write partial sums to workspace slabs, and a second
+// kernel (tc_sum_parts) adds the slabs and writes C.
 static_assert(sizeof(StageRec) == 96, "the kernel reads 16-byte pieces");
 
 struct alignas(16) WorkItem {
@@ -123,7 +122,6 @@ struct ProblemDesc {
   void* C;
   int64_t ldc;
   float* slabs;              // partial sums of split panels: [slab][R * bh rows][BN] FP32
-  int32_t* counters;         // [split panels][column tiles][4], zero before the launch
   int32_t N;
   int32_t n_tiles;
   int32_t c_f16;
@@ -165,7 +163,27 @@ struct SpmmArgs {
 enum : int { TC_KIND_PLAIN = 0, TC_KIND_SPLIT = 1, TC_KIND_FP8 = 2 };
 bool tc_variant_supported(int bh, int R, int nsub, int kind);
 int tc_ctas_per_sm(int bh, int R, int nsub, int kind);
-cudaError_t tc_launch(int bh, int R, int nsub, int kind, const SpmmArgs& args, int grid,
+// `behind`: launched right behind the kernel before it in the stream, which is
+// one of this library's; its set-up then overlaps that kernel's end.
+cudaError_t tc_launch(int bh, int R, int nsub, int kind, const SpmmArgs& args, int grid, bool behind,
                       cudaStream_t stream);
+
+// C of the split panels from their parts' slabs. splits: one item per split
+// panel (panel, nparts, slab, prob), and per column tile in a grouped launch;
+// n_units of them, counted as in SpmmArgs. Launched behind the kernel that
+// wrote the slabs.
+struct SumArgs {
+  ProblemDesc one;
+  const ProblemDesc* probs;
+  const WorkItem* splits;
+  int32_t n_units;
+  int32_t bh, R, nsub, nops;
+};
+cudaError_t tc_sum_parts(const SumArgs& args, cudaStream_t stream);
+
+// Launches kernel `fn` behind the one before it in the stream (programmatic
+// dependent launch) or after it.
+cudaError_t launch_kernel(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool behind,
+                          void** args);
 
 }  // namespace smat

@@ -176,6 +176,12 @@ __device__ __forceinline__ __half2 e4m3x2_to_half2(uint16_t v) {
   return *reinterpret_cast<__half2*>(&r);
 }
 
+// Programmatic dependent launch: wait until the kernels this one was launched
+// behind are complete and their writes visible (nothing to wait for in an
+// ordinary launch); let the kernel launched behind this one begin its set-up.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- tcgen05
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem),
