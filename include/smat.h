@@ -83,7 +83,8 @@ typedef struct smat_bcsr_opts {
   int32_t device;         /* CUDA device ordinal */
   int32_t panel_rows;     /* block rows per tensor-core panel: 4, 8 or 16 for bh 16, 4 or 8
                              for bh 32; 0 = the autotuner's cached choice for matrices
-                             like this one, else 256 rows (16, or 8 for bh 32) */
+                             like this one, else 256 rows (16, or 8 for bh 32) where that
+                             makes four panels per SM, 128 rows otherwise */
   float split_frac;       /* a panel costing more than split_frac x the average per-CTA
                              work is split into parts over several CTAs (0 = default 0.5,
                              < 0 = never split) */

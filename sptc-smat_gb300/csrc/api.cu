@@ -115,7 +115,7 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
   const uint32_t forms = h->forms;
   smat_status st;
   // heavy panels are split over CTAs below
-  int R = o.panel_rows ? o.panel_rows : default_panel_rows(bh);
+  int R = o.panel_rows ? o.panel_rows : default_panel_rows(bh, h->host.nbr(), h->num_sms);
   float split_frac = o.split_frac;
   int ntc = o.n_tile_cols, depth = o.pipeline_depth;
   if (o.panel_rows == 0) {

@@ -258,10 +258,20 @@ inline int plan_class_of_kind(int kind, int nsub = 1) {
   return kind == TC_KIND_SPLIT ? 1 : (kind == TC_KIND_FP8 ? 2 : (nsub == 2 ? 3 : 0));
 }
 // Block rows per panel when the caller leaves it to the library: 256 rows
-// (16 blocks of 16 rows, 8 of 32), two TMEM accumulator buffers of 256
-// columns; panels costing more than kDefaultSplitFrac of the average CTA
-// load are split into parts.
-inline int default_panel_rows(int bh) { return bh == 16 ? 16 : 8; }
+// (16 blocks of 16 rows, 8 of 32: two TMEM accumulator buffers of 256 columns)
+// where that makes at least four panels per SM, else 128. Tall panels share
+// more tiles of B, short ones balance better and have half the rows to drain
+// at the end (256 against 128 rows, GB300: 64^3 stencil, 6.7 tall panels per
+// SM, 184 against 192 us; R-MAT 2^16, 1.7, 112 against 113; split stencil, 2.5,
+// 79 against 74; plain graph 2^15, 0.8, 64 against 60; 24 grouped matrices 53
+// against 47; a ragged block matrix, 0.1, 31 against 24). Panels costing more
+// than kDefaultSplitFrac of the average CTA load are split into parts; finer
+// parts cost more than they balance (304 slabs in place of 96: R-MAT 126 us,
+// the graph 83).
+inline int default_panel_rows(int bh, int64_t nbr, int num_sms) {
+  const bool tall = nbr * bh >= (int64_t)1024 * num_sms;
+  return (tall ? 256 : 128) / bh;
+}
 constexpr double kDefaultSplitFrac = 0.5;
 int pick_nsub(const smat_bcsr* h, int64_t N, int kind);
 

@@ -102,6 +102,8 @@ smat_status smat_autotune(const smat_csr* A, const smat_bcsr_opts* opts, int32_t
   int prev = -1;
   cudaGetDevice(&prev);
   if (cudaSetDevice(o.device) != cudaSuccess) return fail(SMAT_ERR_CUDA, "cudaSetDevice failed");
+  int num_sms = 1;
+  cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, o.device);
   // operands: FP32 B (every form packs from it), FP32 C, the largest workspace
   const int64_t K = hb.cols, M = hb.rows;
   void *dB = nullptr, *dC = nullptr, *dW = nullptr;
@@ -175,7 +177,7 @@ smat_status smat_autotune(const smat_csr* A, const smat_bcsr_opts* opts, int32_t
           ok = false;
           break;
         }
-        if (R == default_panel_rows(bh) && f == (float)kDefaultSplitFrac && ntc == 128) ms_default = t;
+        if (R == default_panel_rows(bh, hb.nbr(), num_sms) && f == (float)kDefaultSplitFrac && ntc == 128) ms_default = t;
         consider(t, R, f, ntc, 0);
       }
     }
