@@ -206,7 +206,10 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
     SMAT_TRY(upload(&pd.d_stages, pd.plan.stages.data(), pd.plan.stages.size()));
     SMAT_TRY(upload(&pd.d_panels, pd.plan.panels.data(), pd.plan.panels.size()));
     SMAT_TRY(upload(&pd.d_row_map, pd.plan.row_map.data(), pd.plan.row_map.size()));
-    if (!pd.plan.gcol.empty()) SMAT_TRY(upload(&pd.d_gcol, pd.plan.gcol.data(), pd.plan.gcol.size()));
+    if (!pd.plan.gcol.empty()) {
+      const std::vector<int32_t> list = gather_list(pd.plan, cls == 1 ? 2 : 1);
+      SMAT_TRY(upload(&pd.d_gcol, list.data(), list.size()));
+    }
     if (!pd.plan.poison.empty()) {
       SMAT_TRY(upload(&pd.d_poison_ptr, pd.plan.poison_ptr.data(), pd.plan.poison_ptr.size()));
       SMAT_TRY(upload(&pd.d_poison, pd.plan.poison.data(), pd.plan.poison.size()));

@@ -353,6 +353,8 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
   std::vector<uint32_t> ext_masks;
   const int32_t per_warp = R / kMmaWarps;
   const bool can_cut = R % kMmaWarps == 0;
+  // (rows of B are counted in 128-byte rows of the packed tile, see gather_list)
+  if (gather && b.cols_p > ((int64_t)1 << 31) / 4) gather = false;
   if (gather && (b.bw != 16 || (int64_t)b.colmask.size() != b.nnzb())) gather = false;
   // a block row's weight is its number of MMAs: its blocks, or (gather) about
   // a sixteenth of an MMA per nonzero column of its sparse blocks
@@ -719,6 +721,17 @@ smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan, co
     plan.gcol[q] = s < 0 ? -1 : b.colidx[s / 16] + (int32_t)(s % 16);
   }
   return SMAT_OK;
+}
+
+std::vector<int32_t> gather_list(const Plan& pl, int nops) {
+  std::vector<int32_t> out(pl.gcol.size());
+#pragma omp parallel for schedule(static)
+  for (size_t g = 0; g < pl.gcol.size() / 16; g++)
+    for (int x = 0; x < 16; x++) {
+      const int32_t k = pl.gcol[g * 16 + (x & 3) * 4 + (x >> 2)];
+      out[g * 16 + x] = k < 0 ? -1 : (k >> 4) * (32 * nops) + (k & 15);
+    }
+  return out;
 }
 
 void build_work_items_multi(const std::vector<const Plan*>& plans, const std::vector<int32_t>& bhs, int32_t workers,

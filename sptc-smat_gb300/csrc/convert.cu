@@ -19,7 +19,9 @@
 // byte of `flags`, whether any packed value is infinite or NaN: the SpMM then
 // restores what a block's stored zeros make of such a value (spmm_tc.cu).
 //
-// What bounds it: DRAM and L2 traffic of a copy. Row-major B needs no
+// What bounds it: DRAM and L2 traffic of a copy (268 MB of FP32 in and 134 MB out
+// in 62 us, 6.5 TB/s of the 6.7 a copy reaches; six blocks an SM, 64^3 stencil
+// 183 -> 180 us against four). Row-major B needs no
 // transposition in this layout (a thread moves eight neighbouring columns);
 // column-major B goes through shared memory, 128 x 64 values at a time.
 #include <cuda_bf16.h>
@@ -196,7 +198,7 @@ __device__ __forceinline__ void pack_unit(const T* __restrict__ in, int layout, 
 }
 
 template <typename T, int OUT>
-__global__ void __launch_bounds__(kPackThreads)
+__global__ void __launch_bounds__(kPackThreads, 6)
     pack_b_kernel(const T* __restrict__ in, int layout, int64_t ldi, uint8_t* __restrict__ out, int64_t K, int64_t N,
                   const int32_t* __restrict__ kperm, uint8_t* __restrict__ flags, int32_t* __restrict__ counters) {
   extern __shared__ uint32_t tr[];
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(kPackThreads)
 
 // Many B operands in one launch: block g packs unit g of the list of all
 // jobs' units (jobs sorted by their first unit).
-__global__ void __launch_bounds__(kPackThreads)
+__global__ void __launch_bounds__(kPackThreads, 6)
     pack_b_grouped_kernel(const PackJob* __restrict__ jobs, int njobs, int64_t total, int32_t* __restrict__ counters,
                           int n_counters) {
   extern __shared__ uint32_t tr[];

@@ -135,6 +135,12 @@ struct Plan {
 smat_status build_plan(const HostBcsr& b, int32_t R, int32_t cls, Plan& plan,
                        const std::vector<uint8_t>* skip = nullptr, bool gather = false);
 
+// The device's copy of Plan::gcol for a form with nops operands: columns 4 rr +
+// q of a block at place 4 q + rr, and instead of row k of B its place in the
+// packed column tile, in 128-byte rows (the copy warps then neither shuffle nor
+// divide).
+std::vector<int32_t> gather_list(const Plan& pl, int nops);
+
 // ------------------------------------------------------------------ 2:4 path
 // The structured-sparse path's units, stages and groups (spmm24.h) and the
 // compressed stream, for the blocks with take[k] != 0 (16 x 16 blocks, all

@@ -322,27 +322,30 @@ __device__ __forceinline__ void load_rows(StageView& v, const int32_t* gcol, int
   if (t < v.ngath) v.rows0 = __ldg(reinterpret_cast<const int4*>(gcol + ((int64_t)v.g0 + t) * 16) + (lane & 3));
 }
 
-// A gathered tile: row r of the tile from row k = list[r] of B (zeros for -1).
-// A lane moves 16-byte chunks: 8 lanes bring the 128 bytes of 64 columns of a
-// row, undoing the swizzle of row k & 7 in the packed B and applying that of
-// row r & 7.
+// A gathered tile: row r of the tile from B's row at list[...] (its place in
+// the packed column tile, in 128-byte rows; -1: zeros). A lane moves 16-byte
+// chunks: 8 lanes bring the 128 bytes of 64 columns of a row, undoing the
+// swizzle of the source row (its low three bits) and applying that of row r &
+// 7. The list holds the four rows of a lane side by side (rows q, q + 4, q + 8,
+// q + 12 for lanes 8 q .. 8 q + 7), so one load brings them.
 template <int NOPS>
 __device__ __forceinline__ void gather_tile(uint32_t dst, const uint8_t* b, const int* list, int nh, int lane) {
-  const int c = lane & 7;
+  const int c = lane & 7, q = lane >> 3;
+  const int4 k4 = reinterpret_cast<const int4*>(list)[q];
+  const int k[4] = {k4.x, k4.y, k4.z, k4.w};
 #pragma unroll
   for (int rr = 0; rr < 4; ++rr) {
-    const int r = rr * 4 + (lane >> 3);
-    const int k = list[r];
-    const int kk = k < 0 ? 0 : k;
-    const uint8_t* src = b + (int64_t)(kk >> 4) * (4096 * NOPS) + (kk & 15) * 128 + ((c ^ (kk & 7)) << 4);
-    const uint32_t d = dst + r * 128 + ((c ^ (r & 7)) << 4);
+    const uint32_t n = k[rr] < 0 ? 0u : 16u;
+    const int kk = max(k[rr], 0);
+    const uint8_t* src = b + (int64_t)kk * 128 + ((c ^ (kk & 7)) << 4);
+    // row r = 4 rr + q: its swizzle is 4 (rr & 1) + q
+    const uint32_t d = dst + (rr * 4 + q) * 128 + ((c ^ ((rr & 1) * 4 + q)) << 4);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (h < nh) {
+    for (int o = 0; o < NOPS; ++o) cp_async16(d + o * 2048, src + o * 2048, n);
+    if (nh > 1) {
 #pragma unroll
-        for (int o = 0; o < NOPS; ++o)
-          cp_async16(d + h * (2048 * NOPS) + o * 2048, src + h * (2048 * NOPS) + o * 2048, k < 0 ? 0u : 16u);
-      }
+      for (int o = 0; o < NOPS; ++o)
+        cp_async16(d + 2048 * NOPS + o * 2048, src + 2048 * NOPS + o * 2048, n);
     }
   }
 }
@@ -662,7 +665,6 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
         if (wi.panel < 0) break;
         const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
         const uint32_t idesc0 = P.idesc;  // without the N field
-        const bool gathers = P.gcol != nullptr;
         const int nstages = wi.s1 - wi.s0;
         {
           const uint32_t buf = k & 1;
@@ -691,14 +693,15 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
               ok = false;
               break;
             }
-            if (gathers) fence_proxy_async_smem();  // gathered rows were written through the generic proxy
             const uint8_t* stp = smem + s * C::STAGE;
-            const uint2 hd = *reinterpret_cast<const uint2*>(stp);  // (first, count) of each warp
+            // (first, count) of each warp, block and tile counts, gathered blocks
+            const uint4 hd = *reinterpret_cast<const uint4*>(stp);
+            if (hd.w != 0) fence_proxy_async_smem();  // gathered rows were written through the generic proxy
             const uint32_t wl = ((warp & 2 ? hd.y : hd.x) >> (16 * (warp & 1))) & 0xffffu;
             const uint32_t first = wl & 0xffu, cnt = wl >> 8;
             const uint32_t* ent = reinterpret_cast<const uint32_t*>(stp + kStageHdrFixed) + first;
             // lo blocks follow the stage's nblk hi blocks (split form)
-            const uint32_t lo_off = KIND == KIND_SPLIT ? *reinterpret_cast<const uint16_t*>(stp + 8) * C::ABLK : 0;
+            const uint32_t lo_off = KIND == KIND_SPLIT ? (hd.z & 0xffffu) * C::ABLK : 0;
             // descriptors of operands inside the stage = stage descriptor + offset / 16
             const uint64_t sdesc = desc_kmajor_sw32(smem0 + s * C::STAGE + C::OFF_A);
             const uint64_t bdesc = desc_mnmajor_sw128(smem0 + s * C::STAGE + C::OFF_B, C::HALF);
