@@ -421,7 +421,11 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   grid_release();  // the kernel that sums split panels may be set up
-  grid_wait();     // B is packed, the next-unit counter is zero, C is free
+  // What the launch before this one makes (the packed B and its flags, the
+  // zero next-unit counter, a C nobody reads any more) is first used by the
+  // copy warps and the epilogue, which wait for it there; the plan and A's
+  // stream are the handle's own, so the first unit's lookups overlap the
+  // packing of B.
 
   int* err = args.err;
   const uint32_t smem0 = smem_u32(smem);
@@ -544,19 +548,12 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
         break;
       }
       if (wi.panel < 0) {
+        if (kk == 0) grid_wait();
         // the end, once more for the other set of epilogue warps
         if (pw == 0 && elect_one())
           put_unit(args, taken, itemfull, itemempty, item_ring, abort_flag, err, lim);
         __syncwarp();
         break;
-      }
-      // a short unit: take the next one now, so that its copies follow
-      // without a wait (a long one would be taken from a CTA that is free
-      // earlier)
-      if (pw == 0 && wi.s1 - wi.s0 <= kShortUnit) {
-        if (elect_one()) put_unit(args, taken, itemfull, itemempty, item_ring, abort_flag, err, lim);
-        __syncwarp();
-        ++taken;
       }
       const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
       // fields used after shared-memory stores, held in registers (the stores
@@ -584,6 +581,15 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       load_stage(cur, p_stages, i, nst, bt);
       load_stage(nxt, p_stages, i + (int)np, nst, bt);
       load_rows(cur, p_gcol, hf, lane);
+      if (kk == 0) grid_wait();
+      // a short unit: take the next one now, so that its copies follow
+      // without a wait (a long one would be taken from a CTA that is free
+      // earlier)
+      if (pw == 0 && wi.s1 - wi.s0 <= kShortUnit) {
+        if (elect_one()) put_unit(args, taken, itemfull, itemempty, item_ring, abort_flag, err, lim);
+        __syncwarp();
+        ++taken;
+      }
       for (; i < nst; i += (int)np) {
         const int na = cur.ntiles - cur.ngath, ng = (cur.ngath + 1 - hf) / 2;  // gathered tiles of this warp
         const int nb = (na + 1 - hf) / 2;                                     // and bulk ones
@@ -807,6 +813,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
         full |= ((there & 0xffffu) == 0xffffu ? 1u : 0u) << (x / 16);
         full |= ((there >> 16) == 0xffffu ? 1u : 0u) << (x / 16 + 1);
       }
+      if (kk == buf) grid_wait();  // the warp's first unit
       const int32_t* const p_pois = P.poison_ptr;
       // does the packed B of these columns hold infinite or NaN values?
       // (looked up once per problem and column tile)
