@@ -213,9 +213,24 @@ def csr_to_bcsr_split_host(csr: Csr, block_cols: int = 16, row_perm=None):
             grid[:nbr * nbc].reshape(nbr, nbc))
 
 
+_TORCH_DT = {}
+
+
 def _torch_dt(dt):
+    """The library's code of a torch dtype (KeyError where it has none)."""
+    if not _TORCH_DT:
+        import torch
+        _TORCH_DT.update({torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16})
+    return _TORCH_DT[dt]
+
+
+def _current_stream(device):
+    """The raw current stream of a torch device."""
     import torch
-    return {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}[dt]
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None or device.index is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return raw(device.index)
 
 
 def _torch_layout(t):
@@ -223,10 +238,11 @@ def _torch_layout(t):
     if t.dim() != 2:
         raise ValueError("B must be 2-D (K, N)")
     s0, s1 = t.stride()
-    if s0 == 1 and (s1 >= t.shape[0] or t.shape[1] == 1):
-        return COL_MAJOR, max(s1, t.shape[0])
+    rows, cols = t.shape
+    if s0 == 1 and (s1 >= rows or cols == 1):
+        return COL_MAJOR, max(s1, rows)
     if s1 == 1:
-        return ROW_MAJOR, max(s0, t.shape[1])
+        return ROW_MAJOR, max(s0, cols)
     raise ValueError("B must have a unit stride in one dimension")
 
 
@@ -257,6 +273,7 @@ class Bcsr:
         self._h = h
         self.device = device
         self.forms = tuple(forms)
+        self._ws_sizes = {}             # (form, b_dtype, N) -> workspace bytes: fixed for a handle
         inf = BcsrInfo()
         check(lib().smat_bcsr_get_info(self._h, C.byref(inf)))
         self.info = {k: getattr(inf, k) for k, _ in BcsrInfo._fields_}
@@ -298,9 +315,15 @@ class Bcsr:
         check(lib().smat_bcsr_debug_stall(self._h, int(stage)))
 
     def workspace_size(self, form: int, b_dtype: int, N: int) -> int:
-        n = C.c_size_t()
-        check(lib().smat_spmm_workspace_size(self._h, form, b_dtype, N, C.byref(n)))
-        return n.value
+        key = (form, b_dtype, N)
+        size = self._ws_sizes.get(key)
+        if size is None:
+            n = C.c_size_t()
+            check(lib().smat_spmm_workspace_size(self._h, form, b_dtype, N, C.byref(n)))
+            if len(self._ws_sizes) >= 256:
+                self._ws_sizes.clear()
+            size = self._ws_sizes[key] = n.value
+        return size
 
     def spmm_raw(self, form, B, b_dtype, b_layout, ldb, Cmat, c_dtype, ldc, N, workspace=None,
                  workspace_bytes=0, stream=0):
@@ -321,20 +344,31 @@ class Bcsr:
         """C = A @ B for a torch CUDA tensor B of shape (K, N); returns C (rows, N)."""
         import torch
         K, N = B.shape
-        if K != self.info["cols"]:
-            raise ValueError(f"B has {K} rows, A has {self.info['cols']} columns")
-        b_dtype = {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}[B.dtype]
+        info = self.info
+        if K != info["cols"]:
+            raise ValueError(f"B has {K} rows, A has {info['cols']} columns")
+        b_dtype = _torch_dt(B.dtype)
         layout, ldb = _torch_layout(B)
+        dev = B.device
         if out is None:
-            out = torch.empty((self.info["rows"], N), device=B.device,
-                              dtype=out_dtype if out_dtype is not None else torch.float32)
-        c_dtype = {torch.float32: F32, torch.float16: F16}[out.dtype]
-        ws_bytes = self.workspace_size(form, b_dtype, N)
-        if workspace is None and ws_bytes:
-            workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=B.device)
-        s = stream if stream is not None else torch.cuda.current_stream(B.device).cuda_stream
-        self.spmm_raw(form, B, b_dtype, layout, ldb, out, c_dtype, out.stride(0), N,
-                      workspace, 0 if workspace is None else workspace.numel(), s)
+            c_dt = out_dtype if out_dtype is not None else torch.float32
+            out = torch.empty((info["rows"], N), device=dev, dtype=c_dt)
+            ldc = max(N, 1)
+        else:
+            c_dt = out.dtype
+            ldc = out.stride(0)
+        c_dtype = _torch_dt(c_dt)
+        if c_dtype == BF16:
+            raise KeyError(c_dt)        # C is FP32 or FP16
+        if workspace is None:
+            ws_bytes = self.workspace_size(form, b_dtype, N)
+            if ws_bytes:
+                workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+        else:
+            ws_bytes = workspace.numel()
+        s = stream if stream is not None else _current_stream(dev)
+        check(lib().smat_spmm(self._h, form, B.data_ptr(), b_dtype, layout, ldb, out.data_ptr(), c_dtype, ldc, N,
+                              None if workspace is None else workspace.data_ptr(), ws_bytes, s))
         return out
 
     def spmm_host(self, B: np.ndarray, form: int = FORM_F16, out_dtype=np.float32, out=None,
