@@ -79,7 +79,7 @@ static void free_handle(smat_bcsr* h) {
   cudaGetDevice(&prev);
   cudaSetDevice(h->device);
   void* ptrs[] = {h->d_kperm, h->d_aval[0], h->d_aval[1], h->d_aval[2], h->d_aval[3], h->d_err,
-                  h->d_bstage, h->d_cstage, h->d_ws, h->d_sp24_stages, h->d_sp24_groups,
+                  h->d_bstage, h->d_cstage, h->d_ws, h->d_sp24_stages, h->d_sp24_groups, h->d_sp24_items, h->d_sp24_split,
                   h->d_sp24_unit_window, h->d_sp24_stream[0], h->d_sp24_stream[1], h->d_bcsr_row_map,
                   h->d_aval_wide[0], h->d_aval_wide[1]};
   for (void* p : ptrs)
@@ -190,6 +190,14 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
     // (some block is routed to the 2:4 path, so every list below has an entry)
     SMAT_TRY(upload(&h->d_sp24_stages, sp.stages.data(), sp.stages.size()));
     SMAT_TRY(upload(&h->d_sp24_groups, sp.groups.data(), sp.groups.size()));
+    std::vector<Sp24Group> items, split;
+    split_sp24(sp, h->num_sms, items, split, h->sp24_nslabs);
+    if (!split.empty()) {
+      h->sp24_nitems = (int32_t)items.size();
+      h->sp24_nsplit = (int32_t)split.size();
+      SMAT_TRY(upload(&h->d_sp24_items, items.data(), items.size()));
+      SMAT_TRY(upload(&h->d_sp24_split, split.data(), split.size()));
+    }
     SMAT_TRY(upload(&h->d_sp24_unit_window, sp.unit_window.data(), sp.unit_window.size()));
     SMAT_TRY(upload(&h->d_bcsr_row_map, b.row_map.data(), b.row_map.size()));
     h->sp24_ngroups = (int32_t)sp.groups.size();
@@ -580,7 +588,10 @@ WsLayout smat::ws_layout(const smat_bcsr* A, int32_t form, int64_t N, bool whole
   const int64_t bn = 128 * nsub, n_tiles = (std::max<int64_t>(N, 1) + bn - 1) / bn;
   const size_t n_slabs = whole ? 0 : sc.n_slabs;
   w.slabs = w.counters + 256;
-  w.flags = w.slabs + n_slabs * n_tiles * A->R * A->host.bh * bn * sizeof(float);
+  w.slabs24 = w.slabs + n_slabs * n_tiles * A->R * A->host.bh * bn * sizeof(float);
+  w.flags = w.slabs24;
+  if (uses_sp24(A, form) && !whole)
+    w.flags += (size_t)A->sp24_nslabs * ((std::max<int64_t>(N, 1) + 127) / 128) * 128 * 128 * sizeof(float);
   w.total = w.flags + (pack_flag_bytes(A->host.cols, std::max<int64_t>(N, 1)) + 255) / 256 * 256;
   return w;
 }
@@ -731,6 +742,7 @@ static smat_status packed_impl(const smat_bcsr* A, int32_t form, const void* pac
   SpmmArgs args;
   std::memset(&args, 0, sizeof(args));
   const WsLayout wl = ws_layout(A, form, N, whole);
+  const bool whole24 = whole;
   whole = whole && sc.n_split > 0;  // else the list has no split panel
   fill_problem(A, form, packed_b, N, C, c_dtype, ldc, nsub, wl, args.one);
   const int64_t units = (int64_t)(whole ? sc.n_whole : sc.n_items) * args.one.n_tiles;
@@ -772,7 +784,11 @@ static smat_status packed_impl(const smat_bcsr* A, int32_t form, const void* pac
     const int fmt = form == SMAT_FORM_BF16 ? 1 : 0;
     a24.stream = A->d_sp24_stream[fmt];
     a24.stages = A->d_sp24_stages;
-    a24.groups = A->d_sp24_groups;
+    const bool parts = !whole24 && A->sp24_nsplit > 0;
+    a24.groups = parts ? A->d_sp24_items : A->d_sp24_groups;
+    a24.n_split = parts ? A->sp24_nsplit : 0;
+    a24.split = A->d_sp24_split;
+    a24.slabs = reinterpret_cast<float*>(static_cast<uint8_t*>(const_cast<void*>(packed_b)) + wl.slabs24);
     a24.unit_window = A->d_sp24_unit_window;
     a24.row_map = A->d_bcsr_row_map;
     a24.bpack64 = static_cast<const uint8_t*>(packed_b) + wl.b64;
@@ -781,14 +797,14 @@ static smat_status packed_impl(const smat_bcsr* A, int32_t form, const void* pac
     a24.ldc = ldc;
     a24.N = (int32_t)N;
     a24.n_tiles = (int32_t)((N + 127) / 128);
-    a24.n_groups = A->sp24_ngroups;
+    a24.n_groups = parts ? A->sp24_nitems : A->sp24_ngroups;
     a24.c_f16 = c_dtype == SMAT_F16 ? 1 : 0;
     // kind::f16 instruction descriptor without N: sparse (bit 2), FP32
     // accumulator, A and B FP16 (0) or BF16 (1), K-major, M = 128
     a24.idesc = (1u << 2) | (1u << 4) | ((uint32_t)fmt << 7) | ((uint32_t)fmt << 10) | ((uint32_t)(128 >> 4) << 24);
     a24.err = A->d_err;
     a24.wait_ns = A->wait_ns;
-    const int grid = std::max(1, std::min<int>(A->num_sms, A->sp24_ngroups));
+    const int grid = std::max(1, std::min<int>(A->num_sms, a24.n_groups));
     e = sp24_launch(a24, grid, static_cast<cudaStream_t>(stream_));
     if (e != cudaSuccess) return cuda_fail(e, "2:4 spmm kernel launch");
   }

@@ -153,6 +153,11 @@ struct Sp24Host {
   int64_t n_blocks = 0, n_units = 0;
 };
 smat_status build_sp24(const HostBcsr& b, const std::vector<uint8_t>& take, int fmt, Sp24Host& out);
+// The work list of `workers` CTAs: groups with more than the average share of
+// units are cut at stage boundaries into parts (heaviest first; `split` gets
+// the first part of each cut group, n_slabs their number of parts).
+void split_sp24(const Sp24Host& sp, int32_t workers, std::vector<Sp24Group>& items, std::vector<Sp24Group>& split,
+                int32_t& n_slabs);
 // Blocks routed to the 2:4 path: exactly 2:4 (is24), in a unit (8 block
 // rows x one 32-column window) holding at least min_unit such blocks.
 void route_sp24(const HostBcsr& b, int min_unit, std::vector<uint8_t>& take);
@@ -216,6 +221,9 @@ struct SmatBcsrBody {
   // (shared by the forms) and one compressed stream per form (FP16, BF16)
   int sp24_on = 0;
   int32_t sp24_ngroups = 0;
+  int32_t sp24_nitems = 0, sp24_nsplit = 0, sp24_nslabs = 0;  // the list with split groups
+  Sp24Group* d_sp24_items = nullptr;
+  Sp24Group* d_sp24_split = nullptr;
   int64_t sp24_units = 0;
   Sp24Stage* d_sp24_stages = nullptr;
   Sp24Group* d_sp24_groups = nullptr;
@@ -285,10 +293,12 @@ int pick_nsub(const smat_bcsr* h, int64_t N, int kind);
 // [the 2:4 path's copy of B, when the handle uses it for this form]
 // [the launch's next-unit counter, 256 bytes]
 // [per part of a split panel and column tile: an R*bh x BN FP32 slab]
+// [per part of a split 2:4 group and column tile: a 128 x 128 FP32 slab]
 // [a byte per packing unit of B: it holds infinite or NaN values].
 struct WsLayout {
   size_t counters = 0, slabs = 0, flags = 0, total = 0;
   size_t b64 = 0;  // the 2:4 path's copy of B (0: none)
+  size_t slabs24 = 0;  // the 2:4 path's partial sums
 };
 WsLayout ws_layout(const smat_bcsr* A, int32_t form, int64_t N, bool whole = false);
 

@@ -89,6 +89,8 @@ smat_status build_sp24(const HostBcsr& b, const std::vector<uint8_t>& take, int 
     Sp24Group G{};
     G.group = (int32_t)g;
     G.row_mask = row_mask;
+    G.slab = -1;
+    G.nparts = 1;
     G.stage0 = (int32_t)out.stages.size();
     G.unit0 = (int32_t)out.unit_window.size();
     // units, then stages of whole units
@@ -161,6 +163,42 @@ smat_status build_sp24(const HostBcsr& b, const std::vector<uint8_t>& take, int 
                    [](const Sp24Group& x, const Sp24Group& y) { return x.nunits > y.nunits; });
   if (out.stream.empty()) out.stream.resize(16, 0);
   return SMAT_OK;
+}
+
+void split_sp24(const Sp24Host& sp, int32_t workers, std::vector<Sp24Group>& items, std::vector<Sp24Group>& split,
+                int32_t& n_slabs) {
+  items.clear();
+  split.clear();
+  n_slabs = 0;
+  // as many parts as make about one average CTA's units each
+  const int64_t per = std::max<int64_t>(kSp24StageUnits, (sp.n_units + workers - 1) / std::max(1, workers));
+  for (const Sp24Group& g : sp.groups) {
+    const int32_t parts = (int32_t)std::min<int64_t>((g.nunits + per / 2) / per, g.nstages);
+    if (parts < 2) {
+      items.push_back(g);
+      continue;
+    }
+    int32_t s0 = 0, part = 0;
+    const size_t first = items.size();
+    for (int32_t st = 0; st < g.nstages; st++) {
+      const Sp24Stage& S = sp.stages[g.stage0 + st];
+      const int64_t done = S.unit0 + S.nunits;  // units of the group up to here
+      if (st + 1 < g.nstages && done * parts < (int64_t)g.nunits * (part + 1)) continue;
+      Sp24Group p = g;
+      p.stage0 = g.stage0 + s0;
+      p.nstages = st + 1 - s0;
+      p.unit0 = g.unit0 + sp.stages[p.stage0].unit0;
+      p.nunits = (int32_t)(done - sp.stages[p.stage0].unit0);
+      p.slab = n_slabs + part++;
+      items.push_back(p);
+      s0 = st + 1;
+    }
+    for (size_t i = first; i < items.size(); i++) items[i].nparts = part;
+    split.push_back(items[first]);
+    n_slabs += part;
+  }
+  std::stable_sort(items.begin(), items.end(),
+                   [](const Sp24Group& x, const Sp24Group& y) { return x.nunits > y.nunits; });
 }
 
 }  // namespace smat

@@ -11,7 +11,7 @@
 //
 // Roles (384 threads), one CTA per SM, groups taken round-robin from a list
 // sorted by decreasing work:
-//   warp 0        MMA issuer (lane 0); owns TMEM (two 128-column
+//   warp 0        MMA issuer (one lane); owns TMEM (two 128-column
 //                 accumulators, then the metadata column of each A-tile
 //                 slot, 64 columns apart: the MMA's metadata address is
 //                 kept on a 64-column boundary).
@@ -24,6 +24,13 @@
 //                 writes its 16 kept values into the zero-filled A tile in
 //                 shared memory (32-byte swizzle) and its 32-bit metadata word
 //                 into the unit's TMEM column (tcgen05.st).
+// Units go from the converters to the MMA issuer in batches of two (half the
+// A-tile slots each), with one wait, one fence and one arrival per batch. What
+// bounds the kernel is the latency of the converters' work (330 cycles a unit)
+// and of that hand-off, not the tensor cores; groups with more than an average
+// CTA's units are therefore cut into parts over several CTAs (8192 x 8192, 12 %
+// of the blocks, N = 128, 64 groups on 152 SMs: the whole step 135 us without
+// parts and batches, 68 with them).
 // Waits are bounded like the dense kernel's; an expired wait aborts the CTA
 // after its copies and MMAs in flight have landed.
 #include <cuda.h>
@@ -34,6 +41,7 @@
 #include <cstdint>
 
 #include "spmm24.h"
+#include "spmm_tc.h"
 #include "tc_ptx.cuh"
 
 namespace smat {
@@ -54,14 +62,16 @@ struct Sp24Cfg {
       kSp24StageUnits * sizeof(Sp24Unit) + kSp24StageBlocks * kSp24BlockBytes;
   static constexpr uint32_t STAGE_SLOT = (STAGE_MAX + 1023) / 1024 * 1024;
   static constexpr int NT = 4;                                   // A tile slots (and metadata columns)
+  static constexpr int NB = 2;                                   // batches of slots
+  static constexpr int UB = NT / NB;                             // units per batch, at most
   static constexpr uint32_t ATILE = 128 * 32;                    // 128 rows x 16 kept values
   static constexpr int NBT = 12;                                 // B tile slots (8 KB copies from L2 in flight)
   static constexpr uint32_t BTILE = 128 * 64;                    // 128 columns x 32 k
   static constexpr uint32_t OFF_A = NS * STAGE_SLOT;
   static constexpr uint32_t OFF_B = OFF_A + NT * ATILE;
   static constexpr uint32_t RING = OFF_B + NBT * BTILE;
-  static constexpr uint32_t NBARS = 2 * NS + 2 * NT + 2 * NBT + 4 + 1;
-  static constexpr uint32_t SMEM_BYTES = 1024 + RING + 8 * NBARS + 16;
+  static constexpr uint32_t NBARS = 2 * NS + 2 * NB + 2 * NBT + 4 + 1;
+  static constexpr uint32_t SMEM_BYTES = 1024 + RING + 8 * NBARS + 8 + 4 * NB + 8;
   static constexpr uint32_t META_COL0 = 256;                     // metadata column of A slot t: META_COL0 + 64 t
   static constexpr uint32_t META_STRIDE = 64;
   static constexpr uint32_t TMEM_COLS = 512;                     // 2 x 128 accumulator + NT metadata
@@ -73,14 +83,13 @@ struct Sp24Cfg {
 
 __device__ __forceinline__ bool w24(uint32_t bar, uint32_t parity, volatile int* abort, int* err, int where,
                                     uint64_t lim) {
-  return mbar_try_wait(bar, parity) || mbar_wait(bar, parity, abort, err, where, lim);
+  return mbar_poll(bar, parity) || mbar_wait(bar, parity, abort, err, where, lim);
 }
 
-__device__ __forceinline__ bool w24_warp(uint32_t bar, uint32_t parity, int lane, volatile int* abort, int* err,
-                                         int where, uint64_t lim) {
-  int got = 1;
-  if (lane == 0) got = w24(bar, parity, abort, err, where, lim) ? 1 : 0;
-  return __shfl_sync(0xffffffffu, got, 0) != 0;
+// For a whole warp: every lane polls, the vote makes the outcome uniform.
+__device__ __forceinline__ bool w24_warp(uint32_t bar, uint32_t parity, volatile int* abort, int* err, int where,
+                                         uint64_t lim) {
+  return __all_sync(0xffffffffu, w24(bar, parity, abort, err, where, lim));
 }
 
 __device__ __noinline__ void drain24(uint32_t bar, uint32_t parity, int* err, uint64_t lim) {
@@ -124,16 +133,17 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
   uint64_t* s_full = reinterpret_cast<uint64_t*>(smem + C::RING);
   uint64_t* s_free = s_full + C::NS;
   uint64_t* a_ready = s_free + C::NS;
-  uint64_t* a_free = a_ready + C::NT;
-  uint64_t* b_full = a_free + C::NT;
+  uint64_t* a_free = a_ready + C::NB;
+  uint64_t* b_full = a_free + C::NB;
   uint64_t* b_free = b_full + C::NBT;
   uint64_t* accfull = b_free + C::NBT;
   uint64_t* accempty = accfull + 2;
   uint64_t* drainbar = accempty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drainbar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* batch_n = abort_flag + 1;  // [NB] units of the batch
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint64_t lim = args.wait_ns ? args.wait_ns : kWaitTimeoutNs;
   int* err = args.err;
 
@@ -142,7 +152,7 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
       mbar_init(smem_u32(&s_full[i]), 1);
       mbar_init(smem_u32(&s_free[i]), 4);
     }
-    for (int i = 0; i < C::NT; i++) {
+    for (int i = 0; i < C::NB; i++) {
       mbar_init(smem_u32(&a_ready[i]), 4);
       mbar_init(smem_u32(&a_free[i]), 1);
     }
@@ -168,10 +178,11 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
   const uint32_t tmem = *tmem_slot;
   const uint32_t smem0 = smem_u32(smem);
   const int G = (int)gridDim.x;
+  grid_release();  // the kernel that sums split groups may be set up
 
   if (warp == 1) {
     // ---------------------------------------------------------- stage copies
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t sc = 0;
       bool ok = true;
       for (int gi = blockIdx.x; gi < args.n_groups && ok; gi += G) {
@@ -197,35 +208,43 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
     }
   } else if (warp == 2) {
     // -------------------------------------------------------------- B copies
-    if (lane == 0) {
-      uint32_t u = 0;
-      bool ok = true;
-      for (int gi = blockIdx.x; gi < args.n_groups && ok; gi += G) {
-        const Sp24Group g = args.groups[gi];
-        for (int nt = 0; nt < args.n_tiles && ok; ++nt)
-          for (int i = 0; i < g.nunits; ++i, ++u) {
+    // The whole warp, one unit at a time; the windows of 32 units are read
+    // together and ahead.
+    const uint64_t pol = make_l2_policy_evict_last();
+    uint32_t u = 0;
+    bool ok = true;
+    for (int gi = blockIdx.x; gi < args.n_groups && ok; gi += G) {
+      const Sp24Group g = args.groups[gi];
+      for (int nt = 0; nt < args.n_tiles && ok; ++nt) {
+        int ahead = lane < g.nunits ? __ldg(args.unit_window + g.unit0 + lane) : 0;
+        for (int i0 = 0; i0 < g.nunits && ok; i0 += 32) {
+          const int mine = ahead;
+          if (i0 + 32 + lane < g.nunits) ahead = __ldg(args.unit_window + g.unit0 + i0 + 32 + lane);
+          const int cnt = min(32, g.nunits - i0);
+          for (int i = 0; i < cnt; ++i, ++u) {
             const uint32_t x = u % C::NBT;
             if (u >= (uint32_t)C::NBT &&
-                !w24(smem_u32(&b_free[x]), ((u - C::NBT) / C::NBT) & 1, abort_flag, err, ERR24_B, lim)) {
+                !w24_warp(smem_u32(&b_free[x]), ((u - C::NBT) / C::NBT) & 1, abort_flag, err, ERR24_B, lim)) {
               ok = false;
               break;
             }
-            const int w = args.unit_window[g.unit0 + i];
+            const int w = __shfl_sync(0xffffffffu, mine, i);
             const uint32_t fb = smem_u32(&b_full[x]);
-            mbar_arrive_expect_tx(fb, C::BTILE);
-            bulk_load(smem0 + C::OFF_B + x * C::BTILE, args.bpack64 + ((int64_t)nt * args.kw + w) * C::BTILE,
-                      C::BTILE, fb);
+            mbar_arrive_expect_tx_if(fb, C::BTILE, lane == 0);
+            bulk_load_hint_if(smem0 + C::OFF_B + x * C::BTILE, args.bpack64 + ((int64_t)nt * args.kw + w) * C::BTILE,
+                              C::BTILE, fb, pol, lane == 0);
           }
+        }
       }
-      if (!ok) {
-        const uint32_t lo = u > (uint32_t)C::NBT ? u - C::NBT : 0;
-        for (uint32_t k = lo; k < u; ++k) drain24(smem_u32(&b_full[k % C::NBT]), (k / C::NBT) & 1, err, lim);
-      }
+    }
+    if (!ok && lane == 0) {
+      const uint32_t lo = u > (uint32_t)C::NBT ? u - C::NBT : 0;
+      for (uint32_t k = lo; k < u; ++k) drain24(smem_u32(&b_full[k % C::NBT]), (k / C::NBT) & 1, err, lim);
     }
   } else if (warp == 0) {
     // ----------------------------------------------------------------- MMAs
-    if (lane == 0) {
-      uint32_t u = 0, k = 0;
+    if (elect_one()) {
+      uint32_t u = 0, k = 0, bc = 0;
       bool ok = true, issued = false;
       for (int gi = blockIdx.x; gi < args.n_groups && ok; gi += G) {
         const Sp24Group g = args.groups[gi];
@@ -236,20 +255,28 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
             break;
           }
           tc_fence_after();
-          for (int i = 0; i < g.nunits; ++i, ++u) {
-            const uint32_t t = u % C::NT, x = u % C::NBT;
-            if (!w24(smem_u32(&a_ready[t]), (u / C::NT) & 1, abort_flag, err, ERR24_MMA, lim) ||
-                !w24(smem_u32(&b_full[x]), (u / C::NBT) & 1, abort_flag, err, ERR24_MMA, lim)) {
+          for (int i = 0; i < g.nunits && ok; ++bc) {
+            const uint32_t bt = bc % C::NB;
+            if (!w24(smem_u32(&a_ready[bt]), (bc / C::NB) & 1, abort_flag, err, ERR24_MMA, lim)) {
               ok = false;
               break;
             }
             tc_fence_after();
-            const uint64_t ad = desc_kmajor_sw32(smem0 + C::OFF_A + t * C::ATILE);
-            const uint64_t bd = desc_kmajor_sw64(smem0 + C::OFF_B + x * C::BTILE);
-            umma_sp_f16(tmem + buf * 128, ad, bd, tmem + C::META_COL0 + C::META_STRIDE * t, args.idesc | ((128u >> 3) << 17), i > 0 ? 1u : 0u);
-            issued = true;
-            umma_commit(smem_u32(&a_free[t]));
-            umma_commit(smem_u32(&b_free[x]));
+            const int n = batch_n[bt];
+            for (int j = 0; j < n; ++j, ++i, ++u) {
+              const uint32_t t = bt * C::UB + (uint32_t)j, x = u % C::NBT;
+              if (!w24(smem_u32(&b_full[x]), (u / C::NBT) & 1, abort_flag, err, ERR24_MMA, lim)) {
+                ok = false;
+                break;
+              }
+              const uint64_t ad = desc_kmajor_sw32(smem0 + C::OFF_A + t * C::ATILE);
+              const uint64_t bd = desc_kmajor_sw64(smem0 + C::OFF_B + x * C::BTILE);
+              umma_sp_f16(tmem + buf * 128, ad, bd, tmem + C::META_COL0 + C::META_STRIDE * t,
+                          args.idesc | ((128u >> 3) << 17), i > 0 ? 1u : 0u);
+              issued = true;
+              umma_commit(smem_u32(&b_free[x]));
+            }
+            if (ok) umma_commit(smem_u32(&a_free[bt]));
           }
           if (!ok) break;
           umma_commit(smem_u32(&accfull[buf]));
@@ -274,14 +301,14 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
     const int q = warp - 8;
     const int r = q * 32 + lane;
     const int j = r >> 4, rr = r & 15;
-    uint32_t u = 0, sc = 0;
+    uint32_t bc = 0, sc = 0;
     bool ok = true;
     for (int gi = blockIdx.x; gi < args.n_groups && ok; gi += G) {
       const Sp24Group g = args.groups[gi];
       for (int nt = 0; nt < args.n_tiles && ok; ++nt)
         for (int st = 0; st < g.nstages && ok; ++st, ++sc) {
           const uint32_t slot = sc % C::NS;
-          if (!w24_warp(smem_u32(&s_full[slot]), (sc / C::NS) & 1, lane, abort_flag, err, ERR24_CONV, lim)) {
+          if (!w24_warp(smem_u32(&s_full[slot]), (sc / C::NS) & 1, abort_flag, err, ERR24_CONV, lim)) {
             ok = false;
             break;
           }
@@ -291,28 +318,32 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
           const Sp24Unit* units = reinterpret_cast<const Sp24Unit*>(sp);
           const uint8_t* vals = sp + nunits * sizeof(Sp24Unit);
           const uint8_t* metas = vals + (size_t)nblk * 256;
-          for (int i = 0; i < nunits; ++i, ++u) {
-            const uint32_t t = u % C::NT;
-            if (u >= (uint32_t)C::NT &&
-                !w24_warp(smem_u32(&a_free[t]), ((u - C::NT) / C::NT) & 1, lane, abort_flag, err, ERR24_CONV, lim)) {
+          for (int i0 = 0; i0 < nunits; i0 += C::UB, ++bc) {
+            const uint32_t bt = bc % C::NB;
+            const int n = min(C::UB, nunits - i0);
+            if (bc >= (uint32_t)C::NB &&
+                !w24_warp(smem_u32(&a_free[bt]), ((bc - C::NB) / C::NB) & 1, abort_flag, err, ERR24_CONV, lim)) {
               ok = false;
               break;
             }
-            const uint32_t mask = units[i].mask;
-            const uint32_t first = units[i].first;
-            uint8_t* arow = smem + C::OFF_A + t * C::ATILE + r * 32;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const uint32_t bit = 2u * j + h;
-              uint4 v = make_uint4(0, 0, 0, 0);
-              if ((mask >> bit) & 1u) {
-                const uint32_t blk = first + __popc(mask & ((1u << bit) - 1u));
-                v = *reinterpret_cast<const uint4*>(vals + (size_t)blk * 256 + rr * 16);
+            for (int y = 0; y < C::UB; ++y) {
+              if (y >= n) break;
+              const uint32_t t = bt * C::UB + (uint32_t)y;
+              const uint32_t mask = units[i0 + y].mask;
+              const uint32_t first = units[i0 + y].first;
+              uint8_t* arow = smem + C::OFF_A + t * C::ATILE + r * 32;
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const uint32_t bit = 2u * j + h;
+                uint4 v = make_uint4(0, 0, 0, 0);
+                if ((mask >> bit) & 1u) {
+                  const uint32_t blk = first + __popc(mask & ((1u << bit) - 1u));
+                  v = *reinterpret_cast<const uint4*>(vals + (size_t)blk * 256 + rr * 16);
+                }
+                *reinterpret_cast<uint4*>(arow + ((h ^ ((r >> 2) & 1)) << 4)) = v;
               }
-              *reinterpret_cast<uint4*>(arow + ((h ^ ((r >> 2) & 1)) << 4)) = v;
-            }
-            uint32_t word = 0x44444444u;
-            {
+              uint32_t word = 0x44444444u;
               const uint32_t mh = (r >> 3) & 1u, mi = r & 7u;  // K-half and slab row of this lane
               const uint32_t bit = 2u * j + mh;
               if ((mask >> bit) & 1u) {
@@ -320,13 +351,16 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
                 const uint16_t* mp = reinterpret_cast<const uint16_t*>(metas + (size_t)blk * 32);
                 word = (uint32_t)mp[mi] | ((uint32_t)mp[mi + 8] << 16);
               }
+              __syncwarp();
+              tmem_st_x1(tmem + ((uint32_t)(q * 32) << 16) + C::META_COL0 + C::META_STRIDE * t, word);
             }
-            tmem_st_x1(tmem + ((uint32_t)(q * 32) << 16) + C::META_COL0 + C::META_STRIDE * t, word);
+            if (q == 0 && lane == 0) batch_n[bt] = n;
+            __syncwarp();
             tmem_st_wait();
             fence_proxy_async_smem();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&a_ready[t]));
+            if (lane == 0) mbar_arrive(smem_u32(&a_ready[bt]));
           }
           __syncwarp();
           if (lane == 0 && ok) mbar_arrive(smem_u32(&s_free[slot]));
@@ -348,7 +382,7 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
       const int crow = ((g.row_mask >> (r >> 4)) & 1u) ? args.row_map[prow] : -1;
       for (int nt = 0; nt < args.n_tiles; ++nt, ++k) {
         const uint32_t buf = k & 1;
-        if (!w24_warp(smem_u32(&accfull[buf]), (k >> 1) & 1, lane, abort_flag, err, ERR24_EPI, lim)) {
+        if (!w24_warp(smem_u32(&accfull[buf]), (k >> 1) & 1, abort_flag, err, ERR24_EPI, lim)) {
           ok = false;
           break;
         }
@@ -356,8 +390,13 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
 #pragma unroll 1
         for (int c = 0; c < 128; c += 32) {
           float v[32];
+          __syncwarp();
           tmem_ld_x32(tmem + ((uint32_t)(q * 32) << 16) + buf * 128 + c, v);
-          if (crow >= 0) {
+          if (g.slab >= 0) {
+            float4* sp = reinterpret_cast<float4*>(args.slabs + (((int64_t)g.slab * args.n_tiles + nt) * 128 + r) * 128 + c);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) __stcg(sp + m, make_float4(v[4 * m], v[4 * m + 1], v[4 * m + 2], v[4 * m + 3]));
+          } else if (crow >= 0) {
             const int n0 = nt * 128 + c;
             if (args.c_f16) {
               __half* cp = reinterpret_cast<__half*>(args.C) + (int64_t)crow * args.ldc + n0;
@@ -387,6 +426,41 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
   }
 }
 
+// The split groups' parts, added in order and then into C: a block per 16 rows
+// of a group, a thread per column.
+__global__ void __launch_bounds__(128) sum24_kernel(const __grid_constant__ Sp24Args args) {
+  grid_wait();
+  const int u = (int)blockIdx.x / args.n_tiles, nt = (int)blockIdx.x % args.n_tiles;
+  const Sp24Group g = args.split[u];
+  const int j = (int)blockIdx.y;  // block row of the group
+  const int n = nt * 128 + (int)threadIdx.x;
+  if (!((g.row_mask >> j) & 1u) || n >= args.N) return;
+  const float* src = args.slabs + (((int64_t)g.slab * args.n_tiles + nt) * 128 + 16 * j) * 128 + threadIdx.x;
+  const int64_t step = (int64_t)args.n_tiles * 128 * 128;
+  float acc[16];
+#pragma unroll
+  for (int m = 0; m < 16; ++m) acc[m] = 0.0f;
+  for (int p = 0; p < g.nparts; ++p, src += step) {
+    float t[16];
+#pragma unroll
+    for (int m = 0; m < 16; ++m) t[m] = __ldcg(src + m * 128);
+#pragma unroll
+    for (int m = 0; m < 16; ++m) acc[m] += t[m];
+  }
+#pragma unroll
+  for (int m = 0; m < 16; ++m) {
+    const int row = args.row_map[(int64_t)g.group * 128 + 16 * j + m];
+    if (row < 0) continue;
+    const int64_t off = (int64_t)row * args.ldc + n;
+    if (args.c_f16) {
+      __half* cp = reinterpret_cast<__half*>(args.C) + off;
+      *cp = __float2half_rn(__half2float(*cp) + acc[m]);
+    } else {
+      reinterpret_cast<float*>(args.C)[off] += acc[m];
+    }
+  }
+}
+
 }  // namespace dev
 
 int sp24_threads() { return dev::Sp24Cfg::THREADS; }
@@ -406,7 +480,11 @@ cudaError_t sp24_launch(const Sp24Args& args, int grid, cudaStream_t stream) {
     done.fetch_or(bit);
   }
   dev::spmm24_kernel<<<grid, dev::Sp24Cfg::THREADS, dev::Sp24Cfg::SMEM_BYTES, stream>>>(args);
-  return cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || args.n_split == 0) return e;
+  void* params[] = {const_cast<Sp24Args*>(&args)};
+  return launch_kernel(reinterpret_cast<const void*>(dev::sum24_kernel),
+                       dim3((unsigned)(args.n_split * args.n_tiles), kSp24GroupRows), dim3(128), 0, stream, true, params);
 }
 
 }  // namespace smat

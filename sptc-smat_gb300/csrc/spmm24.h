@@ -49,13 +49,16 @@ struct Sp24Stage {
   int32_t pad[2];
 };
 
-// A group (32 bytes): its stages and units.
+// A group (32 bytes), or a part of one: its stages and units. The parts of a
+// group that is split over several CTAs write partial sums, and a second
+// kernel adds them into C.
 struct Sp24Group {
   int32_t stage0, nstages;
   int32_t unit0, nunits;    // units in the device unit-window array
   int32_t group;            // group index (block rows 8 * group ..)
   uint32_t row_mask;        // bit j: block row j has a 2:4 block
-  int32_t pad[2];
+  int32_t slab;             // the part's partial sums, or -1: the whole group, added into C
+  int32_t nparts;           // parts of the group (their slabs are consecutive)
 };
 
 struct Sp24Args {
@@ -72,7 +75,9 @@ struct Sp24Args {
   int32_t n_groups;
   int32_t c_f16;
   uint32_t idesc;             // sparse instruction descriptor without N
-  int32_t pad_;
+  int32_t n_split;            // split groups
+  const Sp24Group* split;     // the first part of each
+  float* slabs;               // [slab][column tile][128 rows][128 columns]
   int* err;
   uint64_t wait_ns;
 };
