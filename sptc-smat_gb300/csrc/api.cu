@@ -168,6 +168,7 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
   }
   if (h->sp24_on)
     for (uint8_t v : take24) h->n_24 += v;
+  h->sp24_all = h->sp24_on && h->n_24 == h->host.nnzb();
 
 #define SMAT_TRY(x)              \
   do {                           \
@@ -755,16 +756,19 @@ static smat_status packed_impl(const smat_bcsr* A, int32_t form, const void* pac
   args.depth = A->depth;
   uint8_t* ctr = static_cast<uint8_t*>(const_cast<void*>(packed_b)) + wl.counters;
   args.next_item = reinterpret_cast<int32_t*>(ctr);
-  if (!behind_pack) {
+  const bool all24 = uses_sp24(A, form) && A->sp24_all;  // nothing for the dense kernel
+  cudaError_t e = cudaSuccess;
+  if (!behind_pack && !all24) {
     // the next-unit counter starts at zero in every launch (packing B sets it
     // to zero for the launch right behind)
-    cudaError_t e = cudaMemsetAsync(ctr, 0, 16, static_cast<cudaStream_t>(stream_));
+    e = cudaMemsetAsync(ctr, 0, 16, static_cast<cudaStream_t>(stream_));
     if (e != cudaSuccess) return cuda_fail(e, "clearing the work counter");
   }
-  cudaError_t e = tc_launch(bh, R, nsub, kind, args, (int)std::min<int64_t>(sc.workers, std::max<int64_t>(units, 1)),
-                            behind_pack, static_cast<cudaStream_t>(stream_));
+  if (!all24)
+    e = tc_launch(bh, R, nsub, kind, args, (int)std::min<int64_t>(sc.workers, std::max<int64_t>(units, 1)), behind_pack,
+                  static_cast<cudaStream_t>(stream_));
   if (e != cudaSuccess) return cuda_fail(e, "spmm kernel launch");
-  if (!whole && sc.n_split > 0) {
+  if (!all24 && !whole && sc.n_split > 0) {
     SumArgs sa;
     std::memset(&sa, 0, sizeof(sa));
     sa.one = args.one;
@@ -778,7 +782,9 @@ static smat_status packed_impl(const smat_bcsr* A, int32_t form, const void* pac
     if (e != cudaSuccess) return cuda_fail(e, "split panel sums");
   }
   if (uses_sp24(A, form)) {
-    // the exact-2:4 blocks, added into the C the dense kernel wrote
+    // the exact-2:4 blocks, added into the C the dense kernel wrote; C itself
+    // where they are all there is (8192 x 8192, 12 % of the blocks, N = 128: 60.7 us
+    // a call with the dense kernel storing zeros first, 52.6 without)
     Sp24Args a24;
     std::memset(&a24, 0, sizeof(a24));
     const int fmt = form == SMAT_FORM_BF16 ? 1 : 0;
@@ -804,8 +810,10 @@ static smat_status packed_impl(const smat_bcsr* A, int32_t form, const void* pac
     a24.idesc = (1u << 2) | (1u << 4) | ((uint32_t)fmt << 7) | ((uint32_t)fmt << 10) | ((uint32_t)(128 >> 4) << 24);
     a24.err = A->d_err;
     a24.wait_ns = A->wait_ns;
+    a24.whole_c = all24 ? 1 : 0;
+    a24.n_brows = (int32_t)hb.nbr();
     const int grid = std::max(1, std::min<int>(A->num_sms, a24.n_groups));
-    e = sp24_launch(a24, grid, static_cast<cudaStream_t>(stream_));
+    e = sp24_launch(a24, grid, behind_pack || !all24, static_cast<cudaStream_t>(stream_));
     if (e != cudaSuccess) return cuda_fail(e, "2:4 spmm kernel launch");
   }
   return SMAT_OK;

@@ -31,6 +31,7 @@
 #include <cstdint>
 
 #include "convert.h"
+#include "spmm_tc.h"
 #include "tc_ptx.cuh"
 
 namespace smat {
@@ -269,6 +270,8 @@ static cudaError_t run_pack(const void* in, int layout, int64_t ldi, uint8_t* ou
 // lanes of a warp read neighbouring columns of one row k.
 __global__ void pack_b_sw64_kernel(const uint8_t* __restrict__ p, uint8_t* __restrict__ out, int64_t kbs,
                                    int64_t kw) {
+  grid_release();  // the kernels launched behind may be set up
+  grid_wait();     // the packed tiles
   const int64_t w = blockIdx.x;
   const int64_t t = blockIdx.y;
   const int n = threadIdx.x;
@@ -300,8 +303,8 @@ cudaError_t pack_b_sw64(const uint8_t* packed, int64_t K, int64_t N, uint8_t* ou
   const int64_t kbs = (K + 15) / 16, kw = (kbs + 1) / 2, nt = packed_b_tiles(N);
   if (kw == 0 || nt == 0) return cudaSuccess;
   dim3 grid((unsigned)kw, (unsigned)nt);
-  dev::pack_b_sw64_kernel<<<grid, 128, 0, s>>>(packed, out, kbs, kw);
-  return cudaGetLastError();
+  void* params[] = {&packed, &out, const_cast<int64_t*>(&kbs), const_cast<int64_t*>(&kw)};
+  return launch_kernel(reinterpret_cast<const void*>(dev::pack_b_sw64_kernel), grid, dim3(128), 0, s, true, params);
 }
 
 int64_t packed_b_tiles(int64_t N) {

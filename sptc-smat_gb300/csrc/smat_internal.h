@@ -220,6 +220,7 @@ struct SmatBcsrBody {
   // 2:4 path (use24 and 16 x 16 blocks): the groups, stages and unit windows
   // (shared by the forms) and one compressed stream per form (FP16, BF16)
   int sp24_on = 0;
+  int sp24_all = 0;  // no block is left to the dense plan of the FP16 / BF16 forms
   int32_t sp24_ngroups = 0;
   int32_t sp24_nitems = 0, sp24_nsplit = 0, sp24_nslabs = 0;  // the list with split groups
   Sp24Group* d_sp24_items = nullptr;

@@ -64,6 +64,9 @@ smat_status build_sp24(const HostBcsr& b, const std::vector<uint8_t>& take, int 
   if (b.bh != 16 || b.bw != 16) return fail(SMAT_ERR_UNSUPPORTED, "2:4 path: 16 x 16 blocks only");
   const int64_t nbr = b.nbr();
   const int64_t ngroups = (nbr + kSp24GroupRows - 1) / kSp24GroupRows;
+  // no block is left to the dense kernel, so this path writes C: groups without
+  // a block are listed too, for their rows of zeros
+  const bool all = std::all_of(take.begin(), take.end(), [](uint8_t v) { return v != 0; });
   struct Ent {
     int32_t window, bit;
     int64_t k;
@@ -83,7 +86,7 @@ smat_status build_sp24(const HostBcsr& b, const std::vector<uint8_t>& take, int 
           row_mask |= 1u << j;
         }
     }
-    if (ent.empty()) continue;
+    if (ent.empty() && !all) continue;
     std::sort(ent.begin(), ent.end(),
               [](const Ent& x, const Ent& y) { return x.window != y.window ? x.window < y.window : x.bit < y.bit; });
     Sp24Group G{};

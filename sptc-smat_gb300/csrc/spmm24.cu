@@ -19,18 +19,21 @@
 //   warp 2        B copies: one 8 KB tile (32 rows of B x 128 columns,
 //                 64-byte swizzle) per unit.
 //   warps 4..7    epilogue: tcgen05.ld of the accumulator (lane = row) and
-//                 C[row, :] += it, rows through the row map.
-//   warps 8..11   converters: each thread owns one of the 128 rows of a unit,
-//                 writes its 16 kept values into the zero-filled A tile in
-//                 shared memory (32-byte swizzle) and its 32-bit metadata word
-//                 into the unit's TMEM column (tcgen05.st).
+//                 C[row, :] += it, rows through the row map; C[row, :] = it
+//                 where every block is on this path and no dense kernel ran.
+//   warps 8..15   converters, two sets of four: each thread owns one of the 128
+//                 rows of a unit, writes its 16 kept values into the zero-filled
+//                 A tile in shared memory (32-byte swizzle) and its 32-bit
+//                 metadata word into the unit's TMEM column (tcgen05.st).
 // Units go from the converters to the MMA issuer in batches of two (half the
-// A-tile slots each), with one wait, one fence and one arrival per batch. What
-// bounds the kernel is the latency of the converters' work (330 cycles a unit)
-// and of that hand-off, not the tensor cores; groups with more than an average
-// CTA's units are therefore cut into parts over several CTAs (8192 x 8192, 12 %
-// of the blocks, N = 128, 64 groups on 152 SMs: the whole step 135 us without
-// parts and batches, 68 with them).
+// A-tile slots each), with one wait, one fence and one arrival per batch; the
+// sets take every other batch. What bounds the kernel is the latency of the
+// converters' work (330 cycles a unit) and of that hand-off, not the tensor
+// cores; groups with more than an average CTA's units are therefore cut into
+// parts over several CTAs (8192 x 8192, 12 % of the blocks, N = 128, 64 groups
+// on 152 SMs, the whole step: 135 us without parts and batches, 68 with them, 61
+// with the second set of converters and every launch a programmatic dependent of
+// the one before, 53 without the dense kernel's pass).
 // Waits are bounded like the dense kernel's; an expired wait aborts the CTA
 // after its copies and MMAs in flight have landed.
 #include <cuda.h>
@@ -75,7 +78,7 @@ struct Sp24Cfg {
   static constexpr uint32_t META_COL0 = 256;                     // metadata column of A slot t: META_COL0 + 64 t
   static constexpr uint32_t META_STRIDE = 64;
   static constexpr uint32_t TMEM_COLS = 512;                     // 2 x 128 accumulator + NT metadata
-  static constexpr int THREADS = 384;
+  static constexpr int THREADS = 512;
   static_assert(STAGE_MAX % 16 == 0, "stage bytes");
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
   static_assert(META_COL0 + META_STRIDE * (NT - 1) < TMEM_COLS, "metadata columns inside the allocation");
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::NS; i++) {
       mbar_init(smem_u32(&s_full[i]), 1);
-      mbar_init(smem_u32(&s_free[i]), 4);
+      mbar_init(smem_u32(&s_free[i]), 4 * C::NB);
     }
     for (int i = 0; i < C::NB; i++) {
       mbar_init(smem_u32(&a_ready[i]), 4);
@@ -213,6 +216,7 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
     const uint64_t pol = make_l2_policy_evict_last();
     uint32_t u = 0;
     bool ok = true;
+    grid_wait();  // the windows, made by the launches before this one
     for (int gi = blockIdx.x; gi < args.n_groups && ok; gi += G) {
       const Sp24Group g = args.groups[gi];
       for (int nt = 0; nt < args.n_tiles && ok; ++nt) {
@@ -298,7 +302,8 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
     // 16-bit metadata of K-half h (the window's block h) for row i of the
     // slab in bits 0..15 and for row i + 8 in bits 16..31 (0x4444 for an
     // absent block: indices 0 and 1 of zero values).
-    const int q = warp - 8;
+    const int q = (warp - 8) & 3;
+    const uint32_t set = (uint32_t)(warp - 8) >> 2;
     const int r = q * 32 + lane;
     const int j = r >> 4, rr = r & 15;
     uint32_t bc = 0, sc = 0;
@@ -320,6 +325,7 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
           const uint8_t* metas = vals + (size_t)nblk * 256;
           for (int i0 = 0; i0 < nunits; i0 += C::UB, ++bc) {
             const uint32_t bt = bc % C::NB;
+            if (bt != set) continue;  // the other set's batch
             const int n = min(C::UB, nunits - i0);
             if (bc >= (uint32_t)C::NB &&
                 !w24_warp(smem_u32(&a_free[bt]), ((bc - C::NB) / C::NB) & 1, abort_flag, err, ERR24_CONV, lim)) {
@@ -376,10 +382,13 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
     }
     uint32_t k = 0;
     bool ok = true;
+    grid_wait();  // C of the dense kernel; the slabs of the call before
     for (int gi = blockIdx.x; gi < args.n_groups && ok; gi += G) {
       const Sp24Group g = args.groups[gi];
       const int64_t prow = (int64_t)g.group * 128 + r;
-      const int crow = ((g.row_mask >> (r >> 4)) & 1u) ? args.row_map[prow] : -1;
+      const bool has = (g.row_mask >> (r >> 4)) & 1u;
+      const bool mine = has || (args.whole_c && g.group * kSp24GroupRows + (r >> 4) < args.n_brows);
+      const int crow = mine ? args.row_map[prow] : -1;
       for (int nt = 0; nt < args.n_tiles; ++nt, ++k) {
         const uint32_t buf = k & 1;
         if (!w24_warp(smem_u32(&accfull[buf]), (k >> 1) & 1, abort_flag, err, ERR24_EPI, lim)) {
@@ -398,16 +407,20 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
             for (int m = 0; m < 8; ++m) __stcg(sp + m, make_float4(v[4 * m], v[4 * m + 1], v[4 * m + 2], v[4 * m + 3]));
           } else if (crow >= 0) {
             const int n0 = nt * 128 + c;
+            if (!has) {
+#pragma unroll
+              for (int m = 0; m < 32; ++m) v[m] = 0.0f;
+            }
             if (args.c_f16) {
               __half* cp = reinterpret_cast<__half*>(args.C) + (int64_t)crow * args.ldc + n0;
 #pragma unroll
               for (int m = 0; m < 32; ++m)
-                if (n0 + m < args.N) cp[m] = __float2half_rn(__half2float(cp[m]) + v[m]);
+                if (n0 + m < args.N) cp[m] = __float2half_rn(args.whole_c ? v[m] : __half2float(cp[m]) + v[m]);
             } else {
               float* cp = reinterpret_cast<float*>(args.C) + (int64_t)crow * args.ldc + n0;
 #pragma unroll
               for (int m = 0; m < 32; ++m)
-                if (n0 + m < args.N) cp[m] += v[m];
+                if (n0 + m < args.N) cp[m] = args.whole_c ? v[m] : cp[m] + v[m];
             }
           }
         }
@@ -434,13 +447,14 @@ __global__ void __launch_bounds__(128) sum24_kernel(const __grid_constant__ Sp24
   const Sp24Group g = args.split[u];
   const int j = (int)blockIdx.y;  // block row of the group
   const int n = nt * 128 + (int)threadIdx.x;
-  if (!((g.row_mask >> j) & 1u) || n >= args.N) return;
+  const bool has = (g.row_mask >> j) & 1u;
+  if (n >= args.N || !(has || (args.whole_c && g.group * kSp24GroupRows + j < args.n_brows))) return;
   const float* src = args.slabs + (((int64_t)g.slab * args.n_tiles + nt) * 128 + 16 * j) * 128 + threadIdx.x;
   const int64_t step = (int64_t)args.n_tiles * 128 * 128;
   float acc[16];
 #pragma unroll
   for (int m = 0; m < 16; ++m) acc[m] = 0.0f;
-  for (int p = 0; p < g.nparts; ++p, src += step) {
+  for (int p = 0; has && p < g.nparts; ++p, src += step) {
     float t[16];
 #pragma unroll
     for (int m = 0; m < 16; ++m) t[m] = __ldcg(src + m * 128);
@@ -454,9 +468,10 @@ __global__ void __launch_bounds__(128) sum24_kernel(const __grid_constant__ Sp24
     const int64_t off = (int64_t)row * args.ldc + n;
     if (args.c_f16) {
       __half* cp = reinterpret_cast<__half*>(args.C) + off;
-      *cp = __float2half_rn(__half2float(*cp) + acc[m]);
+      *cp = __float2half_rn(args.whole_c ? acc[m] : __half2float(*cp) + acc[m]);
     } else {
-      reinterpret_cast<float*>(args.C)[off] += acc[m];
+      float* cp = reinterpret_cast<float*>(args.C) + off;
+      *cp = args.whole_c ? acc[m] : *cp + acc[m];
     }
   }
 }
@@ -465,7 +480,7 @@ __global__ void __launch_bounds__(128) sum24_kernel(const __grid_constant__ Sp24
 
 int sp24_threads() { return dev::Sp24Cfg::THREADS; }
 
-cudaError_t sp24_launch(const Sp24Args& args, int grid, cudaStream_t stream) {
+cudaError_t sp24_launch(const Sp24Args& args, int grid, bool behind, cudaStream_t stream) {
   static std::atomic<uint64_t> done{0};
   int d = 0;
   if (cudaGetDevice(&d) != cudaSuccess) return cudaErrorInvalidDevice;
@@ -479,10 +494,10 @@ cudaError_t sp24_launch(const Sp24Args& args, int grid, cudaStream_t stream) {
     }
     done.fetch_or(bit);
   }
-  dev::spmm24_kernel<<<grid, dev::Sp24Cfg::THREADS, dev::Sp24Cfg::SMEM_BYTES, stream>>>(args);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess || args.n_split == 0) return e;
   void* params[] = {const_cast<Sp24Args*>(&args)};
+  const cudaError_t e = launch_kernel(reinterpret_cast<const void*>(dev::spmm24_kernel), dim3((unsigned)grid),
+                                      dim3(dev::Sp24Cfg::THREADS), dev::Sp24Cfg::SMEM_BYTES, stream, behind, params);
+  if (e != cudaSuccess || args.n_split == 0) return e;
   return launch_kernel(reinterpret_cast<const void*>(dev::sum24_kernel),
                        dim3((unsigned)(args.n_split * args.n_tiles), kSp24GroupRows), dim3(128), 0, stream, true, params);
 }

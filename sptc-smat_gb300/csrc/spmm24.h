@@ -80,9 +80,13 @@ struct Sp24Args {
   float* slabs;               // [slab][column tile][128 rows][128 columns]
   int* err;
   uint64_t wait_ns;
+  int32_t whole_c;            // every block is on this path: C is written, not added to
+  int32_t n_brows;            // block rows
 };
 
-cudaError_t sp24_launch(const Sp24Args& args, int grid, cudaStream_t stream);
+// behind: a programmatic dependent of the launch before it, which is one of the
+// same call.
+cudaError_t sp24_launch(const Sp24Args& args, int grid, bool behind, cudaStream_t stream);
 int sp24_threads();
 
 }  // namespace smat
