@@ -24,8 +24,8 @@
 // both), so the hand-off between the copies and the tensor cores is one
 // full/empty barrier pair per stage.
 //
-// Roles (640 threads):
-//   warps 12..19    copy warps, in pairs that own whole stages: bulk copies for
+// Roles (576 threads, FP8 640):
+//   warps 12..17    copy warps, in pairs that own whole stages: bulk copies for
 //                   the list, the A blocks and the B tiles, 16-byte copies
 //                   through the load path for the rows of gathered tiles.
 //   warps 0..3      MMA issuers, one elected lane each, one per quarter of the
@@ -42,14 +42,15 @@
 // What bounds it (GB300; time of the whole step with the packing of B):
 //   R-MAT, 2^16 rows, 816K blocks, N = 128: 256 us at first; 216 with waits
 //     that branch on the barrier's own predicate, elected issue and no barrier
-//     among the copy warps; 148 with gathered blocks (600K -> 266K MMAs, 1.85
-//     -> 1.0 GB into shared memory); 115 with the drain as a loop, (item,
-//     column tile) units and the roles above. Now the turn of a stage slot
-//     (copy issue, landing, MMAs) sets the pace: 47 bytes a cycle into an SM of
-//     the 70 it can take, tensor pipe busy 30 %.
-//   64^3 stencil, N = 256: 358 -> 187 us, 63 of them packing the FP32 B at 6.4
-//     TB/s; the kernel moves 450 MB of DRAM data in 125.
-//   plain graph, 2^15 rows, 600K entries, N = 256: 231 -> 76 us.
+//     among the copy warps; 148 with gathered blocks (615K -> 284K MMAs, 1.6 ->
+//     1.0 GB into shared memory); 115 with the drain as a loop, (item, column
+//     tile) units and the roles above; 109 with the parts of split panels added
+//     by a kernel of its own and the launches overlapping. The turn of a stage
+//     slot (copy issue, landing, MMAs) sets the pace: 34 bytes a cycle into an SM
+//     of the 70 it can take, tensor pipe busy 30 %.
+//   64^3 stencil, N = 256: 358 -> 178 us, 62 of them packing the FP32 B at 6.5
+//     TB/s; the kernel moves 450 MB of DRAM data in 116.
+//   plain graph, 2^15 rows, 600K entries, N = 256: 231 -> 54 us.
 //
 // Every wait is bounded (see tc_ptx.cuh); on a timeout the kernel raises the
 // CTA's abort flag, records the site in the global error word, lets the
@@ -122,7 +123,7 @@ struct Cfg {
   static constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
   static constexpr int NMMA = kMmaWarps;                  // MMA-issuing warps
   static constexpr int NEPI = 8;                          // epilogue warps: a set of four per accumulator buffer
-  static constexpr int NPROD = FP8 ? 4 : 8;               // copy warps, in pairs
+  static constexpr int NPROD = FP8 ? 4 : 6;               // copy warps, in pairs (3 stages in flight)
   static constexpr int NCONV = FP8 ? 4 : 0;               // FP8 converter warps (16..19)
   static constexpr uint32_t SMEM_BARS = 8 * (2 * NS + 4 + NMMA + (FP8 ? 2 * NS : 0) + 2 * kItemRing + 1);
   static constexpr int GLIST = (ST + 1) / 2 * 16 * 4;     // bytes of a copy warp's rows of gathered tiles
@@ -301,25 +302,25 @@ __device__ __forceinline__ void put_unit(const SpmmArgs& args, uint32_t k, uint6
 // tile's k-block in each lane, and (after load_rows) a 16-byte piece of the
 // rows of B of the warp's gathered tiles (every other one, from hf).
 struct StageView {
-  int nblk, ngath, ntiles, aoff, kb, g0;
+  int4 r1;  // nblk | ntiles, hdr_bytes | ngath, g0, aoff256: as loaded (unpacking them would wait for the load)
+  int kb;
   int4 rows0;
+  __device__ __forceinline__ int nblk() const { return r1.x & 0xffff; }
+  __device__ __forceinline__ int ntiles() const { return r1.x >> 16; }
+  __device__ __forceinline__ int ngath() const { return r1.y >> 16; }
 };
 __device__ __forceinline__ void load_stage(StageView& v, const StageRec* recs, int i, int n, int tile) {
-  v.nblk = v.ngath = v.ntiles = v.aoff = v.kb = v.g0 = 0;
+  v.r1 = make_int4(0, 0, 0, 0);
+  v.kb = 0;
   if (i >= 0 && i < n) {
     const StageRec* rp = recs + i;
-    const int4 r1 = __ldg(reinterpret_cast<const int4*>(rp) + 1);  // nblk | ntiles, hdr_bytes | ngath, g0, aoff256
-    v.nblk = r1.x & 0xffff;
-    v.ntiles = r1.x >> 16;
-    v.ngath = r1.y >> 16;
-    v.g0 = r1.z;
-    v.aoff = r1.w;
+    v.r1 = __ldg(reinterpret_cast<const int4*>(rp) + 1);
     v.kb = __ldg(rp->kb + min(tile, kMaxStageTiles - 1));
   }
 }
 __device__ __forceinline__ void load_rows(StageView& v, const int32_t* gcol, int hf, int lane) {
   const int t = (lane >> 2) * 2 + hf;  // four pieces per tile
-  if (t < v.ngath) v.rows0 = __ldg(reinterpret_cast<const int4*>(gcol + ((int64_t)v.g0 + t) * 16) + (lane & 3));
+  if (t < v.ngath()) v.rows0 = __ldg(reinterpret_cast<const int4*>(gcol + ((int64_t)v.r1.z + t) * 16) + (lane & 3));
 }
 
 // A gathered tile: row r of the tile from B's row at list[...] (its place in
@@ -591,10 +592,11 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
         ++taken;
       }
       for (; i < nst; i += (int)np) {
-        const int na = cur.ntiles - cur.ngath, ng = (cur.ngath + 1 - hf) / 2;  // gathered tiles of this warp
+        const int nblk = cur.nblk(), ngath = cur.ngath(), na = cur.ntiles() - ngath;
+        const int ng = (ngath + 1 - hf) / 2;  // gathered tiles of this warp
         const int nb = (na + 1 - hf) / 2;                                     // and bulk ones
-        const int kb = cur.kb, aoff = cur.aoff;
-        const uint32_t abytes = (uint32_t)stage_a_bytes(C::CLS, BH, cur.nblk, cur.ngath);
+        const int kb = cur.kb, aoff = cur.r1.w;
+        const uint32_t abytes = (uint32_t)stage_a_bytes(C::CLS, BH, nblk, ngath);
         if (lane < ng * 4) reinterpret_cast<int4*>(glist)[lane] = cur.rows0;  // for every lane to look up
         cur = nxt;
         load_rows(cur, p_gcol, hf, lane);
@@ -630,6 +632,16 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
         }
         cp_async_arrive(fb);
         __syncwarp();
+        if (!C::FP8) {
+          // The A region of the pair's next stage on its way from HBM into L2,
+          // a line per lane: the stage's copy then waits for L2 alone (R-MAT,
+          // 2^16 rows: 109 us a call without, 104 with; with bulk prefetches
+          // 106). Not for FP8, whose regions are half as large: 117.6 without,
+          // 121 with.
+          const int abytes_next = cur.nblk() ? stage_a_bytes(C::CLS, BH, cur.nblk(), cur.ngath()) : 0;
+          const uint8_t* const a_next = p_aval + (int64_t)cur.r1.w * 256;
+          for (int x = (lane + 32 * hf) * 128; x < abytes_next; x += 64 * 128) prefetch_l2(a_next + x);
+        }
         last_mine = my_c;
         mine = true;
         my_c += np;
@@ -796,22 +808,26 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       void* const p_C = P.C;
       const int panel = wi.panel, nt = wi.nt;
       const bool split = wi.split >= 0;
-      const uint32_t slot_mask = P.panels[panel].slot_mask;
+      // the panel's C rows, loaded before the accumulators are ready, side by
+      // side (one after the other, each behind the shared-memory store of the
+      // one before, they were 10,000 cycles a unit on the 64^3 stencil, now 3,300)
+      int row[R * BH / 32];
+#pragma unroll
+      for (int x = 0; x < R * BH / 32; ++x) row[x] = __ldg(P.row_map + (int64_t)panel * R * BH + x * 32 + lane);
+      const uint32_t slot_mask = __ldg(&P.panels[panel].slot_mask);
       // a hub row cut over the issuing warps has its parts in slots s, s + PW,
       // s + 2 PW, ...; the parts after the first are added into it here
-      const uint32_t ext_mask = P.panels[panel].ext_mask;
-      // the panel's C rows, loaded before the accumulators are ready; bit x of
-      // `full`: rows 16 x .. 16 x + 15 are all there
+      const uint32_t ext_mask = __ldg(&P.panels[panel].ext_mask);
+      // bit x of `full`: rows 16 x .. 16 x + 15 are all there
       uint32_t full = 0;
       const int elt = p_f16 ? 2 : 4;
       const int64_t ldb = p_ldc * elt;
 #pragma unroll
-      for (int x = 0; x < R * BH; x += 32) {
-        const int row = P.row_map[(int64_t)panel * R * BH + x + lane];
-        rows[x + lane] = row;
-        const uint32_t there = __ballot_sync(0xffffffffu, row >= 0);
-        full |= ((there & 0xffffu) == 0xffffu ? 1u : 0u) << (x / 16);
-        full |= ((there >> 16) == 0xffffu ? 1u : 0u) << (x / 16 + 1);
+      for (int x = 0; x < R * BH / 32; ++x) {
+        rows[x * 32 + lane] = row[x];
+        const uint32_t there = __ballot_sync(0xffffffffu, row[x] >= 0);
+        full |= ((there & 0xffffu) == 0xffffu ? 1u : 0u) << (2 * x);
+        full |= ((there >> 16) == 0xffffu ? 1u : 0u) << (2 * x + 1);
       }
       if (kk == buf) grid_wait();  // the warp's first unit
       const int32_t* const p_pois = P.poison_ptr;

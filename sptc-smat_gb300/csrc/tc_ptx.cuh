@@ -176,6 +176,9 @@ __device__ __forceinline__ __half2 e4m3x2_to_half2(uint16_t v) {
   return *reinterpret_cast<__half2*>(&r);
 }
 
+// The 128-byte line of `p` into L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Programmatic dependent launch: wait until the kernels this one was launched
 // behind are complete and their writes visible (nothing to wait for in an
 // ordinary launch); let the kernel launched behind this one begin its set-up.
