@@ -32,8 +32,8 @@
 //                   panel's block rows (one thread issues at most one
 //                   tcgen05.mma per 64-75 cycles, the tensor pipe takes one of
 //                   this width every 39); warp 0 also owns TMEM.
-//   warps 4..11     epilogue, a set of four per accumulator buffer: tcgen05.ld
-//                   -> row scatter through row_map -> FP32 or FP16 stores of C
+//   warps 4..11     epilogue, two per TMEM lane quadrant: tcgen05.ld -> row
+//                   scatter through row_map -> FP32 or FP16 stores of C
 //                   (coalesced along N).
 //
 // Consecutive block rows with a block at the same column form one MMA
@@ -45,12 +45,13 @@
 //     among the copy warps; 148 with gathered blocks (615K -> 284K MMAs, 1.6 ->
 //     1.0 GB into shared memory); 115 with the drain as a loop, (item, column
 //     tile) units and the roles above; 109 with the parts of split panels added
-//     by a kernel of its own and the launches overlapping. The turn of a stage
-//     slot (copy issue, landing, MMAs) sets the pace: 34 bytes a cycle into an SM
-//     of the 70 it can take, tensor pipe busy 30 %.
-//   64^3 stencil, N = 256: 358 -> 178 us, 62 of them packing the FP32 B at 6.5
-//     TB/s; the kernel moves 450 MB of DRAM data in 116.
-//   plain graph, 2^15 rows, 600K entries, N = 256: 231 -> 54 us.
+//     by a kernel of its own and the launches overlapping; 103 with A prefetched
+//     into L2. The turn of a stage slot (copy issue, landing, MMAs) sets the
+//     pace: 36 bytes a cycle into an SM of the 70 it can take, tensor pipe busy
+//     30 %.
+//   64^3 stencil, N = 256: 358 -> 170 us, 62 of them packing the FP32 B at 6.5
+//     TB/s; the kernel moves 450 MB of DRAM data in 108.
+//   plain graph, 2^15 rows, 600K entries, N = 256: 231 -> 52 us.
 //
 // Every wait is bounded (see tc_ptx.cuh); on a timeout the kernel raises the
 // CTA's abort flag, records the site in the global error word, lets the
@@ -122,7 +123,7 @@ struct Cfg {
   static constexpr uint32_t ACC_COLS = NSUB * SUB_COLS;   // TMEM columns per buffer
   static constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
   static constexpr int NMMA = kMmaWarps;                  // MMA-issuing warps
-  static constexpr int NEPI = 8;                          // epilogue warps: a set of four per accumulator buffer
+  static constexpr int NEPI = 8;                          // epilogue warps: two per TMEM lane quadrant
   static constexpr int NPROD = FP8 ? 4 : 6;               // copy warps, in pairs (3 stages in flight)
   static constexpr int NCONV = FP8 ? 4 : 0;               // FP8 converter warps (16..19)
   static constexpr uint32_t SMEM_BARS = 8 * (2 * NS + 4 + NMMA + (FP8 ? 2 * NS : 0) + 2 * kItemRing + 1);
@@ -130,7 +131,7 @@ struct Cfg {
   // then the TMEM address, the abort flag, the ring of work items, the
   // epilogue warps' row tables and the copy warps' gather lists
   static constexpr uint32_t SMEM_BYTES = 1024 + NS * STAGE + SMEM_BARS + 24 + kItemRing * sizeof(WorkItem) +
-                                         NEPI * R * BH * 4 + NPROD * GLIST;
+                                         NEPI * (R * BH / 2) * 4 + NPROD * GLIST;
   static constexpr int THREADS = 32 * (4 + NEPI + NPROD + NCONV);  // MMA, epilogue, copy, converter warps
   static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0,
                 "TMEM allocation must be a power of two in [32, 512]");
@@ -378,8 +379,8 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
   // [kItemRing] work items (panel -1: no more work), 16-byte aligned
   WorkItem* item_ring = reinterpret_cast<WorkItem*>((reinterpret_cast<uintptr_t>(tmem_slot + 2) + 15) &
                                                     ~static_cast<uintptr_t>(15));
-  int* row_tab = reinterpret_cast<int*>(item_ring + kItemRing);  // [NEPI][R * BH] C rows, a table per epilogue warp
-  int* glists = row_tab + C::NEPI * R * BH;                      // [NPROD][GLIST / 4] rows of B of gathered tiles
+  int* row_tab = reinterpret_cast<int*>(item_ring + kItemRing);  // [NEPI][R * BH / 2] C rows, a table per epilogue warp
+  int* glists = row_tab + C::NEPI * (R * BH / 2);                    // [NPROD][GLIST / 4] rows of B of gathered tiles
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // uniform for the compiler
   const int lane = threadIdx.x & 31;
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     }
     for (int i = 0; i < 2; i++) {
       mbar_init(smem_u32(&accfull[i]), C::NMMA);
-      mbar_init(smem_u32(&accempty[i]), 4);
+      mbar_init(smem_u32(&accempty[i]), C::NEPI);
     }
     for (int i = 0; i < C::NMMA; i++) mbar_init(smem_u32(&drainbar[i]), 1);
     if (C::FP8)
@@ -407,7 +408,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       }
     for (int i = 0; i < kItemRing; i++) {
       mbar_init(smem_u32(&itemfull[i]), 1);
-      mbar_init(smem_u32(&itemempty[i]), C::NMMA + 4 + C::NCONV + C::NPROD);  // one lane of every warp
+      mbar_init(smem_u32(&itemempty[i]), C::NMMA + C::NEPI + C::NCONV + C::NPROD);  // one lane of every warp
     }
     mbar_init(smem_u32(stallbar), 1);
     *abort_flag = 0;
@@ -550,10 +551,6 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       }
       if (wi.panel < 0) {
         if (kk == 0) grid_wait();
-        // the end, once more for the other set of epilogue warps
-        if (pw == 0 && elect_one())
-          put_unit(args, taken, itemfull, itemempty, item_ring, abort_flag, err, lim);
-        __syncwarp();
         break;
       }
       const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
@@ -763,43 +760,65 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     }
   } else if (warp >= 4) {
     // -------------------------------------------------------------- epilogue
-    // Two sets of four warps, one per accumulator buffer: while one drains a
-    // unit, the other looks up the next one's rows (8,000 cycles of dependent
-    // global loads a unit on the 64^3 stencil) and drains it as soon as its
-    // MMAs are done. Warp q of a set drains TMEM lane quadrant q (C columns
-    // q*32 .. q*32+31 of each 128-column subtile) for every slot, and writes
-    // zeros back: the accumulators are all zero whenever the MMA warps receive
-    // a buffer, so a part that starts in the middle of a panel accumulates
-    // onto zero.
-    const uint32_t q = warp & 3;
-    const uint32_t buf = (uint32_t)(warp - 4) >> 2;
+    // Eight warps drain a unit together, while the MMAs of the next one fill
+    // the other accumulator buffer: warp (q, h) takes TMEM lane quadrant q (C
+    // columns q*32 .. q*32+31 of each 128-column subtile) of half h of the
+    // slots, and writes zeros back: the accumulators are all zero whenever the
+    // MMA warps receive a buffer, so a part that starts in the middle of a panel
+    // accumulates onto zero. The next unit's rows are on their way meanwhile.
+    // (A set of four warps per buffer took 18,000 cycles for a unit of the 64^3
+    // stencil, with the MMAs' 10,000 before them in the same buffer, and the
+    // lookups, one row load behind the other, 10,000 more: 177 us a call against
+    // 170.)
+    const uint32_t q = warp & 3, h = (uint32_t)(warp - 4) >> 2;
     const uint32_t lane_base = tmem + ((q * 32u) << 16);
-    const uint32_t dbase = lane_base + buf * C::ACC_COLS;
-    for (uint32_t c = 0; c < C::ACC_COLS; c += 16) tmem_st_x16_zero(dbase + c);
+    for (uint32_t c = h * C::ACC_COLS; c < (h + 1) * C::ACC_COLS; c += 16) tmem_st_x16_zero(lane_base + c);
     tmem_st_wait();
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&accempty[buf]));
+    if (lane == 0) {
+      mbar_arrive(smem_u32(&accempty[0]));
+      mbar_arrive(smem_u32(&accempty[1]));
+    }
     constexpr int SLAB = R * BH * C::BN;  // floats per slab
     constexpr int PW = (R % kMmaWarps == 0) ? R / kMmaWarps : 0;  // slots per issuing warp
-    // A drain step takes 32 TMEM columns (a 32-row slot, or two adjacent
-    // 16-row ones) with one load; 16 where a hub row's later parts may be in
-    // its first part's pair (one slot per issuing warp). The steps are a loop:
-    // unrolled, the drain was about 16,000 instructions a pass, and fetching
-    // them set the kernel's pace (64^3 stencil, N = 256: 235 us with every
-    // copy and MMA in place, 190 us with none).
-    constexpr int STEP = 16;
-    int* const rows = row_tab + (warp - 4) * (R * BH);  // this warp's table of the panel's C rows
+    // A drain step takes 16 TMEM columns (a 16-row slot, half a 32-row one) with
+    // one load. The steps are a loop: unrolled, the drain was about 16,000
+    // instructions a pass, and fetching them set the kernel's pace (64^3 stencil,
+    // N = 256: 235 us with every copy and MMA in place, 190 us with none).
+    constexpr int STEP = 16, HALF_ROWS = R * BH / 2, NROW = HALF_ROWS / 32;
+    static_assert(HALF_ROWS % 32 == 0, "a lane per row");
+    int* const rows = row_tab + (warp - 4) * HALF_ROWS;  // this warp's table of its half's C rows
     bool ok = true;
     int odd_prob = -1;                      // problem that odd_known and odd_val are about
     uint64_t odd_known = 0, odd_val = 0;  // a bit per column tile below 64
-    for (uint32_t kk = buf; ok; kk += 2) {
-      WorkItem wi;
-      if (!take_item_warp(itemfull, itemempty, item_ring, kk, lane, abort_flag, err, ERR_ITEM_EPI, lim, true, wi)) {
-        ok = false;
-        break;
-      }
-      if (wi.panel < 0) break;
+    // what the drain of a unit looks up: its half's C rows and the slot masks
+    int row[NROW];
+    uint32_t slot_mask = 0, ext_mask = 0;
+    bool more = true;  // not the end of the work
+    auto look_up = [&](uint32_t kk) {
+      const uint32_t bar = smem_u32(&itemfull[kk % kItemRing]);
+      ok = __all_sync(0xffffffffu, wait_phase_sleepy(bar, (kk / kItemRing) & 1, abort_flag, err, ERR_ITEM_EPI, lim));
+      if (!ok) return;
+      const WorkItem* const it = item_ring + kk % kItemRing;
+      const int panel = it->panel;
+      more = panel >= 0;
+      if (!more) return;
+      const ProblemDesc& P = args.probs ? args.probs[it->prob] : args.one;
+      const int32_t* const rm = P.row_map + (int64_t)panel * R * BH + h * HALF_ROWS + lane;
+#pragma unroll
+      for (int x = 0; x < NROW; ++x) row[x] = __ldg(rm + x * 32);
+      slot_mask = __ldg(&P.panels[panel].slot_mask);
+      // a hub row cut over the issuing warps has its parts in slots s, s + PW,
+      // s + 2 PW, ...; the parts after the first are added into it here
+      ext_mask = __ldg(&P.panels[panel].ext_mask);
+    };
+    look_up(0);
+    for (uint32_t kk = 0; ok && more; ++kk) {
+      const WorkItem wi = item_ring[kk % kItemRing];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&itemempty[kk % kItemRing]));
+      const uint32_t buf = kk & 1, dbase = lane_base + buf * C::ACC_COLS;
       const ProblemDesc& P = args.probs ? args.probs[wi.prob] : args.one;
       // fields used between the stores to C, held in registers (the stores
       // could alias P for the compiler and force reloads of every field)
@@ -808,28 +827,19 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       void* const p_C = P.C;
       const int panel = wi.panel, nt = wi.nt;
       const bool split = wi.split >= 0;
-      // the panel's C rows, loaded before the accumulators are ready, side by
-      // side (one after the other, each behind the shared-memory store of the
-      // one before, they were 10,000 cycles a unit on the 64^3 stencil, now 3,300)
-      int row[R * BH / 32];
-#pragma unroll
-      for (int x = 0; x < R * BH / 32; ++x) row[x] = __ldg(P.row_map + (int64_t)panel * R * BH + x * 32 + lane);
-      const uint32_t slot_mask = __ldg(&P.panels[panel].slot_mask);
-      // a hub row cut over the issuing warps has its parts in slots s, s + PW,
-      // s + 2 PW, ...; the parts after the first are added into it here
-      const uint32_t ext_mask = __ldg(&P.panels[panel].ext_mask);
-      // bit x of `full`: rows 16 x .. 16 x + 15 are all there
-      uint32_t full = 0;
       const int elt = p_f16 ? 2 : 4;
       const int64_t ldb = p_ldc * elt;
+      // bit x of `full`: the half's rows 16 x .. 16 x + 15 are all there
+      uint32_t full = 0;
 #pragma unroll
-      for (int x = 0; x < R * BH / 32; ++x) {
+      for (int x = 0; x < NROW; ++x) {
         rows[x * 32 + lane] = row[x];
         const uint32_t there = __ballot_sync(0xffffffffu, row[x] >= 0);
         full |= ((there & 0xffffu) == 0xffffu ? 1u : 0u) << (2 * x);
         full |= ((there >> 16) == 0xffffu ? 1u : 0u) << (2 * x + 1);
       }
-      if (kk == buf) grid_wait();  // the warp's first unit
+      const uint32_t slots = slot_mask, exts = ext_mask;
+      if (kk == 0) grid_wait();  // the warp's first unit
       const int32_t* const p_pois = P.poison_ptr;
       // does the packed B of these columns hold infinite or NaN values?
       // (looked up once per problem and column tile)
@@ -865,66 +875,60 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       tc_fence_after();
       // slab of (part, column tile): (first slab of the panel + part) * n_tiles + nt
       float* const slab = split ? P.slabs + ((size_t)(wi.slab + wi.part) * n_tiles + nt) * SLAB : nullptr;
+      look_up(kk + 1);
+      if (!ok) break;
 #pragma unroll 1
       for (int j = 0; j < NSUB; ++j) {
         const int nl = j * 128 + (int)q * 32 + lane;  // column inside the tile
         const int n = nt * C::BN + nl;
         uint8_t* const col = static_cast<uint8_t*>(p_C) + (int64_t)n * elt;
 #pragma unroll 1
-        for (int r0 = 0; r0 < R * BH; r0 += STEP) {
+        for (int x = 0; x < HALF_ROWS; x += STEP) {
+          const int r0 = (int)h * HALF_ROWS + x;      // row of the panel
+          const int sl = r0 / BH, off = r0 % BH;      // slot, row inside it
+          if ((exts >> sl) & 1u) continue;            // its first part's warp adds it and writes the zeros
           float v[STEP];
           const uint32_t ta = dbase + j * C::SUB_COLS + r0;
           __syncwarp();  // lanes past N skipped the stores: together again for the aligned loads
           // an empty slot reads zeros: slots are zeroed after every drain and
           // no MMA writes an empty one
-          if ((slot_mask >> (r0 / BH)) & (STEP > BH ? 3u : 1u)) {
-            if constexpr (STEP == 32) {
-              tmem_ld_x32(ta, v);
-              tmem_st_x32_zero(ta);
-            } else {
-              tmem_ld_x16(ta, v);
-              tmem_st_x16_zero(ta);
-            }
+          if ((slots >> sl) & 1u) {
+            tmem_ld_x16(ta, v);
+            tmem_st_x16_zero(ta);
           } else {
 #pragma unroll
             for (int m = 0; m < STEP; ++m) v[m] = 0.0f;
           }
-#pragma unroll
-          for (int g = 0; g < STEP; g += 16) {
-            const int sl = (r0 + g) / BH, h = (r0 + g) % BH;  // slot, row inside it
-            if ((ext_mask >> sl) & 1u) continue;
-            __syncwarp();
-            float* const w = v + g;
-            if constexpr (PW > 0) {
+          __syncwarp();
+          if constexpr (PW > 0) {
 #pragma unroll 1
-              for (int t = sl + PW; t < R && ((ext_mask >> t) & 1u); t += PW) {
-                if (((slot_mask >> t) & 1u) == 0) continue;
-                float u[16];
-                const uint32_t tb = dbase + j * C::SUB_COLS + t * BH + h;
-                tmem_ld_x16(tb, u);
-                tmem_st_x16_zero(tb);
+            for (int t = sl + PW; t < R && ((exts >> t) & 1u); t += PW) {
+              if (((slots >> t) & 1u) == 0) continue;
+              float u[16];
+              const uint32_t tb = dbase + j * C::SUB_COLS + t * BH + off;
+              tmem_ld_x16(tb, u);
+              tmem_st_x16_zero(tb);
 #pragma unroll
-                for (int m = 0; m < 16; ++m) w[m] += u[m];
+              for (int m = 0; m < 16; ++m) v[m] += u[m];
+            }
+          }
+          if (split) {
+            if (((slots >> sl) & 1u) == 0) continue;  // taken as zeros
+            float* const dst = slab + (size_t)r0 * C::BN + nl;
+#pragma unroll
+            for (int m = 0; m < 16; ++m) __stcg(dst + (size_t)m * C::BN, v[m]);
+          } else {
+            if (odd) {
+              const int q0 = p_pois[panel * R + sl], q1 = p_pois[panel * R + sl + 1];
+              if (q0 < q1 && n < p_N && poisoned(P, C::NOPS, q0, q1, n)) {
+#pragma unroll
+                for (int m = 0; m < 16; ++m) v[m] = __int_as_float(0x7fffffff);
               }
             }
-            if (split) {
-              if (((slot_mask >> sl) & 1u) == 0) continue;  // taken as zeros
-              float* const dst = slab + (size_t)(r0 + g) * C::BN + nl;
-#pragma unroll
-              for (int m = 0; m < 16; ++m) __stcg(dst + (size_t)m * C::BN, w[m]);
-            } else {
-              if (odd) {
-                const int q0 = p_pois[panel * R + sl], q1 = p_pois[panel * R + sl + 1];
-                if (q0 < q1 && n < p_N && poisoned(P, C::NOPS, q0, q1, n)) {
-#pragma unroll
-                  for (int m = 0; m < 16; ++m) w[m] = __int_as_float(0x7fffffff);
-                }
-              }
-              const bool fl = (full >> ((r0 + g) / 16)) & 1u;
-              if (n < p_N) {
-                if (p_f16) store_rows16<__half>(col, ldb, rows + r0 + g, fl, w);
-                else store_rows16<float>(col, ldb, rows + r0 + g, fl, w);
-              }
+            const bool fl = (full >> (x / 16)) & 1u;
+            if (n < p_N) {
+              if (p_f16) store_rows16<__half>(col, ldb, rows + x, fl, v);
+              else store_rows16<float>(col, ldb, rows + x, fl, v);
             }
           }
         }
