@@ -114,6 +114,10 @@ smat_status build_sp24(const HostBcsr& b, const std::vector<uint8_t>& take, int 
         nblk += (int)(units[v].second - units[v].first);
         v++;
       }
+      // whole batches (a unit has at most 16 blocks, so one always fits)
+      if (v < units.size()) {
+        for (; (v - u) % kSp24Batch != 0; v--) nblk -= (int)(units[v - 1].second - units[v - 1].first);
+      }
       const int nu = (int)(v - u);
       Sp24Stage S{};
       S.off = (int64_t)out.stream.size();

@@ -9,7 +9,7 @@
 // spmm24.h). It runs after the dense kernel, which writes every row of C from
 // the other blocks, and adds its products into C.
 //
-// Roles (384 threads), one CTA per SM, groups taken round-robin from a list
+// Roles (512 threads), one CTA per SM, groups taken round-robin from a list
 // sorted by decreasing work:
 //   warp 0        MMA issuer (one lane); owns TMEM (two 128-column
 //                 accumulators, then the metadata column of each A-tile
@@ -17,7 +17,7 @@
 //                 kept on a 64-column boundary).
 //   warp 1        stage copies: the compact unit data (values, metadata).
 //   warp 2        B copies: one 8 KB tile (32 rows of B x 128 columns,
-//                 64-byte swizzle) per unit.
+//                 64-byte swizzle) per unit, a batch of two at a time.
 //   warps 4..7    epilogue: tcgen05.ld of the accumulator (lane = row) and
 //                 C[row, :] += it, rows through the row map; C[row, :] = it
 //                 where every block is on this path and no dense kernel ran.
@@ -27,13 +27,14 @@
 //                 metadata word into the unit's TMEM column (tcgen05.st).
 // Units go from the converters to the MMA issuer in batches of two (half the
 // A-tile slots each), with one wait, one fence and one arrival per batch; the
-// sets take every other batch. What bounds the kernel is the latency of the
-// converters' work (330 cycles a unit) and of that hand-off, not the tensor
-// cores; groups with more than an average CTA's units are therefore cut into
+// sets take every other batch, and a batch's B tiles share a barrier. What
+// bounds the kernel is the latency of the converters' work (330 cycles a unit)
+// and of that hand-off, not the tensor cores; groups with more than an average CTA's units are therefore cut into
 // parts over several CTAs (8192 x 8192, 12 % of the blocks, N = 128, 64 groups
 // on 152 SMs, the whole step: 135 us without parts and batches, 68 with them, 61
 // with the second set of converters and every launch a programmatic dependent of
-// the one before, 53 without the dense kernel's pass).
+// the one before, 53 without the dense kernel's pass, 44 with one wait and one
+// release of B a batch instead of a unit).
 // Waits are bounded like the dense kernel's; an expired wait aborts the CTA
 // after its copies and MMAs in flight have landed.
 #include <cuda.h>
@@ -68,13 +69,13 @@ struct Sp24Cfg {
   static constexpr int NB = 2;                                   // batches of slots
   static constexpr int UB = NT / NB;                             // units per batch, at most
   static constexpr uint32_t ATILE = 128 * 32;                    // 128 rows x 16 kept values
-  static constexpr int NBT = 12;                                 // B tile slots (8 KB copies from L2 in flight)
+  static constexpr int NBT = 6;                                  // slots of a batch's B tiles (8 KB copies from L2)
   static constexpr uint32_t BTILE = 128 * 64;                    // 128 columns x 32 k
   static constexpr uint32_t OFF_A = NS * STAGE_SLOT;
   static constexpr uint32_t OFF_B = OFF_A + NT * ATILE;
-  static constexpr uint32_t RING = OFF_B + NBT * BTILE;
+  static constexpr uint32_t RING = OFF_B + NBT * UB * BTILE;
   static constexpr uint32_t NBARS = 2 * NS + 2 * NB + 2 * NBT + 4 + 1;
-  static constexpr uint32_t SMEM_BYTES = 1024 + RING + 8 * NBARS + 8 + 4 * NB + 8;
+  static constexpr uint32_t SMEM_BYTES = 1024 + RING + 8 * NBARS + 8 + 8;
   static constexpr uint32_t META_COL0 = 256;                     // metadata column of A slot t: META_COL0 + 64 t
   static constexpr uint32_t META_STRIDE = 64;
   static constexpr uint32_t TMEM_COLS = 512;                     // 2 x 128 accumulator + NT metadata
@@ -82,6 +83,7 @@ struct Sp24Cfg {
   static_assert(STAGE_MAX % 16 == 0, "stage bytes");
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
   static_assert(META_COL0 + META_STRIDE * (NT - 1) < TMEM_COLS, "metadata columns inside the allocation");
+  static_assert(UB == kSp24Batch, "stages hold whole batches");
 };
 
 __device__ __forceinline__ bool w24(uint32_t bar, uint32_t parity, volatile int* abort, int* err, int where,
@@ -144,7 +146,6 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
   uint64_t* drainbar = accempty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drainbar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* batch_n = abort_flag + 1;  // [NB] units of the batch
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint64_t lim = args.wait_ns ? args.wait_ns : kWaitTimeoutNs;
@@ -211,8 +212,8 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
     }
   } else if (warp == 2) {
     // -------------------------------------------------------------- B copies
-    // The whole warp, one unit at a time; the windows of 32 units are read
-    // together and ahead.
+    // The whole warp, a batch of units at a time (a lane each); the windows of
+    // 32 units are read together and ahead.
     const uint64_t pol = make_l2_policy_evict_last();
     uint32_t u = 0;
     bool ok = true;
@@ -225,18 +226,20 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
           const int mine = ahead;
           if (i0 + 32 + lane < g.nunits) ahead = __ldg(args.unit_window + g.unit0 + i0 + 32 + lane);
           const int cnt = min(32, g.nunits - i0);
-          for (int i = 0; i < cnt; ++i, ++u) {
+          for (int i = 0; i < cnt; i += C::UB, ++u) {
             const uint32_t x = u % C::NBT;
             if (u >= (uint32_t)C::NBT &&
                 !w24_warp(smem_u32(&b_free[x]), ((u - C::NBT) / C::NBT) & 1, abort_flag, err, ERR24_B, lim)) {
               ok = false;
               break;
             }
-            const int w = __shfl_sync(0xffffffffu, mine, i);
+            const int n = min(C::UB, cnt - i);
+            const int w = __shfl_sync(0xffffffffu, mine, (i + lane) & 31);
             const uint32_t fb = smem_u32(&b_full[x]);
-            mbar_arrive_expect_tx_if(fb, C::BTILE, lane == 0);
-            bulk_load_hint_if(smem0 + C::OFF_B + x * C::BTILE, args.bpack64 + ((int64_t)nt * args.kw + w) * C::BTILE,
-                              C::BTILE, fb, pol, lane == 0);
+            mbar_arrive_expect_tx_if(fb, (uint32_t)n * C::BTILE, lane == 0);
+            __syncwarp();
+            bulk_load_hint_if(smem0 + C::OFF_B + (x * C::UB + (lane & (C::UB - 1))) * C::BTILE,
+                              args.bpack64 + ((int64_t)nt * args.kw + w) * C::BTILE, C::BTILE, fb, pol, lane < n);
           }
         }
       }
@@ -248,7 +251,7 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
   } else if (warp == 0) {
     // ----------------------------------------------------------------- MMAs
     if (elect_one()) {
-      uint32_t u = 0, k = 0, bc = 0;
+      uint32_t k = 0, bc = 0;
       bool ok = true, issued = false;
       for (int gi = blockIdx.x; gi < args.n_groups && ok; gi += G) {
         const Sp24Group g = args.groups[gi];
@@ -260,27 +263,25 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
           }
           tc_fence_after();
           for (int i = 0; i < g.nunits && ok; ++bc) {
-            const uint32_t bt = bc % C::NB;
-            if (!w24(smem_u32(&a_ready[bt]), (bc / C::NB) & 1, abort_flag, err, ERR24_MMA, lim)) {
+            const uint32_t bt = bc % C::NB, x = bc % C::NBT;
+            if (!w24(smem_u32(&a_ready[bt]), (bc / C::NB) & 1, abort_flag, err, ERR24_MMA, lim) ||
+                !w24(smem_u32(&b_full[x]), (bc / C::NBT) & 1, abort_flag, err, ERR24_MMA, lim)) {
               ok = false;
               break;
             }
             tc_fence_after();
-            const int n = batch_n[bt];
-            for (int j = 0; j < n; ++j, ++i, ++u) {
-              const uint32_t t = bt * C::UB + (uint32_t)j, x = u % C::NBT;
-              if (!w24(smem_u32(&b_full[x]), (u / C::NBT) & 1, abort_flag, err, ERR24_MMA, lim)) {
-                ok = false;
-                break;
-              }
-              const uint64_t ad = desc_kmajor_sw32(smem0 + C::OFF_A + t * C::ATILE);
-              const uint64_t bd = desc_kmajor_sw64(smem0 + C::OFF_B + x * C::BTILE);
-              umma_sp_f16(tmem + buf * 128, ad, bd, tmem + C::META_COL0 + C::META_STRIDE * t,
-                          args.idesc | ((128u >> 3) << 17), i > 0 ? 1u : 0u);
-              issued = true;
-              umma_commit(smem_u32(&b_free[x]));
-            }
-            if (ok) umma_commit(smem_u32(&a_free[bt]));
+            const uint64_t ad = desc_kmajor_sw32(smem0 + C::OFF_A + bt * C::UB * C::ATILE);
+            const uint64_t bd = desc_kmajor_sw64(smem0 + C::OFF_B + x * C::UB * C::BTILE);
+#pragma unroll
+            for (int j = 0; j < C::UB; ++j)
+              if (i + j < g.nunits)
+                umma_sp_f16(tmem + buf * 128, ad + ((j * C::ATILE) >> 4), bd + ((j * C::BTILE) >> 4),
+                            tmem + C::META_COL0 + C::META_STRIDE * (bt * C::UB + j), args.idesc | ((128u >> 3) << 17),
+                            i + j > 0 ? 1u : 0u);
+            i += C::UB;
+            issued = true;
+            umma_commit(smem_u32(&b_free[x]));
+            umma_commit(smem_u32(&a_free[bt]));
           }
           if (!ok) break;
           umma_commit(smem_u32(&accfull[buf]));
@@ -360,7 +361,6 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
               __syncwarp();
               tmem_st_x1(tmem + ((uint32_t)(q * 32) << 16) + C::META_COL0 + C::META_STRIDE * t, word);
             }
-            if (q == 0 && lane == 0) batch_n[bt] = n;
             __syncwarp();
             tmem_st_wait();
             fence_proxy_async_smem();

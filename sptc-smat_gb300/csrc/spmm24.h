@@ -26,9 +26,11 @@
 namespace smat {
 
 constexpr int kSp24GroupRows = 8;      // block rows per group (M = 128)
-constexpr int kSp24StageUnits = 16;    // units per stage, at most
+constexpr int kSp24Batch = 2;          // units handed from role to role together
+constexpr int kSp24StageUnits = 16;    // units per stage, at most; whole batches but in a group's last stage
 constexpr int kSp24StageBlocks = 32;   // blocks per stage, at most
 constexpr int kSp24BlockBytes = 256 + 32;
+static_assert(kSp24StageBlocks >= 2 * kSp24GroupRows * kSp24Batch, "a batch fits in a stage");
 
 // A unit (16 bytes): its window, blocks and where they are in the stage.
 struct Sp24Unit {
