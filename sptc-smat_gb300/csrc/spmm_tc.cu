@@ -24,7 +24,7 @@
 // both), so the hand-off between the copies and the tensor cores is one
 // full/empty barrier pair per stage.
 //
-// Roles (576 threads, FP8 640):
+// Roles (576 threads, FP8 768):
 //   warps 12..17    copy warps, in pairs that own whole stages: bulk copies for
 //                   the list, the A blocks and the B tiles, 16-byte copies
 //                   through the load path for the rows of gathered tiles.
@@ -125,7 +125,7 @@ struct Cfg {
   static constexpr int NMMA = kMmaWarps;                  // MMA-issuing warps
   static constexpr int NEPI = 8;                          // epilogue warps: two per TMEM lane quadrant
   static constexpr int NPROD = FP8 ? 4 : 6;               // copy warps, in pairs (3 stages in flight)
-  static constexpr int NCONV = FP8 ? 4 : 0;               // FP8 converter warps (16..19)
+  static constexpr int NCONV = FP8 ? 8 : 0;               // FP8 converter warps, two sets of four
   static constexpr uint32_t SMEM_BARS = 8 * (2 * NS + 4 + NMMA + (FP8 ? 2 * NS : 0) + 2 * kItemRing + 1);
   static constexpr int GLIST = (ST + 1) / 2 * 16 * 4;     // bytes of a copy warp's rows of gathered tiles
   // then the TMEM address, the abort flag, the ring of work items, the
@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     for (int i = 0; i < C::NMMA; i++) mbar_init(smem_u32(&drainbar[i]), 1);
     if (C::FP8)
       for (int i = 0; i < C::NS; i++) {
-        mbar_init(smem_u32(&conv[i]), C::NCONV);
+        mbar_init(smem_u32(&conv[i]), C::NCONV / 2);
         mbar_init(smem_u32(&afull[i]), 1);
       }
     for (int i = 0; i < kItemRing; i++) {
@@ -435,11 +435,17 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
   if (C::FP8 && warp >= 4 + C::NEPI + C::NPROD) {
     // ------------------------------------------------------ FP8 converters
     // Each stage's e4m3 blocks and FP32 scales land in the staging area;
-    // these four warps write them to the stage's A area as FP16 (value times
+    // a set of four warps writes them to the stage's A area as FP16 (value times
     // its block's scale, one rounding) in the 32-byte-swizzled layout the
     // MMA reads, make the writes visible to the tensor core's async proxy,
-    // and release the stage to the MMA warps (conv barrier).
-    const int ct = threadIdx.x - 32 * (4 + C::NEPI + C::NPROD);
+    // and release the stage to the MMA warps (conv barrier). One set of four
+    // warps took 1,750 cycles a stage, more than half of them in the fence, and
+    // set the pace; two sets take every other slot (48^3 stencil, N = 256: 115 us
+    // a call with one set, 106 with two, 101 with stages of 9 tiles, four in
+    // flight, instead of 12). A slot always goes to the same set: a set that met
+    // a slot every other time only could take the phase before last for its own.
+    const int ct = (threadIdx.x - 32 * (4 + C::NEPI + C::NPROD)) & 127;
+    const uint32_t set = (uint32_t)(warp - 4 - C::NEPI - C::NPROD) >> 2;
     uint32_t ci = 0;
     bool ok = true;
     for (uint32_t kk = 0; ok; ++kk) {
@@ -452,6 +458,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       {
         for (int c = wi.s0; c < wi.s1; ++c, ++ci) {
           const uint32_t s = ci % nsr;
+          if ((s & 1) != set) continue;
           if (!warp_wait(smem_u32(&afull[s]), (ci / nsr) & 1, lane, abort_flag, err, ERR_CONV, false, lim)) {
             ok = false;
             break;
