@@ -48,8 +48,8 @@ WORKLOAD = {
     "B": "65536x128 FP16 U[-1,1], column-major",
     "C": "FP32, original row order",
     "form": "plain FP16 (tcgen05 kind::f16, FP32 accumulate)",
-    "l2": "no flush: A (~0.4 GB) is larger than the 129 MB L2",
-    "step": "pack B into 4 KB tiles + tensor-core SpMM (2 launches), replayed as one captured CUDA graph",
+    "l2": "no flush: the A stream (0.15 GB) is larger than the 129 MB L2",
+    "step": "pack B into 4 KB tiles + tensor-core SpMM + sum of the split panels (3 launches), replayed as one captured CUDA graph",
 }
 
 
@@ -412,7 +412,7 @@ def run_smat(args):
     for _ in range(max(args.warmup, 3)):
         step()
     torch.cuda.synchronize(dev)
-    # the step (work-counter memset, B packing, contraction) captured once as
+    # the step (B packing, contraction, sums) captured once as
     # a CUDA graph and replayed: the library's calls are capture-safe
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=stream):
@@ -457,7 +457,7 @@ def run_smat(args):
         ms, kern_ms = float(t[0]), float(t[1])
 
     # the same step with the structured-sparse path on: exact-2:4 blocks on
-    # tcgen05.mma.sp (second launch), the others on the dense kernel
+    # tcgen05.mma.sp, the others on the dense kernel
     sp24 = []
     for unit_min in ([] if args.no_sp24 else [1, 8]):
         M24 = smat.Bcsr(A, block=(16, 16), forms=(smat.FORM_F16,), row_perm=perm, device=local, use_24=unit_min)
@@ -499,7 +499,7 @@ def run_smat(args):
                 "n_blocks_24": n24, "nnzb": i24["nnzb"], "rel_err_vs_fp64": err24,
                 "a_bytes": (i24["nnzb"] - n24) * 512 + n24 * 288, "a_bytes_dense_path": i24["nnzb"] * 512,
                 "step": "pack B (4 KB tiles, then 8 KB 2:4 windows) + dense SpMM over the other blocks + "
-                        "tcgen05.mma.sp over the routed exact-2:4 blocks (4 launches), one CUDA graph"})
+                        "tcgen05.mma.sp over the routed exact-2:4 blocks, one CUDA graph"})
         log(f"[bench] 2:4 path (units of >= {unit_min}): {n24} of {i24['nnzb']} blocks on mma.sp, "
             f"{ms24:.4f} ms/step, rel err {err24:.3e}")
         M24.close()
@@ -582,10 +582,10 @@ def run_smat(args):
     peak, peak_kind = peaks()
     achieved = alg_bytes / (kern_ms * 1e-3) / 1e9
     tr = profile_traffic()
-    # the contraction's staging traffic through L2: every stage's A region
-    # (blocks + MMA list) and one 4 KB B tile per distinct block column of a
-    # panel (n_union_cols per 128-column pass)
-    staged = nnzb * 512 + info["n_union_cols"] * 4096 * ((N + 127) // 128)
+    # B through L2 into shared memory: a 4 KB tile per kept block column of a
+    # panel and one per gathered block (n_union_cols per 128-column pass); the
+    # A stream comes on top
+    staged = info["n_union_cols"] * 4096 * ((N + 127) // 128)
     line = {
         "metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
@@ -604,13 +604,13 @@ def run_smat(args):
         "staging": {"bytes_per_launch": staged, "achieved_gbs": staged / (kern_ms * 1e-3) / 1e9,
                     "bytes_per_clk_per_sm": staged / (kern_ms * 1e-3) / 152 / (clk["sm_mhz"] * 1e6)
                     if clk.get("sm_mhz") else None,
-                    "note": "what the stages pull from L2 into shared memory: every A block once plus one 4 KB B "
-                            "tile per distinct block column of a 16-row panel (ncu: 1.86 GB L2->SM per launch); "
-                            "the roofline above counts B once"},
+                    "note": "B tiles the stages pull from L2 into shared memory, 4 KB per kept block column of a "
+                            "panel and per gathered block; the A stream (0.15 GB) comes on top; the roofline "
+                            "above counts B once"},
         "clocks": clk,
         "e2e": {"value": world * useful / (e2e_ms * 1e-3) / 1e12, "unit": "TFLOP/s",
                 "h2d_bytes_per_step": A.cols * N * 2, "d2h_bytes_per_step": A.rows * N * 4, "ms_per_step": e2e_ms},
-        "gpu_launches": 2 * args.steps,
+        "gpu_launches": 3 * args.steps,  # packing, SpMM, sum of the split panels
     }
     if sp24:
         line["sp24_path"] = sp24

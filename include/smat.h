@@ -99,7 +99,7 @@ typedef struct smat_bcsr_opts {
                              once per 256 columns; one more copy of A on the device);
                              with panel_rows = 0 the autotuner's cached choice */
   int32_t pipeline_depth; /* pipeline stages in flight (2..): 0 = as many as fit in shared
-                             memory (3 for the default stage shapes), or the autotuner's
+                             memory (3; FP8 4), or the autotuner's
                              cached choice when panel_rows = 0 */
 } smat_bcsr_opts;
 
@@ -114,7 +114,7 @@ typedef struct smat_bcsr_info {
   int32_t block_rows, block_cols;
   int32_t panel_rows;
   int32_t n_panels;
-  int64_t n_union_cols;         /* B tiles one SpMM pass loads (per N tile) */
+  int64_t n_union_cols;         /* B tiles one SpMM pass loads (per N tile), gathered ones included */
   double fill;                  /* nnz / (nnzb * bh * bw) */
   int32_t n_tile_cols;          /* widest N tile the handle runs: 128, or 256 (FP16 / BF16, N > 128) */
   int32_t pipeline_depth;       /* stages in flight requested (0: all that fit) */
@@ -277,8 +277,8 @@ smat_status smat_tiles_destroy(smat_tiles* t);
 /* ---------------------------------------------------------------- step 3 */
 
 /* Bytes of device scratch smat_spmm needs for this form / B dtype / N: the
- * packed copy of B (twice that for the split form), for panels split over
- * several CTAs for load balance one counter per split panel and a partial-sum
+ * packed copy of B (twice that for the split form), the launch's next-unit
+ * counter, for panels split over several CTAs for load balance a partial-sum
  * slab per part, and a byte per 128 x 64 values of B that says whether they
  * hold an infinite or NaN one. */
 smat_status smat_spmm_workspace_size(const smat_bcsr* A, int32_t form, int32_t b_dtype, int64_t N,
@@ -414,9 +414,9 @@ typedef struct smat_group smat_group;
  * descriptors and scratch (device memory owned by the group); B and C
  * pointers are fixed here. All handles must be on one device. */
 smat_status smat_group_create(const smat_problem* problems, int32_t count, smat_group** out);
-/* Runs the group on `stream`: one grouped B-packing launch, one counter
- * clear, one SpMM launch per kernel variant among the problems (one for
- * FP16/BF16 problems with N <= 128). Allocates and synchronises nothing, so
+/* Runs the group on `stream`: one grouped B-packing launch, then per kernel
+ * variant among the problems (one for FP16/BF16 problems with N <= 128) one
+ * SpMM launch and, where panels are split, one that sums their parts. Allocates and synchronises nothing, so
  * it can be captured in a CUDA graph (after a first run outside capture). */
 smat_status smat_group_run(smat_group* g, void* stream);
 /* As smat_bcsr_check_device_error, for the group's launches. */
