@@ -441,14 +441,23 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
 
 // The split groups' parts, added in order and then into C: a block per 16 rows
 // of a group, a thread per column.
+// What is the handle's own is looked up before the wait for the parts (the step
+// of 8192 x 8192, 12 % of the blocks: 44.4 us with the lookups behind it, 43.5).
 __global__ void __launch_bounds__(128) sum24_kernel(const __grid_constant__ Sp24Args args) {
-  grid_wait();
   const int u = (int)blockIdx.x / args.n_tiles, nt = (int)blockIdx.x % args.n_tiles;
   const Sp24Group g = args.split[u];
   const int j = (int)blockIdx.y;  // block row of the group
   const int n = nt * 128 + (int)threadIdx.x;
   const bool has = (g.row_mask >> j) & 1u;
-  if (n >= args.N || !(has || (args.whole_c && g.group * kSp24GroupRows + j < args.n_brows))) return;
+  const bool mine = n < args.N && (has || (args.whole_c && g.group * kSp24GroupRows + j < args.n_brows));
+  int4 rows[4] = {};
+  if (mine) {
+    const int4* const row4 = reinterpret_cast<const int4*>(args.row_map + (int64_t)g.group * 128 + 16 * j);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) rows[m] = __ldg(row4 + m);
+  }
+  grid_wait();
+  if (!mine) return;
   const float* src = args.slabs + (((int64_t)g.slab * args.n_tiles + nt) * 128 + 16 * j) * 128 + threadIdx.x;
   const int64_t step = (int64_t)args.n_tiles * 128 * 128;
   float acc[16];
@@ -463,7 +472,8 @@ __global__ void __launch_bounds__(128) sum24_kernel(const __grid_constant__ Sp24
   }
 #pragma unroll
   for (int m = 0; m < 16; ++m) {
-    const int row = args.row_map[(int64_t)g.group * 128 + 16 * j + m];
+    const int4 r4 = rows[m / 4];
+    const int row = m % 4 == 0 ? r4.x : (m % 4 == 1 ? r4.y : (m % 4 == 2 ? r4.z : r4.w));
     if (row < 0) continue;
     const int64_t off = (int64_t)row * args.ldc + n;
     if (args.c_f16) {
