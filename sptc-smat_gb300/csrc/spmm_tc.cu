@@ -47,8 +47,8 @@
 //     tile) units and the roles above; 109 with the parts of split panels added
 //     by a kernel of its own and the launches overlapping; 103 with A prefetched
 //     into L2. The turn of a stage slot (copy issue, landing, MMAs) sets the
-//     pace: 36 bytes a cycle into an SM of the 70 it can take, tensor pipe busy
-//     30 %.
+//     pace: 36 bytes a cycle into an SM of the 70 it can take, 44 % of the narrow
+//     MMAs that the tensor pipe could issue.
 //   64^3 stencil, N = 256: 358 -> 170 us, 62 of them packing the FP32 B at 6.5
 //     TB/s; the kernel moves 450 MB of DRAM data in 108.
 //   plain graph, 2^15 rows, 600K entries, N = 256: 231 -> 52 us.
