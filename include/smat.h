@@ -412,7 +412,9 @@ typedef struct smat_group smat_group;
  * reference, which runs one matrix at a time). smat_group_create builds, once,
  * one load-balanced work list over all the problems' block-row panels, their
  * descriptors and scratch (device memory owned by the group); B and C
- * pointers are fixed here. All handles must be on one device. */
+ * pointers are fixed here. All handles must be on one device, and built with
+ * use_24 = 0: a group runs the dense kernel alone, so the blocks that a handle
+ * keeps for the 2:4 path would be left out. */
 smat_status smat_group_create(const smat_problem* problems, int32_t count, smat_group** out);
 /* Runs the group on `stream`: one grouped B-packing launch, then per kernel
  * variant among the problems (one for FP16/BF16 problems with N <= 128) one
