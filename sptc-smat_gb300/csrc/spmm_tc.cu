@@ -352,8 +352,8 @@ __device__ __forceinline__ void gather_tile(uint32_t dst, const uint8_t* b, cons
   }
 }
 
-// Warp roles: 0..3 MMA issuers (0 also owns TMEM), 4..7 epilogue (TMEM lane
-// quadrants 0..3), then NPROD copy warps, then (FP8) the converter warps.
+// Warp roles: 0..3 MMA issuers (0 also owns TMEM), 4..11 epilogue (two per TMEM
+// lane quadrant), then NPROD copy warps, then (FP8) the converter warps.
 template <int BH, int R, int NSUB, int KIND>
 __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     spmm_tc_kernel(const __grid_constant__ SpmmArgs args) {
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     // by the lanes side by side (about 55 cycles each; two warps reach the SM's
     // 74-78 bytes a cycle), and the rows of the gathered tiles with 16-byte
     // copies through the load path. The warps of a pair take every other tile;
-    // as many pairs are at work as stages are in flight. (Eight warps that each
+    // as many pairs are at work as stages are in flight (FP8: two). (Eight that each
     // brought two of every stage's tiles spent 940 cycles a stage on waits,
     // shuffles and arrivals.) A stage's record is read two of the pair's stages
     // ahead, its rows of B one.
