@@ -610,6 +610,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
           ok = false;
           break;
         }
+        __syncwarp();  // the gather list is read by other lanes than those that wrote it; a vote orders no memory
         const uint32_t st = smem0 + slot_s * C::STAGE;
         const uint32_t fb = smem_u32(&full[slot_s]);
         // One bulk copy per lane: the warp's B tiles on the stage's barrier, and

@@ -1,0 +1,33 @@
+"""Shared memory that one lane of a warp writes and another reads needs a
+__syncwarp (or a barrier) in between: votes and shuffles order no memory. The
+order holds by chance where a warp's accesses issue in program order, so no run
+shows the mistake; this reads the source instead."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sptc-smat_gb300", "csrc")
+
+
+def code(name):
+    text = open(os.path.join(CSRC, name)).read()
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def between(text, first, second):
+    """The text from the only match of `first` to the next match of `second`."""
+    starts = list(re.finditer(first, text))
+    assert len(starts) == 1, first
+    tail = text[starts[0].end():]
+    end = re.search(second, tail)
+    assert end, second
+    return tail[:end.start()]
+
+
+def test_gather_list_is_ordered():
+    part = between(code("spmm_tc.cu"), r"reinterpret_cast<int4\*>\(glist\)\[lane\]\s*=", r"gather_tile<")
+    assert "__syncwarp()" in part
+
+
+def test_row_table_is_ordered():
+    part = between(code("spmm_tc.cu"), r"rows\[x \* 32 \+ lane\]\s*=", r"store_rows16<")
+    assert "__syncwarp()" in part
