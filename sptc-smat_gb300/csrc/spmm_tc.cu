@@ -228,6 +228,8 @@ __device__ __noinline__ bool poisoned(const ProblemDesc& P, int nops, int q0, in
 // Bounded wait for a whole warp: lane 0 polls, the warp learns the outcome
 // by shuffle and leaves converged (lanes that each polled would leave the
 // loop on different iterations and could run the code after it diverged).
+// The __syncwarp puts the other lanes behind what lane 0 acquired; a shuffle
+// orders no memory.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int lane, volatile int* abort, int* err,
                                           int where, bool sleepy, uint64_t lim) {
   int got = 1;
@@ -236,6 +238,7 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int lan
                   : wait_phase(bar, parity, abort, err, where, lim))
               ? 1
               : 0;
+  __syncwarp();
   return __shfl_sync(0xffffffffu, got, 0) != 0;
 }
 

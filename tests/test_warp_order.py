@@ -31,3 +31,8 @@ def test_gather_list_is_ordered():
 def test_row_table_is_ordered():
     part = between(code("spmm_tc.cu"), r"rows\[x \* 32 \+ lane\]\s*=", r"store_rows16<")
     assert "__syncwarp()" in part
+
+
+def test_warp_wait_orders_the_other_lanes():
+    part = between(code("spmm_tc.cu"), r"__device__ __forceinline__ bool warp_wait\(", r"\n}")
+    assert "__syncwarp()" in part
