@@ -412,14 +412,16 @@ typedef struct smat_group smat_group;
  * reference, which runs one matrix at a time). smat_group_create builds, once,
  * one load-balanced work list over all the problems' block-row panels, their
  * descriptors and scratch (device memory owned by the group); B and C
- * pointers are fixed here. All handles must be on one device, and built with
- * use_24 = 0: a group runs the dense kernel alone, so the blocks that a handle
- * keeps for the 2:4 path would be left out. */
+ * pointers are fixed here. All handles must be on one device. */
 smat_status smat_group_create(const smat_problem* problems, int32_t count, smat_group** out);
 /* Runs the group on `stream`: one grouped B-packing launch, then per kernel
- * variant among the problems (one for FP16/BF16 problems with N <= 128) one
- * SpMM launch and, where panels are split, one that sums their parts. Allocates and synchronises nothing, so
- * it can be captured in a CUDA graph (after a first run outside capture). */
+ * variant among the problems one SpMM launch and, where panels are split, one
+ * that sums their parts. Problems share a variant when their handles have one
+ * block height, panel height and pass width and their forms one kind (FP16 and
+ * BF16 are one). A problem with blocks on the 2:4 path (use_24) adds that path's
+ * launches: one that packs its B, one or two for its blocks. Allocates and
+ * synchronises nothing, so it can be captured in a CUDA graph (after a first
+ * run outside capture). */
 smat_status smat_group_run(smat_group* g, void* stream);
 /* As smat_bcsr_check_device_error, for the group's launches. */
 smat_status smat_group_check_device_error(smat_group* g);

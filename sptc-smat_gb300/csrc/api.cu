@@ -571,8 +571,12 @@ smat_status smat_csr_to_bcsr_host(const smat_csr* A, int32_t block_rows, int32_t
 }  // extern "C"
 
 // The 2:4 path runs for this form (the exact-2:4 blocks are not in its plan).
-static bool uses_sp24(const smat_bcsr* A, int32_t form) {
+bool smat::uses_sp24(const smat_bcsr* A, int32_t form) {
   return A->sp24_on && (form == SMAT_FORM_F16 || form == SMAT_FORM_BF16);
+}
+
+size_t smat::sp24_slab_bytes(const smat_bcsr* A, int64_t N) {
+  return (size_t)A->sp24_nslabs * ((std::max<int64_t>(N, 1) + 127) / 128) * 128 * 128 * sizeof(float);
 }
 
 WsLayout smat::ws_layout(const smat_bcsr* A, int32_t form, int64_t N, bool whole) {
@@ -592,7 +596,7 @@ WsLayout smat::ws_layout(const smat_bcsr* A, int32_t form, int64_t N, bool whole
   w.slabs24 = w.slabs + n_slabs * n_tiles * A->R * A->host.bh * bn * sizeof(float);
   w.flags = w.slabs24;
   if (uses_sp24(A, form) && !whole)
-    w.flags += (size_t)A->sp24_nslabs * ((std::max<int64_t>(N, 1) + 127) / 128) * 128 * 128 * sizeof(float);
+    w.flags += sp24_slab_bytes(A, N);
   w.total = w.flags + (pack_flag_bytes(A->host.cols, std::max<int64_t>(N, 1)) + 255) / 256 * 256;
   return w;
 }
@@ -628,6 +632,33 @@ void smat::fill_problem(const smat_bcsr* A, int32_t form, const void* ws_, int64
   const uint32_t fmt = (form == SMAT_FORM_F16 || form == SMAT_FORM_FP8) ? 0u : 1u;
   P.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 15) | ((uint32_t)(128 >> 4) << 24);
   P.b_bf16 = (int32_t)fmt;
+}
+
+void smat::fill_sp24(const smat_bcsr* A, int32_t form, const uint8_t* b64, float* slabs, int64_t N, void* C,
+                     int32_t c_dtype, int64_t ldc, Sp24Args& a) {
+  std::memset(&a, 0, sizeof(a));
+  const int fmt = form == SMAT_FORM_BF16 ? 1 : 0;
+  a.stream = A->d_sp24_stream[fmt];
+  a.stages = A->d_sp24_stages;
+  const bool parts = slabs && A->sp24_nsplit > 0;
+  a.groups = parts ? A->d_sp24_items : A->d_sp24_groups;
+  a.n_groups = parts ? A->sp24_nitems : A->sp24_ngroups;
+  a.n_split = parts ? A->sp24_nsplit : 0;
+  a.split = A->d_sp24_split;
+  a.slabs = slabs;
+  a.unit_window = A->d_sp24_unit_window;
+  a.row_map = A->d_bcsr_row_map;
+  a.bpack64 = b64;
+  a.kw = ((A->host.cols + 15) / 16 + 1) / 2;
+  a.C = C;
+  a.ldc = ldc;
+  a.N = (int32_t)N;
+  a.n_tiles = (int32_t)((N + 127) / 128);
+  a.c_f16 = c_dtype == SMAT_F16 ? 1 : 0;
+  // kind::f16 instruction descriptor without N: sparse (bit 2), FP32
+  // accumulator, A and B FP16 (0) or BF16 (1), K-major, M = 128
+  a.idesc = (1u << 2) | (1u << 4) | ((uint32_t)fmt << 7) | ((uint32_t)fmt << 10) | ((uint32_t)(128 >> 4) << 24);
+  a.n_brows = (int32_t)A->host.nbr();
 }
 
 extern "C" {
@@ -786,32 +817,11 @@ static smat_status packed_impl(const smat_bcsr* A, int32_t form, const void* pac
     // where they are all there is (8192 x 8192, 12 % of the blocks, N = 128: 60.7 us
     // a call with the dense kernel storing zeros first, 52.6 without)
     Sp24Args a24;
-    std::memset(&a24, 0, sizeof(a24));
-    const int fmt = form == SMAT_FORM_BF16 ? 1 : 0;
-    a24.stream = A->d_sp24_stream[fmt];
-    a24.stages = A->d_sp24_stages;
-    const bool parts = !whole24 && A->sp24_nsplit > 0;
-    a24.groups = parts ? A->d_sp24_items : A->d_sp24_groups;
-    a24.n_split = parts ? A->sp24_nsplit : 0;
-    a24.split = A->d_sp24_split;
-    a24.slabs = reinterpret_cast<float*>(static_cast<uint8_t*>(const_cast<void*>(packed_b)) + wl.slabs24);
-    a24.unit_window = A->d_sp24_unit_window;
-    a24.row_map = A->d_bcsr_row_map;
-    a24.bpack64 = static_cast<const uint8_t*>(packed_b) + wl.b64;
-    a24.kw = ((hb.cols + 15) / 16 + 1) / 2;
-    a24.C = C;
-    a24.ldc = ldc;
-    a24.N = (int32_t)N;
-    a24.n_tiles = (int32_t)((N + 127) / 128);
-    a24.n_groups = parts ? A->sp24_nitems : A->sp24_ngroups;
-    a24.c_f16 = c_dtype == SMAT_F16 ? 1 : 0;
-    // kind::f16 instruction descriptor without N: sparse (bit 2), FP32
-    // accumulator, A and B FP16 (0) or BF16 (1), K-major, M = 128
-    a24.idesc = (1u << 2) | (1u << 4) | ((uint32_t)fmt << 7) | ((uint32_t)fmt << 10) | ((uint32_t)(128 >> 4) << 24);
+    uint8_t* const ws = static_cast<uint8_t*>(const_cast<void*>(packed_b));
+    fill_sp24(A, form, ws + wl.b64, whole24 ? nullptr : reinterpret_cast<float*>(ws + wl.slabs24), N, C, c_dtype, ldc, a24);
     a24.err = A->d_err;
     a24.wait_ns = A->wait_ns;
     a24.whole_c = all24 ? 1 : 0;
-    a24.n_brows = (int32_t)hb.nbr();
     const int grid = std::max(1, std::min<int>(A->num_sms, a24.n_groups));
     e = sp24_launch(a24, grid, behind_pack || !all24, static_cast<cudaStream_t>(stream_));
     if (e != cudaSuccess) return cuda_fail(e, "2:4 spmm kernel launch");

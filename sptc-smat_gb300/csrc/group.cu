@@ -7,9 +7,11 @@
 // the per-problem descriptors the kernel reads, the packed-B / partial-sum
 // scratch and the jobs of the grouped B packing. smat_group_run then issues
 // one grouped B-packing launch, one SpMM launch per kernel variant among the
-// problems (one for a group of FP16 / BF16 problems with N <= 128) and one that
+// problems (block height, panel height, pass width, kind of form) and one that
 // sums each variant's split panels, and allocates nothing, so it can be captured
-// in a CUDA graph. The pointers B and C are fixed at creation.
+// in a CUDA graph. A problem whose handle keeps blocks for the 2:4 path (use_24)
+// adds that path's launches: its copy of B behind the packing, its products at
+// the end. The pointers B and C are fixed at creation.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -35,6 +37,15 @@ struct Launch {
   int32_t n_splits = 0;
 };
 
+// A problem with blocks on the 2:4 path.
+struct Part24 {
+  Sp24Args args;
+  const uint8_t* packed = nullptr;  // its packed B, and the path's copy of it
+  uint8_t* b64 = nullptr;
+  int64_t K = 0;
+  int grid = 1;
+};
+
 }  // namespace
 
 struct smat_group {
@@ -48,6 +59,7 @@ struct smat_group {
   bool pack_col = false, pack_split = false;  // column-major / split-form operands among them
   int* d_err = nullptr;
   std::vector<Launch> launches;
+  std::vector<Part24> parts24;
 };
 
 static void group_free(smat_group* g) {
@@ -128,7 +140,7 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
 
   // work lists per variant; per problem its scratch sizes
   struct Scratch {
-    size_t packed = 0, slabs = 0, flags = 0, ws_off = 0;
+    size_t packed = 0, slabs = 0, flags = 0, b64 = 0, slabs24 = 0, ws_off = 0;
   };
   std::vector<Scratch> sc(count);
   std::vector<std::vector<WorkItem>> v_items, v_splits;
@@ -154,7 +166,11 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
       const size_t one = (packed_b_bytes(p.A->host.cols, p.N) + 255) / 256 * 256;
       s.packed = kind == TC_KIND_SPLIT ? 2 * one : one;
       s.slabs = (size_t)n_slabs[m] * n_tiles * p.A->R * p.A->host.bh * bn * sizeof(float);
-      s.flags = pack_flag_bytes(p.A->host.cols, p.N);
+      s.flags = (pack_flag_bytes(p.A->host.cols, p.N) + 255) / 256 * 256;
+      if (uses_sp24(p.A, p.form)) {
+        s.b64 = (packed_b64_bytes(p.A->host.cols, p.N) + 255) / 256 * 256;
+        s.slabs24 = sp24_slab_bytes(p.A, p.N);
+      }
     }
     Launch l;
     l.bh = bh;
@@ -173,7 +189,7 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
   size_t ws_total = 0;
   for (Scratch& s : sc) {
     s.ws_off = ws_total;
-    ws_total += (s.packed + s.slabs + s.flags + 255) / 256 * 256;
+    ws_total += (s.packed + s.slabs + s.flags + s.b64 + s.slabs24 + 255) / 256 * 256;
   }
   GTRY(cudaMalloc(reinterpret_cast<void**>(&g->d_ws), std::max<size_t>(ws_total, 256)));
   GTRY(cudaMalloc(reinterpret_cast<void**>(&g->d_counters), std::max<size_t>(16 * g->launches.size(), 256)));
@@ -199,6 +215,16 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
     g->pack_col |= j.layout == 1;
     g->pack_split |= j.out_mode == 2;
     blocks += pack_halves(j.N) * pack_units_k(j.K);
+    if (sc[i].b64 > 0) {
+      Part24 q;
+      q.packed = j.out;
+      q.b64 = j.flags + sc[i].flags;
+      q.K = j.K;
+      fill_sp24(p.A, p.form, q.b64, reinterpret_cast<float*>(q.b64 + sc[i].b64), p.N, p.C, p.c_dtype, p.ldc, q.args);
+      q.args.err = g->d_err;
+      q.grid = std::max(1, std::min<int>(g->num_sms, q.args.n_groups));
+      g->parts24.push_back(q);
+    }
   }
   g->njobs = count;
   g->pack_blocks = blocks;
@@ -233,6 +259,11 @@ smat_status smat_group_run(smat_group* g, void* stream_) {
   cudaError_t e = pack_b_grouped(g->d_jobs, g->njobs, g->pack_blocks, g->pack_col, g->pack_split, g->num_sms,
                                  g->d_counters, (int)(4 * g->launches.size()), s);
   if (e != cudaSuccess) st = fail(SMAT_ERR_CUDA, std::string("grouped B packing: ") + cudaGetErrorString(e));
+  for (size_t v = 0; v < g->parts24.size() && st == SMAT_OK; v++) {
+    const Part24& q = g->parts24[v];
+    e = pack_b_sw64(q.packed, q.K, q.args.N, q.b64, s);
+    if (e != cudaSuccess) st = fail(SMAT_ERR_CUDA, std::string("grouped 2:4 B packing: ") + cudaGetErrorString(e));
+  }
   for (size_t v = 0; v < g->launches.size() && st == SMAT_OK; v++) {
     const Launch& l = g->launches[v];
     SpmmArgs args;
@@ -258,6 +289,12 @@ smat_status smat_group_run(smat_group* g, void* stream_) {
     sa.nops = l.kind == TC_KIND_SPLIT ? 2 : 1;
     e = tc_sum_parts(sa, s);
     if (e != cudaSuccess) st = fail(SMAT_ERR_CUDA, std::string("grouped split panel sums: ") + cudaGetErrorString(e));
+  }
+  // added into the C that the dense kernel and the sums wrote
+  for (size_t v = 0; v < g->parts24.size() && st == SMAT_OK; v++) {
+    const Part24& q = g->parts24[v];
+    e = sp24_launch(q.args, q.grid, true, s);
+    if (e != cudaSuccess) st = fail(SMAT_ERR_CUDA, std::string("grouped 2:4 spmm launch: ") + cudaGetErrorString(e));
   }
   if (prev >= 0 && prev != g->device) cudaSetDevice(prev);
   return st;

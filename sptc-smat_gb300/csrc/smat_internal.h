@@ -303,6 +303,15 @@ struct WsLayout {
 };
 WsLayout ws_layout(const smat_bcsr* A, int32_t form, int64_t N, bool whole = false);
 
+// The 2:4 path of a handle for a form: whether it takes blocks of that form,
+// the bytes of its partial sums, and its launch arguments for the B windows at
+// `b64` (pack_b_sw64); without slabs no group is cut into parts. err, wait_ns and
+// whole_c are the caller's to set.
+bool uses_sp24(const smat_bcsr* A, int32_t form);
+size_t sp24_slab_bytes(const smat_bcsr* A, int64_t N);
+void fill_sp24(const smat_bcsr* A, int32_t form, const uint8_t* b64, float* slabs, int64_t N, void* C, int32_t c_dtype,
+               int64_t ldc, Sp24Args& a);
+
 // smat_spmm; `whole`: with no panel split over CTAs, so that the workspace
 // needs no partial sums.
 smat_status spmm_impl(const smat_bcsr* A, int32_t form, const void* B, int32_t b_dtype, int32_t b_layout, int64_t ldb,
