@@ -616,6 +616,7 @@ void smat::fill_problem(const smat_bcsr* A, int32_t form, const void* ws_, int64
   P.stages = A->pc[cls].d_stages;
   P.row_map = A->pc[cls].d_row_map;
   P.bflags = ws + wl.flags;
+  P.bcols = reinterpret_cast<const uint32_t*>(P.bflags + pack_cols_offset(A->host.cols, N));
   P.gcol = A->pc[cls].d_gcol;
   P.poison_ptr = A->pc[cls].d_poison_ptr;
   P.poison = reinterpret_cast<const int2*>(A->pc[cls].d_poison);

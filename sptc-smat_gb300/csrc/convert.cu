@@ -16,8 +16,9 @@
 // is neither written nor read.
 //
 // A block packs one UNIT: 8 k-blocks of one half. It also says, in the unit's
-// byte of `flags`, whether any packed value is infinite or NaN: the SpMM then
-// restores what a block's stored zeros make of such a value (spmm_tc.cu).
+// byte of `flags`, whether any packed value is infinite or NaN, and in the unit's
+// two words of `cols` in which columns: the SpMM then restores what a block's
+// stored zeros make of such a value (spmm_tc.cu).
 //
 // What bounds it: DRAM and L2 traffic of a copy (268 MB of FP32 in and 134 MB out
 // in 62 us, 6.5 TB/s of the 6.7 a copy reaches; six blocks an SM, 64^3 stencil
@@ -115,8 +116,9 @@ __device__ __forceinline__ void row_chunk(const T* __restrict__ in, int64_t ldi,
 
 // One unit: k-blocks 8 * kc .. 8 * kc + 7 of half hx (columns 64 * hx ..).
 // `tr`: kUnitK * kStride words of shared memory per operand (column-major).
+// Returns, to every thread, whether the unit holds infinite or NaN values.
 template <typename T, int OUT>
-__device__ __forceinline__ void pack_unit(const T* __restrict__ in, int layout, int64_t ldi, uint8_t* __restrict__ out,
+__device__ __forceinline__ bool pack_unit(const T* __restrict__ in, int layout, int64_t ldi, uint8_t* __restrict__ out,
                                           int64_t K, int64_t N, int64_t kc, int64_t hx,
                                           const int32_t* __restrict__ kperm, uint8_t* __restrict__ flags,
                                           uint32_t* tr) {
@@ -196,16 +198,47 @@ __device__ __forceinline__ void pack_unit(const T* __restrict__ in, int layout, 
   const int64_t fs = pack_flag_stride(K);
   if (tid == 0) flags[hx * fs + kc] = any ? 1 : 0;
   if (kc == pack_units_k(K) - 1 && tid > 0 && kc + tid < fs) flags[hx * fs + kc + tid] = 0;  // the unused bytes
+  return any != 0;
+}
+
+// The unit's words of `cols`: the columns in which it holds such values. A thread
+// looks at the chunks it wrote, all of columns 8 * (tid % 8) .. (A call of its own:
+// packing keeps its registers.)
+__device__ __noinline__ void unit_columns(const uint8_t* out, int out_mode, int64_t K, int64_t kc, int64_t hx,
+                                             uint32_t* cols) {
+  __shared__ uint32_t bits[2];
+  const int tid = threadIdx.x;
+  const uint32_t E = out_mode == OUT_F16 ? 0x7c00u : 0x7f80u;
+  const int nops = out_mode == OUT_SPLIT ? 2 : 1;
+  const int64_t kbs = (K + 15) / 16;
+  const uint8_t* const half = out + ((hx >> 1) * kbs + kc * kPackUnitBlocks) * (4096 * nops) + (hx & 1) * (2048 * nops);
+  if (tid < 2) bits[tid] = 0;
+  __syncthreads();
+  uint32_t m = 0;
+#pragma unroll 1
+  for (int kr = tid >> 3; kr < kUnitK && kc * kPackUnitBlocks + (kr >> 4) < kbs; kr += kPackThreads / 8) {
+    const uint32_t* const w = reinterpret_cast<const uint32_t*>(half + (kr >> 4) * (4096 * nops) + (kr & 15) * 128 +
+                                                                (((tid & 7) ^ (kr & 7)) << 4));
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      m |= ((w[i] & E) == E ? 1u : 0u) << (2 * i) | (((w[i] >> 16) & E) == E ? 2u : 0u) << (2 * i);
+  }
+  if (m) atomicOr(&bits[(tid & 7) >> 2], m << (8 * (tid & 3)));
+  __syncthreads();
+  if (tid < 2) cols[(hx * pack_units_k(K) + kc) * 2 + tid] = bits[tid];
 }
 
 template <typename T, int OUT>
 __global__ void __launch_bounds__(kPackThreads, 6)
     pack_b_kernel(const T* __restrict__ in, int layout, int64_t ldi, uint8_t* __restrict__ out, int64_t K, int64_t N,
-                  const int32_t* __restrict__ kperm, uint8_t* __restrict__ flags, int32_t* __restrict__ counters) {
+                  const int32_t* __restrict__ kperm, uint8_t* __restrict__ flags, uint32_t* __restrict__ cols,
+                  int32_t* __restrict__ counters) {
   extern __shared__ uint32_t tr[];
   grid_release();  // the SpMM launched behind may be set up
   if (counters && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kLaunchCounters) counters[threadIdx.x] = 0;
-  pack_unit<T, OUT>(in, layout, ldi, out, K, N, blockIdx.x, blockIdx.y, kperm, flags, tr);
+  const bool any = pack_unit<T, OUT>(in, layout, ldi, out, K, N, blockIdx.x, blockIdx.y, kperm, flags, tr);
+  if (threadIdx.x < 2) cols[((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 2 + threadIdx.x] = 0;
+  if (any) unit_columns(out, OUT, K, blockIdx.x, blockIdx.y, cols);
 }
 
 // Many B operands in one launch: block g packs unit g of the list of all
@@ -225,11 +258,12 @@ __global__ void __launch_bounds__(kPackThreads, 6)
     }
     const PackJob& j = jobs[lo];
     const int64_t nkc = pack_units_k(j.K), kc = (g - j.begin) % nkc, hx = (g - j.begin) / nkc;
+    bool any = false;
 #define SMAT_GPACK(T)                                                                                        \
   switch (j.out_mode) {                                                                                      \
-    case OUT_F16: pack_unit<T, OUT_F16>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, kc, hx, j.kperm, j.flags, tr); break; \
-    case OUT_BF16: pack_unit<T, OUT_BF16>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, kc, hx, j.kperm, j.flags, tr); break; \
-    default: pack_unit<T, OUT_SPLIT>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, kc, hx, j.kperm, j.flags, tr); break; \
+    case OUT_F16: any = pack_unit<T, OUT_F16>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, kc, hx, j.kperm, j.flags, tr); break; \
+    case OUT_BF16: any = pack_unit<T, OUT_BF16>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, kc, hx, j.kperm, j.flags, tr); break; \
+    default: any = pack_unit<T, OUT_SPLIT>((const T*)j.in, j.layout, j.ldi, j.out, j.K, j.N, kc, hx, j.kperm, j.flags, tr); break; \
   }
     switch (j.in_dtype) {
       case 0: SMAT_GPACK(float) break;
@@ -237,6 +271,9 @@ __global__ void __launch_bounds__(kPackThreads, 6)
       default: SMAT_GPACK(__nv_bfloat16) break;
     }
 #undef SMAT_GPACK
+    // every column or none: the exact words, of whichever form, cost the 24 jobs of
+    // 512..8192 rows 0.6-3 us of their 8.7 here (registers), and are a filter only
+    if (threadIdx.x < 2) j.cols[(g - j.begin) * 2 + threadIdx.x] = any ? 0xffffffffu : 0u;
   }
 }
 
@@ -250,13 +287,14 @@ static cudaError_t run_pack(const void* in, int layout, int64_t ldi, uint8_t* ou
                             const int32_t* kperm, uint8_t* flags, int32_t* counters, cudaStream_t s) {
   const int64_t nkc = pack_units_k(K), halves = pack_halves(N);
   if (nkc == 0 || halves == 0) return cudaSuccess;
+  uint32_t* const cols = reinterpret_cast<uint32_t*>(flags + pack_cols_offset(K, N));
   // grid.y is limited to 65,535 halves: wider B goes in several launches
   for (int64_t h0 = 0; h0 < halves; h0 += 65534) {
     const int64_t hn = halves - h0 < 65534 ? halves - h0 : 65534;
     const T* src = (const T*)in + (layout == 1 ? h0 * 64 * ldi : h0 * 64);
     uint8_t* dst = out + (h0 >> 1) * ((K + 15) / 16) * (OUT == OUT_SPLIT ? 8192 : 4096);
     pack_b_kernel<T, OUT><<<dim3((unsigned)nkc, (unsigned)hn), kPackThreads, pack_smem(layout, OUT == OUT_SPLIT), s>>>(
-        src, layout, ldi, dst, K, N - h0 * 64, kperm, flags + h0 * pack_flag_stride(K), counters);
+        src, layout, ldi, dst, K, N - h0 * 64, kperm, flags + h0 * pack_flag_stride(K), cols + h0 * nkc * 2, counters);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -316,7 +354,9 @@ size_t packed_b_bytes(int64_t K, int64_t N) {
   return (size_t)((K + 15) / 16) * (size_t)packed_b_tiles(N) * 4096;
 }
 
-size_t pack_flag_bytes(int64_t K, int64_t N) { return (size_t)pack_halves(N) * (size_t)pack_flag_stride(K); }
+size_t pack_flag_bytes(int64_t K, int64_t N) {
+  return (size_t)pack_cols_offset(K, N) + (size_t)pack_halves(N) * (size_t)pack_units_k(K) * 8;
+}
 
 cudaError_t pack_b(const void* in, int in_dtype, int layout, int64_t ldi, int out_mode, uint8_t* out,
                    int64_t K, int64_t N, const int32_t* kperm, uint8_t* flags, int32_t* counters, cudaStream_t s) {

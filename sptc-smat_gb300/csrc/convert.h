@@ -16,16 +16,20 @@ int64_t packed_b_tiles(int64_t N);
 size_t packed_b_bytes(int64_t K, int64_t N);
 
 // B is packed in units of kPackUnitBlocks k-blocks of one 64-column half tile;
-// each unit has a byte that says whether it holds an infinite or NaN value.
-// The bytes of a half (pack_flag_stride of them, zeros after the last unit)
-// lie one after the other.
+// each unit has a byte that says whether it holds an infinite or NaN value, and
+// a word per 32 columns with a bit for each column that does. The bytes of a half
+// (pack_flag_stride of them, zeros after the last unit) lie one after the other,
+// behind those of all halves the words (two per unit, half by half).
 constexpr int kPackUnitBlocks = 8;
 __host__ __device__ constexpr int64_t pack_units_k(int64_t K) {
   return ((K + 15) / 16 + kPackUnitBlocks - 1) / kPackUnitBlocks;
 }
 __host__ __device__ constexpr int64_t pack_halves(int64_t N) { return (N + 63) / 64; }
 __host__ __device__ constexpr int64_t pack_flag_stride(int64_t K) { return (pack_units_k(K) + 15) / 16 * 16; }
-size_t pack_flag_bytes(int64_t K, int64_t N);
+__host__ __device__ constexpr int64_t pack_cols_offset(int64_t K, int64_t N) {
+  return pack_halves(N) * pack_flag_stride(K);
+}
+size_t pack_flag_bytes(int64_t K, int64_t N);  // the bytes and the words
 
 // Packs B into 4 KB tiles of 16 rows x 128 columns ordered [128-column
 // tile][k-block] (layout: convert.cu), so that the tiles of consecutive
@@ -35,7 +39,7 @@ size_t pack_flag_bytes(int64_t K, int64_t N);
 // tile, twice packed_b_bytes).
 // kperm (device, optional): row kperm[k] of `in` feeds packed row k (a
 // column permutation of A; gathered with scalar loads).
-// flags: pack_flag_bytes() bytes; the units' bytes are written.
+// flags: pack_flag_bytes() bytes; the units' bytes and words are written.
 // counters (optional): kLaunchCounters integers set to zero, for the SpMM
 // launched behind.
 constexpr int kLaunchCounters = 4;
@@ -57,6 +61,7 @@ struct PackJob {
   uint8_t* out;
   const int32_t* kperm;  // column permutation of A (device), or null
   uint8_t* flags;
+  uint32_t* cols;        // flags + pack_cols_offset
   int64_t ldi, K, N, begin;
   int32_t in_dtype, layout, out_mode, pad;
 };

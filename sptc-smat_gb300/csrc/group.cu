@@ -212,6 +212,7 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
     j.layout = p.b_layout == SMAT_COL_MAJOR ? 1 : 0;
     j.out_mode = (p.form == SMAT_FORM_F16 || p.form == SMAT_FORM_FP8) ? 0 : (p.form == SMAT_FORM_SPLIT_BF16 ? 2 : 1);
     j.flags = j.out + sc[i].packed + sc[i].slabs;
+    j.cols = reinterpret_cast<uint32_t*>(j.flags + pack_cols_offset(j.K, j.N));
     g->pack_col |= j.layout == 1;
     g->pack_split |= j.out_mode == 2;
     blocks += pack_halves(j.N) * pack_units_k(j.K);
@@ -238,6 +239,7 @@ smat_status smat_group_create(const smat_problem* probs, int32_t count, smat_gro
       WsLayout wl;  // offsets are replaced below
       fill_problem(p.A, p.form, g->d_ws + sc[i].ws_off, p.N, p.C, p.c_dtype, p.ldc, l.nsub, wl, descs[m]);
       descs[m].bflags = g->d_ws + sc[i].ws_off + sc[i].packed + sc[i].slabs;
+      descs[m].bcols = reinterpret_cast<const uint32_t*>(descs[m].bflags + pack_cols_offset(p.A->host.cols, p.N));
       descs[m].slabs = reinterpret_cast<float*>(g->d_ws + sc[i].ws_off + sc[i].packed);
     }
     GTRY(upload_vec(&l.d_probs, descs));

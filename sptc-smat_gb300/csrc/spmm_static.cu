@@ -40,9 +40,10 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 
-// The limit counts the packed B and the partial sums; a byte per packing unit
-// (at most one per 128 bytes of packed B) comes on top.
-constexpr size_t kFlagRoom = SMAT_SPMM_STATIC_SCRATCH_BYTES / 128 + 4096;
+// The limit counts the packed B and the partial sums; the bytes and words of the
+// packing units (at most 24 bytes per 2,048 of packed B: one k-block in 64 columns)
+// come on top.
+constexpr size_t kFlagRoom = SMAT_SPMM_STATIC_SCRATCH_BYTES / 2048 * 24 + 4096;
 static __device__ __align__(256) uint8_t g_spmm_scratch[SMAT_SPMM_STATIC_SCRATCH_BYTES + kFlagRoom];
 
 std::mutex g_scratch_mu;

@@ -95,6 +95,9 @@ enum : int {
 // Entries of the CTA's ring of work items (the copy warps take items from
 // the launch's counter and run up to a few items ahead of the other roles).
 constexpr int kItemRing = 8;
+// Units of a CTA that it takes note of, so that it can come back to those whose
+// columns of B hold infinite or NaN values.
+constexpr int kNotedUnits = 512;
 
 template <int BH, int R, int NSUB, int KIND>
 struct Cfg {
@@ -129,9 +132,10 @@ struct Cfg {
   static constexpr uint32_t SMEM_BARS = 8 * (2 * NS + 4 + NMMA + (FP8 ? 2 * NS : 0) + 2 * kItemRing + 1);
   static constexpr int GLIST = (ST + 1) / 2 * 16 * 4;     // bytes of a copy warp's rows of gathered tiles
   // then the TMEM address, the abort flag, the ring of work items, the
-  // epilogue warps' row tables and the copy warps' gather lists
+  // epilogue warps' row tables, the copy warps' gather lists and the notes of units
   static constexpr uint32_t SMEM_BYTES = 1024 + NS * STAGE + SMEM_BARS + 24 + kItemRing * sizeof(WorkItem) +
-                                         NEPI * (R * BH / 2) * 4 + NPROD * GLIST;
+                                         NEPI * (R * BH / 2) * 4 + NPROD * GLIST + kNotedUnits * 4 +
+                                         (kNotedUnits / 32 + 1) * 4;
   static constexpr int THREADS = 32 * (4 + NEPI + NPROD + NCONV);  // MMA, epilogue, copy, converter warps
   static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0,
                 "TMEM allocation must be a power of two in [32, 512]");
@@ -203,18 +207,105 @@ __device__ __forceinline__ bool take_item_warp(uint64_t* itemfull, uint64_t* ite
   return true;
 }
 
+// Unit `pos` of the launch; panel -1 past the last one.
+__device__ __forceinline__ WorkItem unit_at(const SpmmArgs& args, int pos) {
+  WorkItem w;
+  w.panel = -1;
+  if (pos < args.n_items) {
+    if (args.probs) {
+      w = args.items[pos];
+    } else {  // one problem: every item once per column tile
+      const uint32_t it = (uint32_t)pos / (uint32_t)args.one.n_tiles;
+      w = args.items[it];
+      w.nt = pos - (int)(it * (uint32_t)args.one.n_tiles);
+    }
+  }
+  return w;
+}
+
 // Infinite and NaN values of B. A block's stored zeros count: zero times such
 // a value is NaN in every row of the block. The columns that gathering left
 // out (all zero in the block) are looked up here, for a launch whose packed B
-// says that it holds such values: whether column n of C is NaN in the rows of
-// the plan slot whose all-zero columns are poison[q0 .. q1).
-__device__ __noinline__ bool poisoned(const ProblemDesc& P, int nops, int q0, int q1, int64_t n) {
+// says that it holds such values: which of the columns `open` of n0 .. n0 + 63 of C
+// (n0 a multiple of 64; all of them below N) are NaN in the rows of the plan slot
+// whose all-zero columns are poison[q0 .. q1). For a whole warp.
+//
+// What bounds it: latency, two loads behind each other for 128 entries. An entry (16
+// rows of B) is looked at only for columns that its packing unit holds such a
+// value in and that are not known yet, so that few are: a lane per entry and the
+// unit's two words of columns, then a lane per 16 bytes of the rows. (One infinity
+// in B, R-MAT of 2^16 rows and 1M entries, N = 128: 140 us a call, 50 without; a
+// thread per column that read every zero column's value took 17,400.)
+__device__ __forceinline__ uint64_t poisoned64(const ProblemDesc& P, int nops, int q0, int q1, int n0, uint64_t open,
+                                               int lane) {
+  const uint32_t E = P.b_bf16 ? 0x7f80u : 0x7c00u;
+  const uint64_t* const cols = reinterpret_cast<const uint64_t*>(P.bcols) + (int64_t)(n0 >> 6) * pack_units_k(P.K);
+  const int r = lane >> 3, c = lane & 7;  // rows r, r + 4, .. of an entry, columns n0 + 8 c ..
+  const uint8_t* const tile = P.bpack + (int64_t)(n0 >> 7) * P.bp_kbs * (4096 * nops) + ((n0 >> 6) & 1) * (2048 * nops);
+  uint64_t bad = 0;
+  for (int q = q0 + lane; q - lane < q1 && open != 0; q += 32 * 4) {
+    int kbs[4];
+    uint64_t in[4], any = 0;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) kbs[x] = q + 32 * x < q1 ? __ldg(&P.poison[q + 32 * x].x) : -1;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) in[x] = kbs[x] >= 0 ? __ldcg(cols + kbs[x] / kPackUnitBlocks) : 0ull;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) any |= in[x];
+    if (!__any_sync(0xffffffffu, (any & open) != 0)) continue;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      for (uint32_t m = __ballot_sync(0xffffffffu, (in[x] & open) != 0); m != 0; m &= m - 1) {
+        const int src = __ffs((int)m) - 1;
+        if ((__shfl_sync(0xffffffffu, in[x], src) & open) == 0) continue;
+        const int kb = __shfl_sync(0xffffffffu, kbs[x], src);
+        const uint32_t mask = (uint32_t)__ldg(&P.poison[q - lane + 32 * x + src].y);
+        const uint8_t* const p = tile + (int64_t)kb * (4096 * nops);
+        uint32_t b = 0;  // bit i: column n0 + 8 c + i
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int k = r + 4 * x;
+          if (((mask >> k) & 1u) == 0) continue;
+          const uint4 v = __ldcg(reinterpret_cast<const uint4*>(p + k * 128 + ((c ^ (k & 7)) << 4)));
+          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int z = 0; z < 4; ++z)
+            b |= ((w[z] & E) == E ? 1u : 0u) << (2 * z) | (((w[z] >> 16) & E) == E ? 2u : 0u) << (2 * z);
+        }
+        b <<= 8 * (c & 3);
+        const uint32_t lo = __reduce_or_sync(0xffffffffu, c < 4 ? b : 0u);
+        const uint32_t hi = __reduce_or_sync(0xffffffffu, c < 4 ? 0u : b);
+        bad |= (lo | (uint64_t)hi << 32) & open;
+        open &= ~bad;
+      }
+    }
+  }
+  return bad;
+}
+
+__device__ __noinline__ uint64_t poisoned64_call(const ProblemDesc& P, int nops, int q0, int q1, int n0, uint64_t open,
+                                               int lane) {
+  return poisoned64(P, nops, q0, q1, n0, open, lane);
+}
+
+// The columns n0 .. n0 + 63 below N, of which `part` (a mask) is wanted.
+__device__ __forceinline__ uint64_t columns64(int n0, int N, uint64_t part) {
+  return N - n0 >= 64 ? part : (N > n0 ? part & ((1ull << (N - n0)) - 1) : 0ull);
+}
+
+// The same for column n alone, by one thread, one load behind the other: in the
+// drain, for units beyond those that a CTA takes note of. (The search above called
+// there, or given to two more warps, took 1-8 % of the time of calls with finite B;
+// at the kernel's end it is inlined for the same reason.)
+__device__ __noinline__ bool poisoned1(const ProblemDesc& P, int nops, int q0, int q1, int64_t n) {
   const uint32_t E = P.b_bf16 ? 0x7f80u : 0x7c00u;
   const uint8_t* base =
       P.bpack + (n >> 7) * P.bp_kbs * (4096 * nops) + ((n >> 6) & 1) * (2048 * nops) + (n & 7) * 2;
+  const uint32_t* const cols = P.bcols + (n >> 6) * pack_units_k(P.K) * 2 + ((n >> 5) & 1);
   const uint32_t c = (uint32_t)(n >> 3) & 7u;
   for (int q = q0; q < q1; ++q) {
     const int2 e = P.poison[q];
+    if (((cols[e.x / kPackUnitBlocks * 2] >> (n & 31)) & 1u) == 0) continue;
     for (uint32_t m = (uint32_t)e.y; m != 0; m &= m - 1) {
       const uint32_t k = (uint32_t)__ffs((int)m) - 1;
       const uint32_t v = *reinterpret_cast<const uint16_t*>(base + (int64_t)e.x * (4096 * nops) + k * 128 +
@@ -223,6 +314,75 @@ __device__ __noinline__ bool poisoned(const ProblemDesc& P, int nops, int q0, in
     }
   }
   return false;
+}
+
+// Whether the packed B of a column tile holds infinite or NaN values, for a whole
+// warp, looked up once per problem and column tile.
+struct OddTiles {
+  int prob = -1;                // problem that known and val are about
+  uint64_t known = 0, val = 0;  // a bit per column tile below 64
+  __device__ __forceinline__ bool look(const ProblemDesc& P, int nsub, int p, int nt, int lane) {
+    if (p != prob) {
+      prob = p;
+      known = val = 0;
+    }
+    const uint64_t bit = nt < 64 ? 1ull << nt : 0ull;
+    if (known & bit) return (val & bit) != 0;
+    const int64_t fs = pack_flag_stride(P.K);
+    const int h0 = nt * (2 * nsub), h1 = min(h0 + 2 * nsub, (P.N + 63) >> 6);
+    const uint4* fl = reinterpret_cast<const uint4*>(P.bflags + (int64_t)h0 * fs);
+    uint32_t any = 0;
+#pragma unroll 4
+    for (int64_t x = lane; x < (h1 - h0) * fs / 16; x += 32) {
+      const uint4 f = __ldcg(fl + x);
+      any |= f.x | f.y | f.z | f.w;
+    }
+    const bool odd = __any_sync(0xffffffffu, any != 0);
+    known |= bit;
+    if (odd) val |= bit;
+    return odd;
+  }
+};
+
+// NaN into what gathering left out of a plan slot's rows (`bh` of them) of C,
+// columns n0 .. n0 + 63, when finite values are stored there.
+__device__ __forceinline__ void poison_slot(const ProblemDesc& P, int nops, int slot, int bh, int n0, uint64_t part,
+                                            int lane) {
+  const int q0 = __ldg(P.poison_ptr + slot), q1 = __ldg(P.poison_ptr + slot + 1);
+  part = columns64(n0, P.N, part);
+  const uint64_t bad = q0 < q1 && part != 0 ? poisoned64(P, nops, q0, q1, n0, part, lane) : 0ull;
+  if (bad == 0) return;
+  const int32_t* const rows = P.row_map + (int64_t)slot * bh;
+  for (int m = 0; m < bh; ++m) {
+    const int row = __ldg(rows + m);
+    for (int n = lane; n < 64; n += 32) {
+      if (row < 0 || ((bad >> n) & 1ull) == 0) continue;
+      const int64_t at = (int64_t)row * P.ldc + n0 + n;
+      if (P.c_f16) static_cast<__half*>(P.C)[at] = __float2half_rn(__int_as_float(0x7fffffff));
+      else static_cast<float*>(P.C)[at] = __int_as_float(0x7fffffff);
+    }
+  }
+  __syncwarp();
+}
+
+// The same for the units whose bits are set in `odd` (units[k]: the CTA's k-th
+// unit), when all of the CTA's units are stored. The CTA's warps share the slots and
+// 64-column pieces of a unit.
+__device__ __forceinline__ void poison_units(const SpmmArgs& args, const int* units, const uint32_t* odd, int nops,
+                                             int bh, int R, int nsub, int warp, int nwarps, int lane) {
+  for (int k = 0; k < kNotedUnits; ++k) {
+    if (((odd[k >> 5] >> (k & 31)) & 1u) == 0) continue;
+    const WorkItem w = unit_at(args, units[k]);
+    const ProblemDesc& P = args.probs ? args.probs[w.prob] : args.one;
+    for (int t = warp; t < 2 * nsub * R; t += nwarps)
+      poison_slot(P, nops, w.panel * R + t % R, bh, w.nt * 128 * nsub + t / R * 64, ~0ull, lane);
+  }
+}
+
+// For an epilogue warp of the FP8 form, behind a unit's drain: its half of the slots
+// and its 32 columns.
+__device__ __noinline__ void poison_half(const ProblemDesc& P, int s0, int nslots, int n0, uint64_t part, int lane) {
+  for (int s = s0; s < s0 + nslots; ++s) poison_slot(P, 1, s, 16, n0, part, lane);
 }
 
 // Bounded wait for a whole warp: lane 0 polls, the warp learns the outcome
@@ -283,22 +443,12 @@ constexpr int kShortUnit = 24;
 // Unit `k` of the CTA into the item ring (one thread): the launch's unit
 // blockIdx.x first, then the next one nobody has taken; panel -1 at the end.
 __device__ __forceinline__ void put_unit(const SpmmArgs& args, uint32_t k, uint64_t* itemfull, uint64_t* itemempty,
-                                         WorkItem* ring, volatile int* abort, int* err, uint64_t lim) {
+                                         WorkItem* ring, int* units, volatile int* abort, int* err, uint64_t lim) {
   const uint32_t r = k % kItemRing;
   if (!wait_phase(smem_u32(&itemempty[r]), ((k / kItemRing) & 1) ^ 1, abort, err, ERR_ITEM_TAKE, lim)) return;
   const int pos = k == 0 ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(args.next_item, 1);
-  WorkItem nw;
-  nw.panel = -1;
-  if (pos < args.n_items) {
-    if (args.probs) {
-      nw = args.items[pos];
-    } else {  // one problem: every item once per column tile
-      const uint32_t it = (uint32_t)pos / (uint32_t)args.one.n_tiles;
-      nw = args.items[it];
-      nw.nt = pos - (int)(it * (uint32_t)args.one.n_tiles);
-    }
-  }
-  ring[r] = nw;
+  if (k < (uint32_t)kNotedUnits) units[k] = pos;
+  ring[r] = unit_at(args, pos);
   mbar_arrive(smem_u32(&itemfull[r]));
 }
 
@@ -384,6 +534,9 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
                                                     ~static_cast<uintptr_t>(15));
   int* row_tab = reinterpret_cast<int*>(item_ring + kItemRing);  // [NEPI][R * BH / 2] C rows, a table per epilogue warp
   int* glists = row_tab + C::NEPI * (R * BH / 2);                    // [NPROD][GLIST / 4] rows of B of gathered tiles
+  int* units = glists + C::NPROD * (C::GLIST / 4);                   // [kNotedUnits] the CTA's first units
+  // [kNotedUnits / 32 + 1] a bit per unit: to come back to; then whether any bit is set
+  volatile uint32_t* odd_units = reinterpret_cast<uint32_t*>(units + kNotedUnits);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // uniform for the compiler
   const int lane = threadIdx.x & 31;
@@ -415,6 +568,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     }
     mbar_init(smem_u32(stallbar), 1);
     *abort_flag = 0;
+    for (int i = 0; i <= kNotedUnits / 32; i++) odd_units[i] = 0;
     fence_barrier_init();
   }
   if (warp == 0) {
@@ -550,7 +704,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       // list (the CTA's own index first, then the shared counter) and puts it
       // in the item ring once every role has read the entry it replaces.
       if (pw == 0 && taken == kk) {
-        if (elect_one()) put_unit(args, taken, itemfull, itemempty, item_ring, abort_flag, err, lim);
+        if (elect_one()) put_unit(args, taken, itemfull, itemempty, item_ring, units, abort_flag, err, lim);
         __syncwarp();
         ++taken;
       }
@@ -594,7 +748,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       // without a wait (a long one would be taken from a CTA that is free
       // earlier)
       if (pw == 0 && wi.s1 - wi.s0 <= kShortUnit) {
-        if (elect_one()) put_unit(args, taken, itemfull, itemempty, item_ring, abort_flag, err, lim);
+        if (elect_one()) put_unit(args, taken, itemfull, itemempty, item_ring, units, abort_flag, err, lim);
         __syncwarp();
         ++taken;
       }
@@ -801,8 +955,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     static_assert(HALF_ROWS % 32 == 0, "a lane per row");
     int* const rows = row_tab + (warp - 4) * HALF_ROWS;  // this warp's table of its half's C rows
     bool ok = true;
-    int odd_prob = -1;                      // problem that odd_known and odd_val are about
-    uint64_t odd_known = 0, odd_val = 0;  // a bit per column tile below 64
+    OddTiles odds;
     // what the drain of a unit looks up: its half's C rows and the slot masks
     int row[NROW];
     uint32_t slot_mask = 0, ext_mask = 0;
@@ -852,31 +1005,16 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       const uint32_t slots = slot_mask, exts = ext_mask;
       if (kk == 0) grid_wait();  // the warp's first unit
       const int32_t* const p_pois = P.poison_ptr;
-      // does the packed B of these columns hold infinite or NaN values?
-      // (looked up once per problem and column tile)
-      bool odd = false;
-      if (p_pois != nullptr) {
-        if (wi.prob != odd_prob) {
-          odd_prob = wi.prob;
-          odd_known = odd_val = 0;
+      // Does the packed B of these columns hold infinite or NaN values? Then the CTA
+      // comes back to the unit at its end (FP8: the warp does so behind the drain,
+      // 48^3 stencil 100 us a call that way and 103 the other, 101 before).
+      bool odd = p_pois != nullptr && !split && odds.look(P, NSUB, wi.prob, nt, lane);
+      if (!C::FP8 && odd && kk < (uint32_t)kNotedUnits) {
+        if (warp == 4 && lane == 0) {
+          odd_units[kk >> 5] |= 1u << (kk & 31);
+          odd_units[kNotedUnits / 32] = 1;
         }
-        const uint64_t bit = nt < 64 ? 1ull << nt : 0ull;
-        if ((odd_known & bit) == 0) {
-          const int64_t fs = pack_flag_stride(P.K);
-          const int h0 = nt * (2 * NSUB), h1 = min(h0 + 2 * NSUB, (p_N + 63) >> 6);
-          const uint4* fl = reinterpret_cast<const uint4*>(P.bflags + (int64_t)h0 * fs);
-          uint32_t any = 0;
-#pragma unroll 4
-          for (int64_t x = lane; x < (h1 - h0) * fs / 16; x += 32) {
-            const uint4 f = __ldcg(fl + x);
-            any |= f.x | f.y | f.z | f.w;
-          }
-          odd = __any_sync(0xffffffffu, any != 0);
-          odd_known |= bit;
-          if (odd) odd_val |= bit;
-        } else {
-          odd = (odd_val & bit) != 0;
-        }
+        odd = false;
       }
       __syncwarp();
       if (!warp_wait(smem_u32(&accfull[buf]), (kk >> 1) & 1, lane, abort_flag, err, ERR_EPI, true, lim)) {
@@ -929,9 +1067,9 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
 #pragma unroll
             for (int m = 0; m < 16; ++m) __stcg(dst + (size_t)m * C::BN, v[m]);
           } else {
-            if (odd) {
+            if (!C::FP8 && odd) {
               const int q0 = p_pois[panel * R + sl], q1 = p_pois[panel * R + sl + 1];
-              if (q0 < q1 && n < p_N && poisoned(P, C::NOPS, q0, q1, n)) {
+              if (q0 < q1 && n < p_N && poisoned1(P, C::NOPS, q0, q1, n)) {
 #pragma unroll
                 for (int m = 0; m < 16; ++m) v[m] = __int_as_float(0x7fffffff);
               }
@@ -949,6 +1087,9 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&accempty[buf]));
+      if (C::FP8 && odd)
+        poison_half(P, panel * R + (int)h * (R / 2), R / 2, nt * C::BN + (int)(q >> 1) * 64, 0xffffffffull << (32 * (q & 1)),
+                    lane);
     }
   }
 
@@ -961,6 +1102,8 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     tc_fence_after();
     tmem_dealloc(tmem, C::TMEM_COLS);
   }
+  if (!C::FP8 && odd_units[kNotedUnits / 32] != 0 && *abort_flag == 0)
+    poison_units(args, units, const_cast<const uint32_t*>(odd_units), C::NOPS, BH, R, NSUB, warp, C::THREADS / 32, lane);
 }
 
 // C of the split panels: block (unit, 16 plan rows) adds the parts' slab rows
@@ -1017,7 +1160,10 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ 
         const uint4 f = __ldcg(fl + x);
         any |= f.x | f.y | f.z | f.w;
       }
-      if (__syncthreads_or((int)any) && n < P.N && poisoned(P, a.nops, q0, q1, n)) {
+      const int lane = (int)threadIdx.x & 31, n64 = n & ~63;
+      const uint64_t part = columns64(n64, P.N, 0xffffffffull << (n & 32));
+      if (__syncthreads_or((int)any) && part != 0 &&
+          ((poisoned64_call(P, a.nops, q0, q1, n64, part, lane) >> (n & 63)) & 1ull)) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) acc[m] = __int_as_float(0x7fffffff);
       }

@@ -112,6 +112,7 @@ struct alignas(16) WorkItem {
 struct ProblemDesc {
   const uint8_t* bpack;      // B in 4 KB tiles [128-column tile][k-block] (pack_b), 8 KB in the split form
   const uint8_t* bflags;     // a byte per packing unit: holds infinite or NaN values
+  const uint32_t* bcols;     // a bit per packing unit and column: the same
   const int32_t* gcol;       // [16 g + x]: rows of B of gathered block g (gather_list), or -1
   const int32_t* poison_ptr; // [panels * R + 1] per plan slot: its range of `poison`; null without gathering
   const int2* poison;        // k-block and mask of its all-zero columns, per gathered block
