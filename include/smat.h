@@ -443,7 +443,8 @@ smat_status smat_spmm_host(const smat_bcsr* A, int32_t form, const void* B_host,
 smat_status smat_bcsr_check_device_error(const smat_bcsr* A);
 
 /* Limit, in nanoseconds, of every device-side wait in this handle's SpMM
- * launches (0: the default, 4 s). A wait that runs out aborts the launch:
+ * launches (0: the default, 4 s), counted from when the launches before are
+ * done. A wait that runs out aborts the launch:
  * the kernel drains its own copies and MMAs, frees its tensor memory and
  * returns, and smat_bcsr_check_device_error reports SMAT_ERR_TIMEOUT; the
  * handle stays usable. No counterpart in the reference, whose waits are

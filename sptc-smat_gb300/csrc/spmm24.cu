@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
         for (int nt = 0; nt < args.n_tiles && ok; ++nt)
           for (int st = 0; st < g.nstages; ++st, ++sc) {
             const uint32_t slot = sc % C::NS;
+            if (sc == (uint32_t)C::NS) grid_wait();  // slots are freed behind it
             if (sc >= (uint32_t)C::NS &&
                 !w24(smem_u32(&s_free[slot]), ((sc - C::NS) / C::NS) & 1, abort_flag, err, ERR24_STAGE, lim)) {
               ok = false;
@@ -253,6 +254,7 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
     if (elect_one()) {
       uint32_t k = 0, bc = 0;
       bool ok = true, issued = false;
+      grid_wait();  // the limit of its waits is not for the launches before
       for (int gi = blockIdx.x; gi < args.n_groups && ok; gi += G) {
         const Sp24Group g = args.groups[gi];
         for (int nt = 0; nt < args.n_tiles && ok; ++nt, ++k) {
@@ -308,12 +310,19 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
     const int r = q * 32 + lane;
     const int j = r >> 4, rr = r & 15;
     uint32_t bc = 0, sc = 0;
-    bool ok = true;
+    bool ok = true, behind = false;
+    // what the first batches and stages need is there without the launches before;
+    // the rest comes when MMAs have freed their slots
+    auto wait_before = [&](bool first) {
+      if (!first && !behind) grid_wait();
+      behind |= !first;
+    };
     for (int gi = blockIdx.x; gi < args.n_groups && ok; gi += G) {
       const Sp24Group g = args.groups[gi];
       for (int nt = 0; nt < args.n_tiles && ok; ++nt)
         for (int st = 0; st < g.nstages && ok; ++st, ++sc) {
           const uint32_t slot = sc % C::NS;
+          wait_before(sc < (uint32_t)C::NS);
           if (!w24_warp(smem_u32(&s_full[slot]), (sc / C::NS) & 1, abort_flag, err, ERR24_CONV, lim)) {
             ok = false;
             break;
@@ -328,6 +337,7 @@ __global__ void __launch_bounds__(Sp24Cfg::THREADS, 1) spmm24_kernel(const __gri
             const uint32_t bt = bc % C::NB;
             if (bt != set) continue;  // the other set's batch
             const int n = min(C::UB, nunits - i0);
+            wait_before(bc < (uint32_t)C::NB);
             if (bc >= (uint32_t)C::NB &&
                 !w24_warp(smem_u32(&a_free[bt]), ((bc - C::NB) / C::NB) & 1, abort_flag, err, ERR24_CONV, lim)) {
               ok = false;

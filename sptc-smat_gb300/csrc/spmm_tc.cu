@@ -584,7 +584,8 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
   // zero next-unit counter, a C nobody reads any more) is first used by the
   // copy warps and the epilogue, which wait for it there; the plan and A's
   // stream are the handle's own, so the first unit's lookups overlap the
-  // packing of B.
+  // packing of B. The other roles wait for it too, before their first bounded
+  // wait: a limit is for this kernel's work, not for the launch before it.
 
   int* err = args.err;
   const uint32_t smem0 = smem_u32(smem);
@@ -605,6 +606,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
     const uint32_t set = (uint32_t)(warp - 4 - C::NEPI - C::NPROD) >> 2;
     uint32_t ci = 0;
     bool ok = true;
+    grid_wait();
     for (uint32_t kk = 0; ok; ++kk) {
       WorkItem wi;
       if (!take_item_warp(itemfull, itemempty, item_ring, kk, lane, abort_flag, err, ERR_ITEM_CONV, lim, false, wi)) {
@@ -836,6 +838,7 @@ __global__ void __launch_bounds__(Cfg<BH, R, NSUB, KIND>::THREADS, 1)
       uint32_t ci = 0, k = 0, slot_s = 0, phase_s = 0;
       bool ok = true, issued = false;
       const uint32_t stall = (blockIdx.x == 0 && warp == 0) ? (uint32_t)args.stall_stage : 0u;
+      grid_wait();
       for (uint32_t kk = 0; ok; ++kk) {
         WorkItem wi;
         if (!take_item_one(itemfull, itemempty, item_ring, kk, abort_flag, err, ERR_ITEM_MMA, lim, wi)) {

@@ -36,3 +36,17 @@ def test_row_table_is_ordered():
 def test_warp_wait_orders_the_other_lanes():
     part = between(code("spmm_tc.cu"), r"__device__ __forceinline__ bool warp_wait\(", r"\n}")
     assert "__syncwarp()" in part
+
+
+def test_roles_wait_for_the_launch_before_ahead_of_their_limits():
+    """A kernel launched behind another one starts while that one runs. A role's bounded
+    waits must not count it (they are too coarse to see that in a run: the launch
+    before would have to take milliseconds with all of its blocks resident)."""
+    tc, s24 = code("spmm_tc.cu"), code("spmm24.cu")
+    assert "grid_wait();" in between(tc, r"const int ct = \(threadIdx\.x", r"take_item_warp\(")        # converters
+    assert "grid_wait();" in between(tc, r"const uint32_t stall =", r"take_item_one\(")                # MMAs
+    assert "grid_wait();" in between(s24, r"bool ok = true, issued = false;", r"w24\(")                # MMAs
+    part = between(s24, r"bool ok = true, behind = false;", r"!w24_warp\(smem_u32\(&a_free")           # converters
+    assert "grid_wait();" in part and part.count("wait_before(") == 2
+    stages = between(s24, r"if \(warp == 1\) \{", r"!w24\(smem_u32\(&s_free")                          # stage copies
+    assert "grid_wait();" in stages
