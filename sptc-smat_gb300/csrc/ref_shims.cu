@@ -83,26 +83,34 @@ Key make_key(int dev, size_t M, size_t K, size_t nnzb, int bw, std::initializer_
   return Key{dev, M, K, nnzb, bw, a};
 }
 
-// The SpMM of a cached entry on the legacy default stream: the static
-// scratch when it is large enough, else the entry's own workspace.
+// The SpMM of a cached entry on the legacy default stream: the static scratch
+// when it holds the packed B and the partial sums of split panels, else the
+// entry's own workspace (4096 x 8192 with eight heavy panels, N = 1024: 76 us a
+// call; 86 in the static scratch, with whole panels), and where that cannot be
+// allocated the static scratch all the same.
 smat_status spmm_entry(Entry& e, const half* B, half* C, size_t N, size_t K) {
   size_t need = 0;
   smat_status st = smat_spmm_workspace_size(e.h, SMAT_FORM_F16, SMAT_F16, (int64_t)N, &need);
   if (st != SMAT_OK) return st;
   bool whole = false;
-  if (smat::static_scratch_fits(e.h, SMAT_FORM_F16, (int64_t)N, &whole))
-    return smat_spmm_static_scratch(e.h, SMAT_FORM_F16, B, SMAT_F16, SMAT_COL_MAJOR, (int64_t)K, C, SMAT_F16,
-                                    (int64_t)N, (int64_t)N, nullptr);
-  if (need > e.ws_bytes) {
+  const bool fits = smat::static_scratch_fits(e.h, SMAT_FORM_F16, (int64_t)N, &whole);
+  bool use_static = fits && !whole;
+  if (!use_static && need > e.ws_bytes) {
     if (e.ws) cudaFree(e.ws);
     e.ws = nullptr;
     e.ws_bytes = 0;
-    if (cudaMalloc(&e.ws, need) != cudaSuccess) {
+    if (cudaMalloc(&e.ws, need) == cudaSuccess) {
+      e.ws_bytes = need;
+    } else {
       cudaGetLastError();
-      return smat::fail(SMAT_ERR_NOMEM, "workspace for the packed B: cudaMalloc failed");
+      e.ws = nullptr;
+      if (!fits) return smat::fail(SMAT_ERR_NOMEM, "workspace for the packed B: cudaMalloc failed");
+      use_static = true;
     }
-    e.ws_bytes = need;
   }
+  if (use_static)
+    return smat_spmm_static_scratch(e.h, SMAT_FORM_F16, B, SMAT_F16, SMAT_COL_MAJOR, (int64_t)K, C, SMAT_F16,
+                                    (int64_t)N, (int64_t)N, nullptr);
   return smat_spmm(e.h, SMAT_FORM_F16, B, SMAT_F16, SMAT_COL_MAJOR, (int64_t)K, C, SMAT_F16, (int64_t)N, (int64_t)N,
                    e.ws, e.ws_bytes, nullptr);
 }
