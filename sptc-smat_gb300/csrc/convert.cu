@@ -305,14 +305,16 @@ static cudaError_t run_pack(const void* in, int layout, int64_t ldi, uint8_t* ou
 // 2w and 2w+1 of column tile t side by side, 128 rows (n) of 64 bytes (32
 // k-values) in the 64-byte swizzle (inside every 8-row group, 16-byte chunk
 // c of row n sits at chunk c ^ ((n >> 1) & 3)). One thread per row n; the
-// lanes of a warp read neighbouring columns of one row k.
+// lanes of a warp read neighbouring columns of one row k. Zeros for a half
+// without a column below N, which is not packed.
 __global__ void pack_b_sw64_kernel(const uint8_t* __restrict__ p, uint8_t* __restrict__ out, int64_t kbs,
-                                   int64_t kw) {
+                                   int64_t kw, int64_t N) {
   grid_release();  // the kernels launched behind may be set up
   grid_wait();     // the packed tiles
   const int64_t w = blockIdx.x;
   const int64_t t = blockIdx.y;
   const int n = threadIdx.x;
+  const bool packed = t * 128 + (n & 64) < N;
   uint4 c[4];
   uint16_t* const v = reinterpret_cast<uint16_t*>(c);
 #pragma unroll
@@ -321,8 +323,9 @@ __global__ void pack_b_sw64_kernel(const uint8_t* __restrict__ p, uint8_t* __res
     const uint8_t* src = p + (t * kbs + kb) * 4096 + (n >> 6) * 2048 + (n & 7) * 2;
 #pragma unroll
     for (int k = 0; k < 16; ++k)
-      v[hb * 16 + k] = kb < kbs ? *reinterpret_cast<const uint16_t*>(src + k * 128 + ((((n >> 3) & 7) ^ (k & 7)) << 4))
-                                : (uint16_t)0;
+      v[hb * 16 + k] = packed && kb < kbs
+                           ? *reinterpret_cast<const uint16_t*>(src + k * 128 + ((((n >> 3) & 7) ^ (k & 7)) << 4))
+                           : (uint16_t)0;
   }
   uint4* dst = reinterpret_cast<uint4*>(out + (t * kw + w) * 8192 + n * 64);
   const int sw = (n >> 1) & 3;
@@ -338,10 +341,10 @@ size_t packed_b64_bytes(int64_t K, int64_t N) {
 }
 
 cudaError_t pack_b_sw64(const uint8_t* packed, int64_t K, int64_t N, uint8_t* out, cudaStream_t s) {
-  const int64_t kbs = (K + 15) / 16, kw = (kbs + 1) / 2, nt = packed_b_tiles(N);
+  const int64_t kbs = (K + 15) / 16, kw = (kbs + 1) / 2, nt = (N + 127) / 128;
   if (kw == 0 || nt == 0) return cudaSuccess;
   dim3 grid((unsigned)kw, (unsigned)nt);
-  void* params[] = {&packed, &out, const_cast<int64_t*>(&kbs), const_cast<int64_t*>(&kw)};
+  void* params[] = {&packed, &out, const_cast<int64_t*>(&kbs), const_cast<int64_t*>(&kw), &N};
   return launch_kernel(reinterpret_cast<const void*>(dev::pack_b_sw64_kernel), grid, dim3(128), 0, s, true, params);
 }
 
