@@ -107,7 +107,8 @@ smat_status smat_spmm_static_scratch(const smat_bcsr* A, int32_t form, const voi
   bool whole = false;
   if (!smat::static_scratch_fits(A, form, N, &whole))
     return smat::fail(SMAT_ERR_UNSUPPORTED,
-                      "packed B needs " + std::to_string(need) + " bytes but the static scratch holds " +
+                      "packed B needs " + std::to_string(smat::ws_layout(A, form, N, true).flags) +
+                          " bytes but the static scratch holds " +
                           std::to_string((size_t)SMAT_SPMM_STATIC_SCRATCH_BYTES) +
                           "; use smat_spmm with a caller-provided workspace");
   void* scratch = nullptr;
