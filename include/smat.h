@@ -97,7 +97,7 @@ typedef struct smat_bcsr_opts {
                              panel_rows <= 8 the handle also holds a plan for 256-column
                              passes, which the FP16 and BF16 forms use for N > 128 (A read
                              once per 256 columns; one more copy of A on the device);
-                             with panel_rows = 0 the autotuner's cached choice */
+                             with panel_rows = 0 the autotuner's cached choice, else 128 */
   int32_t pipeline_depth; /* pipeline stages in flight (2..): 0 = as many as fit in shared
                              memory (3; FP8 4), or the autotuner's
                              cached choice when panel_rows = 0 */

@@ -118,6 +118,7 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
   int R = o.panel_rows ? o.panel_rows : default_panel_rows(bh, h->host.nbr(), h->num_sms);
   float split_frac = o.split_frac;
   int ntc = o.n_tile_cols, depth = o.pipeline_depth;
+  bool chosen = o.panel_rows != 0;  // the caller's or the autotuner's panel height
   if (o.panel_rows == 0) {
     // a configuration the autotuner measured for matrices like this one
     // (measured for N <= 128 first, else for N <= 256)
@@ -126,6 +127,7 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
       TuneVal tv;
       if (tune_key_of(h->host, kind_of(SMAT_FORM_F16), n_try, key) && tune_lookup(key, tv)) {
         R = tv.panel_rows;
+        chosen = true;
         if (o.split_frac == 0.0f) split_frac = tv.split_frac;
         if (o.n_tile_cols == 0) ntc = tv.n_tile_cols;
         if (o.pipeline_depth == 0) depth = tv.depth;
@@ -153,7 +155,9 @@ static smat_status finish_handle(smat_bcsr* h, const smat_bcsr_opts& o, smat_bcs
   if (h->use24 > 0 && bh == 16 && bw == 16 && (forms & ((1u << SMAT_FORM_F16) | (1u << SMAT_FORM_BF16))))
     route_sp24(h->host, h->use24, take24);
   h->sp24_on = std::any_of(take24.begin(), take24.end(), [](uint8_t v) { return v != 0; });
-  const bool wide = ntc == 256 && (forms & ((1u << SMAT_FORM_F16) | (1u << SMAT_FORM_BF16))) &&
+  // (the library's own panel height leaves it at 128 columns: whether a matrix then
+  // gets a second copy of A does not hang on how many panels it has)
+  const bool wide = ntc == 256 && chosen && (forms & ((1u << SMAT_FORM_F16) | (1u << SMAT_FORM_BF16))) &&
                     tc_variant_supported(bh, R, 2, TC_KIND_PLAIN);
   for (int cls = 0; cls < kPlanClasses; cls++) {
     if (cls == 1 && !(forms & (1u << SMAT_FORM_SPLIT_BF16))) continue;
