@@ -498,8 +498,6 @@ __global__ void __launch_bounds__(128) sum24_kernel(const __grid_constant__ Sp24
 
 }  // namespace dev
 
-int sp24_threads() { return dev::Sp24Cfg::THREADS; }
-
 cudaError_t sp24_launch(const Sp24Args& args, int grid, bool behind, cudaStream_t stream) {
   static std::atomic<uint64_t> done{0};
   int d = 0;

@@ -89,6 +89,5 @@ struct Sp24Args {
 // behind: a programmatic dependent of the launch before it, which is one of the
 // same call.
 cudaError_t sp24_launch(const Sp24Args& args, int grid, bool behind, cudaStream_t stream);
-int sp24_threads();
 
 }  // namespace smat

@@ -78,7 +78,6 @@ enum : int { KIND_PLAIN = 0, KIND_SPLIT = 1, KIND_FP8 = 2 };
 // Error sites recorded in the global error word.
 enum : int {
   ERR_PROD_A = 102,
-  ERR_PROD_B = 101,
   ERR_MMA_ACC = 201,
   ERR_MMA_A = 202,
   ERR_MMA_B = 203,
@@ -401,8 +400,6 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int lan
   __syncwarp();
   return __shfl_sync(0xffffffffu, got, 0) != 0;
 }
-
-__device__ __forceinline__ int shfl_i(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 
 // Stores a column of 16 rows of C: v[m] to row rows[m] (in shared memory, the
 // same for every lane; -1: none) of rows `ldb` bytes apart, base = the

@@ -1,5 +1,5 @@
 // tc_ptx.cuh — inline-PTX building blocks for sm_103a: mbarriers with bounded
-// waits, TMA tiled loads, tcgen05 (TMEM alloc, MMA, commit, loads) and the
+// waits, bulk copies, tcgen05 (TMEM alloc, MMA, commit, loads) and the
 // shared-memory matrix descriptors the MMA reads its operands through.
 #pragma once
 
@@ -114,39 +114,12 @@ static __device__ __noinline__ bool mbar_wait_sleepy(uint32_t bar, uint32_t pari
   }
 }
 
-// Named barrier `id` over `nthreads` threads (whole warps); also orders the
-// participants' shared-memory accesses. The warp reconverges first and the
-// barrier is the non-aligned form, which counts every thread's own arrival,
-// so a lane still busy (say, waiting on an mbarrier) holds the barrier.
-__device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t nthreads) {
-  __syncwarp();
-  asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
-// 2-D tiled TMA load into this CTA's shared memory, completing on `bar`.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm, int32_t x,
-                                            int32_t y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
 // 1-D bulk copy global -> this CTA's shared memory, completing on `bar`.
 // Both addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
-      : "memory");
-}
-// Same, with an L2 eviction-priority policy from make_l2_policy_*.
-__device__ __forceinline__ void bulk_load_hint(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar,
-                                               uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::
-          "r"(dst),
-      "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar), "l"(policy)
       : "memory");
 }
 __device__ __forceinline__ uint64_t make_l2_policy_evict_first() {
@@ -159,10 +132,6 @@ __device__ __forceinline__ uint64_t make_l2_policy_evict_last() {
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
-__device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* tm) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tm)) : "memory");
-}
-
 // Generic-proxy writes to shared memory made visible to the async proxy
 // (the tensor core's operand reads) before a barrier hands them over.
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -266,16 +235,6 @@ __device__ __forceinline__ void tmem_ld_x32(uint32_t taddr, float* v) {
   for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// Each thread of the warp writes zeros to 32 consecutive 32-bit TMEM columns.
-__device__ __forceinline__ void tmem_st_x32_zero(uint32_t taddr) {
-  const uint32_t z = 0;
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,"
-      "%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
-      "r"(z)
-      : "memory");
-}
-
 // Shared-memory matrix descriptor of a K-major operand stored with the
 // 32-byte swizzle: rows of 32 bytes (16 x 16-bit elements = one MMA K step),
 // 8-row groups 256 bytes apart. The tile must start on a 256-byte boundary.
@@ -338,13 +297,6 @@ __device__ __forceinline__ void bulk_load_hint_if(uint32_t dst, const void* src,
       "%4;\n}" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar), "l"(policy), "r"((uint32_t)pred)
       : "memory");
-}
-
-// Instruction descriptor, kind::f16: FP32 accumulator, both operands
-// K-major, A/B format 0 = FP16, 1 = BF16.
-__host__ __device__ constexpr uint32_t idesc_f16(int M, int N, uint32_t ab_format) {
-  return (1u << 4) | (ab_format << 7) | (ab_format << 10) | (static_cast<uint32_t>(N >> 3) << 17) |
-         (static_cast<uint32_t>(M >> 4) << 24);
 }
 
 }  // namespace dev
