@@ -279,8 +279,8 @@ smat_status smat_tiles_destroy(smat_tiles* t);
 /* Bytes of device scratch smat_spmm needs for this form / B dtype / N: the
  * packed copy of B (twice that for the split form), the launch's next-unit
  * counter, for panels split over several CTAs for load balance a partial-sum
- * slab per part, and a byte per 128 x 64 values of B that says whether they
- * hold an infinite or NaN one. */
+ * slab per part, and per 128 x 64 values of B a byte that says whether they
+ * hold an infinite or NaN one and 64 bits that say in which columns. */
 smat_status smat_spmm_workspace_size(const smat_bcsr* A, int32_t form, int32_t b_dtype, int64_t N,
                                      size_t* bytes);
 

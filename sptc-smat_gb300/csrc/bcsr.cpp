@@ -314,6 +314,10 @@ smat_status quantize_fp8(const HostBcsr& b, std::vector<uint8_t>& q, std::vector
 // tile: 64 cycles), an MMA of one block 39 cycles, 12 for a block that
 // widens its neighbour's MMA, and a 512-byte A block 8. A gathered column
 // costs a 256-byte row of B (4) and a sixteenth of an MMA and an A block (3).
+// They are those of the FP16 and BF16 forms with 16-row blocks and serve the
+// others too: the split form (8 KB tiles, three MMAs a block), FP8 (a conversion
+// behind each block) and 32-row blocks have other ones. Costs of its own took the
+// split form's stencils 1-4 % down and a 30 % 2:4 R-MAT 1-3.5 % up.
 namespace {
 constexpr int kCostTile = 64, kCostBlock = 47, kCostJoin = 12, kCostCol = 8;
 inline int cols_of(uint32_t mask) { return __builtin_popcount(mask); }
@@ -755,9 +759,9 @@ void build_work_items_multi(const std::vector<const Plan*>& plans, const std::ve
     }
   }
   double max_item = std::max(1.0, max_item_frac * total / std::max(1, workers));
-  // a part costs a full epilogue, a slab write and a share of the fixup
-  // whatever its size: never cut a panel into parts of fewer than
-  // kMinPartStages stages (small matrices then keep whole panels)
+  // a part costs a full epilogue into its slab whatever its size, and the
+  // kernel that sums the parts reads it: never cut a panel into parts of fewer
+  // than kMinPartStages stages (small matrices then keep whole panels)
   constexpr int32_t kMinPartStages = 4;
   auto max_parts = [](int32_t nstages) { return std::max<int32_t>(1, nstages / kMinPartStages); };
   // bound the partial-sum slabs: at most kMaxSlabs parts of split panels per
@@ -808,7 +812,9 @@ void build_work_items_multi(const std::vector<const Plan*>& plans, const std::ve
         items[i].nparts = part;
         double c = 0.0;
         for (int32_t st = items[i].s0; st < items[i].s1; st++) c += stage_cost(pl.stages[pi.stage_off + st]);
-        icost.push_back(c + 2.0 * epi);  // a part writes its slab; the last one also reads all parts back
+        // a part writes its slab; the second epilogue keeps parts ahead of whole panels
+        // of the same work (with one: the same times within 0.1 %)
+        icost.push_back(c + 2.0 * epi);
       }
       n_split[q]++;
       n_slabs[q] += part;

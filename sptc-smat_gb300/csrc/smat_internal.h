@@ -295,7 +295,8 @@ int pick_nsub(const smat_bcsr* h, int64_t N, int kind);
 // [the launch's next-unit counter, 256 bytes]
 // [per part of a split panel and column tile: an R*bh x BN FP32 slab]
 // [per part of a split 2:4 group and column tile: a 128 x 128 FP32 slab]
-// [a byte per packing unit of B: it holds infinite or NaN values].
+// [a byte per packing unit of B, then two words: whether and in which columns it
+// holds infinite or NaN values].
 struct WsLayout {
   size_t counters = 0, slabs = 0, flags = 0, total = 0;
   size_t b64 = 0;  // the 2:4 path's copy of B (0: none)
@@ -360,7 +361,7 @@ bool tune_lookup(const TuneKey& key, TuneVal& val);
 void tune_store(const TuneKey& key, const TuneVal& val);
 
 // The device's list: the items in `order`, their stage ranges counted from
-// the plan's first stage (a role then reads one 32-byte item, not an index,
+// the plan's first stage (a role then reads one 48-byte item, not an index,
 // an item and the panel's record one after the other).
 // n_tiles (grouped launches): column tiles per problem, each a unit of its own.
 std::vector<WorkItem> device_items(const std::vector<const Plan*>& plans, const std::vector<WorkItem>& items,
